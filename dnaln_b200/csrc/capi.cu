@@ -494,24 +494,28 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
   bool tune = false;
   const int bucket = rows_max <= 256 ? 0 : (rows_max <= 1024 ? 1 : 2);
   const int key = sp.W | (tb ? 1 : 0) << 10 | bucket << 11;
-  if (forms.size() > 1) {
-    const SwForm pinned = c->sw_mode == 1 ? kSwInter : (c->sw_mode == 2 ? kSwIntra : (c->sw_mode == 3 ? kSwIntraNarrow
-                                                                                                      : kSwInter));
-    if (c->sw_mode != 0 && std::find(forms.begin(), forms.end(), pinned) != forms.end()) {
-      form = pinned;
-    } else {
-      auto it = c->sw_tune.find(key);
-      if (it != c->sw_tune.end()) form = static_cast<SwForm>(it->second.form);
-      else if (c->capturing) return fail(c, DNALN_ERR_CUDA, "capture stopped: a kernel form is still to be tuned");
-      else tune = true;
-    }
+  if (c->sw_mode != 0 && sw_has_form(sp.W, bytes_ok, static_cast<SwForm>(c->sw_mode - 1))) {
+    form = static_cast<SwForm>(c->sw_mode - 1);
+  } else if (forms.size() > 1) {
+    auto it = c->sw_tune.find(key);
+    if (it != c->sw_tune.end()) form = static_cast<SwForm>(it->second.form);
+    else if (c->capturing) return fail(c, DNALN_ERR_CUDA, "capture stopped: a kernel form is still to be tuned");
+    else tune = true;
+  }
+  // short lists: the host's count picks the form, or the kernels read the device's (the
+  // first chunk then holds the whole of a short list)
+  int few = 0;
+  if (!tune && c->sw_mode == 0 && sw_has_form(sp.W, bytes_ok, kSwIntraFew)) {
+    const int limit = sw_few_tasks(sp.W);
+    if (n_max <= limit) form = kSwIntraFew;
+    else if (n_dev && chunk >= limit) few = limit;
   }
   for (int64_t b = 0; b < n_max; b += chunk) {
     const int cnt = static_cast<int>(n_max - b < chunk ? n_max - b : chunk);
     const auto run = [&](SwForm f) {
       const bool ok = launch_sw(c->st, tb, bytes_ok, tasks, static_cast<int>(b), cnt, n_max, n_dev, qbase, tbase, sp,
-                                res, dir, rows_max, cig, cig_off, band, fb, c->d_err, &kt, f);
-      c->stats.launches += static_cast<uint64_t>(sw_launches(sp.W, bytes_ok, tb));
+                                res, dir, rows_max, cig, cig_off, band, fb, c->d_err, &kt, f, b == 0 ? few : 0);
+      c->stats.launches += static_cast<uint64_t>(sw_launches(sp.W, bytes_ok, tb)) + (b == 0 && few > 0 ? 1 : 0);
       return ok;
     };
     if (b == 0 && tune) {
@@ -1499,7 +1503,7 @@ int dnaln_gpu_set_option(dnaln_ctx* c, const char* name, int64_t value) {
     return DNALN_OK;
   }
   if (k == "sw_form") {
-    if (value < 0 || value > 3) return fail(c, DNALN_ERR_INVALID_ARG, "sw_form must be 0 (tuned), 1, 2 or 3");
+    if (value < 0 || value > 4) return fail(c, DNALN_ERR_INVALID_ARG, "sw_form must be 0 (tuned) or 1 to 4");
     c->sw_mode = static_cast<int>(value);
     return DNALN_OK;
   }

@@ -38,6 +38,7 @@
 // takes the reference's steps. The best cell is the first strict maximum in row-major
 // order (per-row maximum with its first column, then strict across rows).
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "common.cuh"
@@ -434,7 +435,7 @@ __device__ bool window_has_n(const SwTask& tk, int W, const uint8_t* __restrict_
 // 2.56 ms per 1,000,000 x 150 bp reads.
 template <int W, bool TB>
 __global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
-    k_sw_u2(const SwTask* __restrict__ tasks, int base, int n, const int* __restrict__ n_dev,
+    k_sw_u2(const SwTask* __restrict__ tasks, int base, int n, const int* __restrict__ n_dev, int few,
              const uint8_t* __restrict__ qbase, const uint8_t* __restrict__ tbase, SwParams p,
              SwResult* __restrict__ res, uint32_t* __restrict__ dir, int rows_max, int* __restrict__ fb) {
   static_assert(W >= 3, "a window of at least two columns past an empty query");
@@ -445,7 +446,7 @@ __global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
   const int lt = blockIdx.x * blockDim.x + threadIdx.x;  // pair index within this launch
   const int nn = n_dev ? min(n, *n_dev) : n;
   const int ia = base + 2 * lt, ib = ia + 1;
-  if (ia >= nn) return;
+  if (ia >= nn || (n_dev && *n_dev <= few)) return;  // a short list is the narrowest form's
   const bool has_b = ib < nn;
   uint32_t* DP = TB ? pair_base(dir, 2 * lt, rows_max, WQ) : nullptr;
   const SwTask ta = tasks[ia];
@@ -594,13 +595,14 @@ __global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
 // the first strict maximum of the whole band in row-major order. Pairs k_sw_u2 would
 // hand to the int32 kernel are listed in fb the same way.
 template <int LANES, int CH, bool TB>
-__global__ void __launch_bounds__(kSwThreads, TB ? (CH == 16 ? 4 : 3) : 1)
-    k_sw_wide(const SwTask* __restrict__ tasks, int base, int n, const int* __restrict__ n_dev,
+__global__ void __launch_bounds__(kSwThreads, TB ? (CH <= 16 ? 4 : 3) : 1)
+    k_sw_wide(const SwTask* __restrict__ tasks, int base, int n, const int* __restrict__ n_dev, int above, int upto,
               const uint8_t* __restrict__ qbase, const uint8_t* __restrict__ tbase, SwParams p,
               SwResult* __restrict__ res, uint32_t* __restrict__ dir, int rows_max, int* __restrict__ fb) {
-  static_assert(CH % 4 == 0 && CH >= 8, "a lane's cells fill whole direction words");
+  static_assert(CH % 4 == 0, "a lane's cells fill whole direction words");
   constexpr int W = CH * LANES + 1, WQ = (W + 3) / 4;
   constexpr unsigned FULL = 0xffffffffu;
+  if (n_dev && (*n_dev <= above || *n_dev > upto)) return;  // a list of another form's length
   __shared__ uint32_t s_prof[8];  // profile words of the five query codes
   if (threadIdx.x < 5) s_prof[threadIdx.x] = prof_biased(p, threadIdx.x);
   __syncthreads();
@@ -986,11 +988,19 @@ __global__ void __launch_bounds__(kSwThreads)
   }
 }
 
-// Traceback of every task of the launch from the stashed best cell (one task per thread;
-// the DP kernels are done with the scratch). The walk waits on memory, so the launch bound
-// asks for seven resident blocks (72 registers, no spills) rather than the six that 80
-// registers allow: 0.52 -> 0.48 ms per 1,000,000 150-bp walks (eight blocks, 64 registers
-// with spills: 0.51 ms).
+// Traceback of every task of the launch from the stashed best cell (the DP kernels are done
+// with the scratch), src/align.cpp:87-143. A walk is a chain of dependent memory latencies,
+// so kWalkLanes lanes share a task: on a diagonal run lane l fetches the codes and bases of
+// rows i - 8l .. i - 8l - 7, a prefix sum over the lanes gives each the score its block
+// starts from, and all leading blocks that are diagonal throughout, with the score above
+// what their steps can use up, are taken at once, 64 rows per memory latency instead of 8.
+// The first block that is not is stepped through by its lane as the one-cell walk would.
+// Against one thread per task: 4,001 reads of 1-5 kbp 1,789 -> 236 us, 200,003 of 50-1000 bp
+// 398 -> 258, 64 of 100-300 bp 43 -> 17. Where short walks fill the SMs by themselves
+// (262,144 of 150 bp) the lanes' extra instructions cost more than the latencies they hide
+// (122 -> 181 us), so those run one thread per task.
+constexpr int kWalkLanes = 8;
+constexpr int kWalkMany = 98304, kWalkShort = 256;  // more tasks of at most this many rows: one thread each
 template <int W>
 __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restrict__ tasks, int base, int count, int n,
                                                         const int* __restrict__ n_dev,
@@ -1001,18 +1011,168 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
                                                         const int64_t* __restrict__ cig_off,
                                                         uint32_t* __restrict__ err) {
   constexpr int WQ = (W + 3) / 4;
-  const int lt = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nn = n_dev ? min(n, *n_dev) : n;
-  if (lt >= count || base + lt >= nn) return;
-  const SwTask tk = tasks[base + lt];
-  const SwResult s = res[tk.slot];
-  SwResult r{s.score, 0, 0, 0, 0, 0, 0, 0};
-  if (s.score > 0) {
-    const PairCodes codes{pair_base(const_cast<uint32_t*>(dir), lt, rows_max, WQ), WQ, lt & 1};
-    traceback(codes, W, s.qb, s.qe, s.score, qbase + tk.q_off, tbase, tk, p, r, cig + cig_off[tk.slot],
-              2 * tk.qlen + 1, err);
+  constexpr int G = kWalkLanes;
+  const int nn = min(base + count, n_dev ? min(n, *n_dev) : n) - base;  // tasks of this launch
+  if (rows_max <= kWalkShort && nn > kWalkMany) {  // the launch has a thread per task then
+    const int lt = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lt >= nn) return;
+    const SwTask tk = tasks[base + lt];
+    const SwResult s = res[tk.slot];
+    SwResult r{s.score, 0, 0, 0, 0, 0, 0, 0};
+    if (s.score > 0) {
+      const PairCodes codes{pair_base(const_cast<uint32_t*>(dir), lt, rows_max, WQ), WQ, lt & 1};
+      traceback(codes, W, s.qb, s.qe, s.score, qbase + tk.q_off, tbase, tk, p, r, cig + cig_off[tk.slot],
+                2 * tk.qlen + 1, err);
+    }
+    res[tk.slot] = r;
+    return;
   }
-  res[tk.slot] = r;
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+  const unsigned gm = ((1u << G) - 1u) << (lane & ~(G - 1));
+  const int smax = max(p.match, max(-p.mismatch, -p.ambig));  // the most one step can lower v
+  const int stride = static_cast<int>(gridDim.x * blockDim.x) / G;
+  for (int lt = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x) / G; lt < nn; lt += stride) {
+    const SwTask tk = tasks[base + lt];
+    const SwResult s = res[tk.slot];
+    __syncwarp(gm);  // every lane has the best cell before the group's first lane overwrites it
+    SwResult r{s.score, 0, 0, 0, 0, 0, 0, 0};
+    if (s.score > 0) {
+      const PairCodes code{pair_base(const_cast<uint32_t*>(dir), lt, rows_max, WQ), WQ, lt & 1};
+      const uint8_t* __restrict__ q = qbase + tk.q_off;
+      const int cap = 2 * tk.qlen + 1;
+      CigarWriter cw{cig + cig_off[tk.slot], gl == 0 ? cap : 0, 0, 0xFu, 0};  // the first lane writes
+      int i = s.qb, d = s.qe, v = s.score, nm = 0;
+      bool broken = d < 0 || d >= W || i >= tk.qlen;
+      while (!broken) {
+        int run = 0;
+        uint32_t x = 0;
+        bool stop = false;
+        while (!stop && i >= 0 && v > 0) {
+          const int top = i - kAhead * gl;  // this lane's block: rows top, top - 1, .. top - 7
+          const int sh = code.shift(d);
+          uint32_t cx = 0;  // the block's codes, row top - k in bits 4k
+          uint64_t qw = 0, tw = 0;  // its bases, row top - k in byte 7 - k; N past any end
+          int lost = 0;             // what the block takes from v, and 256ths of it its mismatches
+          bool clean = false;
+          if (top >= 0) {
+            const int64_t x0 = tk.t_start + (top - (kAhead - 1)) + d;  // target of row top - 7
+            if (top >= kAhead - 1 && x0 >= tk.t_lo && x0 + kAhead <= tk.t_hi) {
+              qw = load8u(q + top - (kAhead - 1));
+              tw = load8u(tbase + x0);
+#pragma unroll
+              for (int k = 0; k < kAhead; ++k) cx |= ((code.word(top - k, d) >> sh) & 0xFu) << (4 * k);
+              clean = (cx & 0x11111111u * (kNotDiagE | kFromF)) == 0;
+              // bytes equal and both below 4: match; either above 3: ambiguous; else mismatch
+              const uint64_t ok_amb = zero_bytes((qw | tw) & 0xFCFCFCFCFCFCFCFCull);
+              const int n_match = __popcll(zero_bytes(qw ^ tw) & ok_amb);
+              const int n_amb = kAhead - __popcll(ok_amb);
+              lost = (n_match * p.match - (kAhead - n_match - n_amb) * p.mismatch - n_amb * p.ambig) * 256 +
+                     (kAhead - n_match);
+            } else {
+#pragma unroll
+              for (int k = 0; k < kAhead; ++k) {
+                if (top - k >= 0) {
+                  cx |= code(top - k, d) << (4 * k);
+                  qw |= static_cast<uint64_t>(q[top - k]) << (8 * (kAhead - 1 - k));
+                  tw |= static_cast<uint64_t>(tcode(tbase, tk, static_cast<int64_t>(top - k) + d))
+                        << (8 * (kAhead - 1 - k));
+                }
+              }
+            }
+          }
+          int sum = lost;  // inclusive prefix over the lanes (mismatches stay below 256)
+#pragma unroll
+          for (int o = 1; o < G; o <<= 1) {
+            const int y = __shfl_up_sync(gm, sum, o, G);
+            if (gl >= o) sum += y;
+          }
+          const int before = (sum - lost) >> 8;  // the arithmetic shift drops the mismatches
+          const bool take = clean && v - before > (kAhead - 1) * smax;
+          const unsigned not_ok = (__ballot_sync(gm, !take) & gm) >> (lane & ~(G - 1));
+          const int c = not_ok ? __ffs(not_ok) - 1 : G;
+          if (c > 0) {
+            const int t = __shfl_sync(gm, sum, c - 1, G);
+            v -= t >> 8;
+            nm += t & 255;
+            run += kAhead * c;
+            i -= kAhead * c;
+          }
+          if (c == G) continue;
+          if (gl == c) {  // top == i
+#pragma unroll 1
+            for (int k = 0; k < kAhead; ++k) {
+              if (i < 0 || v <= 0) {
+                stop = true;
+                break;
+              }
+              x = (cx >> (4 * k)) & 0xFu;
+              if (x & (kNotDiagE | kFromF)) {  // not from the diagonal
+                stop = true;
+                break;
+              }
+              const int qa = static_cast<int>((qw >> (8 * (kAhead - 1 - k))) & 0xFFu);
+              const int t8 = static_cast<int>((tw >> (8 * (kAhead - 1 - k))) & 0xFFu);
+              const int tt = t8 > 3 ? 4 : t8;
+              v -= sub_score(p, qa, tt);
+              nm += (qa != tt || qa > 3) ? 1 : 0;
+              ++run;
+              --i;
+            }
+          }
+          i = __shfl_sync(gm, i, c, G);
+          v = __shfl_sync(gm, v, c, G);
+          nm = __shfl_sync(gm, nm, c, G);
+          run = __shfl_sync(gm, run, c, G);
+          x = __shfl_sync(gm, x, c, G);
+          stop = __shfl_sync(gm, static_cast<int>(stop), c, G) != 0;
+        }
+        if (run && gl == 0) cw.push(0u /* M */, run);
+        if (i < 0 || v <= 0) break;
+        run = 0;
+        bool ext = true;
+        if (!(x & kFromF)) {  // from E, an insertion: E(i,d) <- (i-1, d+1)
+          while (ext) {
+            if (i < 0 || d >= W) {
+              broken = true;
+              break;
+            }
+            ext = (code(i, d) & kExtE) != 0;
+            v += ext ? p.ge : p.oe;
+            ++run;
+            --i;
+            ++d;
+          }
+          if (!broken && gl == 0) cw.push(1u /* I */, run);
+        } else {  // from F, a deletion: F(i,d) <- (i, d-1)
+          while (ext) {
+            if (d < 0 || d >= W) {
+              broken = true;
+              break;
+            }
+            ext = (code(i, d) & kExtF) != 0;
+            v += ext ? p.ge : p.oe;
+            ++run;
+            --d;
+          }
+          if (!broken && gl == 0) cw.push(2u /* D */, run);
+        }
+        nm += run;
+        broken = broken || (i >= 0 && v > 0 && (d < 0 || d >= W));
+      }
+      if (gl == 0) {
+        if (broken) atomicOr(err, kErrTracebackBounds);
+        cw.flush();
+        if (cw.n > cap) atomicOr(err, kErrCigarOverflow);
+        r.qb = i + 1;
+        r.tb = i + 1 + d;
+        r.qe = s.qb + 1;
+        r.te = s.qb + s.qe + 1;
+        r.nm = nm;
+        r.n_ops = cw.n < cap ? cw.n : cap;
+      }
+    }
+    if (gl == 0) res[tk.slot] = r;
+  }
 }
 
 // Any band width and any scores: one alignment per thread, int32, band rows H, E in
@@ -1085,102 +1245,109 @@ __global__ void __launch_bounds__(kSwThreads) k_sw_any(const SwTask* __restrict_
   res[tk.slot] = r;
 }
 
+// What a launch hands to its kernels.
+struct SwLaunch {
+  cudaStream_t st;
+  bool tb;
+  const SwTask* tasks;
+  int base, count, n;
+  const int* n_dev;
+  const uint8_t* qbase;
+  const uint8_t* tbase;
+  const SwParams& p;
+  SwResult* res;
+  uint32_t* dir;
+  int rows_max;
+  uint32_t* cig;
+  const int64_t* cig_off;
+  int* fb;
+  uint32_t* err;
+  const KernelTrace& kt;
+};
+
+template <int LANES, int CH>
+void run_wide(const SwLaunch& a, int count, int above, int upto) {
+  const int64_t pairs = (static_cast<int64_t>(count) + 1) / 2;
+  const int blocks = static_cast<int>((pairs * LANES + kSwThreads - 1) / kSwThreads);
+  constexpr int kRowBytes = 2 * (CH + 1) * kSwThreads * 4;  // the two saved best rows of each lane
+  a.kt.begin(a.st, a.tb ? "k_sw_wide<tb>" : "k_sw_wide<score>");
+  if (a.tb)
+    k_sw_wide<LANES, CH, true><<<blocks, kSwThreads, kRowBytes, a.st>>>(
+        a.tasks, a.base, a.n, a.n_dev, above, upto, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb);
+  else
+    k_sw_wide<LANES, CH, false><<<blocks, kSwThreads, 0, a.st>>>(
+        a.tasks, a.base, a.n, a.n_dev, above, upto, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb);
+  a.kt.end(a.st);
+}
+
 template <int W>
-void launch_u2(cudaStream_t st, bool tb, const SwTask* tasks, int base, int count, int n, const int* n_dev,
-               const uint8_t* qbase, const uint8_t* tbase, const SwParams& p, SwResult* res, uint32_t* dir,
-               int rows_max, uint32_t* cig, const int64_t* cig_off, int* fb, uint32_t* err, const KernelTrace* kt) {
-  const int pairs = (count + 1) / 2;
-  const int blocks_pairs = (pairs + kSwThreads - 1) / kSwThreads;
-  const int blocks_tasks = (count + kSwThreads - 1) / kSwThreads;
-  // W = 33 and 65: the fallback list runs four lanes per alignment (k_sw_fb_lanes), the
-  // other widths the one-thread kernel, whose band fits in registers
-  constexpr bool kLanesFb = W == 33 || W == 65;
-  constexpr int kFbCh = (W - 1) / 4;
-  // the fallback kernels stride over a list whose length only the device knows (usually
-  // short or empty): a few resident waves, not one block per possible entry
-  const int fb_cap = 8 * device_sm_count();
-  const int blocks_fb =
-      std::min(fb_cap, static_cast<int>((static_cast<int64_t>(count) * 4 + kSwThreads - 1) / kSwThreads));
-  const int blocks_fb1 = std::min(fb_cap, blocks_tasks);
-  const KernelTrace none;
-  const KernelTrace& t = kt ? *kt : none;
-  cudaMemsetAsync(fb, 0, sizeof(int), st);
-  if (tb) {
+void run_u2(const SwLaunch& a, int above) {
+  const int blocks = ((a.count + 1) / 2 + kSwThreads - 1) / kSwThreads;
+  a.kt.begin(a.st, a.tb ? "k_sw_u2<tb>" : "k_sw_u2<score>");
+  if (a.tb) {
     constexpr int kRowBytes = 2 * W * kSwThreads * 4;  // the two saved best rows of each thread
     if (kRowBytes > 48 * 1024) {
       static std::atomic<bool> attr_set[kMaxDevices];
       set_smem_limit_once(k_sw_u2<W, true>, kRowBytes, attr_set);
     }
-    t.begin(st, "k_sw_u2<tb>");
-    k_sw_u2<W, true><<<blocks_pairs, kSwThreads, kRowBytes, st>>>(tasks, base, n, n_dev, qbase, tbase, p, res, dir,
-                                                                  rows_max, fb);
-    t.end(st);
-    t.begin(st, "k_sw_fb<tb>");
-    if constexpr (kLanesFb)
-      k_sw_fb_lanes<4, kFbCh, true><<<blocks_fb, kSwThreads, 0, st>>>(tasks, base, qbase, tbase, p, res, dir,
-                                                                      rows_max, fb);
-    else
-      k_sw_fb<W, true><<<blocks_fb1, kSwThreads, 0, st>>>(tasks, base, qbase, tbase, p, res, dir, rows_max, fb);
-    t.end(st);
-    t.begin(st, "k_sw_walk");
-    k_sw_walk<W><<<blocks_tasks, kSwThreads, 0, st>>>(tasks, base, count, n, n_dev, qbase, tbase, p, res, dir,
-                                                      rows_max, cig, cig_off, err);
-    t.end(st);
+    k_sw_u2<W, true><<<blocks, kSwThreads, kRowBytes, a.st>>>(a.tasks, a.base, a.n, a.n_dev, above, a.qbase, a.tbase,
+                                                              a.p, a.res, a.dir, a.rows_max, a.fb);
   } else {
-    t.begin(st, "k_sw_u2<score>");
-    k_sw_u2<W, false><<<blocks_pairs, kSwThreads, 0, st>>>(tasks, base, n, n_dev, qbase, tbase, p, res, dir, rows_max,
-                                                           fb);
-    t.end(st);
-    t.begin(st, "k_sw_fb<score>");
-    if constexpr (kLanesFb)
-      k_sw_fb_lanes<4, kFbCh, false><<<blocks_fb, kSwThreads, 0, st>>>(tasks, base, qbase, tbase, p, res, dir,
-                                                                       rows_max, fb);
-    else
-      k_sw_fb<W, false><<<blocks_fb1, kSwThreads, 0, st>>>(tasks, base, qbase, tbase, p, res, dir, rows_max, fb);
-    t.end(st);
+    k_sw_u2<W, false><<<blocks, kSwThreads, 0, a.st>>>(a.tasks, a.base, a.n, a.n_dev, above, a.qbase, a.tbase, a.p,
+                                                       a.res, a.dir, a.rows_max, a.fb);
   }
+  a.kt.end(a.st);
 }
 
-template <int LANES, int CH = 32>
-void launch_wide(cudaStream_t st, bool tb, const SwTask* tasks, int base, int count, int n, const int* n_dev,
-                 const uint8_t* qbase, const uint8_t* tbase, const SwParams& p, SwResult* res, uint32_t* dir,
-                 int rows_max, uint32_t* cig, const int64_t* cig_off, int* fb, uint32_t* err, const KernelTrace* kt) {
-  constexpr int W = CH * LANES + 1;
-  constexpr int FBCH = W == 33 ? 8 : 16;  // cells per lane of the int32 fallback kernel
-  constexpr int FBL = (W - 1) / FBCH;     // its lanes per alignment
-  const int pairs = (count + 1) / 2;
-  const int blocks_pairs = static_cast<int>((static_cast<int64_t>(pairs) * LANES + kSwThreads - 1) / kSwThreads);
-  const int blocks_tasks = (count + kSwThreads - 1) / kSwThreads;
-  // the fallback list holds at most `count` tasks (its length is known on the device only;
-  // the kernel strides over it, so a few resident waves suffice)
-  const int blocks_fb = std::min(8 * device_sm_count(),
-                                 static_cast<int>((static_cast<int64_t>(count) * FBL + kSwThreads - 1) / kSwThreads));
-  const KernelTrace none;
-  const KernelTrace& t = kt ? *kt : none;
-  cudaMemsetAsync(fb, 0, sizeof(int), st);
-  if (tb) {
-    constexpr int kRowBytes = 2 * (CH + 1) * kSwThreads * 4;  // the two saved best rows of each lane
-    t.begin(st, "k_sw_wide<tb>");
-    k_sw_wide<LANES, CH, true><<<blocks_pairs, kSwThreads, kRowBytes, st>>>(tasks, base, n, n_dev, qbase, tbase, p,
-                                                                            res, dir, rows_max, fb);
-    t.end(st);
-    t.begin(st, "k_sw_fb<tb>");
-    k_sw_fb_lanes<FBL, FBCH, true><<<blocks_fb, kSwThreads, 0, st>>>(tasks, base, qbase, tbase, p, res, dir, rows_max,
-                                                                     fb);
-    t.end(st);
-    t.begin(st, "k_sw_walk");
-    k_sw_walk<W><<<blocks_tasks, kSwThreads, 0, st>>>(tasks, base, count, n, n_dev, qbase, tbase, p, res, dir,
-                                                      rows_max, cig, cig_off, err);
-    t.end(st);
-  } else {
-    t.begin(st, "k_sw_wide<score>");
-    k_sw_wide<LANES, CH, false><<<blocks_pairs, kSwThreads, 0, st>>>(tasks, base, n, n_dev, qbase, tbase, p, res, dir,
-                                                                     rows_max, fb);
-    t.end(st);
-    t.begin(st, "k_sw_fb<score>");
-    k_sw_fb_lanes<FBL, FBCH, false><<<blocks_fb, kSwThreads, 0, st>>>(tasks, base, qbase, tbase, p, res, dir,
-                                                                      rows_max, fb);
-    t.end(st);
+// The int32 kernel over the listed tasks: several lanes per alignment at W = 33, 65 and 129
+// (narrow chunks: its time is one task's serial latency), else one thread, whose band fits
+// in registers. The list's length is known on the device only (usually short or empty), so
+// the kernel strides over it with a few resident waves.
+template <int W>
+void run_fb(const SwLaunch& a) {
+  constexpr int CH = W == 33 ? 8 : 16;
+  constexpr bool kLanes = W == 33 || W == 65 || W == 129;
+  constexpr int L = kLanes ? (W - 1) / CH : 1;
+  const int blocks = std::min(
+      8 * device_sm_count(), static_cast<int>((static_cast<int64_t>(a.count) * L + kSwThreads - 1) / kSwThreads));
+  const auto run = [&](auto kernel) {
+    kernel<<<blocks, kSwThreads, 0, a.st>>>(a.tasks, a.base, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb);
+  };
+  a.kt.begin(a.st, a.tb ? "k_sw_fb<tb>" : "k_sw_fb<score>");
+  if constexpr (kLanes) a.tb ? run(k_sw_fb_lanes<L, CH, true>) : run(k_sw_fb_lanes<L, CH, false>);
+  else a.tb ? run(k_sw_fb<W, true>) : run(k_sw_fb<W, false>);
+  a.kt.end(a.st);
+}
+
+// One band width: the form for short lists (few > 0: it takes a device count of at most
+// `few`, the main form any other), the main form, the int32 kernel, the walk.
+template <int W>
+void launch_band(const SwLaunch& a, SwForm form, int few) {
+  constexpr bool kFew = W == 17 || W == 33 || W == 65 || W == 129;
+  cudaMemsetAsync(a.fb, 0, sizeof(int), a.st);
+  if constexpr (kFew) {
+    if (form == kSwIntraFew) run_wide<(W - 1) / 4, 4>(a, a.count, 0, INT_MAX);
+    else if (few > 0) run_wide<(W - 1) / 4, 4>(a, std::min(a.count, few), 0, few);
+  }
+  if constexpr (W == 33 || W == 65 || W == 129) {
+    if (form == kSwIntra) run_wide<(W - 1) / 32, 32>(a, a.count, few, INT_MAX);
+    if (form == kSwIntraNarrow) run_wide<(W - 1) / 16, 16>(a, a.count, few, INT_MAX);
+  }
+  if constexpr (W != 129) {
+    if (form == kSwInter) run_u2<W>(a, few);
+  }
+  run_fb<W>(a);
+  if (a.tb) {
+    const int lane_blocks = std::min(
+        16 * device_sm_count(),
+        static_cast<int>((static_cast<int64_t>(a.count) * kWalkLanes + kSwThreads - 1) / kSwThreads));
+    const int blocks = a.rows_max <= kWalkShort && a.count > kWalkMany
+                           ? std::max(lane_blocks, (a.count + kSwThreads - 1) / kSwThreads)
+                           : lane_blocks;
+    a.kt.begin(a.st, "k_sw_walk");
+    k_sw_walk<W><<<blocks, kSwThreads, 0, a.st>>>(a.tasks, a.base, a.count, a.n, a.n_dev, a.qbase, a.tbase, a.p,
+                                                  a.res, a.dir, a.rows_max, a.cig, a.cig_off, a.err);
+    a.kt.end(a.st);
   }
 }
 
@@ -1216,6 +1383,14 @@ size_t sw_band_bytes_per_task(int W, bool bytes_ok) {
   return sw_uses_generic(W, bytes_ok) ? static_cast<size_t>(2) * (W + 1) * sizeof(int) : 0;
 }
 
+// Up to this many tasks the form of four cells per lane is the fastest: its row step is the
+// shortest serial chain, and a short list leaves lanes idle anyway. Measured against the
+// best other form, us for 150-row tracebacks: W = 33 67 against 113 at 1,024 tasks, 117
+// against 115 at 16,384; W = 65 68 against 114 and, at 8,192, 122 against 118; W = 129 76
+// against 118 and, at 4,096, 136 against 120; W = 17 70 against 105 and, at 32,768, 118
+// against 108.
+int sw_few_tasks(int W) { return W == 17 ? 24576 : (W == 33 ? 16384 : (W == 65 ? 8192 : 3072)); }
+
 int sw_launches(int W, bool bytes_ok, bool tb) { return sw_uses_generic(W, bytes_ok) ? 1 : (tb ? 3 : 2); }
 
 bool sw_has_form(int W, bool bytes_ok, SwForm form) {
@@ -1224,6 +1399,7 @@ bool sw_has_form(int W, bool bytes_ok, SwForm form) {
     case kSwInter: return W != 129;
     case kSwIntra: return W == 33 || W == 65 || W == 129;
     case kSwIntraNarrow: return W == 33 || W == 65 || W == 129;
+    case kSwIntraFew: return W == 17 || W == 33 || W == 65 || W == 129;
     default: return false;
   }
 }
@@ -1231,13 +1407,14 @@ bool sw_has_form(int W, bool bytes_ok, SwForm form) {
 int sw_lanes_per_pair(int W, SwForm form) {
   if (form == kSwIntra) return (W - 1) / 32;
   if (form == kSwIntraNarrow) return (W - 1) / 16;
+  if (form == kSwIntraFew) return (W - 1) / 4;
   return 1;
 }
 
 bool launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int base, int count, int n,
                const int* n_dev, const uint8_t* qbase, const uint8_t* tbase, const SwParams& p, SwResult* res,
                uint32_t* dir, int rows_max, uint32_t* cig, const int64_t* cig_off, int* band, int* fb,
-               uint32_t* err, const KernelTrace* kt, SwForm form) {
+               uint32_t* err, const KernelTrace* kt, SwForm form, int few) {
   if (count <= 0) return true;
   const bool generic = sw_uses_generic(p.W, bytes_ok);
   if ((tb && !dir) || (generic && !band) || (!generic && !fb) || (base % kSwTaskGroup) != 0) return false;
@@ -1245,42 +1422,21 @@ bool launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int
   // [base, base + count) only, so that no thread of a grid rounded up past `count` takes a
   // task of the next chunk, whose scratch this launch does not hold
   if (n > base + count) n = base + count;
-  if (!generic && form != kSwInter && sw_has_form(p.W, bytes_ok, form)) {
-#define DNB_SW_WIDE(L, CHV) \
-  launch_wide<L, CHV>(st, tb, tasks, base, count, n, n_dev, qbase, tbase, p, res, dir, rows_max, cig, cig_off, fb, err, kt)
-    const bool narrow = form == kSwIntraNarrow;
-    if (p.W == 33) {
-      if (narrow) DNB_SW_WIDE(2, 16);
-      else DNB_SW_WIDE(1, 32);
-    } else if (p.W == 65) {
-      if (narrow) DNB_SW_WIDE(4, 16);
-      else DNB_SW_WIDE(2, 32);
-    } else {
-      if (narrow) DNB_SW_WIDE(8, 16);
-      else DNB_SW_WIDE(4, 32);
-    }
-#undef DNB_SW_WIDE
-    return true;
-  }
   if (!generic) {
-#define DNB_SW_U2(WV)                                                                                       \
-  case WV:                                                                                                  \
-    launch_u2<WV>(st, tb, tasks, base, count, n, n_dev, qbase, tbase, p, res, dir, rows_max, cig, cig_off, \
-                  fb, err, kt);                                                                             \
-    return true;
+    const KernelTrace none;
+    const SwLaunch a{st, tb,  tasks,    base, count,   n,  n_dev, qbase, tbase,
+                     p,  res, dir,      rows_max, cig, cig_off, fb, err, kt ? *kt : none};
+    if (!sw_has_form(p.W, bytes_ok, form)) form = p.W == 129 ? kSwIntra : kSwInter;
+    if (!sw_has_form(p.W, bytes_ok, kSwIntraFew)) few = 0;
     switch (p.W) {
-      DNB_SW_U2(11)
-      DNB_SW_U2(17)
-      DNB_SW_U2(33)
-      DNB_SW_U2(43)
-      DNB_SW_U2(65)
-      case 129:  // no inter-sequence form at this width
-        launch_wide<4, 32>(st, tb, tasks, base, count, n, n_dev, qbase, tbase, p, res, dir, rows_max, cig, cig_off, fb,
-                           err, kt);
-        return true;
+      case 11: launch_band<11>(a, form, few); return true;
+      case 17: launch_band<17>(a, form, few); return true;
+      case 33: launch_band<33>(a, form, few); return true;
+      case 43: launch_band<43>(a, form, few); return true;
+      case 65: launch_band<65>(a, form, few); return true;
+      case 129: launch_band<129>(a, form, few); return true;
       default: break;
     }
-#undef DNB_SW_U2
   }
   const int blocks = (count + kSwThreads - 1) / kSwThreads;
   if (kt) kt->begin(st, tb ? "k_sw_any<tb>" : "k_sw_any<score>");

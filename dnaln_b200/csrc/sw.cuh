@@ -29,8 +29,10 @@ int sw_launches(int W, bool bytes_ok, bool tb);
 // sequence (k_sw_wide, the row of a pair spread over lanes in a skewed wavefront: (W - 1) /
 // 32 lanes of 32 cells, or, narrow, (W - 1) / 16 lanes of 16 cells; W = 33, 65, 129). The
 // generic kernel (other widths or scores) has the inter form only.
-enum SwForm : int { kSwInter = 0, kSwIntra = 1, kSwIntraNarrow = 2 };
-constexpr int kSwForms = 3;
+enum SwForm : int { kSwInter = 0, kSwIntra = 1, kSwIntraNarrow = 2, kSwIntraFew = 3 };
+constexpr int kSwForms = 3;  // forms the tuner times: kSwIntraFew is chosen by the task count
+// Task count up to which kSwIntraFew ((W - 1) / 4 lanes of 4 cells) runs.
+int sw_few_tasks(int W);
 bool sw_has_form(int W, bool bytes_ok, SwForm form);
 int sw_lanes_per_pair(int W, SwForm form);
 
@@ -41,11 +43,12 @@ int sw_lanes_per_pair(int W, SwForm form);
 // and `band` must hold count rounded up to kSwTaskGroup tasks of
 // sw_dir_bytes_per_task(W, rows_max) and sw_band_bytes_per_task(W, bytes_ok); `fb`
 // (count + 1 ints) lists the tasks the 16-bit kernel hands to the int32 one; kt (may be
-// null) times each kernel. Returns false, launching nothing, when a needed scratch pointer
+// null) times each kernel; few > 0 (needs n_dev) lets kSwIntraFew take the whole launch when
+// *n_dev <= few. Returns false, launching nothing, when a needed scratch pointer
 // is null or base is misaligned.
 bool launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int base, int count, int n,
                const int* n_dev, const uint8_t* qbase, const uint8_t* tbase, const SwParams& p, SwResult* res,
                uint32_t* dir, int rows_max, uint32_t* cig, const int64_t* cig_off, int* band, int* fb,
-               uint32_t* err, const KernelTrace* kt, SwForm form = kSwInter);
+               uint32_t* err, const KernelTrace* kt, SwForm form = kSwInter, int few = 0);
 
 }  // namespace dnb
