@@ -162,6 +162,7 @@ struct dnaln_ctx {
   bool stop = false;
   bool warp_seed_only = false;  // option: every read through the warp-per-read seeding kernels
   bool length_order = true;     // option: SW tasks of mixed-length batches run longest first
+  bool ungapped = true;         // option: SW tasks proved to have no gap skip the DP
   bool long_thread = true;      // option: listed long reads one thread each before the warp kernels
   // option "work_stealing": the warp chaining kernel takes reads by atomic claims on
   // resident blocks (default) instead of striding over a fixed grid
@@ -423,45 +424,48 @@ int check_device_errors(dnaln_ctx* c, uint32_t bits) {
               !!(bits & kErrProbeLoop), !!(bits & kErrAsyncCopy));
 }
 
-// SW tasks of a batch whose reads differ in length, longest first (a thread's two
-// alignments and a warp's 64 then have similar lengths, so no lane idles through a long
-// partner's rows). *sorted = tasks when there is nothing to gain.
-int sort_tasks_by_length(dnaln_ctx* c, const SwTask* tasks, int n_max, const int* n_dev, const char* tag,
-                         const SwTask** sorted) {
-  *sorted = tasks;
-  if (n_max < 2) return DNALN_OK;
-  const std::string t = tag;
-  DBUF(keys_in, uint32_t, (t + "_kin").c_str(), n_max);
-  DBUF(keys_out, uint32_t, (t + "_kout").c_str(), n_max);
-  DBUF(idx_in, int32_t, (t + "_iin").c_str(), n_max);
-  DBUF(idx_out, int32_t, (t + "_iout").c_str(), n_max);
-  DBUF(out, SwTask, (t + "_sorted").c_str(), n_max);
-  const KernelTrace kt = tracer(c);
-  kt.begin(c->st, "k_task_keys");
-  launch_task_keys(c->st, tasks, n_max, n_dev, keys_in, idx_in);
-  kt.end(c->st);
-  size_t tmp = 0;
-  CK(cub::DeviceRadixSort::SortPairs(nullptr, tmp, keys_in, keys_out, idx_in, idx_out, n_max, 0, 17, c->st));
-  DBUF(tb, uint8_t, "cub_tmp_sort", tmp);
-  kt.begin(c->st, "cub_sort");
-  const cudaError_t e = cub::DeviceRadixSort::SortPairs(tb, tmp, keys_in, keys_out, idx_in, idx_out, n_max, 0, 17,
-                                                        c->st);
-  kt.end(c->st);
-  CK(e);
-  kt.begin(c->st, "k_task_gather");
-  launch_task_gather(c->st, tasks, n_max, n_dev, idx_out, out);
-  kt.end(c->st);
-  c->stats.launches += 2;
-  *sorted = out;
-  return DNALN_OK;
-}
-
-// Launches traceback SW over tasks [0, n_max) (count read on the device from n_dev),
-// chunked so the direction-bit scratch stays within dir_cap_bytes.
+// Banded SW over tasks [0, n_max) (count read on the device from n_dev): first the tasks
+// proved to align without a gap (option "ungapped"), then the DP kernels over the rest, in
+// length order when by_length (a thread's two alignments and a warp's 64 then have similar
+// lengths, so no lane idles through a long partner's rows), chunked so the direction-bit
+// scratch stays within dir_cap_bytes.
 int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks, int n_max, const int* n_dev,
                       const uint8_t* qbase, const uint8_t* tbase, const SwParams& sp, SwResult* res, int rows_max,
-                      uint32_t* cig, const int64_t* cig_off) {
+                      uint32_t* cig, const int64_t* cig_off, bool by_length) {
   if (n_max <= 0) return DNALN_OK;
+  const bool ungapped = c->ungapped && sw_ungapped_supported(sp, bytes_ok);
+  if (ungapped || (by_length && n_max > 1)) {
+    // [0] listed tasks, then the length bins' counts and the places taken of each
+    const KernelTrace kt = tracer(c);
+    DBUF(cnt, int, "sw_todo_n", 2 + 2 * kSwLengthBins);
+    CK(cudaMemsetAsync(cnt, 0, (by_length ? 2 + 2 * kSwLengthBins : 1) * sizeof(int), c->st));
+    int* hist = by_length ? cnt + 2 : nullptr;
+    int bin_shift = 0;
+    while ((rows_max >> bin_shift) >= kSwLengthBins) ++bin_shift;
+    if (ungapped) {
+      DBUF(todo, SwTask, "sw_todo", n_max);
+      kt.begin(c->st, tb ? "k_sw_ungapped<tb>" : "k_sw_ungapped<score>");
+      launch_sw_ungapped(c->st, tb, tasks, n_max, n_dev, qbase, tbase, sp, res, cig, cig_off, todo, cnt, hist,
+                         bin_shift);
+      kt.end(c->st);
+      c->stats.launches += 1;
+      tasks = todo;
+      n_dev = cnt;
+    } else {
+      kt.begin(c->st, "k_length_bins");
+      launch_length_bins(c->st, tasks, n_max, n_dev, hist, bin_shift);
+      kt.end(c->st);
+      c->stats.launches += 1;
+    }
+    if (by_length) {
+      DBUF(sorted, SwTask, "sw_sorted", n_max);
+      kt.begin(c->st, "k_order_tasks");
+      launch_order_tasks(c->st, tasks, n_max, n_dev, hist, hist + kSwLengthBins, bin_shift, sorted);
+      kt.end(c->st);
+      c->stats.launches += 1;
+      tasks = sorted;
+    }
+  }
   const int64_t G = kSwTaskGroup;
   const size_t dir_t = tb ? sw_dir_bytes_per_task(sp.W, rows_max) : 0;
   const size_t band_t = sw_band_bytes_per_task(sp.W, bytes_ok);
@@ -812,12 +816,8 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   kt.begin(st, "k_score_tasks");
   launch_score_tasks(st, n, pofs, d_seq_len, cb, ix.dev, mc, sc_tasks, c->d_count, ctr);
   kt.end(st);
-  // reads of very different lengths: SW tasks longest first (lengths known on the host)
-  const SwTask* sc_run = sc_tasks;
-  if (by_length)
-    if (int e = sort_tasks_by_length(c, sc_tasks, static_cast<int>(n * MC), c->d_count, "sc", &sc_run)) return e;
-  if (int e = launch_sw_chunked(c, false, bytes_ok, sc_run, static_cast<int>(n * MC), c->d_count, codes,
-                                ix.dev.genome, swp, res_sc, static_cast<int>(max_len), nullptr, nullptr))
+  if (int e = launch_sw_chunked(c, false, bytes_ok, sc_tasks, static_cast<int>(n * MC), c->d_count, codes,
+                                ix.dev.genome, swp, res_sc, static_cast<int>(max_len), nullptr, nullptr, by_length))
     return e;
   CK(cudaEventRecord(c->ev[kEvSc1], st));
 
@@ -835,11 +835,8 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   kt.begin(st, "k_cig_slots");
   k_cig_slots<<<nblk(n), 256, 0, st>>>(pofs, n, cig_slot);
   kt.end(st);
-  const SwTask* tb_run = tb_tasks;
-  if (by_length)
-    if (int e = sort_tasks_by_length(c, tb_tasks, static_cast<int>(n), c->d_count + 1, "tb", &tb_run)) return e;
-  if (int e = launch_sw_chunked(c, true, bytes_ok, tb_run, static_cast<int>(n), c->d_count + 1, codes,
-                                ix.dev.genome, swp, res_tb, static_cast<int>(max_len), cig_tb, cig_slot))
+  if (int e = launch_sw_chunked(c, true, bytes_ok, tb_tasks, static_cast<int>(n), c->d_count + 1, codes,
+                                ix.dev.genome, swp, res_tb, static_cast<int>(max_len), cig_tb, cig_slot, by_length))
     return e;
   CK(cudaEventRecord(c->ev[kEvTb1], st));
 
@@ -970,7 +967,7 @@ std::string graph_key(const dnaln_ctx* c, const IndexRes& ix, const char* d_seq,
   put(ptrs, sizeof ptrs);
   const int64_t nums[] = {n, hint.seq_base, hint.bases, hint.max_len, hint.cigar_base, cigar_cap, c->pool_cap,
                           static_cast<int64_t>(c->dir_cap_bytes), c->sw_mode, c->warp_seed_only, c->long_thread,
-                          c->length_order, c->stealing, c->encode_bulk, c->seed_block,
+                          c->length_order, c->ungapped, c->stealing, c->encode_bulk, c->seed_block,
                           c->seed_tune.tuned ? c->seed_tune.reads_per_block : 0};
   put(nums, sizeof nums);
   put(&p, sizeof p);
@@ -1509,6 +1506,10 @@ int dnaln_gpu_set_option(dnaln_ctx* c, const char* name, int64_t value) {
   }
   if (k == "long_thread") {
     c->long_thread = value != 0;
+    return DNALN_OK;
+  }
+  if (k == "ungapped") {
+    c->ungapped = value != 0;
     return DNALN_OK;
   }
   if (k == "length_order") {
@@ -2181,6 +2182,8 @@ int dnaln_gpu_align(dnaln_ctx* c, const uint8_t* q, const int64_t* q_off, const 
   }
   cudaStream_t st = c->st;
   const bool tb = traceback != 0;
+  const bool by_length =  // as for a batch of reads
+      c->length_order && rows_max > 1.25 * static_cast<double>((cig_total - n) / 2) / static_cast<double>(n);
   DBUF(d_q, uint8_t, "al_q", qext);
   DBUF(d_t, uint8_t, "al_t", text);
   DBUF(d_tasks, SwTask, "al_tasks", n);
@@ -2202,7 +2205,7 @@ int dnaln_gpu_align(dnaln_ctx* c, const uint8_t* q, const int64_t* q_off, const 
   c->trace_open = false;
   CK(cudaEventRecord(c->ev[tb ? kEvTb0 : kEvSc0], st));
   if (int e = launch_sw_chunked(c, tb, sw_bytes_ok(*sp), d_tasks, static_cast<int>(n), nullptr, d_q, d_t, swp, d_res,
-                                rows_max, d_cig, d_slot))
+                                rows_max, d_cig, d_slot, by_length))
     return e;
   CK(cudaEventRecord(c->ev[tb ? kEvTb1 : kEvSc1], st));
   int64_t total = 0;

@@ -51,4 +51,26 @@ bool launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int
                uint32_t* dir, int rows_max, uint32_t* cig, const int64_t* cig_off, int* band, int* fb,
                uint32_t* err, const KernelTrace* kt, SwForm form = kSwInter, int few = 0);
 
+// ---- tasks without a gap, proved from bit vectors (sw_ungapped.cu) ------------------------
+// True when the scores and the band meet the proof's preconditions.
+bool sw_ungapped_supported(const SwParams& p, bool bytes_ok);
+// Writes the result (and, with tb, the one-operation CIGAR) of every task proved to align
+// by diagonal steps only, and appends the others to todo (capacity n, *todo_n = 0 before).
+// hist (may be null) counts the listed tasks per length bin.
+void launch_sw_ungapped(cudaStream_t st, bool tb, const SwTask* tasks, int n, const int* n_dev, const uint8_t* qbase,
+                        const uint8_t* tbase, const SwParams& p, SwResult* res, uint32_t* cig, const int64_t* cig_off,
+                        SwTask* todo, int* todo_n, int* hist, int bin_shift);
+
+// Length order of tasks, longest first, by counting over kSwLengthBins bins of
+// 2^bin_shift lengths: launch_length_bins fills hist (zero before), launch_order_tasks
+// writes out (taken: kSwLengthBins zeros).
+constexpr int kSwLengthBins = 1024;
+__host__ __device__ __forceinline__ int sw_length_bin(int len, int bin_shift) {
+  const int x = len >> bin_shift;
+  return kSwLengthBins - 1 - (x < kSwLengthBins ? x : kSwLengthBins - 1);
+}
+void launch_length_bins(cudaStream_t st, const SwTask* tasks, int n, const int* n_dev, int* hist, int bin_shift);
+void launch_order_tasks(cudaStream_t st, const SwTask* tasks, int n, const int* n_dev, const int* hist, int* taken,
+                        int bin_shift, SwTask* out);
+
 }  // namespace dnb

@@ -145,6 +145,8 @@ int dnaln_gpu_set_sub_batch(dnaln_ctx* ctx, int64_t reads);
  *                    the long-read kernel first (default); 0 = straight to the warp kernels;
  *   "length_order"   1 = SW tasks of a batch whose reads differ in length run longest
  *                    first (default); 0 = in read order;
+ *   "ungapped"       1 = banded SW tasks proved from bit vectors to align by diagonal steps
+ *                    only skip the DP kernels (default); 0 = every task runs the DP;
  *   "seed_block"     reads per block of the thread-per-read seeding kernel: 0 = tuned
  *                    (default, dnaln_gpu_seed_tuning), 64 or 128;
  *   "encode_bulk"    1 = the codes of both strands are made in shared memory, tiles of
