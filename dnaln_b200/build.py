@@ -20,7 +20,7 @@ ROOT = PKG.parent
 BUILD = PKG / "_build"
 LIB = PKG / "libdnaln_b200.so"
 
-CUDA_SOURCES = ["csrc/sw.cu", "csrc/sw_ungapped.cu", "csrc/seed.cu", "csrc/seed_thread.cu", "csrc/map.cu", "csrc/capi.cu", "csrc/noalloc.cu",
+CUDA_SOURCES = ["csrc/sw.cu", "csrc/sw_ungapped.cu", "csrc/seed.cu", "csrc/seed_thread.cu", "csrc/seed_colinear.cu", "csrc/map.cu", "csrc/capi.cu", "csrc/noalloc.cu",
                 "csrc/serve.cu", "csrc/index_build.cu",
                 "csrc/seed_long.cu", "csrc/peak.cu", "csrc/encode_bulk.cu"]
 HOST_SOURCES = ["host/sam.cpp", "host/reads.cpp", "host/eval.cpp"]

@@ -163,6 +163,7 @@ struct dnaln_ctx {
   bool warp_seed_only = false;  // option: every read through the warp-per-read seeding kernels
   bool length_order = true;     // option: SW tasks of mixed-length batches run longest first
   bool ungapped = true;         // option: SW tasks proved to have no gap skip the DP
+  bool colinear = true;         // option: reads with one colinear chain skip the full seeding kernels
   bool long_thread = true;      // option: listed long reads one thread each before the warp kernels
   // option "work_stealing": the warp chaining kernel takes reads by atomic claims on
   // resident blocks (default) instead of striding over a fixed grid
@@ -437,11 +438,10 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
   if (ungapped || (by_length && n_max > 1)) {
     // [0] listed tasks, then the length bins' counts and the places taken of each
     const KernelTrace kt = tracer(c);
-    DBUF(cnt, int, "sw_todo_n", 2 + 2 * kSwLengthBins);
-    CK(cudaMemsetAsync(cnt, 0, (by_length ? 2 + 2 * kSwLengthBins : 1) * sizeof(int), c->st));
+    DBUF(cnt, int, "sw_todo_n", 2 + 2 * kLengthBins);
+    CK(cudaMemsetAsync(cnt, 0, (by_length ? 2 + 2 * kLengthBins : 1) * sizeof(int), c->st));
     int* hist = by_length ? cnt + 2 : nullptr;
-    int bin_shift = 0;
-    while ((rows_max >> bin_shift) >= kSwLengthBins) ++bin_shift;
+    const int bin_shift = length_bin_shift(rows_max);
     if (ungapped) {
       DBUF(todo, SwTask, "sw_todo", n_max);
       kt.begin(c->st, tb ? "k_sw_ungapped<tb>" : "k_sw_ungapped<score>");
@@ -460,7 +460,7 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
     if (by_length) {
       DBUF(sorted, SwTask, "sw_sorted", n_max);
       kt.begin(c->st, "k_order_tasks");
-      launch_order_tasks(c->st, tasks, n_max, n_dev, hist, hist + kSwLengthBins, bin_shift, sorted);
+      launch_order_tasks(c->st, tasks, n_max, n_dev, hist, hist + kLengthBins, bin_shift, sorted);
       kt.end(c->st);
       c->stats.launches += 1;
       tasks = sorted;
@@ -570,6 +570,19 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
   return DNALN_OK;
 }
 
+// ord = the reads of a list (or all n), longest first by length bin.
+int order_reads(dnaln_ctx* c, const int32_t* d_seq_len, const int32_t* list, const int* list_n, int64_t n,
+                int64_t max_len, int32_t* ord) {
+  DBUF(bins, int, "read_bins", 2 * kLengthBins);
+  CK(cudaMemsetAsync(bins, 0, 2 * kLengthBins * sizeof(int), c->st));
+  const KernelTrace kt = tracer(c);
+  kt.begin(c->st, "k_read_order");
+  launch_read_order(c->st, d_seq_len, list, list_n, static_cast<int>(n), max_len, bins, ord);
+  kt.end(c->st);
+  c->stats.launches += 2;
+  return DNALN_OK;
+}
+
 // Checks that need no index.
 int validate_map_params_basic(dnaln_ctx* c, const dnaln_map_params* p) {
   if (!p) return fail(c, DNALN_ERR_INVALID_ARG, "null map params");
@@ -610,12 +623,12 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   // info: [0] longest read, [1..3] cells, mapped, candidates (map.cuh), [4] minimizers,
   // [5] anchors of the thread path
   // [6] minimizers, [7] bases and [9] anchors of the reads left for the warp path, [8] the
-  // chaining pool's fill
-  DBUF(info, unsigned long long, "info", 10);
-  CK(cudaMemsetAsync(info, 0, 10 * sizeof(unsigned long long), st));
+  // chaining pool's fill, [10] long reads the colinear kernel finished
+  DBUF(info, unsigned long long, "info", 11);
+  CK(cudaMemsetAsync(info, 0, 11 * sizeof(unsigned long long), st));
   CK(cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), st));
   CK(cudaMemsetAsync(c->d_count, 0, 4 * sizeof(int), st));
-  // work-stealing claim counters: [1] warp chaining kernel ([0] spare)
+  // [0] reads the colinear kernel listed, [1] work-stealing claims of the warp chaining kernel
   DBUF(claims, int, "claims", 2);
   CK(cudaMemsetAsync(claims, 0, 2 * sizeof(int), st));
   unsigned long long* ctr = info + 1;  // cells, mapped, candidates (map.cuh)
@@ -635,7 +648,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   if (max_len > (1 << 28)) return fail(c, DNALN_ERR_INVALID_ARG, "read longer than 2^28 bases");
 
   // pass 1: encode, sketch, probe
-  DBUF(codes, uint8_t, "codes", 2 * B);
+  DBUF(codes, uint8_t, "codes", 2 * B + 64);  // the sketch reads whole 16-byte chunks around a read
   MinBuf mb;
   mb.hash = dbuf<uint64_t>(c, "m_hash", B);
   mb.pos = dbuf<uint32_t>(c, "m_pos", B);
@@ -676,8 +689,32 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       launch_encode_reads(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, codes);
     kt.end(st);
     c->stats.launches += 1;
+    // reads whose anchors form one colinear chain; the others are listed for the full kernels
+    const int32_t* full_list = nullptr;
+    const int* full_n = nullptr;
+    if (c->colinear && seed_colinear_supported(sp, cp, ix.dev)) {
+      DBUF(rest, int32_t, "colinear_rest", n);
+      const int32_t* order = nullptr;
+      if (by_length && n > 1) {
+        DBUF(ord, int32_t, "read_order", n);
+        if (int e = order_reads(c, d_seq_len, nullptr, nullptr, n, max_len, ord)) return e;
+        order = ord;
+      }
+      const int lanes = seed_colinear_lanes(n, max_len);
+      DBUF(sk_counts, int32_t, "sketch_counts", n * lanes);
+      kt.begin(st, "k_sketch_reads");
+      launch_sketch_reads(st, codes, pofs, d_seq_len, order, n, lanes, sp, mb.hash, sk_counts);
+      kt.end(st);
+      kt.begin(st, "k_probe_reads");
+      launch_probe_reads(st, pofs, d_seq_len, n, lanes, mb.hash, sk_counts, ix.dev, sp, cp, cand, cb, n_min, n_anchor,
+                         n_anc_t, rest, claims, seed_thread_max_len(), info + 10, c->d_err);
+      kt.end(st);
+      c->stats.launches += 2;
+      full_list = rest;
+      full_n = claims;
+    }
     const auto seed_t = [&](int rpb) {
-      return launch_seed_chain_thread(st, codes, pofs, d_seq_len, n, ix.dev, sp, cp, cand, cb,
+      return launch_seed_chain_thread(st, codes, pofs, d_seq_len, full_list, full_n, n, ix.dev, sp, cp, cand, cb,
                                       n_min, n_anchor, n_anc_t, big_list, big_n, c->d_err, rpb);
     };
     int rpb = c->seed_block ? c->seed_block : (c->seed_tune.tuned ? c->seed_tune.reads_per_block : 0);
@@ -718,22 +755,9 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       DBUF(big2, int32_t, "big2_list", n);
       const int32_t* order = big_list;
       if (by_length && n > 1) {
-        DBUF(lk_in, uint32_t, "long_kin", n);
-        DBUF(lk_out, uint32_t, "long_kout", n);
-        DBUF(lv_in, int32_t, "long_vin", n);
-        DBUF(lv_out, int32_t, "long_vout", n);
-        kt.begin(st, "k_long_keys");
-        const int key_bits = launch_long_order(st, big_list, big_n, static_cast<int>(n), d_seq_len, max_len, lk_in, lv_in);
-        kt.end(st);
-        size_t tmp = 0;
-        CK(cub::DeviceRadixSort::SortPairs(nullptr, tmp, lk_in, lk_out, lv_in, lv_out, static_cast<int>(n), 0, key_bits,
-                                           st));
-        DBUF(tb, uint8_t, "cub_tmp_lsort", tmp);
-        kt.begin(st, "cub_sort");
-        CK(cub::DeviceRadixSort::SortPairs(tb, tmp, lk_in, lk_out, lv_in, lv_out, static_cast<int>(n), 0, key_bits, st));
-        kt.end(st);
-        order = lv_out;
-        c->stats.launches += 1;
+        DBUF(ord, int32_t, "long_order", n);
+        if (int e = order_reads(c, d_seq_len, big_list, big_n, n, max_len, ord)) return e;
+        order = ord;
       }
       kt.begin(st, "k_seed_chain_tl");
       if (!launch_seed_chain_long(st, d_seq_len, pofs, codes, order, big_n, lt, ix.dev, sp, cp, cand, cb, n_min,
@@ -867,7 +891,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   CK(cudaMemcpyAsync(h + 1, c->d_count, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(h + 3, c->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(h + 4, ctr, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(h + 7, info + 4, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(h + 7, info + 4, 7 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   run.B = B;
   run.max_len = max_len;
   run.cigar_cap = cigar_cap;
@@ -901,7 +925,7 @@ int map_finish(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_s
   const uint64_t n_cells = static_cast<uint64_t>(h[4]), n_mapped = static_cast<uint64_t>(h[5]),
                  n_cands = static_cast<uint64_t>(h[6]);
   const int64_t n_minimizers = h[7], n_anchors_thread = h[8], n_minimizers_warp_l = h[9], n_bases_warp_l = h[10];
-  const int64_t pool_used = h[11], n_anchors_warp = h[12];
+  const int64_t pool_used = h[11], n_anchors_warp = h[12], n_long_colinear = h[13];
   if (errbits & kErrChainPool) {
     // the chaining pool was too small for this batch: grow it to what the batch asked for
     // and map the batch again (outputs are rewritten in full; counters are not yet added)
@@ -935,7 +959,7 @@ int map_finish(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_s
   s.warp_minimizers += static_cast<uint64_t>(thread_path ? n_minimizers_warp_l : n_minimizers);
   s.warp_anchors += static_cast<uint64_t>(n_anchors_warp);
   s.warp_bases += static_cast<uint64_t>(thread_path ? n_bases_warp_l : B);
-  s.long_reads += static_cast<uint64_t>(thread_path && run.long_used ? n_listed - n_warp : 0);
+  s.long_reads += static_cast<uint64_t>(n_long_colinear + (thread_path && run.long_used ? n_listed - n_warp : 0));
   s.sw_tasks_score += static_cast<uint64_t>(counts[0]);
   s.sw_tasks_tb += static_cast<uint64_t>(counts[1]);
   s.cells += n_cells;
@@ -967,7 +991,7 @@ std::string graph_key(const dnaln_ctx* c, const IndexRes& ix, const char* d_seq,
   put(ptrs, sizeof ptrs);
   const int64_t nums[] = {n, hint.seq_base, hint.bases, hint.max_len, hint.cigar_base, cigar_cap, c->pool_cap,
                           static_cast<int64_t>(c->dir_cap_bytes), c->sw_mode, c->warp_seed_only, c->long_thread,
-                          c->length_order, c->ungapped, c->stealing, c->encode_bulk, c->seed_block,
+                          c->length_order, c->ungapped, c->colinear, c->stealing, c->encode_bulk, c->seed_block,
                           c->seed_tune.tuned ? c->seed_tune.reads_per_block : 0};
   put(nums, sizeof nums);
   put(&p, sizeof p);
@@ -996,7 +1020,7 @@ int run_map(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_seq_
     cudaStream_t st = c->st;
     DBUF(len64, int64_t, "len64", n + 1);
     DBUF(pofs, int64_t, "pofs", n + 1);
-    DBUF(info, unsigned long long, "info", 10);
+    DBUF(info, unsigned long long, "info", 11);
     CK(cudaMemsetAsync(info, 0, sizeof(unsigned long long), st));
     k_len64<<<nblk(n + 1), 256, 0, st>>>(d_seq_len, n, len64, info);
     if (int e = exclusive_scan(c, len64, pofs, n + 1)) return e;
@@ -1506,6 +1530,10 @@ int dnaln_gpu_set_option(dnaln_ctx* c, const char* name, int64_t value) {
   }
   if (k == "long_thread") {
     c->long_thread = value != 0;
+    return DNALN_OK;
+  }
+  if (k == "colinear") {
+    c->colinear = value != 0;
     return DNALN_OK;
   }
   if (k == "ungapped") {

@@ -168,4 +168,38 @@ __device__ __forceinline__ int warp_exclusive_scan(int v, int* total) {
   return x - v;
 }
 
+// Length order by counting: bins of 2^bin_shift lengths, bin 0 the longest.
+constexpr int kLengthBins = 1024;
+__host__ __device__ __forceinline__ int length_bin(int len, int bin_shift) {
+  const int x = len >> bin_shift;
+  return kLengthBins - 1 - (x < 0 ? 0 : (x < kLengthBins ? x : kLengthBins - 1));
+}
+inline int length_bin_shift(int64_t max_len) {
+  int s = 0;
+  while ((max_len >> s) >= kLengthBins) ++s;
+  return s;
+}
+// first[b] (shared memory) = the elements of the bins before b; called by a block of 256.
+__device__ __forceinline__ void scan_length_bins(const int* __restrict__ hist, int* first) {
+  constexpr int kPer = kLengthBins / 256;
+  __shared__ int warp_total[8];
+  int v[kPer], sum = 0;
+#pragma unroll
+  for (int x = 0; x < kPer; ++x) {
+    v[x] = hist[threadIdx.x * kPer + x];
+    sum += v[x];
+  }
+  int total;
+  int ex = warp_exclusive_scan(sum, &total);
+  if ((threadIdx.x & 31) == 31) warp_total[threadIdx.x >> 5] = total;
+  __syncthreads();
+  for (int w = 0; w < static_cast<int>(threadIdx.x >> 5); ++w) ex += warp_total[w];
+#pragma unroll
+  for (int x = 0; x < kPer; ++x) {
+    first[threadIdx.x * kPer + x] = ex;
+    ex += v[x];
+  }
+  __syncthreads();
+}
+
 }  // namespace dnb

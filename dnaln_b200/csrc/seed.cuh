@@ -155,7 +155,30 @@ void launch_encode_reads(cudaStream_t st, const char* seq, const int64_t* seq_of
 void launch_encode_reads_bulk(cudaStream_t st, const char* seq, const int64_t* seq_off, int64_t seq_base,
                               const int32_t* seq_len, const int64_t* pofs, int64_t n, uint8_t* codes, uint32_t* err);
 
-// One thread per read (seed_thread.cu): passes 1 and 2 of the reads the per-thread budgets
+// Passes 1 and 2 of the reads whose anchors form one colinear chain (seed_colinear.cu), from
+// their forward codes (whose buffer has 64 bytes of padding). launch_sketch_reads: the
+// minimizers of every read, lanes (from seed_colinear_lanes) lanes each, in the order `order`
+// gives (may be null), to mins (total bases entries) and counts (n * lanes).
+// launch_probe_reads: candidates, n_min, n_anc_t and n_anchor = 0 of the reads found to have
+// one chain; the others are appended to list (*list_n = 0 before). *long_done += finished
+// reads longer than long_len.
+bool seed_colinear_supported(const SeedParams& sp, const ChainParamsDev& cp, const DevIndex& ix);
+int seed_colinear_lanes(int64_t n, int64_t max_len);
+void launch_sketch_reads(cudaStream_t st, const uint8_t* codes, const int64_t* pofs, const int32_t* seq_len,
+                         const int32_t* order, int64_t n, int lanes, const SeedParams& sp, uint64_t* mins,
+                         int32_t* counts);
+void launch_probe_reads(cudaStream_t st, const int64_t* pofs, const int32_t* seq_len, int64_t n, int lanes,
+                        const uint64_t* mins, const int32_t* counts, const DevIndex& ix, const SeedParams& sp,
+                        const ChainParamsDev& cp, const CandParams& cand, CandBuf cb, int32_t* n_min,
+                        int64_t* n_anchor, int32_t* n_anc_t, int32_t* list, int* list_n, int long_len,
+                        unsigned long long* long_done, uint32_t* err);
+// order = the reads of list[0, *list_n) (all n without a list; n at least the list's
+// length), longest first by length bin; bins: 2 * kLengthBins zeros.
+void launch_read_order(cudaStream_t st, const int32_t* seq_len, const int32_t* list, const int* list_n, int n,
+                       int64_t max_len, int* bins, int32_t* order);
+
+// One thread per read (seed_thread.cu), of the reads list[0, *list_n) or, without a list, of
+// all n: passes 1 and 2 of the reads the per-thread budgets
 // admit, from their forward codes (codes + 2 * pofs[r], written by launch_encode_reads on
 // the same stream before), writing
 // candidates of the admitted reads, n_min, n_anc_t (their anchor counts, for statistics)
@@ -166,7 +189,8 @@ void launch_encode_reads_bulk(cudaStream_t st, const char* seq, const int64_t* s
 bool seed_thread_supported(const SeedParams& sp, const ChainParamsDev& cp);
 int seed_thread_max_len();  // the longest read the short thread kernel stages
 bool launch_seed_chain_thread(cudaStream_t st, const uint8_t* codes, const int64_t* pofs,
-                              const int32_t* seq_len, int64_t n, const DevIndex& ix, const SeedParams& sp,
+                              const int32_t* seq_len, const int32_t* list, const int* list_n, int64_t n,
+                              const DevIndex& ix, const SeedParams& sp,
                               const ChainParamsDev& cp,
                               const CandParams& cand, CandBuf cb, int32_t* n_min, int64_t* n_anchor,
                               int32_t* n_anc_t, int32_t* big_list, int* big_n, uint32_t* err,
@@ -185,12 +209,6 @@ bool launch_seed_chain_long(cudaStream_t st, const int32_t* seq_len, const int64
                             const SeedParams& sp, const ChainParamsDev& cp, const CandParams& cand, CandBuf cb,
                             int32_t* n_min, int64_t* n_anchor, int32_t* n_anc_t, uint32_t* scratch,
                             int32_t* next_list, int* next_n, int min_len, uint32_t* err);
-// Sort keys (longest first; slots at or past *list_n last) and values (read ids) of a list
-// whose length is only known on the device; n_max = the list buffer's size, max_len at
-// least the longest read. Returns the number of low key bits the sort must cover.
-int launch_long_order(cudaStream_t st, const int32_t* list, const int* list_n, int n_max, const int32_t* seq_len,
-                      int64_t max_len, uint32_t* keys, int32_t* vals);
-
 // Stage entry points: sketch of code sequences, lookups, chaining of given anchor sets.
 void launch_sketch_codes(cudaStream_t st, const uint8_t* codes, const int64_t* seq_off, const int32_t* seq_len,
                          const uint32_t* pos_offset, int64_t n, int32_t k, int32_t w, uint64_t* out_hash,

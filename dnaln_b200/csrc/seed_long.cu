@@ -33,6 +33,9 @@ constexpr int kLBlocksPerSm = 8;  // blocks per SM the grid is sized for: 6 resi
 constexpr int kLMaxMin = 256;
 constexpr int kLMaxAnc = 256;
 constexpr int kLMaxChains = 32;
+// A list of at most this many reads goes on to the warp kernels as it is: one thread takes
+// 1.2 ms for a 1,000 bp read and its global columns, however few there are.
+constexpr int kLFew = 4096;
 constexpr int kLMaxBand = 256;    // chaining band of the shared gap-cost table
 // column words per thread: A = anchor keys (hi, lo); B = minimizer slots (hash, pos |
 // strand << 31), later the DP words (f | maxf << 16, prev + 1) and the chain table;
@@ -42,26 +45,6 @@ constexpr int kLWordsB = 2 * kLMaxAnc + 4 * kLMaxChains + kLMaxAnc;  // DP words
 constexpr int kLWordsU = kLMaxAnc / 32;
 static_assert(2 * kLMaxMin <= kLWordsB, "minimizer slots must fit region B");
 constexpr int kLWords = kLWordsA + kLWordsB + kLWordsU;
-
-// Sort keys of the listed reads, longest first; slots at or past the device count last.
-// Keys are top - length with top = 2^bits - 1 (every length of the batch at most top), the
-// empty slots 2^bits: a sort over bits + 1 key bits.
-__global__ void k_long_keys(const int32_t* __restrict__ list, const int* __restrict__ list_n, int n_max,
-                            const int32_t* __restrict__ seq_len, uint32_t top, uint32_t* __restrict__ keys,
-                            int32_t* __restrict__ vals) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= n_max) return;
-  const int m = *list_n;
-  if (x < m) {
-    const int32_t r = list[x];
-    const uint32_t len = static_cast<uint32_t>(seq_len[r]);
-    keys[x] = len < top ? top - len : 0u;  // a length past top (not expected) still sorts first
-    vals[x] = r;
-  } else {
-    keys[x] = top + 1u;
-    vals[x] = -1;
-  }
-}
 
 template <int W>
 __global__ void __launch_bounds__(kLT, 6)
@@ -91,6 +74,13 @@ __global__ void __launch_bounds__(kLT, 6)
     return reinterpret_cast<int32_t&>(B(2 * kLMaxAnc + field * kLMaxChains + c));
   };
   const int m_list = *list_n;
+  if (m_list <= kLFew) {
+    for (int64_t x = tid; x < m_list; x += stride) {
+      next_list[x] = list[x];
+      if (x == 0) *next_n = m_list;
+    }
+    return;
+  }
   const int k = sp.k;
   // The grid is more blocks than are resident: the first wave takes the longest reads of
   // the (longest-first) list, and the later blocks start as the first's finish. A thread
@@ -488,15 +478,6 @@ int64_t seed_long_threads(int64_t n_max) {
 }
 
 size_t seed_long_scratch_words(int64_t threads) { return static_cast<size_t>(threads) * kLWords; }
-
-int launch_long_order(cudaStream_t st, const int32_t* list, const int* list_n, int n_max, const int32_t* seq_len,
-                      int64_t max_len, uint32_t* keys, int32_t* vals) {
-  int bits = 16;  // 16 bits cover reads up to 65,535 bp: two radix passes instead of four
-  while (bits < 31 && max_len > (int64_t{1} << bits) - 1) ++bits;
-  if (n_max > 0)
-    k_long_keys<<<(n_max + 255) / 256, 256, 0, st>>>(list, list_n, n_max, seq_len, (1u << bits) - 1u, keys, vals);
-  return bits + 1;
-}
 
 bool launch_seed_chain_long(cudaStream_t st, const int32_t* seq_len, const int64_t* pofs, const uint8_t* codes,
                             const int32_t* list, const int* list_n, int64_t threads, const DevIndex& ix,

@@ -73,6 +73,11 @@ struct TLayout {
   static constexpr int kSmem = kRegionA + kRegionB + (kTMaxBand + 1) * 4;
 };
 
+// A list of at most this many reads goes on to the next kernels as it is: one thread per read
+// takes as long for a few reads as for a wave of 56,832 (112 us at 150 bp), one warp per read
+// 30 us for 1,500 and 200 us for 20,000.
+constexpr int kTFew = 4096;
+
 // 4-byte asynchronous copy global -> shared (both 4-byte aligned).
 __device__ __forceinline__ void cp_async4(uint32_t* dst_smem, const void* src) {
   const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst_smem));
@@ -113,7 +118,8 @@ __global__ void __launch_bounds__(256)
 template <int W, int TT>
 __global__ void __launch_bounds__(TT)
     k_seed_chain_t(const uint8_t* __restrict__ codes, const int64_t* __restrict__ pofs,
-                   const int32_t* __restrict__ seq_len, int64_t n, DevIndex ix, SeedParams sp, ChainParamsDev cp,
+                   const int32_t* __restrict__ seq_len, const int32_t* __restrict__ list,
+                   const int* __restrict__ list_n, int64_t n, DevIndex ix, SeedParams sp, ChainParamsDev cp,
                    CandParams cand,
                    CandBuf cb, int32_t* __restrict__ n_min, int64_t* __restrict__ n_anchor,
                    int32_t* __restrict__ n_anc_t, int32_t* __restrict__ big_list, int* __restrict__ big_n,
@@ -123,6 +129,20 @@ __global__ void __launch_bounds__(TT)
   uint32_t* const stg = reinterpret_cast<uint32_t*>(smem);  // region A (all columns, for the staging)
   int32_t* const lut = reinterpret_cast<int32_t*>(smem + L::kRegionA + L::kRegionB);  // chaining gap costs
   const int T = threadIdx.x, lane = T & 31;
+  if (list_n) n = *list_n;
+  if (static_cast<int64_t>(blockIdx.x) * TT >= n) return;
+  if (list_n && n <= kTFew) {
+    const int64_t x = static_cast<int64_t>(blockIdx.x) * TT + T;
+    if (x < n) {
+      const int32_t r = list[x];
+      n_min[r] = 0;
+      n_anc_t[r] = 0;
+      n_anchor[r] = 0;
+      big_list[x] = r;
+      if (x == 0) *big_n = static_cast<int>(n);
+    }
+    return;
+  }
   for (int d = T; d <= cp.band; d += TT) lut[d] = cp.cost[d];
   __syncthreads();
   uint32_t* const ca = stg + T;                                                   // this thread's A column
@@ -143,12 +163,12 @@ __global__ void __launch_bounds__(TT)
     return reinterpret_cast<int32_t&>(cbw[(kTMaxAnc + field * kTMaxChains + c) * TT]);
   };
 
-  const int64_t r0 = static_cast<int64_t>(blockIdx.x) * TT + (T & ~31);  // first read of this warp
-  const int64_t r = r0 + lane;
+  const int64_t x = static_cast<int64_t>(blockIdx.x) * TT + T;  // place in the list, or the read
+  const int64_t r = x < n ? (list ? list[x] : x) : 0;
   int len = 0;
   uint64_t a_word = 0;  // this read's first code byte rounded down to a 4-byte boundary
   int offb = 0, nwords = 0;
-  if (r < n) {
+  if (x < n) {
     len = seq_len[r];
     const uint64_t a = reinterpret_cast<uint64_t>(codes) + 2 * static_cast<uint64_t>(pofs[r]);  // forward codes
     offb = static_cast<int>(a & 3u);
@@ -169,7 +189,7 @@ __global__ void __launch_bounds__(TT)
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncwarp();
-  if (r >= n) return;
+  if (x >= n) return;
 
   const int k = sp.k;
   bool big = len > kTMaxLen;
@@ -483,14 +503,14 @@ __global__ void __launch_bounds__(TT)
 
 template <int TT>
 bool launch_thread_tt(cudaStream_t st, const uint8_t* codes, const int64_t* pofs,
-                      const int32_t* seq_len, int64_t n, const DevIndex& ix, const SeedParams& sp,
-                      const ChainParamsDev& cp, const CandParams& cand, CandBuf cb, int32_t* n_min, int64_t* n_anchor,
+                      const int32_t* seq_len, const int32_t* list, const int* list_n, int64_t n, const DevIndex& ix,
+                      const SeedParams& sp, const ChainParamsDev& cp, const CandParams& cand, CandBuf cb, int32_t* n_min, int64_t* n_anchor,
                       int32_t* n_anc_t, int32_t* big_list, int* big_n, uint32_t* err) {
   static std::atomic<bool> attr_set[kMaxDevices];
   if (!set_smem_limit_once(k_seed_chain_t<kTW, TT>, TLayout<TT>::kSmem, attr_set)) return false;
   const int64_t blocks = (n + TT - 1) / TT;
   k_seed_chain_t<kTW, TT><<<static_cast<unsigned>(blocks), TT, TLayout<TT>::kSmem, st>>>(
-      codes, pofs, seq_len, n, ix, sp, cp, cand, cb, n_min, n_anchor, n_anc_t, big_list, big_n, err);
+      codes, pofs, seq_len, list, list_n, n, ix, sp, cp, cand, cb, n_min, n_anchor, n_anc_t, big_list, big_n, err);
   return true;
 }
 
@@ -511,17 +531,17 @@ void launch_encode_reads(cudaStream_t st, const char* seq, const int64_t* seq_of
 }
 
 bool launch_seed_chain_thread(cudaStream_t st, const uint8_t* codes, const int64_t* pofs,
-                              const int32_t* seq_len, int64_t n, const DevIndex& ix, const SeedParams& sp,
-                              const ChainParamsDev& cp,
+                              const int32_t* seq_len, const int32_t* list, const int* list_n, int64_t n,
+                              const DevIndex& ix, const SeedParams& sp, const ChainParamsDev& cp,
                               const CandParams& cand, CandBuf cb, int32_t* n_min, int64_t* n_anchor,
                               int32_t* n_anc_t, int32_t* big_list, int* big_n, uint32_t* err, int reads_per_block) {
   if (!seed_thread_supported(sp, cp)) return false;
   if (n <= 0) return true;
   if (reads_per_block == 64)
-    return launch_thread_tt<64>(st, codes, pofs, seq_len, n, ix, sp, cp, cand, cb, n_min, n_anchor, n_anc_t,
+    return launch_thread_tt<64>(st, codes, pofs, seq_len, list, list_n, n, ix, sp, cp, cand, cb, n_min, n_anchor, n_anc_t,
                                 big_list, big_n, err);
   if (reads_per_block == 128)
-    return launch_thread_tt<128>(st, codes, pofs, seq_len, n, ix, sp, cp, cand, cb, n_min, n_anchor,
+    return launch_thread_tt<128>(st, codes, pofs, seq_len, list, list_n, n, ix, sp, cp, cand, cb, n_min, n_anchor,
                                  n_anc_t, big_list, big_n, err);
   return false;
 }

@@ -61,14 +61,8 @@ void launch_sw_ungapped(cudaStream_t st, bool tb, const SwTask* tasks, int n, co
                         const uint8_t* tbase, const SwParams& p, SwResult* res, uint32_t* cig, const int64_t* cig_off,
                         SwTask* todo, int* todo_n, int* hist, int bin_shift);
 
-// Length order of tasks, longest first, by counting over kSwLengthBins bins of
-// 2^bin_shift lengths: launch_length_bins fills hist (zero before), launch_order_tasks
-// writes out (taken: kSwLengthBins zeros).
-constexpr int kSwLengthBins = 1024;
-__host__ __device__ __forceinline__ int sw_length_bin(int len, int bin_shift) {
-  const int x = len >> bin_shift;
-  return kSwLengthBins - 1 - (x < kSwLengthBins ? x : kSwLengthBins - 1);
-}
+// Length order of tasks, longest first (length_bin): launch_length_bins fills hist
+// (kLengthBins zeros before), launch_order_tasks writes out (taken: kLengthBins zeros).
 void launch_length_bins(cudaStream_t st, const SwTask* tasks, int n, const int* n_dev, int* hist, int bin_shift);
 void launch_order_tasks(cudaStream_t st, const SwTask* tasks, int n, const int* n_dev, const int* hist, int* taken,
                         int bin_shift, SwTask* out);

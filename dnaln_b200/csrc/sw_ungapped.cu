@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kThreads)
       at = __shfl_sync(FULL, at, 0);
       if (lead && !ok) {
         todo[at + __popc(left & ((1u << lane) - 1u))] = tk;
-        if (hist) atomicAdd(hist + sw_length_bin(L, bin_shift), 1);
+        if (hist) atomicAdd(hist + length_bin(L, bin_shift), 1);
       }
     }
   }
@@ -279,7 +279,7 @@ __global__ void k_length_bins(const SwTask* __restrict__ tasks, int n, const int
                               int* __restrict__ hist, int bin_shift) {
   const int nn = n_dev ? min(n, *n_dev) : n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x)
-    atomicAdd(hist + sw_length_bin(tasks[i].qlen, bin_shift), 1);
+    atomicAdd(hist + length_bin(tasks[i].qlen, bin_shift), 1);
 }
 
 // out = the tasks by length bin (bin 0, the longest, first), in any order within a bin: every
@@ -287,31 +287,13 @@ __global__ void k_length_bins(const SwTask* __restrict__ tasks, int n, const int
 __global__ void __launch_bounds__(256)
     k_order_tasks(const SwTask* __restrict__ tasks, int n, const int* __restrict__ n_dev,
                   const int* __restrict__ hist, int* __restrict__ taken, int bin_shift, SwTask* __restrict__ out) {
-  constexpr int kPer = kSwLengthBins / 256;
-  __shared__ int first[kSwLengthBins];
-  __shared__ int warp_sum_s[8];
+  __shared__ int first[kLengthBins];
   const int nn = n_dev ? min(n, *n_dev) : n;
   if (static_cast<int>(blockIdx.x * blockDim.x) >= nn) return;
-  int v[kPer], sum = 0;
-#pragma unroll
-  for (int x = 0; x < kPer; ++x) {
-    v[x] = hist[threadIdx.x * kPer + x];
-    sum += v[x];
-  }
-  int total;
-  int ex = warp_exclusive_scan(sum, &total);
-  if ((threadIdx.x & 31) == 31) warp_sum_s[threadIdx.x >> 5] = total;
-  __syncthreads();
-  for (int w = 0; w < static_cast<int>(threadIdx.x >> 5); ++w) ex += warp_sum_s[w];
-#pragma unroll
-  for (int x = 0; x < kPer; ++x) {
-    first[threadIdx.x * kPer + x] = ex;
-    ex += v[x];
-  }
-  __syncthreads();
+  scan_length_bins(hist, first);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
     const SwTask t = tasks[i];
-    const int b = sw_length_bin(t.qlen, bin_shift);
+    const int b = length_bin(t.qlen, bin_shift);
     out[first[b] + atomicAdd(taken + b, 1)] = t;
   }
 }

@@ -95,7 +95,7 @@ typedef struct {
   /* reads seeded and chained one warp per read (long reads, or past the per-thread
    * budget), their minimizers, anchors and bases */
   uint64_t warp_reads, warp_minimizers, warp_anchors, warp_bases;
-  uint64_t long_reads; /* reads seeded and chained by the long-read thread kernel */
+  uint64_t long_reads; /* reads past the short thread kernel's length seeded and chained without the warp kernels */
   uint64_t graph_launches; /* batches launched as a captured CUDA graph (running total) */
   uint64_t batch_retries;  /* batches mapped again after the chaining pool grew */
 } dnaln_stats;
@@ -145,6 +145,8 @@ int dnaln_gpu_set_sub_batch(dnaln_ctx* ctx, int64_t reads);
  *                    the long-read kernel first (default); 0 = straight to the warp kernels;
  *   "length_order"   1 = SW tasks of a batch whose reads differ in length run longest
  *                    first (default); 0 = in read order;
+ *   "colinear"       1 = reads whose anchors are checked, as they are found, to form one
+ *                    colinear chain skip the chaining DP (default); 0 = every read runs it;
  *   "ungapped"       1 = banded SW tasks proved from bit vectors to align by diagonal steps
  *                    only skip the DP kernels (default); 0 = every task runs the DP;
  *   "seed_block"     reads per block of the thread-per-read seeding kernel: 0 = tuned
