@@ -2186,51 +2186,56 @@ int dnaln_gpu_align(dnaln_ctx* c, const uint8_t* q, const int64_t* q_off, const 
   if (n > (int64_t(1) << 31) - 64) return fail(c, DNALN_ERR_INVALID_ARG, "too many tasks in one call");
   if (int e = set_device(c)) return e;
   const int W = 2 * sp->bw + 1;
-  int64_t qext = 0, text = 0, cig_total = 0;
+  // extents and totals the host needs; the tasks themselves are built on the device
+  int64_t qext = 0, text = 0, bases = 0, neg = 0;
   int rows_max = 0;
-  std::vector<SwTask> tasks(static_cast<size_t>(n));
-  std::vector<int64_t> slot_off(static_cast<size_t>(n));
   for (int64_t i = 0; i < n; ++i) {
-    if (q_len[i] < 0 || t_len[i] < 0 || q_off[i] < 0 || t_off[i] < 0)
-      return fail(c, DNALN_ERR_INVALID_ARG, "negative offset or length in task %lld", static_cast<long long>(i));
-    qext = std::max<int64_t>(qext, q_off[i] + q_len[i]);
-    const int64_t tmax = static_cast<int64_t>(q_len[i]) + W - 1;
-    const int64_t tl = t_len[i] < tmax ? t_len[i] : tmax;
-    text = std::max<int64_t>(text, t_off[i] + tl);
-    SwTask& tk = tasks[static_cast<size_t>(i)];
-    tk.q_off = q_off[i];
-    tk.qlen = q_len[i];
-    tk.t_start = t_off[i];
-    tk.t_lo = t_off[i];
-    tk.t_hi = t_off[i] + tl;
-    tk.slot = static_cast<int32_t>(i);
-    slot_off[static_cast<size_t>(i)] = cig_total;
-    cig_total += 2 * static_cast<int64_t>(q_len[i]) + 1;
+    const int64_t ql = q_len[i], tl = t_len[i], tmax = ql + W - 1;
+    neg |= ql | tl | q_off[i] | t_off[i];
+    qext = std::max(qext, q_off[i] + ql);
+    text = std::max(text, t_off[i] + std::min(tl, tmax));
+    bases += ql;
     rows_max = std::max(rows_max, q_len[i]);
   }
+  if (neg < 0) {
+    int64_t i = 0;
+    while (q_len[i] >= 0 && t_len[i] >= 0 && q_off[i] >= 0 && t_off[i] >= 0) ++i;
+    return fail(c, DNALN_ERR_INVALID_ARG, "negative offset or length in task %lld", static_cast<long long>(i));
+  }
+  const int64_t cig_total = 2 * bases + n;
   cudaStream_t st = c->st;
   const bool tb = traceback != 0;
   const bool by_length =  // as for a batch of reads
-      c->length_order && rows_max > 1.25 * static_cast<double>((cig_total - n) / 2) / static_cast<double>(n);
+      c->length_order && rows_max > 1.25 * static_cast<double>(bases) / static_cast<double>(n);
   DBUF(d_q, uint8_t, "al_q", qext);
   DBUF(d_t, uint8_t, "al_t", text);
+  DBUF(d_off, int64_t, "al_off", 2 * n);
+  DBUF(d_len, int32_t, "al_len", 2 * n);
   DBUF(d_tasks, SwTask, "al_tasks", n);
   DBUF(d_res, SwResult, "al_res", n);
+  DBUF(d_out, dnaln_align_result, "al_out", n);
   CK(cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), st));
+  CK(cudaMemcpyAsync(d_off, q_off, n * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d_off + n, t_off, n * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d_len, q_len, n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d_len + n, t_len, n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
   if (qext) CK(cudaMemcpyAsync(d_q, q, qext, cudaMemcpyHostToDevice, st));
   if (text) CK(cudaMemcpyAsync(d_t, t, text, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(d_tasks, tasks.data(), n * sizeof(SwTask), cudaMemcpyHostToDevice, st));
+  c->trace_n = 0;
+  c->trace_open = false;
   const SwParams swp = make_sw_params(*sp);
   uint32_t* d_cig = nullptr;
   int64_t* d_slot = nullptr;
+  int64_t* d_cnt = nullptr;
   if (tb) {
     d_cig = dbuf<uint32_t>(c, "al_cig", cig_total);
-    d_slot = dbuf<int64_t>(c, "al_slot", n);
-    if (!d_cig || !d_slot) return DNALN_ERR_OOM;
-    CK(cudaMemcpyAsync(d_slot, slot_off.data(), n * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+    d_slot = dbuf<int64_t>(c, "al_slot", n + 1);
+    d_cnt = dbuf<int64_t>(c, "al_cnt", n + 1);
+    if (!d_cig || !d_slot || !d_cnt) return DNALN_ERR_OOM;
   }
-  c->trace_n = 0;
-  c->trace_open = false;
+  launch_align_tasks(st, n, d_off, d_len, W, d_tasks, d_cnt);
+  if (tb)  // each task's room for 2 * qlen + 1 operations
+    if (int e = exclusive_scan(c, d_cnt, d_slot, n + 1)) return e;
   CK(cudaEventRecord(c->ev[tb ? kEvTb0 : kEvSc0], st));
   if (int e = launch_sw_chunked(c, tb, sw_bytes_ok(*sp), d_tasks, static_cast<int>(n), nullptr, d_q, d_t, swp, d_res,
                                 rows_max, d_cig, d_slot, by_length))
@@ -2238,18 +2243,10 @@ int dnaln_gpu_align(dnaln_ctx* c, const uint8_t* q, const int64_t* q_off, const 
   CK(cudaEventRecord(c->ev[tb ? kEvTb1 : kEvSc1], st));
   int64_t total = 0;
   if (!tb) {
-    std::vector<SwResult> res(static_cast<size_t>(n));
-    CK(cudaMemcpyAsync(res.data(), d_res, n * sizeof(SwResult), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    for (int64_t i = 0; i < n; ++i) {
-      dnaln_align_result& o = out[i];
-      std::memset(&o, 0, sizeof o);
-      o.score = res[static_cast<size_t>(i)].score;
-    }
+    launch_align_scores(st, n, d_res, d_out);
+    CK(cudaGetLastError());
   } else {
-    DBUF(d_cnt, int64_t, "al_cnt", n + 1);
     DBUF(d_doff, int64_t, "al_doff", n + 1);
-    DBUF(d_out, dnaln_align_result, "al_out", n);
     launch_align_counts(st, n, d_res, d_cnt);
     if (int e = exclusive_scan(c, d_cnt, d_doff, n + 1)) return e;
     CK(cudaMemcpyAsync(c->h_info, d_doff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -2258,18 +2255,18 @@ int dnaln_gpu_align(dnaln_ctx* c, const uint8_t* q, const int64_t* q_off, const 
     DBUF(d_final, uint32_t, "al_final", total);
     launch_align_gather(st, n, d_res, d_cig, d_slot, d_doff, d_out, d_final);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out, d_out, n * sizeof(dnaln_align_result), cudaMemcpyDeviceToHost, st));
     if (cigar && total <= cigar_cap && total > 0)
       CK(cudaMemcpyAsync(cigar, d_final, total * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
   }
+  CK(cudaMemcpyAsync(out, d_out, n * sizeof(dnaln_align_result), cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(c->h_info, c->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
   trace_collect(c);
-  uint32_t bits = 0;
-  CK(cudaMemcpy(&bits, c->d_err, sizeof bits, cudaMemcpyDeviceToHost));
+  uint32_t bits;
+  std::memcpy(&bits, c->h_info, sizeof bits);
   if (int e = check_device_errors(c, bits)) return e;
   if (cigar_used) *cigar_used = total;
-  c->stats.cells += 0;
-  for (int64_t i = 0; i < n; ++i) c->stats.cells += static_cast<uint64_t>(q_len[i]) * W;
+  c->stats.cells += static_cast<uint64_t>(bases) * W;
   if (tb) {
     c->stats.sw_tasks_tb += static_cast<uint64_t>(n);
     c->stats.ms_sw_tb += ev_ms(c, kEvTb0, kEvTb1);

@@ -195,6 +195,35 @@ __global__ void k_cigar_gather(int64_t n, const int64_t* __restrict__ pofs, cons
   if (seq_len[r] > a.qe) dst[x++] = static_cast<uint32_t>(seq_len[r] - a.qe) << 4 | 4u;
 }
 
+// Tasks of dnaln_gpu_align from its offset and length columns (query at i, target at n + i),
+// the target cut to the band's reach; ops[i] (may be null) = room for the task's CIGAR.
+__global__ void k_align_tasks(int64_t n, const int64_t* __restrict__ off, const int32_t* __restrict__ len, int W,
+                              SwTask* __restrict__ tasks, int64_t* __restrict__ ops) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n) {
+    const int64_t ql = len[i], tl = len[n + i], tmax = ql + W - 1;
+    SwTask t;
+    t.q_off = off[i];
+    t.t_start = t.t_lo = off[n + i];
+    t.t_hi = t.t_start + (tl < tmax ? tl : tmax);
+    t.qlen = static_cast<int32_t>(ql);
+    t.slot = static_cast<int32_t>(i);
+    t.flags = 0;
+    t.pad_ = 0;
+    tasks[i] = t;
+    if (ops) ops[i] = 2 * ql + 1;
+  }
+  if (i == n && ops) ops[n] = 0;
+}
+
+__global__ void k_align_scores(int64_t n, const SwResult* __restrict__ res, dnaln_align_result* __restrict__ out) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  dnaln_align_result o{};
+  o.score = res[i].score;
+  out[i] = o;
+}
+
 __global__ void k_align_counts(int64_t n, const SwResult* __restrict__ res, int64_t* __restrict__ counts) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) counts[i] = res[i].n_ops;
@@ -252,6 +281,15 @@ void launch_cigar_gather(cudaStream_t st, int64_t n, const int64_t* pofs, const 
   if (n <= 0) return;
   k_cigar_gather<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(n, pofs, seq_len, res_tb, cig_src, dst_off,
                                                                          rec_base, out, dst, cap, err);
+}
+
+void launch_align_tasks(cudaStream_t st, int64_t n, const int64_t* off, const int32_t* len, int W, SwTask* tasks,
+                        int64_t* ops) {
+  k_align_tasks<<<blocks_for(n + 1), kThreads, 0, st>>>(n, off, len, W, tasks, ops);
+}
+
+void launch_align_scores(cudaStream_t st, int64_t n, const SwResult* res, dnaln_align_result* out) {
+  if (n > 0) k_align_scores<<<blocks_for(n), kThreads, 0, st>>>(n, res, out);
 }
 
 void launch_align_counts(cudaStream_t st, int64_t n, const SwResult* res, int64_t* counts) {

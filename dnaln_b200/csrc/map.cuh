@@ -38,6 +38,13 @@ void launch_cigar_gather(cudaStream_t st, int64_t n, const int64_t* pofs, const 
                          const SwResult* res_tb, const uint32_t* cig_src, const int64_t* dst_off, int64_t rec_base,
                          dnaln_map_record* out, uint32_t* dst, int64_t cap, uint32_t* err);
 
+// GpuAligner: the tasks of n (offset, length) pairs, queries at [0, n) and targets at [n, 2n)
+// of off and len; ops (n + 1 entries, may be null) = 2 * qlen + 1 each, then 0.
+void launch_align_tasks(cudaStream_t st, int64_t n, const int64_t* off, const int32_t* len, int W, SwTask* tasks,
+                        int64_t* ops);
+// GpuAligner: score-only results.
+void launch_align_scores(cudaStream_t st, int64_t n, const SwResult* res, dnaln_align_result* out);
+
 // GpuAligner: reversed walk ops of task i (slot i, source cig_src + src_off[i]) to
 // dst + dst_off[i]; fills out[i].
 void launch_align_gather(cudaStream_t st, int64_t n, const SwResult* res, const uint32_t* cig_src,
