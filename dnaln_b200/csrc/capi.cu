@@ -57,13 +57,13 @@ struct DevBuf {
 // Device memory of one resident index. Contexts that share the index (index_attach) hold
 // it through a shared pointer; the last holder to release it frees the memory.
 struct IndexMem {
-  DevBuf table, positions, genome, coff, clen, nruns;
+  DevBuf table, positions, genome, coff, clen, nruns;  // views of the allocations below
+  std::vector<void*> own;
   IndexMem() = default;
   IndexMem(const IndexMem&) = delete;
   IndexMem& operator=(const IndexMem&) = delete;
   ~IndexMem() {
-    for (DevBuf* b : {&table, &positions, &genome, &coff, &clen, &nruns})
-      if (b->p) cudaFree(b->p);
+    for (void* p : own) cudaFree(p);
   }
   size_t bytes() const { return table.cap + positions.cap + genome.cap + coff.cap + clen.cap + nruns.cap; }
 };
@@ -207,6 +207,7 @@ struct dnaln_ctx {
 
 namespace {
 
+constexpr size_t kIndexWorkKept = size_t(256) << 20;  // largest index-build workspace a context keeps
 constexpr int64_t kSeedTuneReads = 32768;  // smallest batch the reads-per-block tuner times
 constexpr int64_t kSwTuneMinTasks = 4096;  // smallest SW sample whose timing picks a form
 
@@ -1093,7 +1094,8 @@ IndexRes* find_index(dnaln_ctx* c, int32_t id) {
   return &it->second;
 }
 
-int dalloc(dnaln_ctx* c, DevBuf& b, size_t bytes) {
+// Device memory owned by an index.
+int dalloc(dnaln_ctx* c, IndexMem& m, DevBuf& b, size_t bytes) {
   if (c->fail_alloc_after >= 0 && c->fail_alloc_after-- == 0) {
     b.p = nullptr;
     return fail(c, DNALN_ERR_OOM, "out of device memory allocating %zu bytes for the index (injected)", bytes);
@@ -1103,7 +1105,21 @@ int dalloc(dnaln_ctx* c, DevBuf& b, size_t bytes) {
     b.p = nullptr;
     return fail(c, DNALN_ERR_OOM, "out of device memory allocating %zu bytes for the index", bytes);
   }
+  m.own.push_back(b.p);
   b.cap = bytes;
+  return DNALN_OK;
+}
+
+// The genome and the contig table in one allocation.
+int dalloc_genome(dnaln_ctx* c, IndexMem& m, uint64_t n_bases, int32_t n_contigs) {
+  const auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
+  const size_t off = static_cast<size_t>(n_contigs) * sizeof(uint64_t), len = static_cast<size_t>(n_contigs) * sizeof(uint32_t);
+  DevBuf all;
+  if (int e = dalloc(c, m, all, up(n_bases) + up(off) + len)) return e;
+  auto* p = static_cast<uint8_t*>(all.p);
+  m.genome = DevBuf{p, n_bases};
+  m.coff = DevBuf{p + up(n_bases), off};
+  m.clen = DevBuf{p + up(n_bases) + up(off), len};
   return DNALN_OK;
 }
 
@@ -1627,9 +1643,7 @@ int dnaln_gpu_index_build(dnaln_ctx* c, const uint8_t* genome, uint64_t n_bases,
   r.device = c->device;
   IndexMem& m = *r.mem;
   int e = DNALN_OK;
-  if ((e = dalloc(c, m.genome, n_bases)) || (e = dalloc(c, m.coff, n_contigs * sizeof(uint64_t))) ||
-      (e = dalloc(c, m.clen, n_contigs * sizeof(uint32_t))))
-    return e;
+  if ((e = dalloc_genome(c, m, n_bases, n_contigs))) return e;
   cudaError_t x = cudaSuccess;
   auto up = [&](DevBuf& b, const void* src, size_t bytes) {  // ordered before the build on c->st
     if (x == cudaSuccess && bytes) x = cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, c->st);
@@ -1640,12 +1654,24 @@ int dnaln_gpu_index_build(dnaln_ctx* c, const uint8_t* genome, uint64_t n_bases,
   if (x != cudaSuccess) return fail(c, DNALN_ERR_CUDA, "index upload: %s", cudaGetErrorString(x));
   DeviceIndexBuild b;
   char why[256] = {};
-  e = build_index_on_device(c->st, static_cast<const uint8_t*>(m.genome.p), n_bases, contig_off, contig_len, n_contigs,
-                            k, w, &b, why, sizeof why);
-  // the built arrays belong to the index from here on (freed with it on every path)
+  e = build_index_on_device(
+      c->st, static_cast<const uint8_t*>(m.genome.p), n_bases, static_cast<const uint64_t*>(m.coff.p),
+      static_cast<const uint32_t*>(m.clen.p), contig_len, n_contigs, k, w,
+      [&](size_t bytes) -> void* { return dbuf<uint8_t>(c, "index_work", bytes); },
+      [&](size_t bytes) -> void* {
+        DevBuf built;
+        return dalloc(c, m, built, bytes) == DNALN_OK ? built.p : nullptr;
+      },
+      c->h_info, &b, why, sizeof why);
   m.table = DevBuf{b.table, b.n_buckets * sizeof(ulonglong2)};
   m.positions = DevBuf{b.positions, b.n_pos * sizeof(uint32_t)};
   m.nruns = DevBuf{b.n_runs, static_cast<size_t>(b.n_n_runs) * sizeof(uint2)};
+  // the workspace stays for the next build of a genome this size, unless it is large
+  if (c->bufs["index_work"].cap > kIndexWorkKept) {
+    cudaStreamSynchronize(c->st);
+    cudaFree(c->bufs["index_work"].p);
+    c->bufs.erase("index_work");
+  }
   if (e != DNALN_OK) {
     cudaStreamSynchronize(c->st);
     return fail(c, e, "%s", why);
@@ -1856,10 +1882,10 @@ int dnaln_gpu_index_load(dnaln_ctx* c, const char* path, int32_t* index_id) {
   r.device = c->device;
   IndexMem& m = *r.mem;
   int e = DNALN_OK;
-  if ((e = dalloc(c, m.coff, h.n_contigs * sizeof(uint64_t))) || (e = dalloc(c, m.clen, h.n_contigs * sizeof(uint32_t))) ||
-      (e = dalloc(c, m.genome, h.n_bases)) || (e = dalloc(c, m.table, h.n_buckets * sizeof(ulonglong2))) ||
-      (e = dalloc(c, m.positions, h.n_pos * sizeof(uint32_t))) ||
-      (e = dalloc(c, m.nruns, static_cast<size_t>(h.n_n_runs) * sizeof(uint2))))
+  if ((e = dalloc(c, m, m.coff, h.n_contigs * sizeof(uint64_t))) || (e = dalloc(c, m, m.clen, h.n_contigs * sizeof(uint32_t))) ||
+      (e = dalloc(c, m, m.genome, h.n_bases)) || (e = dalloc(c, m, m.table, h.n_buckets * sizeof(ulonglong2))) ||
+      (e = dalloc(c, m, m.positions, h.n_pos * sizeof(uint32_t))) ||
+      (e = dalloc(c, m, m.nruns, static_cast<size_t>(h.n_n_runs) * sizeof(uint2))))
     return e;
   std::vector<uint64_t> coff(static_cast<size_t>(h.n_contigs));
   std::vector<uint32_t> clen(static_cast<size_t>(h.n_contigs));
@@ -1980,9 +2006,9 @@ int dnaln_gpu_index_upload(dnaln_ctx* c, const uint8_t* genome, uint64_t n_bases
   r.device = c->device;
   IndexMem& m = *r.mem;
   int e = DNALN_OK;
-  if ((e = dalloc(c, m.genome, n_bases)) || (e = dalloc(c, m.coff, n_contigs * sizeof(uint64_t))) ||
-      (e = dalloc(c, m.clen, n_contigs * sizeof(uint32_t))) || (e = dalloc(c, m.table, t.size() * sizeof(ulonglong2))) ||
-      (e = dalloc(c, m.positions, n_pos * sizeof(uint32_t))))
+  if ((e = dalloc(c, m, m.genome, n_bases)) || (e = dalloc(c, m, m.coff, n_contigs * sizeof(uint64_t))) ||
+      (e = dalloc(c, m, m.clen, n_contigs * sizeof(uint32_t))) || (e = dalloc(c, m, m.table, t.size() * sizeof(ulonglong2))) ||
+      (e = dalloc(c, m, m.positions, n_pos * sizeof(uint32_t))))
     return e;
   CK(cudaMemcpy(m.genome.p, genome, n_bases, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(m.coff.p, contig_off, n_contigs * sizeof(uint64_t), cudaMemcpyHostToDevice));
@@ -1994,6 +2020,7 @@ int dnaln_gpu_index_upload(dnaln_ctx* c, const uint8_t* genome, uint64_t n_bases
   char why[256] = {};
   e = find_n_runs_on_device(c->st, static_cast<const uint8_t*>(m.genome.p), n_bases, &runs, &n_runs, why, sizeof why);
   m.nruns = DevBuf{runs, static_cast<size_t>(n_runs) * sizeof(uint2)};
+  if (runs) m.own.push_back(runs);
   if (e != DNALN_OK) return fail(c, e, "%s", why);
   r.n_keys = tc.n_keys;
   r.n_pos = n_pos;
