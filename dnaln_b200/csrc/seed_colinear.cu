@@ -7,8 +7,11 @@
 // The check. A read's anchors split into the main ones and at most kMaxStray strays. The
 // main ones share a strand and are strictly monotone in both coordinates; each consecutive
 // pair is a valid predecessor (dr in (0, max_gap], |dr - dq| <= band) with a gain g =
-// min(dq, dr, k) - cost(|dr - dq|) >= 1. Every stray is on another strand than each other
-// anchor of the read or more than max_gap away from it, so it takes part in no pair. Let
+// min(dq, dr, k) - cost(|dr - dq|) >= 1. No stray makes a valid pair with a main anchor:
+// another strand, more than max_gap away, or more than band diagonals off (|dr - dq| is the
+// difference of the two anchors' diagonals rpos - qpos). A stray that sorts between main
+// anchors only takes a place of their lookback, so there are fewer strays than the lookback
+// is long. Let
 // G(j, i) be the gains summed from anchor j to anchor i. The DP's choice for i is i - 1 (it
 // scans from the nearest and replaces only for a strictly better score) if for every
 // earlier j in reach G(j, i) >= min(dq, dr, k) - cost of the pair (j, i):
@@ -20,9 +23,11 @@
 //    one change to the anchor after the next is at least k.
 // All of this is symmetric in the direction, so it can be checked in the order the
 // minimizers come, although a reverse-strand read's anchors sort the other way round. Then
-// f rises along the main anchors, they are the first chain extracted, with score k + the
-// gains, and each stray is a chain of one anchor with score k, which the filters drop (the
-// host checks min_anchors >= 2 or min_score > k). One chain gives one candidate
+// f rises along the main anchors and they are a chain with score k + the gains. The strays
+// chain among themselves at most: alone with score k, which the filters drop (the host checks
+// min_anchors >= 2 or min_score > k), or, where two k-mers in a row hit the same wrong place,
+// with k + at most the sum of every stray's best gain from a predecessor, which is checked to
+// stay below min_score. One chain gives one candidate
 // (src/mapper.cpp:40-62).
 //
 // Two kernels:
@@ -83,9 +88,9 @@ __device__ __forceinline__ int pair_gain(const ChainParamsDev& cp, const int32_t
 }
 
 // b's anchors after a's (both in minimizer order) into a. Returns false if the two do not
-// make one chain; an anchor left alone goes to *stray (strand << 31 | rpos; *strays += 1).
+// make one chain; an anchor left alone goes to *stray (strand << 31 | rpos, diagonal).
 __device__ __forceinline__ bool append(Run& a, const Run& b, const ChainParamsDev& cp, const int32_t* lut,
-                                       uint32_t* stray, int* strays) {
+                                       uint2* stray, int* strays) {
   if (b.m == 0) return true;
   bool change = false, ok = true;
   const int g = a.m > 0 && a.strand == b.strand
@@ -111,12 +116,12 @@ __device__ __forceinline__ bool append(Run& a, const Run& b, const ChainParamsDe
   }
   if (a.m > 1 && b.m > 1) return false;
   if (a.m > 1) {
-    *stray = b.strand << 31 | b.first_r;
+    *stray = make_uint2(b.strand << 31 | b.first_r, static_cast<uint32_t>(b.dmin));
     *strays += 1;
     return true;
   }
   if (a.m == 1) {  // a's only anchor becomes a stray and b's take over
-    *stray = a.strand << 31 | a.first_r;
+    *stray = make_uint2(a.strand << 31 | a.first_r, static_cast<uint32_t>(a.dmin));
     *strays += 1;
   }
   a = b;
@@ -283,7 +288,7 @@ __global__ void __launch_bounds__(kCThreads)
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int kWarps = kCThreads / 32;
   __shared__ int32_t lut[kMaxBandC + 1];
-  __shared__ uint32_t s_stray[kWarps][kMaxStray];
+  __shared__ uint2 s_stray[kWarps][kMaxStray];  // strand << 31 | rpos, diagonal
   __shared__ int32_t s_list[kWarps][32];  // reads for the full kernels, appended 32 at a time
   for (int d = threadIdx.x; d <= cp.band; d += kCThreads) lut[d] = cp.cost[d];
   __syncthreads();
@@ -291,7 +296,7 @@ __global__ void __launch_bounds__(kCThreads)
   const uint32_t lt = (1u << lane) - 1u;
   const uint32_t mask = static_cast<uint32_t>(ix.mask);
   const int k = sp.k;
-  uint32_t* const stray = s_stray[wid];
+  uint2* const stray = s_stray[wid];
   int32_t* const mine = s_list[wid];
   int listed = 0, long_reads = 0;
   const auto flush = [&]() {
@@ -367,12 +372,13 @@ __global__ void __launch_bounds__(kCThreads)
       na += __reduce_add_sync(FULL, c);
       unsigned in = __ballot_sync(FULL, c == 1);  // lanes with a main anchor
       // ---- keys with several occurrences: the one that pairs with the nearest lane of a
-      // single occurrence is the main one, the others are strays
+      // single occurrence on either side is the main one, the others are strays
       if (__any_sync(FULL, c > 1)) {
         const unsigned left = in & lt, right = in & ~lt;
-        const int ref = left ? 31 - __clz(left) : (right ? __ffs(right) - 1 : lane);
-        const int ref_pos = __shfl_sync(FULL, pos, ref);
-        const uint32_t ref_r = __shfl_sync(FULL, rpos, ref), ref_s = __shfl_sync(FULL, strand, ref);
+        const int lref = left ? 31 - __clz(left) : lane, rref = right ? __ffs(right) - 1 : lane;
+        const int l_pos = __shfl_sync(FULL, pos, lref), r_pos = __shfl_sync(FULL, pos, rref);
+        const uint32_t l_r = __shfl_sync(FULL, rpos, lref), l_s = __shfl_sync(FULL, strand, lref);
+        const uint32_t r_r = __shfl_sync(FULL, rpos, rref), r_s = __shfl_sync(FULL, strand, rref);
         const int most = static_cast<int>(__reduce_max_sync(FULL, c));
         bool found = false;
         uint32_t got_r = 0, got_s = 0;
@@ -381,9 +387,9 @@ __global__ void __launch_bounds__(kCThreads)
           const uint32_t vt = act ? (t ? __ldg(ix.positions + off + t) : v) : 0u;
           const uint32_t st = (vt ^ pw) & 1u, rt = vt >> 1;
           bool change, pairs = false;
-          if (act && !found && in && st == ref_s)
-            pairs = (left ? pair_gain(cp, lut, st, ref_pos, ref_r, pos, rt, change)
-                          : pair_gain(cp, lut, st, pos, rt, ref_pos, ref_r, change)) > 0;
+          if (act && !found && left && st == l_s) pairs = pair_gain(cp, lut, st, l_pos, l_r, pos, rt, change) > 0;
+          if (act && !found && !pairs && right && st == r_s)
+            pairs = pair_gain(cp, lut, st, pos, rt, r_pos, r_r, change) > 0;
           if (pairs) {
             found = true;
             got_r = rt;
@@ -391,7 +397,8 @@ __global__ void __launch_bounds__(kCThreads)
           }
           const unsigned alone = __ballot_sync(FULL, act && !pairs);
           const int x = ns + __popc(alone & lt);
-          if (act && !pairs && x < kMaxStray) stray[x] = st << 31 | rt;
+          if (act && !pairs && x < kMaxStray)
+            stray[x] = make_uint2(vt >> 1 | st << 31, rt - static_cast<uint32_t>(st ? len - pos - k : pos));
           ns += __popc(alone);
         }
         if (found) {
@@ -421,12 +428,17 @@ __global__ void __launch_bounds__(kCThreads)
       };
       link();
       if (__popc(linked) + 1 < __popc(in)) {
-        // anchors that pair with neither neighbour are strays, unless without the others they
-        // pair with a neighbour after all (a stray stood between); the rest must make one chain
+        // runs of one or two anchors (but the longest run) are strays, unless without the
+        // others they pair with a neighbour after all (a stray stood between); the rest must
+        // make one chain
+        const unsigned starts = in & ~linked;
+        const unsigned upto = starts & (lt | 1u << lane), later = starts & ~lt & ~(1u << lane);
+        const int s0 = upto ? 31 - __clz(upto) : 0;  // start of the run this lane's anchor is in
+        const unsigned span = (later ? (later & (0u - later)) - 1u : FULL) & ~((1u << s0) - 1u);
         const bool member = (in >> lane) & 1u;
-        const unsigned after = in & ~lt & ~(1u << lane);
-        const bool next = after && ((linked >> (__ffs(after) - 1)) & 1u);
-        unsigned alone = __ballot_sync(FULL, member && gain == 0 && !next);
+        const int size = member ? __popc(in & span) : 0;
+        const int longest = __reduce_max_sync(FULL, size ? size << 5 | (31 - s0) : 0);
+        unsigned alone = __ballot_sync(FULL, member && size <= 2 && (size << 5 | (31 - s0)) != longest);
         in &= ~alone;
         const unsigned left = in & lt, right = in & ~lt;
         const int ref = left ? 31 - __clz(left) : (right ? __ffs(right) - 1 : lane);
@@ -440,7 +452,8 @@ __global__ void __launch_bounds__(kCThreads)
         alone &= ~back;
         in |= back;
         const int x = ns + __popc(alone & lt);
-        if (((alone >> lane) & 1u) && x < kMaxStray) stray[x] = strand << 31 | rpos;
+        if (((alone >> lane) & 1u) && x < kMaxStray)
+          stray[x] = make_uint2(strand << 31 | rpos, rpos - static_cast<uint32_t>(strand ? len - pos - k : pos));
         ns += __popc(alone);
         link();
         if (ns > kMaxStray || __popc(linked) + 1 < __popc(in)) {
@@ -483,7 +496,7 @@ __global__ void __launch_bounds__(kCThreads)
       } else {
         b.dmin = b.dmax = __shfl_sync(FULL, diag, f);
       }
-      uint32_t one = 0;
+      uint2 one = make_uint2(0, 0);
       int ones = 0;
       if (!append(run, b, cp, lut, &one, &ones)) bad = true;
       if (ones) {
@@ -496,20 +509,28 @@ __global__ void __launch_bounds__(kCThreads)
       }
     }
     __syncwarp();
-    // strays: another strand than, or more than max_gap from, the main anchors and each other
+    // strays: no valid pair with a main anchor, no chain of their own that the filters keep
     const uint32_t r_lo = run.strand ? run.last_r : run.first_r, r_hi = run.strand ? run.first_r : run.last_r;
     if (!bad && ns) {
       const uint32_t gap = static_cast<uint32_t>(cp.max_gap);
-      bool near = false;
+      bool pairs = ns >= cp.lookback;
+      int best = 0;
       if (lane < ns) {
-        const uint32_t rx = stray[lane] & 0x7FFFFFFFu, sx = stray[lane] >> 31;
-        near = run.m > 0 && sx == run.strand && rx + gap >= r_lo && rx <= r_hi + gap;
+        const uint32_t rx = stray[lane].x & 0x7FFFFFFFu, sx = stray[lane].x >> 31;
+        const int dx = static_cast<int>(stray[lane].y);
+        if (run.m > 0 && sx == run.strand && rx + gap >= r_lo && rx <= r_hi + gap && dx >= run.dmin - cp.band &&
+            dx <= run.dmax + cp.band)
+          pairs = true;
         for (int y = 0; y < ns; ++y) {
-          const uint32_t ry = stray[y] & 0x7FFFFFFFu;
-          if (y != lane && sx == stray[y] >> 31 && (rx > ry ? rx - ry : ry - rx) <= gap) near = true;
+          const int dr = static_cast<int>(rx) - static_cast<int>(stray[y].x & 0x7FFFFFFFu);
+          const int shift = dx - static_cast<int>(stray[y].y), dq = dr - shift;
+          const int dd = shift < 0 ? -shift : shift;
+          if (sx == stray[y].x >> 31 && dr > 0 && dq > 0 && dr <= cp.max_gap && dd <= cp.band)
+            best = max(best, min(min(dr, dq), k) - lut[dd]);
         }
       }
-      bad = __any_sync(FULL, near);
+      const int own = __reduce_add_sync(FULL, best);
+      bad = __any_sync(FULL, pairs) || (own > 0 && k + own >= cp.min_score);
       __syncwarp();
     }
     if (bad) {
