@@ -629,9 +629,10 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   CK(cudaMemsetAsync(info, 0, 11 * sizeof(unsigned long long), st));
   CK(cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), st));
   CK(cudaMemsetAsync(c->d_count, 0, 4 * sizeof(int), st));
-  // [0] reads the colinear kernel listed, [1] work-stealing claims of the warp chaining kernel
-  DBUF(claims, int, "claims", 2);
-  CK(cudaMemsetAsync(claims, 0, 2 * sizeof(int), st));
+  // [0] reads the colinear kernels listed, [1] work-stealing claims of the warp chaining kernel,
+  // [2] reads it listed for their anchor count, [3] claims of those, [4] reads with an N
+  DBUF(claims, int, "claims", 5);
+  CK(cudaMemsetAsync(claims, 0, 5 * sizeof(int), st));
   unsigned long long* ctr = info + 1;  // cells, mapped, candidates (map.cuh)
   kt.begin(st, "k_len64");
   k_len64<<<nblk(n + 1), 256, 0, st>>>(d_seq_len, n, len64, info);
@@ -695,6 +696,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
     const int* full_n = nullptr;
     if (c->colinear && seed_colinear_supported(sp, cp, ix.dev)) {
       DBUF(rest, int32_t, "colinear_rest", n);
+      DBUF(with_n, int32_t, "colinear_with_n", n);
       const int32_t* order = nullptr;
       if (by_length && n > 1) {
         DBUF(ord, int32_t, "read_order", n);
@@ -708,7 +710,11 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       kt.end(st);
       kt.begin(st, "k_probe_reads");
       launch_probe_reads(st, pofs, d_seq_len, n, lanes, mb.hash, sk_counts, ix.dev, sp, cp, cand, cb, n_min, n_anchor,
-                         n_anc_t, rest, claims, seed_thread_max_len(), info + 10, c->d_err);
+                         n_anc_t, mb, rest, claims, with_n, claims + 4, seed_thread_max_len(), info + 10, c->d_err);
+      kt.end(st);
+      kt.begin(st, "k_seed<list>");
+      launch_seed_list(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, with_n, claims + 4, codes, ix.dev, sp,
+                       mb, n_min, n_anchor, c->d_err);
       kt.end(st);
       c->stats.launches += 2;
       full_list = rest;
@@ -762,17 +768,20 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       }
       kt.begin(st, "k_seed_chain_tl");
       if (!launch_seed_chain_long(st, d_seq_len, pofs, codes, order, big_n, lt, ix.dev, sp, cp, cand, cb, n_min,
-                                  n_anchor, n_anc_t, lscr, big2, c->d_count + 3, seed_thread_max_len(), c->d_err))
+                                  n_anchor, n_anc_t, lscr, big2, c->d_count + 3, seed_thread_max_len(),
+                                  full_list != nullptr, c->d_err))
         return fail(c, DNALN_ERR_CUDA, "long-read seeding kernel could not be configured");
       kt.end(st);
       warp_list = big2;
       warp_n = c->d_count + 3;
       c->stats.launches += 1;
     }
-    kt.begin(st, "k_seed<list>");
-    launch_seed_list(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, warp_list, warp_n, codes, ix.dev, sp,
-                     mb, n_min, n_anchor, c->d_err);
-    kt.end(st);
+    if (!full_list) {
+      kt.begin(st, "k_seed<list>");
+      launch_seed_list(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, warp_list, warp_n, codes, ix.dev, sp,
+                       mb, n_min, n_anchor, c->d_err);
+      kt.end(st);
+    }
   } else {
     kt.begin(st, "k_seed");
     launch_seed(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, codes, ix.dev, sp, mb, n_min, n_anchor,
@@ -822,11 +831,12 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       !as.ch_dmax || !as.ch_rpos)
     return DNALN_ERR_OOM;
   unsigned long long* pool_top = info + 8;
+  DBUF(chain_big, int32_t, "chain_big", n);
   CK(cudaEventRecord(c->ev[kEvChain0], st));
   kt.begin(st, thread_path ? "k_chain_map<list>" : "k_chain_map");
   launch_chain_map(st, pofs, d_seq_len, n, thread_path ? warp_list : nullptr, thread_path ? warp_n : nullptr, n_min,
                    n_anchor, mb, ix.dev, cp, cand, as, pool_top, pool_cap, cb, c->stealing ? claims + 1 : nullptr,
-                   c->d_err);
+                   chain_big, claims + 2, c->d_err);
   kt.end(st);
   CK(cudaEventRecord(c->ev[kEvChain1], st));
   CK(cudaGetLastError());

@@ -40,7 +40,8 @@ namespace {
 constexpr int kSeedWarps = 8;
 constexpr int kRing = 512;  // >= 32 + max w (255)
 constexpr int kChainWarps = 4;
-constexpr int kSmCap = 256;  // anchors per read held in shared memory
+constexpr int kSmCap = 256;    // anchors per read held in shared memory
+constexpr int kBigCap = 1024;  // the same in k_chain_big
 
 struct SketchSmem {
   uint64_t hash[kRing];
@@ -785,12 +786,13 @@ __device__ void chain_map_small(uint64_t key, int n, const ChainParamsDev& cp, c
   if (lane == 0) cb.n_cand[r] = nd;
 }
 
+template <int CAP>
 struct ChainSmem {
-  uint64_t keys[kSmCap];
-  uint64_t ord[kSmCap];
-  int32_t f[kSmCap];
-  int32_t prev[kSmCap];
-  uint8_t used[kSmCap];
+  uint64_t keys[CAP];
+  uint64_t ord[CAP];
+  int32_t f[CAP];
+  int32_t prev[CAP];
+  uint8_t used[CAP];
 };
 
 // Pass 1 of read r by one warp (codes of both strands unless `encode` is false, because
@@ -860,11 +862,14 @@ __global__ void __launch_bounds__(kSeedWarps * 32)
 // Scratch of a read with more than 32 anchors (chain records, and the anchors themselves
 // past kSmCap) is taken from a pool by one atomic add; a read the pool cannot hold sets
 // kErrChainPool, and the host maps the batch again with a pool of the size asked for.
+// With `big`, a read of more than CAP and at most kBigCap anchors is listed there instead.
+template <int CAP>
 __device__ void chain_read(int64_t r, const int64_t* __restrict__ pofs, const int32_t* __restrict__ seq_len,
                            const int32_t* __restrict__ n_min, const int64_t* __restrict__ n_anchor, const MinBuf& mb,
                            const DevIndex& ix, const ChainParamsDev& cp, const CandParams& cand,
                            const AnchorScratch& as, unsigned long long* __restrict__ pool_top, int64_t pool_cap,
-                           const CandBuf& cb, uint32_t* __restrict__ err, ChainSmem& smw) {
+                           const CandBuf& cb, int32_t* __restrict__ big, int* __restrict__ big_n,
+                           uint32_t* __restrict__ err, ChainSmem<CAP>& smw) {
   const int lane = threadIdx.x & 31;
   const int64_t na64 = n_anchor[r];
   if (na64 > 0x3FFFFFFF) {
@@ -875,6 +880,10 @@ __device__ void chain_read(int64_t r, const int64_t* __restrict__ pofs, const in
     return;
   }
   const int na = static_cast<int>(na64);
+  if (big && na > CAP && na <= kBigCap) {
+    if (lane == 0) big[atomicAdd(big_n, 1)] = static_cast<int32_t>(r);
+    return;
+  }
   int64_t a0 = 0;
   if (na > 32) {
     unsigned long long b = 0;
@@ -888,7 +897,7 @@ __device__ void chain_read(int64_t r, const int64_t* __restrict__ pofs, const in
       return;
     }
   }
-  const bool small = na <= kSmCap;
+  const bool small = na <= CAP;
   ChainArrays a;
   a.keys = small ? smw.keys : as.keys + a0;
   a.ord = small ? smw.ord : as.ord + a0;
@@ -1011,8 +1020,9 @@ __global__ void __launch_bounds__(kChainWarps * 32, 8)
                 const int32_t* __restrict__ list, const int* __restrict__ list_n, const int32_t* __restrict__ n_min,
                 const int64_t* __restrict__ n_anchor, MinBuf mb, DevIndex ix, ChainParamsDev cp, CandParams cand,
                 AnchorScratch as, unsigned long long* __restrict__ pool_top, int64_t pool_cap, CandBuf cb,
-                int* __restrict__ claim, uint32_t* __restrict__ err) {
-  __shared__ ChainSmem sm[kChainWarps];
+                int* __restrict__ claim, int32_t* __restrict__ big, int* __restrict__ big_n,
+                uint32_t* __restrict__ err) {
+  __shared__ ChainSmem<kSmCap> sm[kChainWarps];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t gw = static_cast<int64_t>(blockIdx.x) * kChainWarps + wib;
   const int64_t m = list ? static_cast<int64_t>(*list_n) : n;
@@ -1023,13 +1033,34 @@ __global__ void __launch_bounds__(kChainWarps * 32, 8)
       x = __shfl_sync(0xffffffffu, x, 0);
       if (x >= m) break;
       chain_read(list ? list[x] : x, pofs, seq_len, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb,
-                 err, sm[wib]);
+                 big, big_n, err, sm[wib]);
     }
     return;
   }
   for (int64_t x = gw; x < m; x += static_cast<int64_t>(gridDim.x) * kChainWarps)
-    chain_read(list ? list[x] : x, pofs, seq_len, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, err,
-               sm[wib]);
+    chain_read(list ? list[x] : x, pofs, seq_len, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, big,
+               big_n, err, sm[wib]);
+}
+
+// The reads k_chain_map listed for their anchor count, one warp and 25 KB of shared memory
+// each: in global memory a 900-anchor read's sort, DP and walk waited 650 us on dependent
+// round trips. big_n[1] hands the reads out.
+__global__ void __launch_bounds__(32)
+    k_chain_big(const int64_t* __restrict__ pofs, const int32_t* __restrict__ seq_len,
+                const int32_t* __restrict__ n_min, const int64_t* __restrict__ n_anchor, MinBuf mb, DevIndex ix,
+                ChainParamsDev cp, CandParams cand, AnchorScratch as, unsigned long long* __restrict__ pool_top,
+                int64_t pool_cap, CandBuf cb, const int32_t* __restrict__ big, int* __restrict__ big_n,
+                uint32_t* __restrict__ err) {
+  __shared__ ChainSmem<kBigCap> sm;
+  const int m = big_n[0];
+  for (;;) {
+    int x = 0;
+    if (threadIdx.x == 0) x = atomicAdd(big_n + 1, 1);
+    x = __shfl_sync(0xffffffffu, x, 0);
+    if (x >= m) break;
+    chain_read(big[x], pofs, seq_len, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, nullptr, nullptr,
+               err, sm);
+  }
 }
 
 __global__ void __launch_bounds__(kSeedWarps * 32)
@@ -1111,7 +1142,8 @@ void launch_seed_list(cudaStream_t st, const char* seq, const int64_t* seq_off, 
 void launch_chain_map(cudaStream_t st, const int64_t* pofs, const int32_t* seq_len, int64_t n, const int32_t* list,
                       const int* list_n, const int32_t* n_min, const int64_t* n_anchor, MinBuf mb,
                       const DevIndex& ix, const ChainParamsDev& cp, const CandParams& cand, AnchorScratch as,
-                      unsigned long long* pool_top, int64_t pool_cap, CandBuf cb, int* claim, uint32_t* err) {
+                      unsigned long long* pool_top, int64_t pool_cap, CandBuf cb, int* claim, int32_t* big, int* big_n,
+                      uint32_t* err) {
   if (n <= 0) return;
   // a count that may be known on the device only: with work stealing the resident blocks,
   // otherwise a grid-stride over a few resident waves
@@ -1130,7 +1162,10 @@ void launch_chain_map(cudaStream_t st, const int64_t* pofs, const int32_t* seq_l
   }
   const int64_t blocks = std::min<int64_t>((n + kChainWarps - 1) / kChainWarps, cap);
   k_chain_map<<<static_cast<unsigned>(blocks), kChainWarps * 32, 0, st>>>(
-      pofs, seq_len, n, list, list_n, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, claim, err);
+      pofs, seq_len, n, list, list_n, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, claim, big, big_n,
+      err);
+  k_chain_big<<<static_cast<unsigned>(std::min<int64_t>(n, int64_t{8} * device_sm_count())), 32, 0, st>>>(
+      pofs, seq_len, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, big, big_n, err);
 }
 
 void launch_sketch_codes(cudaStream_t st, const uint8_t* codes, const int64_t* seq_off, const int32_t* seq_len,

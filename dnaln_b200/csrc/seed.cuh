@@ -139,11 +139,14 @@ void launch_seed_list(cudaStream_t st, const char* seq, const int64_t* seq_off, 
 // the pool by an atomic add on *pool_top; past the capacity a read sets kErrChainPool.
 // With `claim` (an int zeroed by the caller) the grid is the resident warps only and each
 // warp takes its next read by an atomic add on *claim (work stealing); without, the warps
-// stride over the reads.
+// stride over the reads. big (n entries) and big_n (two ints zeroed by the caller: its count
+// and its claims) list reads of 257 to 1,024 anchors for a second kernel with as much shared
+// memory per warp.
 void launch_chain_map(cudaStream_t st, const int64_t* pofs, const int32_t* seq_len, int64_t n, const int32_t* list,
                       const int* list_n, const int32_t* n_min, const int64_t* n_anchor, MinBuf mb,
                       const DevIndex& ix, const ChainParamsDev& cp, const CandParams& cand, AnchorScratch as,
-                      unsigned long long* pool_top, int64_t pool_cap, CandBuf cb, int* claim, uint32_t* err);
+                      unsigned long long* pool_top, int64_t pool_cap, CandBuf cb, int* claim, int32_t* big, int* big_n,
+                      uint32_t* err);
 
 // Codes of both strands of reads [0, n) (seed_thread.cu): forward at codes[2*pofs[r]],
 // reverse complement right after it (src/mapper.cpp:88-99), from the ASCII reads.
@@ -160,8 +163,10 @@ void launch_encode_reads_bulk(cudaStream_t st, const char* seq, const int64_t* s
 // minimizers of every read, lanes (from seed_colinear_lanes) lanes each, in the order `order`
 // gives (may be null), to mins (total bases entries) and counts (n * lanes).
 // launch_probe_reads: candidates, n_min, n_anc_t and n_anchor = 0 of the reads found to have
-// one chain; the others are appended to list (*list_n = 0 before). *long_done += finished
-// reads longer than long_len.
+// one chain; the others are appended to list (*list_n = 0 before), with their minimizers in
+// mb, n_min and n_anchor as launch_seed_list leaves them, or, where an N kept them from being
+// sketched, to n_list as well (*n_list_n = 0 before; launch_seed_list is theirs). *long_done
+// += finished reads longer than long_len.
 bool seed_colinear_supported(const SeedParams& sp, const ChainParamsDev& cp, const DevIndex& ix);
 int seed_colinear_lanes(int64_t n, int64_t max_len);
 void launch_sketch_reads(cudaStream_t st, const uint8_t* codes, const int64_t* pofs, const int32_t* seq_len,
@@ -170,8 +175,8 @@ void launch_sketch_reads(cudaStream_t st, const uint8_t* codes, const int64_t* p
 void launch_probe_reads(cudaStream_t st, const int64_t* pofs, const int32_t* seq_len, int64_t n, int lanes,
                         const uint64_t* mins, const int32_t* counts, const DevIndex& ix, const SeedParams& sp,
                         const ChainParamsDev& cp, const CandParams& cand, CandBuf cb, int32_t* n_min,
-                        int64_t* n_anchor, int32_t* n_anc_t, int32_t* list, int* list_n, int long_len,
-                        unsigned long long* long_done, uint32_t* err);
+                        int64_t* n_anchor, int32_t* n_anc_t, MinBuf mb, int32_t* list, int* list_n,
+                        int32_t* n_list, int* n_list_n, int long_len, unsigned long long* long_done, uint32_t* err);
 // order = the reads of list[0, *list_n) (all n without a list; n at least the list's
 // length), longest first by length bin; bins: 2 * kLengthBins zeros.
 void launch_read_order(cudaStream_t st, const int32_t* seq_len, const int32_t* list, const int* list_n, int n,
@@ -183,7 +188,8 @@ void launch_read_order(cudaStream_t st, const int32_t* seq_len, const int32_t* l
 // the same stream before), writing
 // candidates of the admitted reads, n_min, n_anc_t (their anchor counts, for statistics)
 // and n_anchor = 0 (no scratch); the others are appended to big_list (count in *big_n,
-// zeroed by the caller) for launch_seed_list / launch_chain_map. reads_per_block: 64 or
+// zeroed by the caller) for launch_seed_list / launch_chain_map (with a list, their n_min and
+// n_anchor stay as they were). reads_per_block: 64 or
 // 128 (threads per block; same results). Returns false, launching nothing, when the
 // parameters are outside the path's range.
 bool seed_thread_supported(const SeedParams& sp, const ChainParamsDev& cp);
@@ -200,6 +206,7 @@ bool launch_seed_chain_thread(cudaStream_t st, const uint8_t* codes, const int64
 // min_len (typically those the short kernel listed) with their state in `scratch`
 // (seed_long_scratch_words(threads) words); the others, and reads past its bounds, go to
 // next_list (count *next_n) for the warp kernels.
+// keep_mins: leave n_min and n_anchor of the reads that go on as they are.
 // threads = seed_long_threads(upper bound of the list length).
 bool seed_long_supported(const SeedParams& sp, const ChainParamsDev& cp);
 int64_t seed_long_threads(int64_t n_max);
@@ -208,7 +215,7 @@ bool launch_seed_chain_long(cudaStream_t st, const int32_t* seq_len, const int64
                             const int32_t* list, const int* list_n, int64_t threads, const DevIndex& ix,
                             const SeedParams& sp, const ChainParamsDev& cp, const CandParams& cand, CandBuf cb,
                             int32_t* n_min, int64_t* n_anchor, int32_t* n_anc_t, uint32_t* scratch,
-                            int32_t* next_list, int* next_n, int min_len, uint32_t* err);
+                            int32_t* next_list, int* next_n, int min_len, bool keep_mins, uint32_t* err);
 // Stage entry points: sketch of code sequences, lookups, chaining of given anchor sets.
 void launch_sketch_codes(cudaStream_t st, const uint8_t* codes, const int64_t* seq_off, const int32_t* seq_len,
                          const uint32_t* pos_offset, int64_t n, int32_t k, int32_t w, uint64_t* out_hash,

@@ -282,9 +282,9 @@ __global__ void __launch_bounds__(kCThreads)
     k_probe_reads(const int64_t* __restrict__ pofs, const int32_t* __restrict__ seq_len, int64_t n,
                   const uint64_t* __restrict__ mins, const int32_t* __restrict__ counts, DevIndex ix, SeedParams sp,
                   ChainParamsDev cp, CandParams cand, CandBuf cb, int32_t* __restrict__ n_min,
-                  int64_t* __restrict__ n_anchor, int32_t* __restrict__ n_anc_t, int32_t* __restrict__ list,
-                  int* __restrict__ list_n, int long_len, unsigned long long* __restrict__ long_done,
-                  uint32_t* __restrict__ err) {
+                  int64_t* __restrict__ n_anchor, int32_t* __restrict__ n_anc_t, MinBuf mb, int32_t* __restrict__ list,
+                  int* __restrict__ list_n, int32_t* __restrict__ n_list, int* __restrict__ n_list_n, int long_len,
+                  unsigned long long* __restrict__ long_done, uint32_t* __restrict__ err) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int kWarps = kCThreads / 32;
   __shared__ int32_t lut[kMaxBandC + 1];
@@ -308,6 +308,30 @@ __global__ void __launch_bounds__(kCThreads)
     listed = 0;
     __syncwarp();
   };
+  // the bucket of minimizer m (src/index.hpp:24-38), two buckets a round
+  const auto probe = [&](uint64_t m, uint32_t& pw, uint32_t& off, uint32_t& c) {
+    const uint32_t h = static_cast<uint32_t>(m);
+    pw = static_cast<uint32_t>(m >> 32);
+    uint32_t slot = h & mask;
+    for (uint64_t round = 0;; ++round) {
+      const ulonglong2 b0 = __ldg(ix.table + slot), b1 = __ldg(ix.table + ((slot + 1) & mask));
+      // keys are below 2^30, an empty bucket's is ~0
+      const bool in0 = b0.x == h, end0 = static_cast<uint32_t>(b0.x >> 32) != 0;
+      const bool in1 = b1.x == h, end1 = static_cast<uint32_t>(b1.x >> 32) != 0;
+      if (in0 || end0 || in1 || end1) {
+        const uint64_t y = in0 ? b0.y : b1.y;
+        off = static_cast<uint32_t>(y);
+        c = in0 || (in1 && !end0) ? static_cast<uint32_t>(y >> 32) : 0u;
+        break;
+      }
+      slot = (slot + 2) & mask;
+      if (round > ix.mask) {  // the table is at most half full: an empty bucket ends every walk
+        atomicOr(err, kErrProbeLoop);
+        break;
+      }
+    }
+    if (c > sp.max_occ) c = 0;
+  };
   const int64_t warps = static_cast<int64_t>(gridDim.x) * kWarps;
   for (int64_t r = static_cast<int64_t>(blockIdx.x) * kWarps + wid; r < n; r += warps) {
     const int len = seq_len[r];
@@ -322,46 +346,24 @@ __global__ void __launch_bounds__(kCThreads)
       const int c = lane < G ? counts[r * G + lane] : 0;
       bad = __any_sync(FULL, c < 0);
       start = warp_exclusive_scan(c, &total);
+      if (bad) total = -1;
     }
     const int seg = G > 1 ? stretch_windows<W, G>(len, k) : 0;
+    const auto place = [&](int j) {  // of the read's minimizer j
+      if constexpr (G == 1) return base + j;
+      int s = 0;  // the last stretch that starts at or before j
+#pragma unroll
+      for (int step = G / 2; step > 0; step >>= 1)
+        if (__shfl_sync(FULL, start, s + step) <= j) s += step;
+      return base + static_cast<int64_t>(s) * seg + (j - __shfl_sync(FULL, start, s));
+    };
     Run run;
     int na = 0, ns = 0;
     for (int j0 = 0; j0 < total && !bad; j0 += 32) {
       const int j = j0 + lane;
-      int64_t at = base + j;
-      if constexpr (G > 1) {
-        int s = 0;  // the last stretch that starts at or before j
-#pragma unroll
-        for (int step = G / 2; step > 0; step >>= 1)
-          if (__shfl_sync(FULL, start, s + step) <= j) s += step;
-        at = base + static_cast<int64_t>(s) * seg + (j - __shfl_sync(FULL, start, s));
-      }
-      // ---- probe
+      const int64_t at = place(j);
       uint32_t pw = 0, off = 0, c = 0;
-      if (j < total) {
-        const uint64_t m = __ldg(mins + at);
-        const uint32_t h = static_cast<uint32_t>(m);
-        pw = static_cast<uint32_t>(m >> 32);
-        uint32_t slot = h & mask;
-        for (uint64_t round = 0;; ++round) {
-          const ulonglong2 b0 = __ldg(ix.table + slot), b1 = __ldg(ix.table + ((slot + 1) & mask));
-          // keys are below 2^30, an empty bucket's is ~0
-          const bool in0 = b0.x == h, end0 = static_cast<uint32_t>(b0.x >> 32) != 0;
-          const bool in1 = b1.x == h, end1 = static_cast<uint32_t>(b1.x >> 32) != 0;
-          if (in0 || end0 || in1 || end1) {
-            const uint64_t y = in0 ? b0.y : b1.y;
-            off = static_cast<uint32_t>(y);
-            c = in0 || (in1 && !end0) ? static_cast<uint32_t>(y >> 32) : 0u;
-            break;
-          }
-          slot = (slot + 2) & mask;
-          if (round > ix.mask) {  // the table is at most half full: an empty bucket ends every walk
-            atomicOr(err, kErrProbeLoop);
-            break;
-          }
-        }
-        if (c > sp.max_occ) c = 0;
-      }
+      if (j < total) probe(__ldg(mins + at), pw, off, c);
       if (__any_sync(FULL, c > kMaxHits)) {
         bad = true;
         break;
@@ -534,11 +536,27 @@ __global__ void __launch_bounds__(kCThreads)
       __syncwarp();
     }
     if (bad) {
+      // its minimizers and their buckets for the warp kernels (an N read's are still to be made)
+      int64_t anchors = 0;
+      const bool sketched = total >= 0;
+      for (int j0 = 0; j0 < total && sketched; j0 += 32) {
+        const int j = j0 + lane;
+        const int64_t at = place(j);
+        uint32_t pw = 0, off = 0, c = 0;
+        if (j < total) {
+          probe(__ldg(mins + at), pw, off, c);
+          mb.pos[base + j] = pw >> 1 | pw << 31;
+          mb.hit_off[base + j] = off;
+          mb.hit_cnt[base + j] = c;
+        }
+        anchors += __reduce_add_sync(FULL, c);
+      }
       if (lane == 0) {
         mine[listed] = static_cast<int32_t>(r);
-        n_min[r] = 0;
+        if (!sketched) n_list[atomicAdd(n_list_n, 1)] = static_cast<int32_t>(r);
+        n_min[r] = sketched ? total : 0;
+        n_anchor[r] = anchors;
         n_anc_t[r] = 0;
-        n_anchor[r] = 0;
       }
       if (++listed == 32) flush();
       continue;
@@ -629,13 +647,13 @@ void launch_sketch_reads(cudaStream_t st, const uint8_t* codes, const int64_t* p
 void launch_probe_reads(cudaStream_t st, const int64_t* pofs, const int32_t* seq_len, int64_t n, int lanes,
                         const uint64_t* mins, const int32_t* counts, const DevIndex& ix, const SeedParams& sp,
                         const ChainParamsDev& cp, const CandParams& cand, CandBuf cb, int32_t* n_min,
-                        int64_t* n_anchor, int32_t* n_anc_t, int32_t* list, int* list_n, int long_len,
-                        unsigned long long* long_done, uint32_t* err) {
+                        int64_t* n_anchor, int32_t* n_anc_t, MinBuf mb, int32_t* list, int* list_n,
+                        int32_t* n_list, int* n_list_n, int long_len, unsigned long long* long_done, uint32_t* err) {
   const unsigned blocks = static_cast<unsigned>(
       std::min<int64_t>((n + kCThreads / 32 - 1) / (kCThreads / 32), int64_t{32} * device_sm_count()));
   const auto run = [&](auto kernel) {
     kernel<<<blocks, kCThreads, 0, st>>>(pofs, seq_len, n, mins, counts, ix, sp, cp, cand, cb, n_min, n_anchor, n_anc_t,
-                                         list, list_n, long_len, long_done, err);
+                                         mb, list, list_n, n_list, n_list_n, long_len, long_done, err);
   };
   switch (lanes) {
     case 4: return run(k_probe_reads<kCW, 4>);

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kLT, 6)
                     DevIndex ix, SeedParams sp, ChainParamsDev cp, CandParams cand, CandBuf cb,
                     int32_t* __restrict__ n_min, int64_t* __restrict__ n_anchor, int32_t* __restrict__ n_anc_t,
                     uint32_t* __restrict__ scratch, int32_t* __restrict__ next_list, int* __restrict__ next_n,
-                    int min_len, uint32_t* __restrict__ err) {
+                    int min_len, bool keep_mins, uint32_t* __restrict__ err) {
   __shared__ int32_t lut[kLMaxBand + 1];
   for (int d = threadIdx.x; d <= cp.band; d += kLT) lut[d] = cp.cost[d];
   __syncthreads();
@@ -451,13 +451,12 @@ __global__ void __launch_bounds__(kLT, 6)
         }
       }
     }
-    n_anchor[r] = 0;
     if (big) {
-      n_min[r] = 0;
-      n_anc_t[r] = 0;
+      if (!keep_mins) n_min[r] = n_anc_t[r] = n_anchor[r] = 0;
       next_list[atomicAdd(next_n, 1)] = static_cast<int32_t>(r);
       continue;
     }
+    n_anchor[r] = 0;
     n_min[r] = nmin;
     n_anc_t[r] = na;
     cb.n_cand[r] = nd;
@@ -483,12 +482,12 @@ bool launch_seed_chain_long(cudaStream_t st, const int32_t* seq_len, const int64
                             const int32_t* list, const int* list_n, int64_t threads, const DevIndex& ix,
                             const SeedParams& sp, const ChainParamsDev& cp, const CandParams& cand, CandBuf cb,
                             int32_t* n_min, int64_t* n_anchor, int32_t* n_anc_t, uint32_t* scratch,
-                            int32_t* next_list, int* next_n, int min_len, uint32_t* err) {
+                            int32_t* next_list, int* next_n, int min_len, bool keep_mins, uint32_t* err) {
   if (!seed_long_supported(sp, cp)) return false;
   if (threads <= 0) return true;
   const unsigned blocks = static_cast<unsigned>(threads / kLT);
   k_seed_chain_tl<10><<<blocks, kLT, 0, st>>>(seq_len, pofs, codes, list, list_n, ix, sp, cp, cand, cb, n_min,
-                                              n_anchor, n_anc_t, scratch, next_list, next_n, min_len, err);
+                                              n_anchor, n_anc_t, scratch, next_list, next_n, min_len, keep_mins, err);
   return true;
 }
 

@@ -134,11 +134,7 @@ __global__ void __launch_bounds__(TT)
   if (list_n && n <= kTFew) {
     const int64_t x = static_cast<int64_t>(blockIdx.x) * TT + T;
     if (x < n) {
-      const int32_t r = list[x];
-      n_min[r] = 0;
-      n_anc_t[r] = 0;
-      n_anchor[r] = 0;
-      big_list[x] = r;
+      big_list[x] = list[x];
       if (x == 0) *big_n = static_cast<int>(n);
     }
     return;
@@ -489,13 +485,12 @@ __global__ void __launch_bounds__(TT)
       }
     }
   }
-  n_anchor[r] = 0;  // no anchor scratch: this read either finished here or is listed below
   if (big) {
-    n_min[r] = 0;
-    n_anc_t[r] = 0;
+    if (!list) n_min[r] = n_anc_t[r] = n_anchor[r] = 0;
     big_list[atomicAdd(big_n, 1)] = static_cast<int32_t>(r);
     return;
   }
+  n_anchor[r] = 0;  // no anchor scratch
   n_min[r] = nmin;
   n_anc_t[r] = na;
   cb.n_cand[r] = nd;
