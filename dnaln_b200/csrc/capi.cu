@@ -486,7 +486,7 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
     band = dbuf<int>(c, "sw_band", static_cast<size_t>(chunk) * band_t / sizeof(int));
     if (!band) return DNALN_ERR_OOM;
   }
-  int* fb = dbuf<int>(c, "sw_fb", static_cast<size_t>(chunk) + 1);
+  int* fb = dbuf<int>(c, "sw_fb", static_cast<size_t>(chunk) + kSwFbHead);
   if (!fb) return DNALN_ERR_OOM;
   const KernelTrace kt = tracer(c);
   // the kernel form: fixed by the option, or tuned once per (W, traceback, length bucket)

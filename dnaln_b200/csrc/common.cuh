@@ -119,6 +119,7 @@ struct SwResult {
 struct SwParams {
   int32_t match, mismatch, oe, ge, ambig, bw, W;
   uint32_t prof_n;  // 4 bytes of -ambig (table entries 4..7 of the byte-permute profile)
+  uint32_t one, mone;  // 1 and -1: additions as multiply-adds that are not folded (sw.cu)
 };
 
 // Optional per-kernel timing hook of the orchestrator: begin() before a launch and end()

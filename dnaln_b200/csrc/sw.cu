@@ -30,11 +30,13 @@
 //  * k_sw_any: any band width and any scores (int32, band rows in per-warp scratch).
 //
 // Direction code of a cell (4 bits):
-//   bit 3: hd < E            bit 2: max(hd, E) < F
-//   bit 1: E extends E(i-1,d+1) (ee > eo)    bit 0: F extends F(i,d-1) (fe > fo)
-// On every cell the walk reads, H is the positive value being traced; there "H from the
-// diagonal" (h == hd, src/align.cpp:67) is bits 3,2 = 0,0, "H from E" with no diagonal
-// (h == e) is 1,0, and otherwise H came from F — so the walk (src/align.cpp:87-143)
+//   kNotDiag: H > hd                           kNotE: H > E
+//   kExtE: E extends E(i-1,d+1) (ee > eo)      kExtF: F extends F(i,d-1) (fe > fo)
+// The codes of four neighbouring cells share 16 bits, cell c's at bits c (kNotDiag), 4 + c
+// (kExtE), 8 + c (kNotE) and 12 + c (kExtF): the order in which cell2 gets them.
+// On every cell the walk reads, H is the positive value being traced; there it came from the
+// diagonal if h == hd (src/align.cpp:67), else from E if h == e, and otherwise from F — so
+// the walk (src/align.cpp:87-143)
 // takes the reference's steps. The best cell is the first strict maximum in row-major
 // order (per-row maximum with its first column, then strict across rows).
 #include <algorithm>
@@ -49,8 +51,16 @@ namespace dnb {
 namespace {
 
 constexpr int kSwThreads = 128;
-constexpr uint32_t kNotDiagE = 8u, kFromF = 4u, kExtE = 2u, kExtF = 1u;
-constexpr uint32_t kBias = 16384u, kBias2 = 0x40004000u, kOne2 = 0x00010001u;
+// k_sw_u2 and k_sw_wide: blocks of one warp, as many as are resident, which take 32 / LANES
+// pairs at a time: first those of their block index, then the next by an atomic add until
+// none is left. The list is ordered longest first and often counted on the device only.
+// Against a grid over the longest possible list, with blocks of four warps: blocks go to the
+// GPCs in turn, so the SMs of a small GPC held 16 warps where the others held 8 to 12 and set
+// the kernel's time, and an empty list of 262,144 cost 15 us. (Claiming the first pairs too
+// lets the SMs that start first take whole lists: 219 -> 303 us for 58,000 tasks.)
+constexpr int kDpThreads = 32;
+constexpr uint32_t kNotDiag = 1u, kExtE = 0x10u, kNotE = 0x100u, kExtF = 0x1000u, kCode = 0x1111u;
+constexpr uint32_t kBias = 16384u, kBias2 = 0x40004000u;
 constexpr int kScoreBias = 64;  // profile bytes are score + 64, in [0, 127]
 constexpr int kAhead = 8;       // cells of a diagonal run the walk fetches at once
 
@@ -102,8 +112,8 @@ __device__ __forceinline__ uint32_t prof_biased(const SwParams& p, uint32_t qc) 
 
 __device__ __forceinline__ uint32_t pack2(uint32_t v) { return (v & 0xFFFFu) * 0x10001u; }
 
-__device__ __forceinline__ uint32_t dir_code32(bool hd_ge_e, bool m1_ge_f, bool e_not_ext, bool f_not_ext) {
-  return (hd_ge_e ? 0u : kNotDiagE) | (m1_ge_f ? 0u : kFromF) | (e_not_ext ? 0u : kExtE) | (f_not_ext ? 0u : kExtF);
+__device__ __forceinline__ uint32_t dir_code32(bool diag, bool from_e, bool e_not_ext, bool f_not_ext) {
+  return (diag ? 0u : kNotDiag) | (from_e ? 0u : kNotE) | (e_not_ext ? 0u : kExtE) | (f_not_ext ? 0u : kExtF);
 }
 
 // Global store with an L2 evict-first policy: streaming data (the direction codes, read
@@ -115,6 +125,52 @@ __device__ __forceinline__ uint64_t l2_evict_first_policy() {
 }
 __device__ __forceinline__ void st_evict_first(uint32_t* p, uint32_t v, uint64_t pol) {
   asm volatile("st.global.L2::cache_hint.b32 [%0], %1, %2;" ::"l"(p), "r"(v), "l"(pol) : "memory");
+}
+
+// One cell of two alignments in biased 16-bit halves. H is kept as H - (O+E), which is what
+// both neighbours open a gap from: E and F are one DPX add-max each (max(a + b, c), signed
+// 16x2: the biased values lie in [0, 32767], where signed and unsigned order agree).
+//
+// Adds, maxima, prmt and logic run on the ALU pipe at one instruction every two cycles, and
+// integer multiply-adds beside it at the same rate, so the cell's plain additions are written
+// as multiply-adds by 1 or -1 that the compiler cannot fold: about ten instructions each.
+struct CellParams {
+  uint32_t oe, nge, khd;  // O+E; -E in each signed half; O+E - profile bias
+  uint32_t one, mone;     // 1 and -1, as values known at run time only
+};
+__device__ __forceinline__ CellParams cell_params(const SwParams& p) {
+  return {pack2(p.oe), pack2(static_cast<uint32_t>(-p.ge)), pack2(p.oe) - pack2(kScoreBias), p.one, p.mone};
+}
+__device__ __forceinline__ uint32_t mad(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t r;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+  return r;
+}
+// hdiag, hup, hleft, the result: H - (O+E); s: profile value; f: F of the left cell, then of
+// this one. TB: code holds the direction code in the bits of every cell of the word, for
+// insert_code. A flag is x > y for some x >= y, both below 2^14 + 16000, so x - y + 0x7FFF
+// carries it in the sign bit of its half, with no borrow or carry between the halves; two
+// prmt spread the four sign bits over bytes and a select merges them.
+template <bool TB>
+__device__ __forceinline__ uint32_t cell2(const CellParams& c, uint32_t hdiag, uint32_t s, uint32_t hup, uint32_t eup,
+                                          uint32_t hleft, uint32_t& f, uint32_t& e, uint32_t& code) {
+  const uint32_t hd = mad(mad(hdiag, c.one, c.khd), c.one, s);
+  e = __viaddmax_s16x2(eup, c.nge, hup);
+  f = __viaddmax_s16x2(f, c.nge, hleft);
+  const uint32_t h = __vimax3_u16x2(__vmaxu2(hd, e), f, kBias2);
+  if constexpr (TB) {
+    constexpr uint32_t k = 0x7FFF7FFFu;
+    const uint32_t hk = mad(h, c.one, k);
+    const uint32_t de = prmt(mad(hd, c.mone, hk), mad(e, c.mone, hk), 0xFBD9u);  // bytes: A kNotDiag, A kNotE, B, B
+    const uint32_t ex = prmt(mad(e, c.one, mad(hup, c.mone, k)), mad(f, c.one, mad(hleft, c.mone, k)), 0xFBD9u);
+    code = (de & 0x0F0F0F0Fu) | (ex & 0xF0F0F0F0u);
+  }
+  return mad(c.oe, c.mone, h);
+}
+// Cell c (0..3) of its word; c = 0 starts the word.
+__device__ __forceinline__ uint32_t insert_code(uint32_t dw, uint32_t code, int c) {
+  const uint32_t m = 0x11111111u << c;
+  return c == 0 ? code : (dw & ~m) | (code & m);
 }
 
 struct CigarWriter {
@@ -141,24 +197,23 @@ struct CigarWriter {
 };
 
 // Direction codes of the pair layout: word (i, g), g < WQ = ceil(W/4), holds cells 4g..4g+3
-// of both alignments of a thread (A in the low 16 bits, B in the high 16), cell 4g+c at
-// bits 4*(3-c) of its half; the 32 pairs of a warp are interleaved word by word.
+// of both alignments of a thread (A in the low 16 bits, B in the high 16); the 32 pairs of a warp are interleaved word by word.
 struct PairCodes {
   const uint32_t* D;  // this pair's first word
   int WQ, half;
   __device__ uint32_t word(int i, int d) const { return D[(static_cast<size_t>(i) * WQ + (d >> 2)) * 32]; }
-  __device__ int shift(int d) const { return 16 * half + 4 * (3 - (d & 3)); }
-  __device__ uint32_t operator()(int i, int d) const { return (word(i, d) >> shift(d)) & 0xFu; }
+  __device__ int shift(int d) const { return 16 * half + (d & 3); }
+  __device__ uint32_t operator()(int i, int d) const { return (word(i, d) >> shift(d)) & kCode; }
 };
 
 // Direction codes of the generic kernel: word (i, w), w < WW = ceil(W/8), holds cells
-// 8w..8w+7, cell 8w+c at bits 4c; 32 alignments of a warp interleaved word by word.
-struct NibbleCodes {
+// 8w..8w+7, the first four in the low half; 32 alignments of a warp interleaved word by word.
+struct WordCodes {
   const uint32_t* D;
   int WW;
   __device__ uint32_t word(int i, int d) const { return D[(static_cast<size_t>(i) * WW + (d >> 3)) * 32]; }
-  __device__ int shift(int d) const { return 4 * (d & 7); }
-  __device__ uint32_t operator()(int i, int d) const { return (word(i, d) >> shift(d)) & 0xFu; }
+  __device__ int shift(int d) const { return 4 * (d & 4) + (d & 3); }
+  __device__ uint32_t operator()(int i, int d) const { return (word(i, d) >> shift(d)) & kCode; }
 };
 
 // High bit of each byte of x set where that byte is zero, every other bit clear.
@@ -225,7 +280,7 @@ __device__ void traceback(const Codes& code, int W, int bi, int bd, int best, co
         // step lowers v by at most smax), is taken whole: its score and mismatches from the
         // two byte words (bytes equal and both below 4: match; either above 3: ambiguous;
         // else mismatch), exactly the sums of the steps below.
-        if (((any >> sh) & (kNotDiagE | kFromF)) == 0 && v > (kAhead - 1) * smax) {
+        if (((any >> sh) & kNotDiag) == 0 && v > (kAhead - 1) * smax) {
           const uint64_t amb = (qw | tw) & 0xFCFCFCFCFCFCFCFCull;
           const uint64_t ok_amb = zero_bytes(amb);
           const int n_match = __popcll(zero_bytes(qw ^ tw) & ok_amb);
@@ -238,7 +293,7 @@ __device__ void traceback(const Codes& code, int W, int bi, int bd, int best, co
         }
 #pragma unroll
         for (int k = 0; k < kAhead; ++k) {
-          cx[k] = (wk[k] >> sh) & 0xFu;
+          cx[k] = (wk[k] >> sh) & kCode;
           qa[k] = static_cast<int>((qw >> (8 * (kAhead - 1 - k))) & 0xFFu);
           const int t8 = static_cast<int>((tw >> (8 * (kAhead - 1 - k))) & 0xFFu);
           ta[k] = t8 > 3 ? 4 : t8;
@@ -262,7 +317,7 @@ __device__ void traceback(const Codes& code, int W, int bi, int bd, int best, co
           break;
         }
         x = cx[k];
-        if (x & (kNotDiagE | kFromF)) {  // not from the diagonal
+        if (x & kNotDiag) {  // not from the diagonal
           stop = true;
           break;
         }
@@ -276,7 +331,7 @@ __device__ void traceback(const Codes& code, int W, int bi, int bd, int best, co
     if (i < 0 || v <= 0) break;
     run = 0;
     bool ext;
-    if (!(x & kFromF)) {  // from E, an insertion: E(i,d) <- (i-1, d+1)
+    if (!(x & kNotE)) {  // from E, an insertion: E(i,d) <- (i-1, d+1)
       do {
         if (i < 0 || d >= W) {
           atomicOr(err, kErrTracebackBounds);
@@ -326,6 +381,17 @@ __device__ __forceinline__ int row_buffer(bool up_a, bool up_b, int buf_a, int b
   return buf_a == buf_b ? 1 - buf_a : buf_b;
 }
 
+// The fallback list of a launch: fb[0] its length, fb[1] and fb[2] the warps' claims of the short
+// lists' form and of the main one, then local task indices.
+constexpr int kFbList = kSwFbHead;
+
+// The warp's next claim after its first, blockIdx.x, in every lane.
+__device__ __forceinline__ int next_claim(int* claim) {
+  int w = 0;
+  if ((threadIdx.x & 31) == 0) w = static_cast<int>(gridDim.x) + atomicAdd(claim, 1);
+  return __shfl_sync(0xffffffffu, w, 0);
+}
+
 // The DP kernels leave, for the walk, the best cell in the result: qb = its row, qe = its
 // column (the walk kernel then writes the final coordinates).
 __device__ __forceinline__ SwResult stash(int score, int bi, int bd) { return SwResult{score, bi, bd, 0, 0, 0, 0, 0}; }
@@ -372,9 +438,8 @@ __device__ SwResult sw_one_reg(const SwTask& tk, const uint8_t* __restrict__ qba
       H[d] = h;
       E[d] = e;
       if constexpr (TB) {
-        dw = dw * 16u + dir_code32(hd >= e, m1 >= f, eo >= ee, fo >= fe);
+        dw |= dir_code32(h == hd, h == e, eo >= ee, fo >= fe) << (d & 3);
         if ((d & 3) == 3 || d == W - 1) {
-          if ((d & 3) != 3) dw <<= 4 * (3 - (d & 3));
           reinterpret_cast<uint16_t*>(DP + (static_cast<size_t>(i) * WQ + (d >> 2)) * 32)[half] =
               static_cast<uint16_t>(dw);
           dw = 0;
@@ -413,16 +478,10 @@ __device__ bool window_has_n(const SwTask& tk, int W, const uint8_t* __restrict_
   return any;
 }
 
-// Two alignments per thread in biased 16-bit halves (A low, B high). Pairs it cannot take
-// (an N in a target window, or scores/lengths outside the 16-bit range) are listed in fb
-// (fb[0] = count, then local task indices) for k_sw_fb. With traceback at W <= 33 the
-// launch bound asks for three resident blocks (<= 170 registers, no spills): 12 warps per
-// SM instead of 8. Per cell:
-//  * E and F by the DPX add-max (max(a + b, c) in one instruction, signed 16x2: the biased
-//    values lie in [0, 32767], where signed and unsigned order agree), so the open-gap
-//    candidates hup - (O+E) and hleft - (O+E) are never materialised; the extension bits
-//    come from e - hup + (O+E) and f - hleft + (O+E), one 3-input add each (both halves
-//    non-negative, so no borrow crosses them);
+// Two alignments per thread in biased 16-bit halves (A low, B high), a cell at a time by
+// cell2. Pairs it cannot take (an N in a target window, or scores/lengths outside the 16-bit
+// range) are listed in fb for k_sw_fb. With traceback at W <= 33 the launch bound asks for
+// twelve resident warps (<= 170 registers, no spills).
 //  * the substitution scores of both alignments are one prmt.b32 on the row's profile
 //    words, taken from a 5-entry table in shared memory one row ahead;
 //  * target codes are read without range or N checks: the pair reaches the DP only when
@@ -430,23 +489,21 @@ __device__ bool window_has_n(const SwTask& tk, int W, const uint8_t* __restrict_
 //    window are clamped to its last base (a row past a query's end is an N row for it,
 //    whose scores do not depend on the target), so a code is always 0..3 and the prmt
 //    selector of two codes is two multiply-adds.
-// Against the former form (vmax of materialised open/extend candidates, profile words
-// rebuilt per row, range-checked target reads) this took the traceback kernel from 3.06 to
-// 2.56 ms per 1,000,000 x 150 bp reads.
 template <int W, bool TB>
-__global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
-    k_sw_u2(const SwTask* __restrict__ tasks, int base, int n, const int* __restrict__ n_dev, int few,
+__global__ void __launch_bounds__(kDpThreads, (TB && W <= 33) ? 12 : 1)
+    k_sw_u2(const SwTask* __restrict__ tasks, int base, int count, int n, const int* __restrict__ n_dev, int few,
              const uint8_t* __restrict__ qbase, const uint8_t* __restrict__ tbase, SwParams p,
-             SwResult* __restrict__ res, uint32_t* __restrict__ dir, int rows_max, int* __restrict__ fb) {
+             SwResult* __restrict__ res, uint32_t* __restrict__ dir, int rows_max, int* __restrict__ fb,
+             int* __restrict__ claim) {
   static_assert(W >= 3, "a window of at least two columns past an empty query");
   constexpr int WQ = (W + 3) / 4;
   __shared__ uint32_t s_prof[8];
   if (threadIdx.x < 5) s_prof[threadIdx.x] = prof_biased(p, threadIdx.x);
   __syncthreads();
-  const int lt = blockIdx.x * blockDim.x + threadIdx.x;  // pair index within this launch
-  const int nn = n_dev ? min(n, *n_dev) : n;
+  if (n_dev && *n_dev <= few) return;  // a short list is the narrowest form's
+  const int nn = n_dev ? min(n, *n_dev) : n, pairs = (min(nn - base, count) + 1) / 2;
+  const auto align = [&](const int lt) {  // lt: pair index within this launch
   const int ia = base + 2 * lt, ib = ia + 1;
-  if (ia >= nn || (n_dev && *n_dev <= few)) return;  // a short list is the narrowest form's
   const bool has_b = ib < nn;
   uint32_t* DP = TB ? pair_base(dir, 2 * lt, rows_max, WQ) : nullptr;
   const SwTask ta = tasks[ia];
@@ -458,8 +515,8 @@ __global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
                     p.match + kScoreBias <= 127 && p.mismatch <= kScoreBias && p.ambig <= kScoreBias;
   if (!fits || window_has_n(ta, W, tbase) || (has_b && window_has_n(tb, W, tbase))) {
     const int k = atomicAdd(fb, has_b ? 2 : 1);
-    fb[1 + k] = 2 * lt;
-    if (has_b) fb[2 + k] = 2 * lt + 1;
+    fb[kFbList + k] = 2 * lt;
+    if (has_b) fb[kFbList + 1 + k] = 2 * lt + 1;
     return;
   }
   const uint8_t* __restrict__ qa = qbase + ta.q_off;
@@ -477,22 +534,22 @@ __global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
   auto qcode = [&](const uint8_t* __restrict__ q, int ql, int i) {
     return i < ql ? min(static_cast<uint32_t>(q[i]), 4u) : 4u;
   };
+  const CellParams cp = cell_params(p);
+  const uint32_t h_zero = kBias2 - cp.oe;  // H = 0
   uint32_t H[W + 1], E[W + 1], T[W];
 #pragma unroll
   for (int d = 0; d <= W; ++d) {
-    H[d] = kBias2;
+    H[d] = h_zero;
     E[d] = kBias2;
   }
 #pragma unroll
   for (int d = 0; d < W; ++d) T[d] = tc2(d);
-  const uint32_t OE = pack2(p.oe), GE = pack2(p.ge), SB = pack2(kScoreBias);
-  const uint32_t NOE = pack2(static_cast<uint32_t>(-p.oe));  // -(O+E) in each signed half
-  uint32_t best2 = kBias2;
-  uint32_t best_a = kBias, best_b = kBias;
+  const uint32_t zero = kBias - static_cast<uint32_t>(p.oe);
+  uint32_t best2 = h_zero, best_a = zero, best_b = zero;
   int bi_a = -1, bi_b = -1;
   extern __shared__ uint32_t sw_rows[];
   uint32_t* const row_a = sw_rows + threadIdx.x;
-  uint32_t* const row_b = sw_rows + W * kSwThreads + threadIdx.x;
+  uint32_t* const row_b = sw_rows + W * kDpThreads + threadIdx.x;
   int buf_a = 0, buf_b = 1;
   uint32_t plo = s_prof[qcode(qa, qla, 0)], phi = s_prof[qcode(qb, qlb, 0)];
   uint32_t ca = qcode(qa, qla, 1), cb = qcode(qb, qlb, 1);  // codes of the next row
@@ -504,32 +561,22 @@ __global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
     const uint32_t t_next = tc2(i + W);
     const uint32_t plo_next = s_prof[ca], phi_next = s_prof[cb];
     const uint32_t ca_next = qcode(qa, qla, i + 2), cb_next = qcode(qb, qlb, i + 2);
-    uint32_t f = kBias2, hleft = kBias2, hdiag = H[0], rmax = 0, dw = 0;
+    uint32_t f = kBias2, hleft = h_zero, hdiag = H[0], rmax = 0, dw = 0;
 #pragma unroll
     for (int d = 0; d < W; ++d) {
-      const uint32_t hup = H[d + 1], eup = E[d + 1];
-      const uint32_t hd = hdiag + prmt(plo, phi, T[d]) - SB;
-      const uint32_t e = __viaddmax_s16x2(hup, NOE, eup - GE);
-      const uint32_t fn = __viaddmax_s16x2(hleft, NOE, f - GE);
-      const uint32_t m1 = __vmaxu2(hd, e);
-      const uint32_t h = __vimax3_u16x2(m1, fn, kBias2);
+      const uint32_t hup = H[d + 1];
+      uint32_t e, code = 0;
+      const uint32_t h = cell2<TB>(cp, hdiag, prmt(plo, phi, T[d]), hup, E[d + 1], hleft, f, e, code);
       if constexpr (TB) {
-        // each term is >= 0 per half; saturated to 0/1 it is one code bit
-        const uint32_t b3 = __vminu2(m1 - hd, kOne2), b2 = __vminu2(h - m1, kOne2);
-        const uint32_t b1 = __vminu2(e - hup + OE, kOne2), b0 = __vminu2(fn - hleft + OE, kOne2);
-        dw = dw * 16u + ((b3 * 2u + b2) * 4u + (b1 * 2u + b0));
-        if ((d & 3) == 3 || d == W - 1) {
-          if ((d & 3) != 3) dw <<= 4 * (3 - (d & 3));
-          st_evict_first(rowp + (d >> 2) * 32, dw, pol);
-          dw = 0;
-        }
-        rmax = d == 0 ? h : __vmaxu2(rmax, h);
-      } else {
-        best2 = __vmaxu2(best2, h);
+        dw = insert_code(dw, code, d & 3);
+        if ((d & 3) == 3 || d == W - 1) st_evict_first(rowp + (d >> 2) * 32, dw, pol);
       }
+      // the row's maximum (score only: the maximum so far), two cells at a time
+      uint32_t& top = TB ? rmax : best2;
+      if (d & 1) top = __vimax3_u16x2(top, hleft, h);
+      else if (d == W - 1) top = __vmaxu2(top, h);
       H[d] = h;
       E[d] = e;
-      f = fn;
       hleft = h;
       hdiag = hup;
     }
@@ -539,7 +586,7 @@ __global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
         const int dst = row_buffer(up_a, up_b, buf_a, buf_b);
         uint32_t* const row = dst ? row_b : row_a;
 #pragma unroll
-        for (int d = 0; d < W; ++d) row[d * kSwThreads] = H[d];
+        for (int d = 0; d < W; ++d) row[d * kDpThreads] = H[d];
         if (up_a) {
           best_a = rmax & 0xFFFFu;
           bi_a = i;
@@ -572,18 +619,24 @@ __global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
     const uint32_t* const rb = buf_b ? row_b : row_a;
 #pragma unroll 1
     for (int d = W - 1; d >= 0; --d) {
-      if (bi_a >= 0 && (ra[d * kSwThreads] & 0xFFFFu) == best_a) bd_a = d;
-      if (bi_b >= 0 && (rb[d * kSwThreads] >> 16) == best_b) bd_b = d;
+      if (bi_a >= 0 && (ra[d * kDpThreads] & 0xFFFFu) == best_a) bd_a = d;
+      if (bi_b >= 0 && (rb[d * kDpThreads] >> 16) == best_b) bd_b = d;
     }
   }
-  res[ta.slot] = stash(static_cast<int>(best_a) - static_cast<int>(kBias), TB ? bi_a : 0, bd_a);
-  if (has_b) res[tb.slot] = stash(static_cast<int>(best_b) - static_cast<int>(kBias), TB ? bi_b : 0, bd_b);
+  res[ta.slot] = stash(static_cast<int>(best_a - zero), TB ? bi_a : 0, bd_a);
+  if (has_b) res[tb.slot] = stash(static_cast<int>(best_b - zero), TB ? bi_b : 0, bd_b);
+  };
+  for (int w = blockIdx.x; w * 32 < pairs; w = next_claim(claim)) {
+    if (w * 32 + static_cast<int>(threadIdx.x) < pairs) align(w * 32 + threadIdx.x);
+    __syncwarp();
+  }
 }
 
 // Wide bands, W = CH * LANES + 1: LANES consecutive lanes of a warp share one pair of
 // alignments (A and B in the 16-bit halves, as in k_sw_u2), lane c holding band cells
-// [CH c, CH c + CH) of the row in registers (the last lane also cell W - 1); CH = 32, or 16
-// for twice the lanes per pair (fewer registers, more pairs in flight, a longer skew). Lane c works on
+// [CH c, CH c + CH) of the row in registers (the last lane also cell W - 1). Fewer cells a
+// lane: more warps and a shorter row, but its fixed work (shuffles, codes, the best row) is
+// paid for fewer cells, and the skew grows. Lane c works on
 // row t - c at step t, so its left neighbour finished the same row one step earlier: the
 // row's running F and H(left) arrive by one shuffle at the start of the step. The one value
 // a lane needs from its right neighbour — H and E of the previous row at the neighbour's
@@ -594,11 +647,21 @@ __global__ void __launch_bounds__(kSwThreads, (TB && W <= 33) ? 3 : 1)
 // lanes of a pair combine (value, then earliest row, then smallest column) at the end:
 // the first strict maximum of the whole band in row-major order. Pairs k_sw_u2 would
 // hand to the int32 kernel are listed in fb the same way.
+// With a row's codes taken by shuffles, additions spread over two pipes (cell2), the best rows
+// saved by 16-byte stores and warps that claim their pairs, against loads by every lane in
+// every row and a grid over the list, tracebacks: 58,000 tasks of 150 rows at W = 33 214 ->
+// 176 us (now 8 cells a lane, before 32), 150,000 of 50 to 1,000 rows 924 -> 678 (8, before
+// 16); 88,000 at W = 129 1,484 -> 1,200 (32); 4,001 of 1,000 to 5,000 rows at W = 65 1,732 ->
+// 1,218 (4). At 8 cells a lane ALU and multiply-add pipe are each busy about 60 % of the time.
+// Resident warps per SM (sw_wide_warps), same lists: 8 cells 16 / 20 / 24 warps 185 / 176 /
+// 190 us; 32 cells 12 / 10 / 8 warps 1,333 / 1,311 / 1,200; 4 cells 20 / 24 1,262 / 1,218.
+constexpr int sw_wide_warps(int cells) { return cells == 4 ? 24 : (cells == 8 ? 20 : (cells == 16 ? 12 : 8)); }
 template <int LANES, int CH, bool TB>
-__global__ void __launch_bounds__(kSwThreads, TB ? (CH <= 16 ? 4 : 3) : 1)
-    k_sw_wide(const SwTask* __restrict__ tasks, int base, int n, const int* __restrict__ n_dev, int above, int upto,
+__global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
+    k_sw_wide(const SwTask* __restrict__ tasks, int base, int count, int n, const int* __restrict__ n_dev, int above, int upto,
               const uint8_t* __restrict__ qbase, const uint8_t* __restrict__ tbase, SwParams p,
-              SwResult* __restrict__ res, uint32_t* __restrict__ dir, int rows_max, int* __restrict__ fb) {
+              SwResult* __restrict__ res, uint32_t* __restrict__ dir, int rows_max, int* __restrict__ fb,
+              int* __restrict__ claim) {
   static_assert(CH % 4 == 0, "a lane's cells fill whole direction words");
   constexpr int W = CH * LANES + 1, WQ = (W + 3) / 4;
   constexpr unsigned FULL = 0xffffffffu;
@@ -608,12 +671,10 @@ __global__ void __launch_bounds__(kSwThreads, TB ? (CH <= 16 ? 4 : 3) : 1)
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int c = lane % LANES;  // chunk of this lane
-  const int lt = (blockIdx.x * blockDim.x + threadIdx.x) / LANES;  // pair index within this launch
-  const int nn = n_dev ? min(n, *n_dev) : n;
-  const int warp_first = (blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / LANES;
-  if (base + 2 * warp_first >= nn) return;  // the whole warp is past the tasks (warp-uniform)
+  const int nn = n_dev ? min(n, *n_dev) : n, pairs = (min(nn - base, count) + 1) / 2;
+  const auto align = [&](const int lt) {  // lt: pair index within this launch
   const int ia = base + 2 * lt, ib = ia + 1;
-  const bool live = ia < nn, has_b = ib < nn;
+  const bool live = lt < pairs, has_b = live && ib < nn;
   SwTask ta{}, tb{};
   if (live) ta = tasks[ia];
   if (has_b) tb = tasks[ib];
@@ -626,8 +687,8 @@ __global__ void __launch_bounds__(kSwThreads, TB ? (CH <= 16 ? 4 : 3) : 1)
     skip = true;
     if (c == 0) {
       const int k = atomicAdd(fb, has_b ? 2 : 1);
-      fb[1 + k] = 2 * lt;
-      if (has_b) fb[2 + k] = 2 * lt + 1;
+      fb[kFbList + k] = 2 * lt;
+      if (has_b) fb[kFbList + 1 + k] = 2 * lt + 1;
     }
   }
   const int steps = __reduce_max_sync(FULL, skip ? 0 : qmax + LANES - 1);
@@ -650,63 +711,103 @@ __global__ void __launch_bounds__(kSwThreads, TB ? (CH <= 16 ? 4 : 3) : 1)
     return i >= 0 && i < ql ? min(static_cast<uint32_t>(q[i]), 4u) : 4u;
   };
   const int d0 = CH * c;  // band column of local cell 0
-  uint32_t H[CH + 2], E[CH + 2], T[CH + 1];
+  const CellParams cp = cell_params(p);
+  const uint32_t h_zero = kBias2 - cp.oe;  // H = 0
+  uint32_t H[CH + 1], E[CH + 1], T[CH + 1];
 #pragma unroll
-  for (int k = 0; k < CH + 2; ++k) {
-    H[k] = kBias2;
+  for (int k = 0; k <= CH; ++k) {
+    H[k] = h_zero;
     E[k] = kBias2;
   }
 #pragma unroll
   for (int k = 0; k <= CH; ++k) T[k] = skip ? 0u : tc2(d0 + k);  // row 0
-  const uint32_t OE = pack2(p.oe), GE = pack2(p.ge), SB = pack2(kScoreBias);
-  uint32_t best2 = kBias2, best_a = kBias, best_b = kBias;
+  uint32_t best2 = h_zero;
   int bi_a = -1, bi_b = -1;
   extern __shared__ uint32_t sw_rows[];
-  uint32_t* const row_a = sw_rows + threadIdx.x;
-  uint32_t* const row_b = sw_rows + (CH + 1) * kSwThreads + threadIdx.x;
-  int buf_a = 0, buf_b = 1;  // which of the two row buffers holds each half's best row
-  uint32_t hout = kBias2, fout = kBias2;  // this lane's last cell of its previous row
-  // the row's profile words, and the codes of the next step's row: loaded a step ahead so
-  // their latency hides behind the step (row -c of a lane that has not reached row 0 is N)
-  uint32_t plo = s_prof[qcode(qa, qla, -c)], phi = s_prof[qcode(qb, qlb, -c)];
-  uint32_t cna = qcode(qa, qla, 1 - c), cnb = qcode(qb, qlb, 1 - c);
+  uint4* const row_a = reinterpret_cast<uint4*>(sw_rows) + threadIdx.x;  // cells 4g .. 4g + 3 at [g * kDpThreads]
+  uint4* const row_b = row_a + CH / 4 * kDpThreads;
+  uint32_t* const last_a = sw_rows + 2 * CH * kDpThreads + threadIdx.x;  // cell CH
+  uint32_t* const last_b = last_a + kDpThreads;
+  uint32_t hout = h_zero, fout = kBias2;  // this lane's last cell of its previous row
+  // Codes. Narrow chunks (kStream) load them LANES steps at a time: at a block's first step
+  // lane c holds the profile words of row t + c and the target column the last lane shifts in
+  // at step t + c, loaded a block earlier; a step takes row i's words by a shuffle from lane
+  // i mod LANES (rows before 0 are N rows), and the column entering a lane's window is the
+  // right neighbour's T[2] (its row is one behind). Otherwise each lane loads its own row's
+  // codes two steps and its profile words and column one step ahead.
+  constexpr bool kStream = LANES >= 4;
+  uint32_t plo, phi, x_qa, x_qb, x_ta = 0, x_tb = 0, old_lo = 0, old_hi = 0, cur_t = 0;
+  const auto fetch = [&](int t) {
+    x_qa = qcode(qa, qla, t + c);
+    x_qb = qcode(qb, qlb, t + c);
+    if (!skip) {
+      const int j = t + c + 2 - LANES + LANES * CH;
+      x_ta = __ldg(wa + min(j, ja));
+      x_tb = __ldg(wb + min(j, jb));
+    }
+  };
+  if constexpr (kStream) {
+    plo = phi = s_prof[4];
+    fetch(0);
+  } else {
+    // row -c of a lane that has not reached row 0 is N
+    plo = s_prof[qcode(qa, qla, -c)];
+    phi = s_prof[qcode(qb, qlb, -c)];
+    x_qa = qcode(qa, qla, 1 - c);
+    x_qb = qcode(qb, qlb, 1 - c);
+  }
+  const int end = skip ? 0 : qmax;
+  uint32_t* dp = TB ? DP + (d0 >> 2) * 32 - c * (WQ * 32) : nullptr;  // row i's first word of this lane
   const auto step = [&](const int t, auto steady) {
     constexpr bool kSteady = decltype(steady)::value;
     const int i = t - c;
-    const bool act = !skip && i >= 0 && i < qmax;
+    const bool act = static_cast<unsigned>(i) < static_cast<unsigned>(end);
     // H, E and the target window advance once the lane has reached row 0 (rows past the
     // pair's end are N rows: they change no result and no code is stored for them); from
     // step LANES - 1 on every lane has, so the steady steps carry no per-cell guard
     const bool he_ok = kSteady || i >= 0;
     // row i's F and H(left) at column d0 - 1, from the left lane (its step t - 1)
     uint32_t hleft = __shfl_up_sync(FULL, hout, 1), f = __shfl_up_sync(FULL, fout, 1);
-    if (c == 0) hleft = f = kBias2;
-    const uint32_t plo_next = s_prof[cna], phi_next = s_prof[cnb];
-    const uint32_t cna_next = qcode(qa, qla, i + 2), cnb_next = qcode(qb, qlb, i + 2);
-    // past the pair's end the window shifts in a valid selector (code A for both): the
-    // profile of an N row scores every target alike
-    const uint32_t t_next = act ? tc2(i + 1 + d0 + CH) : sel2(0u, 0u);
-    uint32_t hdiag = H[0], rmax = 0, dw = 0;
-    // local cell 0, then hand (H, E) of it to the left lane: the E input of its last cell
-    uint32_t h0, e0;
-    {
-      const uint32_t hup = H[1], eup = E[1];
-      const uint32_t hd = hdiag + prmt(plo, phi, T[0]) - SB;
-      const uint32_t eo = hup - OE, ee = eup - GE, fo = hleft - OE, fe = f - GE;
-      e0 = __vmaxu2(eo, ee);
-      f = __vmaxu2(fo, fe);
-      const uint32_t m1 = __vmaxu2(hd, e0);
-      h0 = __vimax3_u16x2(m1, f, kBias2);
-      if constexpr (TB)
-        dw = ((__vminu2(m1 - hd, kOne2) * 2u + __vminu2(h0 - m1, kOne2)) * 2u + __vminu2(e0 - eo, kOne2)) * 2u +
-             __vminu2(f - fo, kOne2);
-      rmax = h0;
-      hleft = h0;
-      hdiag = hup;
+    if (c == 0) {
+      hleft = h_zero;
+      f = kBias2;
     }
+    uint32_t lo, hi, t_next;
+    if constexpr (kStream) {
+      const int s = t & (LANES - 1);
+      if (s == 0) {  // plo, phi: this block's words; old_lo, old_hi: the last one's
+        old_lo = plo;
+        old_hi = phi;
+        plo = s_prof[x_qa];
+        phi = s_prof[x_qb];
+        cur_t = x_ta * 17u + x_tb * 4352u + 50304u;  // sel2
+        fetch(t + LANES);
+      }
+      const bool now = c <= s;
+      lo = __shfl_sync(FULL, now ? plo : old_lo, i, LANES);
+      hi = __shfl_sync(FULL, now ? phi : old_hi, i, LANES);
+      t_next = __shfl_down_sync(FULL, he_ok ? T[2] : T[1], 1);
+      const uint32_t entering = __shfl_sync(FULL, cur_t, s, LANES);
+      if (c == LANES - 1) t_next = entering;
+    } else {
+      lo = plo;
+      hi = phi;
+      plo = s_prof[x_qa];
+      phi = s_prof[x_qb];
+      x_qa = qcode(qa, qla, i + 2);
+      x_qb = qcode(qb, qlb, i + 2);
+      // past the pair's end the window shifts in a valid selector (code A for both): the
+      // profile of an N row scores every target alike
+      t_next = act ? tc2(i + 1 + d0 + CH) : sel2(0u, 0u);
+    }
+    // local cell 0, then hand (H, E) of it to the left lane: the E input of its last cell
+    uint32_t rmax = 0, dw = 0, e0;
+    const uint32_t h0 = cell2<TB>(cp, H[0], prmt(lo, hi, T[0]), H[1], E[1], hleft, f, e0, dw);
+    uint32_t hdiag = H[1];
+    hleft = h0;
     // a lane that has not reached row 0 passes row -1's values (zero)
-    uint32_t nh = __shfl_down_sync(FULL, i >= 0 ? h0 : kBias2, 1);
-    uint32_t ne = __shfl_down_sync(FULL, i >= 0 ? e0 : kBias2, 1);
+    uint32_t nh = __shfl_down_sync(FULL, he_ok ? h0 : h_zero, 1);
+    uint32_t ne = __shfl_down_sync(FULL, he_ok ? e0 : kBias2, 1);
     if (c == LANES - 1) {
       nh = H[CH];
       ne = E[CH];
@@ -715,72 +816,55 @@ __global__ void __launch_bounds__(kSwThreads, TB ? (CH <= 16 ? 4 : 3) : 1)
       H[0] = h0;
       E[0] = e0;
     }
+    uint32_t& top = TB ? rmax : best2;  // the row's maximum (score only: the maximum so far)
 #pragma unroll
     for (int k = 1; k <= CH; ++k) {
       if (k == CH && c != LANES - 1) break;  // the extra cell W - 1 belongs to the last lane
-      const uint32_t hup = k == CH - 1 ? nh : (k == CH ? kBias2 : H[k + 1]);
+      const uint32_t hup = k == CH - 1 ? nh : (k == CH ? h_zero : H[k + 1]);
       const uint32_t eup = k == CH - 1 ? ne : (k == CH ? kBias2 : E[k + 1]);
-      const uint32_t hd = hdiag + prmt(plo, phi, T[k]) - SB;
-      const uint32_t eo = hup - OE, ee = eup - GE, fo = hleft - OE, fe = f - GE;
-      const uint32_t e = __vmaxu2(eo, ee);
-      f = __vmaxu2(fo, fe);
-      const uint32_t m1 = __vmaxu2(hd, e);
-      const uint32_t h = __vimax3_u16x2(m1, f, kBias2);
+      uint32_t e, code = 0;
+      const uint32_t h = cell2<TB>(cp, hdiag, prmt(lo, hi, T[k]), hup, eup, hleft, f, e, code);
       if (he_ok) {
         H[k] = h;
         E[k] = e;
       }
       if constexpr (TB) {
-        const uint32_t code = ((__vminu2(m1 - hd, kOne2) * 2u + __vminu2(h - m1, kOne2)) * 2u +
-                               __vminu2(e - eo, kOne2)) * 2u + __vminu2(f - fo, kOne2);
-        dw = dw * 16u + code;
-        if ((k & 3) == 3) {
-          if (act) DP[(static_cast<size_t>(i) * WQ + ((d0 + k) >> 2)) * 32] = dw;
-          dw = 0;
-        } else if (k == CH) {  // cell W - 1 opens the last, partial word
-          dw <<= 12;
-          if (act) DP[(static_cast<size_t>(i) * WQ + ((d0 + k) >> 2)) * 32] = dw;
-        }
-        rmax = __vmaxu2(rmax, h);
-      } else {
-        best2 = __vmaxu2(best2, h);
+        dw = insert_code(dw, code, k & 3);
+        if (((k & 3) == 3 || k == CH) && act) dp[(k >> 2) * 32] = dw;
       }
+      if (k & 1) top = __vimax3_u16x2(top, hleft, h);
+      else if (k == CH) top = __vmaxu2(top, h);
       hleft = h;
       hdiag = hup;
     }
-    if constexpr (!TB) best2 = __vmaxu2(best2, h0);
     hout = hleft;
     fout = f;
-    if (act) {
-      if constexpr (TB) {  // a strictly better row of this lane's cells
-        const bool up_a = (rmax & 0xFFFFu) > best_a, up_b = (rmax >> 16) > best_b;
-        if (up_a || up_b) {
-          const int dst = row_buffer(up_a, up_b, buf_a, buf_b);
-          uint32_t* const row = dst ? row_b : row_a;
+    if constexpr (TB) {
+      if (act) {  // a strictly better row of this lane's cells
+        const uint32_t b2 = __vmaxu2(best2, rmax), up = b2 ^ best2;
+        best2 = b2;
+        if (up & 0xFFFFu) {
+          bi_a = i;
 #pragma unroll
-          for (int k = 0; k <= CH; ++k) row[k * kSwThreads] = H[k];
-          if (up_a) {
-            best_a = rmax & 0xFFFFu;
-            bi_a = i;
-            buf_a = dst;
-          }
-          if (up_b) {
-            best_b = rmax >> 16;
-            bi_b = i;
-            buf_b = dst;
-          }
+          for (int g = 0; g < CH / 4; ++g)
+            row_a[g * kDpThreads] = make_uint4(H[4 * g], H[4 * g + 1], H[4 * g + 2], H[4 * g + 3]);
+          *last_a = H[CH];
+        }
+        if (up >> 16) {
+          bi_b = i;
+#pragma unroll
+          for (int g = 0; g < CH / 4; ++g)
+            row_b[g * kDpThreads] = make_uint4(H[4 * g], H[4 * g + 1], H[4 * g + 2], H[4 * g + 3]);
+          *last_b = H[CH];
         }
       }
+      dp += WQ * 32;
     }
     if (he_ok) {
 #pragma unroll
       for (int k = 0; k < CH; ++k) T[k] = T[k + 1];
       T[CH] = t_next;
     }
-    plo = plo_next;
-    phi = phi_next;
-    cna = cna_next;
-    cnb = cnb_next;
   };
   const int ramp = steps < LANES - 1 ? steps : LANES - 1;
   for (int t = 0; t < ramp; ++t) step(t, std::false_type{});
@@ -790,12 +874,13 @@ __global__ void __launch_bounds__(kSwThreads, TB ? (CH <= 16 ? 4 : 3) : 1)
   const int ncell = c == LANES - 1 ? CH + 1 : CH;
   if constexpr (TB) {
     int bd_a = 0xFFF, bd_b = 0xFFF;
-    const uint32_t* const ra = buf_a ? row_b : row_a;
-    const uint32_t* const rb = buf_b ? row_b : row_a;
+    const uint32_t best_a = best2 & 0xFFFFu, best_b = best2 >> 16;
 #pragma unroll 1
     for (int k = ncell - 1; k >= 0; --k) {
-      if (bi_a >= 0 && (ra[k * kSwThreads] & 0xFFFFu) == best_a) bd_a = d0 + k;
-      if (bi_b >= 0 && (rb[k * kSwThreads] >> 16) == best_b) bd_b = d0 + k;
+      const uint32_t a = k == CH ? *last_a : reinterpret_cast<const uint32_t*>(row_a + (k >> 2) * kDpThreads)[k & 3];
+      const uint32_t b = k == CH ? *last_b : reinterpret_cast<const uint32_t*>(row_b + (k >> 2) * kDpThreads)[k & 3];
+      if (bi_a >= 0 && (a & 0xFFFFu) == best_a) bd_a = d0 + k;
+      if (bi_b >= 0 && (b >> 16) == best_b) bd_b = d0 + k;
     }
     key_a = static_cast<uint64_t>(best_a) << 40 | static_cast<uint64_t>(0xFFFFFu - static_cast<uint32_t>(bi_a + 1)) << 12 |
             (0xFFFu - static_cast<uint32_t>(bd_a));
@@ -812,14 +897,21 @@ __global__ void __launch_bounds__(kSwThreads, TB ? (CH <= 16 ? 4 : 3) : 1)
     key_b = xb > key_b ? xb : key_b;
   }
   if (c != 0 || skip) return;
-  const auto unpack = [](uint64_t key) {
-    const int best = static_cast<int>(key >> 40) - static_cast<int>(kBias);
+  const int zero = static_cast<int>(kBias) - p.oe;
+  const auto unpack = [zero](uint64_t key) {
+    const int best = static_cast<int>(key >> 40) - zero;
     const int bi = static_cast<int>(0xFFFFFu - static_cast<uint32_t>((key >> 12) & 0xFFFFFu)) - 1;
     const int bd = static_cast<int>(0xFFFu - static_cast<uint32_t>(key & 0xFFFu));
     return TB ? stash(best, bi, bd) : stash(best, 0, 0);
   };
   res[ta.slot] = unpack(key_a);
   if (has_b) res[tb.slot] = unpack(key_b);
+  };
+  constexpr int kPairs = 32 / LANES;
+  for (int w = blockIdx.x; w * kPairs < pairs; w = next_claim(claim)) {
+    align(w * kPairs + lane / LANES);
+    __syncwarp();
+  }
 }
 
 // The pairs k_sw_u2 listed, one alignment per thread, int32.
@@ -832,7 +924,7 @@ __global__ void __launch_bounds__(kSwThreads) k_sw_fb(const SwTask* __restrict__
   constexpr int WQ = (W + 3) / 4;
   const int nfb = fb[0];
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nfb; j += gridDim.x * blockDim.x) {
-    const int lt = fb[1 + j];
+    const int lt = fb[kFbList + j];
     const SwTask tk = tasks[base + lt];
     res[tk.slot] = sw_one_reg<W, TB>(tk, qbase, tbase, p, TB ? pair_base(dir, lt, rows_max, WQ) : nullptr, lt & 1);
   }
@@ -866,7 +958,7 @@ __global__ void __launch_bounds__(kSwThreads)
   for (int jw = static_cast<int>((blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / LANES); jw < nfb; jw += stride) {
   const int j = jw + lane / LANES;  // entry of the fallback list
   const bool live = j < nfb;
-  const int lt = live ? fb[1 + j] : 0;
+  const int lt = live ? fb[kFbList + j] : 0;
   SwTask tk{};
   if (live) tk = tasks[base + lt];
   const int ql = live ? tk.qlen : 0;
@@ -905,7 +997,7 @@ __global__ void __launch_bounds__(kSwThreads)
       f = max(fo, fe);
       const int m1 = max(hd, e0);
       h0 = max(max(m1, f), 0);
-      if constexpr (TB) dw = dir_code32(hd >= e0, m1 >= f, eo >= ee, fo >= fe);
+      if constexpr (TB) dw = dir_code32(h0 == hd, h0 == e0, eo >= ee, fo >= fe);
       rmax = h0;
       hleft = h0;
       hdiag = hup;
@@ -937,13 +1029,12 @@ __global__ void __launch_bounds__(kSwThreads)
         E[k] = e;
       }
       if constexpr (TB) {
-        dw = dw * 16u + dir_code32(hd >= e, m1 >= f, eo >= ee, fo >= fe);
+        dw |= dir_code32(h == hd, h == e, eo >= ee, fo >= fe) << (k & 3);
         if ((k & 3) == 3) {
           if (act) reinterpret_cast<uint16_t*>(DP + (static_cast<size_t>(i) * WQ + ((d0 + k) >> 2)) * 32)[half] =
               static_cast<uint16_t>(dw);
           dw = 0;
         } else if (k == CH) {  // cell W - 1 opens the last, partial word
-          dw <<= 12;
           if (act) reinterpret_cast<uint16_t*>(DP + (static_cast<size_t>(i) * WQ + ((d0 + k) >> 2)) * 32)[half] =
               static_cast<uint16_t>(dw);
         }
@@ -1050,7 +1141,7 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
         while (!stop && i >= 0 && v > 0) {
           const int top = i - kAhead * gl;  // this lane's block: rows top, top - 1, .. top - 7
           const int sh = code.shift(d);
-          uint32_t cx = 0;  // the block's codes, row top - k in bits 4k
+          uint32_t cx = 0;  // row top - k of the block: kNotDiag in bit k, kNotE in bit 8 + k
           uint64_t qw = 0, tw = 0;  // its bases, row top - k in byte 7 - k; N past any end
           int lost = 0;             // what the block takes from v, and 256ths of it its mismatches
           bool clean = false;
@@ -1060,8 +1151,8 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
               qw = load8u(q + top - (kAhead - 1));
               tw = load8u(tbase + x0);
 #pragma unroll
-              for (int k = 0; k < kAhead; ++k) cx |= ((code.word(top - k, d) >> sh) & 0xFu) << (4 * k);
-              clean = (cx & 0x11111111u * (kNotDiagE | kFromF)) == 0;
+              for (int k = 0; k < kAhead; ++k) cx |= ((code.word(top - k, d) >> sh) & (kNotDiag | kNotE)) << k;
+              clean = (cx & 0xFFu) == 0;
               // bytes equal and both below 4: match; either above 3: ambiguous; else mismatch
               const uint64_t ok_amb = zero_bytes((qw | tw) & 0xFCFCFCFCFCFCFCFCull);
               const int n_match = __popcll(zero_bytes(qw ^ tw) & ok_amb);
@@ -1072,7 +1163,7 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
 #pragma unroll
               for (int k = 0; k < kAhead; ++k) {
                 if (top - k >= 0) {
-                  cx |= code(top - k, d) << (4 * k);
+                  cx |= (code(top - k, d) & (kNotDiag | kNotE)) << k;
                   qw |= static_cast<uint64_t>(q[top - k]) << (8 * (kAhead - 1 - k));
                   tw |= static_cast<uint64_t>(tcode(tbase, tk, static_cast<int64_t>(top - k) + d))
                         << (8 * (kAhead - 1 - k));
@@ -1105,8 +1196,8 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
                 stop = true;
                 break;
               }
-              x = (cx >> (4 * k)) & 0xFu;
-              if (x & (kNotDiagE | kFromF)) {  // not from the diagonal
+              x = cx >> k;
+              if (x & kNotDiag) {  // not from the diagonal
                 stop = true;
                 break;
               }
@@ -1130,7 +1221,7 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
         if (i < 0 || v <= 0) break;
         run = 0;
         bool ext = true;
-        if (!(x & kFromF)) {  // from E, an insertion: E(i,d) <- (i-1, d+1)
+        if (!(x & kNotE)) {  // from E, an insertion: E(i,d) <- (i-1, d+1)
           while (ext) {
             if (i < 0 || d >= W) {
               broken = true;
@@ -1218,7 +1309,7 @@ __global__ void __launch_bounds__(kSwThreads) k_sw_any(const SwTask* __restrict_
       Hs[d * 32] = h;
       Es[d * 32] = e;
       if (TB) {
-        dw |= dir_code32(hd >= e, m1 >= f, eo >= ee, fo >= fe) << (4 * (d & 7));
+        dw |= dir_code32(h == hd, h == e, eo >= ee, fo >= fe) << (4 * (d & 4) + (d & 3));
         if ((d & 7) == 7 || d == W - 1) {
           D[(static_cast<size_t>(i) * WW + (d >> 3)) * 32] = dw;
           dw = 0;
@@ -1241,7 +1332,7 @@ __global__ void __launch_bounds__(kSwThreads) k_sw_any(const SwTask* __restrict_
   }
   SwResult r{best, 0, 0, 0, 0, 0, 0, 0};
   if (TB && best > 0)
-    traceback(NibbleCodes{D, WW}, W, bi, bd, best, q, tbase, tk, p, r, cig + cig_off[tk.slot], 2 * ql + 1, err);
+    traceback(WordCodes{D, WW}, W, bi, bd, best, q, tbase, tk, p, r, cig + cig_off[tk.slot], 2 * ql + 1, err);
   res[tk.slot] = r;
 }
 
@@ -1265,37 +1356,53 @@ struct SwLaunch {
   const KernelTrace& kt;
 };
 
+// Cells per lane of kSwIntraNarrow: 8 against 16, 58,000 tracebacks of 150 rows at W = 33 188
+// and 212 us; 88,000 of 50 to 1,000 rows at W = 129 1,871 and 1,307.
+constexpr int sw_narrow_cells(int W) { return W == 129 ? 16 : 8; }
+
+// Blocks of one warp for `warps` claims: all of them, up to what is resident.
+template <class Kernel>
+int dp_blocks(int64_t warps, Kernel* kernel, int smem, std::atomic<int>* resident) {
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+    v = resident[dev].load(std::memory_order_relaxed);
+    if (v <= 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, kDpThreads, smem) == cudaSuccess && v > 0)
+      resident[dev].store(v, std::memory_order_relaxed);
+  }
+  cudaGetLastError();
+  return static_cast<int>(std::min<int64_t>(warps, int64_t{v > 0 ? v : 8} * device_sm_count()));
+}
+
 template <int LANES, int CH>
 void run_wide(const SwLaunch& a, int count, int above, int upto) {
   const int64_t pairs = (static_cast<int64_t>(count) + 1) / 2;
-  const int blocks = static_cast<int>((pairs * LANES + kSwThreads - 1) / kSwThreads);
-  constexpr int kRowBytes = 2 * (CH + 1) * kSwThreads * 4;  // the two saved best rows of each lane
+  int* const claim = a.fb + (upto == INT_MAX ? 2 : 1);
+  const auto run = [&](auto* kernel, int smem, std::atomic<int>* resident) {
+    kernel<<<dp_blocks((pairs * LANES + 31) / 32, kernel, smem, resident), kDpThreads, smem, a.st>>>(
+        a.tasks, a.base, a.count, a.n, a.n_dev, above, upto, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb,
+        claim);
+  };
+  constexpr int kRowBytes = 2 * (CH + 1) * kDpThreads * 4;  // the two saved best rows of each lane
+  static std::atomic<int> resident[2][kMaxDevices];
   a.kt.begin(a.st, a.tb ? "k_sw_wide<tb>" : "k_sw_wide<score>");
-  if (a.tb)
-    k_sw_wide<LANES, CH, true><<<blocks, kSwThreads, kRowBytes, a.st>>>(
-        a.tasks, a.base, a.n, a.n_dev, above, upto, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb);
-  else
-    k_sw_wide<LANES, CH, false><<<blocks, kSwThreads, 0, a.st>>>(
-        a.tasks, a.base, a.n, a.n_dev, above, upto, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb);
+  if (a.tb) run(k_sw_wide<LANES, CH, true>, kRowBytes, resident[1]);
+  else run(k_sw_wide<LANES, CH, false>, 0, resident[0]);
   a.kt.end(a.st);
 }
 
 template <int W>
 void run_u2(const SwLaunch& a, int above) {
-  const int blocks = ((a.count + 1) / 2 + kSwThreads - 1) / kSwThreads;
+  const auto run = [&](auto* kernel, int smem, std::atomic<int>* resident) {
+    const int64_t warps = ((static_cast<int64_t>(a.count) + 1) / 2 + 31) / 32;
+    kernel<<<dp_blocks(warps, kernel, smem, resident), kDpThreads, smem, a.st>>>(
+        a.tasks, a.base, a.count, a.n, a.n_dev, above, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb, a.fb + 2);
+  };
+  constexpr int kRowBytes = 2 * W * kDpThreads * 4;  // the two saved best rows of each thread
+  static_assert(kRowBytes <= 48 * 1024);
+  static std::atomic<int> resident[2][kMaxDevices];
   a.kt.begin(a.st, a.tb ? "k_sw_u2<tb>" : "k_sw_u2<score>");
-  if (a.tb) {
-    constexpr int kRowBytes = 2 * W * kSwThreads * 4;  // the two saved best rows of each thread
-    if (kRowBytes > 48 * 1024) {
-      static std::atomic<bool> attr_set[kMaxDevices];
-      set_smem_limit_once(k_sw_u2<W, true>, kRowBytes, attr_set);
-    }
-    k_sw_u2<W, true><<<blocks, kSwThreads, kRowBytes, a.st>>>(a.tasks, a.base, a.n, a.n_dev, above, a.qbase, a.tbase,
-                                                              a.p, a.res, a.dir, a.rows_max, a.fb);
-  } else {
-    k_sw_u2<W, false><<<blocks, kSwThreads, 0, a.st>>>(a.tasks, a.base, a.n, a.n_dev, above, a.qbase, a.tbase, a.p,
-                                                       a.res, a.dir, a.rows_max, a.fb);
-  }
+  if (a.tb) run(k_sw_u2<W, true>, kRowBytes, resident[1]);
+  else run(k_sw_u2<W, false>, 0, resident[0]);
   a.kt.end(a.st);
 }
 
@@ -1324,14 +1431,14 @@ void run_fb(const SwLaunch& a) {
 template <int W>
 void launch_band(const SwLaunch& a, SwForm form, int few) {
   constexpr bool kFew = W == 17 || W == 33 || W == 65 || W == 129;
-  cudaMemsetAsync(a.fb, 0, sizeof(int), a.st);
+  cudaMemsetAsync(a.fb, 0, kFbList * sizeof(int), a.st);
   if constexpr (kFew) {
     if (form == kSwIntraFew) run_wide<(W - 1) / 4, 4>(a, a.count, 0, INT_MAX);
     else if (few > 0) run_wide<(W - 1) / 4, 4>(a, std::min(a.count, few), 0, few);
   }
   if constexpr (W == 33 || W == 65 || W == 129) {
     if (form == kSwIntra) run_wide<(W - 1) / 32, 32>(a, a.count, few, INT_MAX);
-    if (form == kSwIntraNarrow) run_wide<(W - 1) / 16, 16>(a, a.count, few, INT_MAX);
+    if (form == kSwIntraNarrow) run_wide<(W - 1) / sw_narrow_cells(W), sw_narrow_cells(W)>(a, a.count, few, INT_MAX);
   }
   if constexpr (W != 129) {
     if (form == kSwInter) run_u2<W>(a, few);
@@ -1371,6 +1478,8 @@ SwParams make_sw_params(const dnaln_score_params& s) {
   p.bw = s.bw;
   p.W = 2 * s.bw + 1;
   p.prof_n = static_cast<uint32_t>(static_cast<uint8_t>(-s.ambig)) * 0x01010101u;
+  p.one = 1u;
+  p.mone = 0u - 1u;
   return p;
 }
 
@@ -1385,11 +1494,11 @@ size_t sw_band_bytes_per_task(int W, bool bytes_ok) {
 
 // Up to this many tasks the form of four cells per lane is the fastest: its row step is the
 // shortest serial chain, and a short list leaves lanes idle anyway. Measured against the
-// best other form, us for 150-row tracebacks: W = 33 67 against 113 at 1,024 tasks, 117
-// against 115 at 16,384; W = 65 68 against 114 and, at 8,192, 122 against 118; W = 129 76
-// against 118 and, at 4,096, 136 against 120; W = 17 70 against 105 and, at 32,768, 118
-// against 108.
-int sw_few_tasks(int W) { return W == 17 ? 24576 : (W == 33 ? 16384 : (W == 65 ? 8192 : 3072)); }
+// best other form, us for 150-row tracebacks: W = 33 51 against 67 at 1,024 tasks, 94
+// against 91 at 16,384; W = 65 51 against 64 and, at 8,192, 97 against 85; W = 129 57
+// against 90 and, at 4,096, 117 against 95; W = 17 55 against 92 and, at 32,768, 99
+// against 97.
+int sw_few_tasks(int W) { return W == 17 ? 28672 : (W == 33 ? 14336 : (W == 65 ? 4608 : 3072)); }
 
 int sw_launches(int W, bool bytes_ok, bool tb) { return sw_uses_generic(W, bytes_ok) ? 1 : (tb ? 3 : 2); }
 
@@ -1406,7 +1515,7 @@ bool sw_has_form(int W, bool bytes_ok, SwForm form) {
 
 int sw_lanes_per_pair(int W, SwForm form) {
   if (form == kSwIntra) return (W - 1) / 32;
-  if (form == kSwIntraNarrow) return (W - 1) / 16;
+  if (form == kSwIntraNarrow) return (W - 1) / sw_narrow_cells(W);
   if (form == kSwIntraFew) return (W - 1) / 4;
   return 1;
 }

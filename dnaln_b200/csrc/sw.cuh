@@ -29,6 +29,7 @@ int sw_launches(int W, bool bytes_ok, bool tb);
 // sequence (k_sw_wide, the row of a pair spread over lanes in a skewed wavefront: (W - 1) /
 // 32 lanes of 32 cells, or, narrow, (W - 1) / 16 lanes of 16 cells; W = 33, 65, 129). The
 // generic kernel (other widths or scores) has the inter form only.
+constexpr int kSwFbHead = 3;  // ints before the fallback list's entries
 enum SwForm : int { kSwInter = 0, kSwIntra = 1, kSwIntraNarrow = 2, kSwIntraFew = 3 };
 constexpr int kSwForms = 3;  // forms the tuner times: kSwIntraFew is chosen by the task count
 // Task count up to which kSwIntraFew ((W - 1) / 4 lanes of 4 cells) runs.
@@ -42,7 +43,7 @@ int sw_lanes_per_pair(int W, SwForm form);
 // cig_off[task.slot], capacity 2*qlen+1. base must be a multiple of kSwTaskGroup; `dir`
 // and `band` must hold count rounded up to kSwTaskGroup tasks of
 // sw_dir_bytes_per_task(W, rows_max) and sw_band_bytes_per_task(W, bytes_ok); `fb`
-// (count + 1 ints) lists the tasks the 16-bit kernel hands to the int32 one; kt (may be
+// (count + kSwFbHead ints) lists the tasks the 16-bit kernel hands to the int32 one; kt (may be
 // null) times each kernel; few > 0 (needs n_dev) lets kSwIntraFew take the whole launch when
 // *n_dev <= few. Returns false, launching nothing, when a needed scratch pointer
 // is null or base is misaligned.
