@@ -132,8 +132,10 @@ __device__ __forceinline__ void st_evict_first(uint32_t* p, uint32_t v, uint64_t
 // 16x2: the biased values lie in [0, 32767], where signed and unsigned order agree).
 //
 // Adds, maxima, prmt and logic run on the ALU pipe at one instruction every two cycles, and
-// integer multiply-adds beside it at the same rate, so the cell's plain additions are written
-// as multiply-adds by 1 or -1 that the compiler cannot fold: about ten instructions each.
+// integer multiply-adds beside it at the same rate, so some of the cell's additions are
+// written as multiply-adds by 1 or -1 that the compiler cannot fold. Measured, 88,000
+// tracebacks at W = 129 and 262,144 of 150 rows at W = 33: as below 1,154 and 631 us; every
+// addition a multiply-add 1,200 and 708; none 1,439 and, in the flags' former form, 677.
 struct CellParams {
   uint32_t oe, nge, khd;  // O+E; -E in each signed half; O+E - profile bias
   uint32_t one, mone;     // 1 and -1, as values known at run time only
@@ -154,7 +156,7 @@ __device__ __forceinline__ uint32_t mad(uint32_t a, uint32_t b, uint32_t c) {
 template <bool TB>
 __device__ __forceinline__ uint32_t cell2(const CellParams& c, uint32_t hdiag, uint32_t s, uint32_t hup, uint32_t eup,
                                           uint32_t hleft, uint32_t& f, uint32_t& e, uint32_t& code) {
-  const uint32_t hd = mad(mad(hdiag, c.one, c.khd), c.one, s);
+  const uint32_t hd = hdiag + c.khd + s;
   e = __viaddmax_s16x2(eup, c.nge, hup);
   f = __viaddmax_s16x2(f, c.nge, hleft);
   const uint32_t h = __vimax3_u16x2(__vmaxu2(hd, e), f, kBias2);
@@ -162,7 +164,7 @@ __device__ __forceinline__ uint32_t cell2(const CellParams& c, uint32_t hdiag, u
     constexpr uint32_t k = 0x7FFF7FFFu;
     const uint32_t hk = mad(h, c.one, k);
     const uint32_t de = prmt(mad(hd, c.mone, hk), mad(e, c.mone, hk), 0xFBD9u);  // bytes: A kNotDiag, A kNotE, B, B
-    const uint32_t ex = prmt(mad(e, c.one, mad(hup, c.mone, k)), mad(f, c.one, mad(hleft, c.mone, k)), 0xFBD9u);
+    const uint32_t ex = prmt(e - hup + k, mad(hleft, c.mone, f) + k, 0xFBD9u);
     code = (de & 0x0F0F0F0Fu) | (ex & 0xF0F0F0F0u);
   }
   return mad(c.oe, c.mone, h);
@@ -650,9 +652,9 @@ __global__ void __launch_bounds__(kDpThreads, (TB && W <= 33) ? 12 : 1)
 // With a row's codes taken by shuffles, additions spread over two pipes (cell2), the best rows
 // saved by 16-byte stores and warps that claim their pairs, against loads by every lane in
 // every row and a grid over the list, tracebacks: 58,000 tasks of 150 rows at W = 33 214 ->
-// 176 us (now 8 cells a lane, before 32), 150,000 of 50 to 1,000 rows 924 -> 678 (8, before
-// 16); 88,000 at W = 129 1,484 -> 1,200 (32); 4,001 of 1,000 to 5,000 rows at W = 65 1,732 ->
-// 1,218 (4). At 8 cells a lane ALU and multiply-add pipe are each busy about 60 % of the time.
+// 179 us (now 8 cells a lane, before 32), 150,000 of 50 to 1,000 rows 924 -> 643 (8, before
+// 16); 88,000 at W = 129 1,484 -> 1,154 (32); 4,001 of 1,000 to 5,000 rows at W = 65 1,732 ->
+// 1,186 (4). At 8 cells a lane ALU and multiply-add pipe are each busy about 60 % of the time.
 // Resident warps per SM (sw_wide_warps), same lists: 8 cells 16 / 20 / 24 warps 185 / 176 /
 // 190 us; 32 cells 12 / 10 / 8 warps 1,333 / 1,311 / 1,200; 4 cells 20 / 24 1,262 / 1,218.
 constexpr int sw_wide_warps(int cells) { return cells == 4 ? 24 : (cells == 8 ? 20 : (cells == 16 ? 12 : 8)); }
