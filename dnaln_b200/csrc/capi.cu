@@ -3,7 +3,7 @@
 // seed.cu, sw.cu and map.cu.
 //
 // One batch (Mapper::map, src/mapper.cpp:75-223) is enqueued on the context's stream as:
-//   k_len64 + scan: packed read offsets, total bases, longest read (read back first only
+//   k_len_scan: packed read offsets, total bases, longest read (read back first only
 //     when the caller did not give the batch's size, so the rest can run as a graph)
 //   k_encode_reads: codes of both strands of every read
 //   k_seed_chain_t: short reads one thread each (sketch, probe, anchors, chaining DP,
@@ -120,6 +120,7 @@ struct MapRun {
   int64_t B = 0, max_len = 0, cigar_cap = 0;
   uint32_t* d_cigar = nullptr;
   bool thread_path = false, long_used = false;
+  bool direct = false;  // the reads the colinear kernels listed went straight to the warp kernels
   uint64_t launches = 0;  // kernels the enqueue issued (counted again at each graph replay)
 };
 
@@ -138,6 +139,7 @@ struct dnaln_ctx {
   std::map<int32_t, IndexRes> idx;
   int32_t next_id = 1;
   std::map<std::string, DevBuf> bufs;
+  int64_t* d_ctl = nullptr;    // kCtlWords counters; the next two point into it
   uint32_t* d_err = nullptr;   // kernel error flags
   int* d_count = nullptr;      // [0] score tasks, [1] traceback tasks, [2] reads listed for the warp path
   int64_t* h_info = nullptr;   // pinned read-back slots
@@ -377,44 +379,14 @@ int chain_lut_dev(dnaln_ctx* c, int k, int band, const int32_t** out) {
   return DNALN_OK;
 }
 
-__global__ void k_len64(const int32_t* __restrict__ len, int64_t n, int64_t* __restrict__ out,
-                        unsigned long long* __restrict__ max_len) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  int32_t l = 0;
-  if (i < n) {
-    l = len[i] < 0 ? 0 : len[i];
-    out[i] = l;
-  } else if (i == n) {
-    out[n] = 0;
-  }
-  l = __reduce_max_sync(0xffffffffu, l);  // one atomic per warp instead of one per read
-  if ((threadIdx.x & 31) == 0 && l > 0) atomicMax(max_len, static_cast<unsigned long long>(l));
-}
-
-__global__ void k_list_sum64(const int64_t* __restrict__ vals, const int32_t* __restrict__ list,
-                             const int* __restrict__ list_n, unsigned long long* __restrict__ out) {
-  const int m = *list_n;
-  long long acc = 0;
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x) acc += vals[list[x]];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, static_cast<unsigned long long>(acc));
-}
-
-// *out += sum of vals[list[x]] for x < *list_n (minimizers of the reads listed for the
-// warp path): a warp sum, then one atomic per warp.
-__global__ void k_list_sum(const int32_t* __restrict__ vals, const int32_t* __restrict__ list,
-                           const int* __restrict__ list_n, unsigned long long* __restrict__ out) {
-  const int m = *list_n;
-  long long acc = 0;
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x) acc += vals[list[x]];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, static_cast<unsigned long long>(acc));
-}
-
-__global__ void k_cig_slots(const int64_t* __restrict__ pofs, int64_t n, int64_t* __restrict__ out) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = 2 * pofs[i] + i;
-}
+// The words a batch's kernels count into (dnaln_ctx::d_ctl), cleared by one memset and read
+// back by one copy.
+constexpr int kCtlOps = 0;      // CIGAR operations written
+constexpr int kCtlInfo = 1;     // 11 words, see map_enqueue
+constexpr int kCtlCount = 12;   // d_count: 4 ints
+constexpr int kCtlClaims = 14;  // 6 ints, see map_enqueue
+constexpr int kCtlErr = 17;     // d_err
+constexpr int kCtlWords = 18;
 
 inline unsigned nblk(int64_t n, int t = 256) { return static_cast<unsigned>((n + t - 1) / t); }
 
@@ -436,6 +408,10 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
                       uint32_t* cig, const int64_t* cig_off, bool by_length) {
   if (n_max <= 0) return DNALN_OK;
   const bool ungapped = c->ungapped && sw_ungapped_supported(sp, bytes_ok);
+  // a list that fills no more than a warp per scheduler takes as long as its longest task
+  // in any order
+  if (sw_has_form(sp.W, bytes_ok, kSwIntraFew) && n_max <= int64_t{4} * device_sm_count() * 256 / (sp.W - 1))
+    by_length = false;
   if (ungapped || (by_length && n_max > 1)) {
     // [0] listed tasks, then the length bins' counts and the places taken of each
     const KernelTrace kt = tracer(c);
@@ -618,26 +594,22 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   const int bw = p.sc.bw, W = 2 * bw + 1, MC = p.max_cand;
   const int chain_band = p.ch.band < bw ? p.ch.band : bw;  // src/mapper.cpp:9
 
-  // packed offsets, total bases, longest read
-  DBUF(len64, int64_t, "len64", n + 1);
-  DBUF(pofs, int64_t, "pofs", n + 1);
   // info: [0] longest read, [1..3] cells, mapped, candidates (map.cuh), [4] minimizers,
   // [5] anchors of the thread path
   // [6] minimizers, [7] bases and [9] anchors of the reads left for the warp path, [8] the
   // chaining pool's fill, [10] long reads the colinear kernel finished
-  DBUF(info, unsigned long long, "info", 11);
-  CK(cudaMemsetAsync(info, 0, 11 * sizeof(unsigned long long), st));
-  CK(cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), st));
-  CK(cudaMemsetAsync(c->d_count, 0, 4 * sizeof(int), st));
+  unsigned long long* info = reinterpret_cast<unsigned long long*>(c->d_ctl + kCtlInfo);
   // [0] reads the colinear kernels listed, [1] work-stealing claims of the warp chaining kernel,
   // [2] reads it listed for their anchor count, [3] claims of those, [4] reads with an N
-  DBUF(claims, int, "claims", 5);
-  CK(cudaMemsetAsync(claims, 0, 5 * sizeof(int), st));
+  int* claims = reinterpret_cast<int*>(c->d_ctl + kCtlClaims);
+  CK(cudaMemsetAsync(c->d_ctl, 0, kCtlWords * sizeof(int64_t), st));
   unsigned long long* ctr = info + 1;  // cells, mapped, candidates (map.cuh)
-  kt.begin(st, "k_len64");
-  k_len64<<<nblk(n + 1), 256, 0, st>>>(d_seq_len, n, len64, info);
+  // packed offsets, total bases, longest read
+  DBUF(pofs, int64_t, "pofs", n + 1);
+  DBUF(len_sums, long long, "len_sums", len_sum_words(n));
+  kt.begin(st, "k_len_scan");
+  c->stats.launches += static_cast<uint64_t>(launch_read_offsets(st, d_seq_len, n, len_sums, pofs, info));
   kt.end(st);
-  if (int e = exclusive_scan(c, len64, pofs, n + 1)) return e;
   int64_t B = hint.bases, max_len = hint.max_len;
   if (B < 0 || max_len < 0) {
     if (c->capturing) return fail(c, DNALN_ERR_CUDA, "capture needs the batch's size");
@@ -681,6 +653,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       c->length_order && static_cast<double>(max_len) > 1.25 * static_cast<double>(B) / static_cast<double>(n);
   // the reads left for the warp kernels: those the thread kernels listed
   int32_t* warp_list = big_list;
+  run.direct = false;
   int* warp_n = big_n;
   CK(cudaEventRecord(c->ev[kEvSeed0], st));
   if (thread_path) {
@@ -694,16 +667,19 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
     // reads whose anchors form one colinear chain; the others are listed for the full kernels
     const int32_t* full_list = nullptr;
     const int* full_n = nullptr;
+    int32_t* rest_list = nullptr;
     if (c->colinear && seed_colinear_supported(sp, cp, ix.dev)) {
       DBUF(rest, int32_t, "colinear_rest", n);
       DBUF(with_n, int32_t, "colinear_with_n", n);
+      const int lanes = seed_colinear_lanes(n, max_len);
+      // in length order a warp's lanes end together; several lanes a read are taken where all
+      // reads are resident at once, and the order only costs its two launches
       const int32_t* order = nullptr;
-      if (by_length && n > 1) {
+      if (by_length && lanes == 1) {
         DBUF(ord, int32_t, "read_order", n);
         if (int e = order_reads(c, d_seq_len, nullptr, nullptr, n, max_len, ord)) return e;
         order = ord;
       }
-      const int lanes = seed_colinear_lanes(n, max_len);
       DBUF(sk_counts, int32_t, "sketch_counts", n * lanes);
       kt.begin(st, "k_sketch_reads");
       launch_sketch_reads(st, codes, pofs, d_seq_len, order, n, lanes, sp, mb.hash, sk_counts);
@@ -717,64 +693,71 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
                        mb, n_min, n_anchor, c->d_err);
       kt.end(st);
       c->stats.launches += 2;
-      full_list = rest;
+      full_list = rest_list = rest;
       full_n = claims;
     }
-    const auto seed_t = [&](int rpb) {
-      return launch_seed_chain_thread(st, codes, pofs, d_seq_len, full_list, full_n, n, ix.dev, sp, cp, cand, cb,
-                                      n_min, n_anchor, n_anc_t, big_list, big_n, c->d_err, rpb);
-    };
-    int rpb = c->seed_block ? c->seed_block : (c->seed_tune.tuned ? c->seed_tune.reads_per_block : 0);
-    if (rpb == 0 && (n < kSeedTuneReads || c->capturing)) rpb = 128;  // too small to time, or no host waits now
-    if (rpb == 0) {
-      // the reads-per-block tuner: each block size once untimed (a kernel's first launch
-      // also loads it), then each timed; every run rewrites the same outputs (the list of
-      // reads handed on is cleared before each), so the last run's stand
-      const int sizes[2] = {64, 128};
-      for (int x = 0; x < 2; ++x) {
-        CK(cudaMemsetAsync(big_n, 0, sizeof(int), st));
-        if (!seed_t(sizes[x])) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
-      }
-      for (int x = 0; x < 2; ++x) {
-        CK(cudaMemsetAsync(big_n, 0, sizeof(int), st));
-        CK(cudaEventRecord(c->tune_ev[x], st));
-        if (!seed_t(sizes[x])) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
-        CK(cudaEventRecord(c->tune_ev[x + 2], st));
-      }
-      CK(cudaEventSynchronize(c->tune_ev[3]));
-      dnaln_seed_tuning& t = c->seed_tune;
-      t.ms_64 = ev_ms(c->tune_ev[0], c->tune_ev[2]);
-      t.ms_128 = ev_ms(c->tune_ev[1], c->tune_ev[3]);
-      t.reads_per_block = t.ms_64 < t.ms_128 ? 64 : 128;
-      t.reads = n;
-      t.tuned = 1;
-      c->stats.launches += 3;
+    if (full_list && n <= kSeedFewReads) {
+      // the thread kernels would hand the whole list on
+      warp_list = rest_list;
+      warp_n = claims;
+      run.direct = true;
     } else {
-      kt.begin(st, "k_seed_chain_t");
-      const bool ok = seed_t(rpb);
-      kt.end(st);
-      if (!ok) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
-    }
-    if (c->long_thread && seed_long_supported(sp, cp) && max_len > seed_thread_max_len()) {
-      // long reads one thread each, in length order; what exceeds its bounds goes on
-      const int64_t lt = seed_long_threads(n);
-      DBUF(lscr, uint32_t, "long_scratch", seed_long_scratch_words(lt));
-      DBUF(big2, int32_t, "big2_list", n);
-      const int32_t* order = big_list;
-      if (by_length && n > 1) {
-        DBUF(ord, int32_t, "long_order", n);
-        if (int e = order_reads(c, d_seq_len, big_list, big_n, n, max_len, ord)) return e;
-        order = ord;
+      const auto seed_t = [&](int rpb) {
+        return launch_seed_chain_thread(st, codes, pofs, d_seq_len, full_list, full_n, n, ix.dev, sp, cp, cand, cb,
+                                        n_min, n_anchor, n_anc_t, big_list, big_n, c->d_err, rpb);
+      };
+      int rpb = c->seed_block ? c->seed_block : (c->seed_tune.tuned ? c->seed_tune.reads_per_block : 0);
+      if (rpb == 0 && (n < kSeedTuneReads || c->capturing)) rpb = 128;  // too small to time, or no host waits now
+      if (rpb == 0) {
+        // the reads-per-block tuner: each block size once untimed (a kernel's first launch
+        // also loads it), then each timed; every run rewrites the same outputs (the list of
+        // reads handed on is cleared before each), so the last run's stand
+        const int sizes[2] = {64, 128};
+        for (int x = 0; x < 2; ++x) {
+          CK(cudaMemsetAsync(big_n, 0, sizeof(int), st));
+          if (!seed_t(sizes[x])) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
+        }
+        for (int x = 0; x < 2; ++x) {
+          CK(cudaMemsetAsync(big_n, 0, sizeof(int), st));
+          CK(cudaEventRecord(c->tune_ev[x], st));
+          if (!seed_t(sizes[x])) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
+          CK(cudaEventRecord(c->tune_ev[x + 2], st));
+        }
+        CK(cudaEventSynchronize(c->tune_ev[3]));
+        dnaln_seed_tuning& t = c->seed_tune;
+        t.ms_64 = ev_ms(c->tune_ev[0], c->tune_ev[2]);
+        t.ms_128 = ev_ms(c->tune_ev[1], c->tune_ev[3]);
+        t.reads_per_block = t.ms_64 < t.ms_128 ? 64 : 128;
+        t.reads = n;
+        t.tuned = 1;
+        c->stats.launches += 3;
+      } else {
+        kt.begin(st, "k_seed_chain_t");
+        const bool ok = seed_t(rpb);
+        kt.end(st);
+        if (!ok) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
       }
-      kt.begin(st, "k_seed_chain_tl");
-      if (!launch_seed_chain_long(st, d_seq_len, pofs, codes, order, big_n, lt, ix.dev, sp, cp, cand, cb, n_min,
-                                  n_anchor, n_anc_t, lscr, big2, c->d_count + 3, seed_thread_max_len(),
-                                  full_list != nullptr, c->d_err))
-        return fail(c, DNALN_ERR_CUDA, "long-read seeding kernel could not be configured");
-      kt.end(st);
-      warp_list = big2;
-      warp_n = c->d_count + 3;
-      c->stats.launches += 1;
+      if (c->long_thread && seed_long_supported(sp, cp) && max_len > seed_thread_max_len()) {
+        // long reads one thread each, in length order; what exceeds its bounds goes on
+        const int64_t lt = seed_long_threads(n);
+        DBUF(lscr, uint32_t, "long_scratch", seed_long_scratch_words(lt));
+        DBUF(big2, int32_t, "big2_list", n);
+        const int32_t* order = big_list;
+        if (by_length && n > 1) {
+          DBUF(ord, int32_t, "long_order", n);
+          if (int e = order_reads(c, d_seq_len, big_list, big_n, n, max_len, ord)) return e;
+          order = ord;
+        }
+        kt.begin(st, "k_seed_chain_tl");
+        if (!launch_seed_chain_long(st, d_seq_len, pofs, codes, order, big_n, lt, ix.dev, sp, cp, cand, cb, n_min,
+                                    n_anchor, n_anc_t, lscr, big2, c->d_count + 3, seed_thread_max_len(),
+                                    full_list != nullptr, c->d_err))
+          return fail(c, DNALN_ERR_CUDA, "long-read seeding kernel could not be configured");
+        kt.end(st);
+        warp_list = big2;
+        warp_n = c->d_count + 3;
+        c->stats.launches += 1;
+      }
     }
     if (!full_list) {
       kt.begin(st, "k_seed<list>");
@@ -790,28 +773,6 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   }
   CK(cudaEventRecord(c->ev[kEvSeed1], st));
   CK(cudaGetLastError());
-  {  // minimizer and anchor totals (MapStats-style counters), read back with the results
-    size_t tmp = 0;
-    int64_t* total = reinterpret_cast<int64_t*>(info + 4);
-    CK(cub::DeviceReduce::Sum(nullptr, tmp, n_min, total, n, st));
-    DBUF(t, uint8_t, "cub_tmp_red", tmp);
-    CK(cub::DeviceReduce::Sum(t, tmp, n_min, total, n, st));
-    if (thread_path) {
-      CK(cub::DeviceReduce::Sum(t, tmp, n_anc_t, total + 1, n, st));
-      kt.begin(st, "k_list_sum");
-      const unsigned lb = nblk(std::min<int64_t>(n, int64_t{256} * device_sm_count()));
-      k_list_sum<<<lb, 256, 0, st>>>(n_min, warp_list, warp_n, info + 6);
-      k_list_sum<<<lb, 256, 0, st>>>(d_seq_len, warp_list, warp_n, info + 7);
-      k_list_sum64<<<lb, 256, 0, st>>>(n_anchor, warp_list, warp_n, info + 9);
-      kt.end(st);
-    } else {
-      size_t tmp2 = 0;
-      CK(cub::DeviceReduce::Sum(nullptr, tmp2, n_anchor, reinterpret_cast<int64_t*>(info + 9), n, st));
-      DBUF(t2, uint8_t, "cub_tmp_red2", tmp2);
-      CK(cub::DeviceReduce::Sum(t2, tmp2, n_anchor, reinterpret_cast<int64_t*>(info + 9), n, st));
-    }
-  }
-
   // pass 2 of the warp path: anchors, chains, candidates; the scratch of reads with many
   // anchors comes from a pool (sized from the previous batches; a batch that outgrows it
   // is mapped again with the size it asked for)
@@ -836,7 +797,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   kt.begin(st, thread_path ? "k_chain_map<list>" : "k_chain_map");
   launch_chain_map(st, pofs, d_seq_len, n, thread_path ? warp_list : nullptr, thread_path ? warp_n : nullptr, n_min,
                    n_anchor, mb, ix.dev, cp, cand, as, pool_top, pool_cap, cb, c->stealing ? claims + 1 : nullptr,
-                   chain_big, claims + 2, c->d_err);
+                   chain_big, claims + 2, info, c->d_err);
   kt.end(st);
   CK(cudaEventRecord(c->ev[kEvChain1], st));
   CK(cudaGetLastError());
@@ -863,12 +824,13 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   DBUF(res_tb, SwResult, "res_tb", n);
   DBUF(cig_tb, uint32_t, "cig_tb", 2 * B + n);
   DBUF(cig_slot, int64_t, "cig_slot", n);
+  DBUF(op_count, int32_t, "op_count", n);
+  DBUF(op_words, long long, "op_sums", op_sum_words(n));
+  const OpSums ops = make_op_sums(n, op_count, op_words);
   CK(cudaEventRecord(c->ev[kEvTb0], st));
   kt.begin(st, "k_choose");
-  launch_choose(st, n, pofs, d_seq_len, cb, res_sc, d_hash, ix.dev, mc, chosen, s2, tb_tasks, c->d_count + 1, ctr);
-  kt.end(st);
-  kt.begin(st, "k_cig_slots");
-  k_cig_slots<<<nblk(n), 256, 0, st>>>(pofs, n, cig_slot);
+  launch_choose(st, n, pofs, d_seq_len, cb, res_sc, d_hash, ix.dev, mc, chosen, s2, tb_tasks, c->d_count + 1,
+                cig_slot, ops, n_min, thread_path ? n_anc_t : nullptr, info + 4, ctr);
   kt.end(st);
   if (int e = launch_sw_chunked(c, true, bytes_ok, tb_tasks, static_cast<int>(n), c->d_count + 1, codes,
                                 ix.dev.genome, swp, res_tb, static_cast<int>(max_len), cig_tb, cig_slot, by_length))
@@ -876,13 +838,10 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   CK(cudaEventRecord(c->ev[kEvTb1], st));
 
   // records, CIGAR offsets and compaction
-  DBUF(cig_cnt, int64_t, "cig_cnt", n + 1);
-  DBUF(cig_off, int64_t, "cig_off", n + 1);
   CK(cudaEventRecord(c->ev[kEvPost0], st));
   kt.begin(st, "k_records");
-  launch_records(st, n, d_seq_len, cb, chosen, s2, res_tb, ix.dev, mc, d_out, cig_cnt, ctr);
+  launch_records(st, n, d_seq_len, cb, chosen, s2, res_tb, ix.dev, mc, d_out, ops, ctr);
   kt.end(st);
-  if (int e = exclusive_scan(c, cig_cnt, cig_off, n + 1)) return e;
   // final CIGARs: into the caller's buffer, or an internal one of the bound 2 * len + 3 per
   // read; the kernel checks the capacity itself, so nothing waits for the total here
   if (!d_cigar) {
@@ -891,24 +850,19 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
     if (!d_cigar) return DNALN_ERR_OOM;
   }
   kt.begin(st, "k_cigar_gather");
-  launch_cigar_gather(st, n, pofs, d_seq_len, res_tb, cig_tb, cig_off, hint.cigar_base, d_out, d_cigar, cigar_cap,
-                      c->d_err);
+  launch_cigar_gather(st, n, pofs, d_seq_len, res_tb, cig_tb, ops, hint.cigar_base, d_out, d_cigar, cigar_cap,
+                      reinterpret_cast<long long*>(c->d_ctl + kCtlOps), c->d_err);
   kt.end(st);
   CK(cudaEventRecord(c->ev[kEvPost1], st));
   CK(cudaGetLastError());
   // the batch's one read-back: totals, task counts, error flags, counters
-  int64_t* h = c->h_info;
-  CK(cudaMemcpyAsync(h, cig_off + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(h + 1, c->d_count, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(h + 3, c->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(h + 4, ctr, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(h + 7, info + 4, 7 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(c->h_info, c->d_ctl, kCtlWords * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   run.B = B;
   run.max_len = max_len;
   run.cigar_cap = cigar_cap;
   run.d_cigar = d_cigar;
   run.thread_path = thread_path;
-  run.long_used = warp_list != big_list;
+  run.long_used = !run.direct && warp_list != big_list;
   run.launches = c->stats.launches - launches0;
   c->stats.launches = launches0;
   return DNALN_OK;
@@ -928,15 +882,17 @@ int map_finish(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_s
   const bool thread_path = run.thread_path;
   int64_t* h = c->h_info;
   CK(cudaStreamSynchronize(st));
-  const int64_t total_ops = h[0];
+  const int64_t total_ops = h[kCtlOps];
   int counts[4];
-  std::memcpy(counts, h + 1, sizeof counts);
+  std::memcpy(counts, h + kCtlCount, sizeof counts);
   uint32_t errbits;
-  std::memcpy(&errbits, h + 3, sizeof errbits);
-  const uint64_t n_cells = static_cast<uint64_t>(h[4]), n_mapped = static_cast<uint64_t>(h[5]),
-                 n_cands = static_cast<uint64_t>(h[6]);
-  const int64_t n_minimizers = h[7], n_anchors_thread = h[8], n_minimizers_warp_l = h[9], n_bases_warp_l = h[10];
-  const int64_t pool_used = h[11], n_anchors_warp = h[12], n_long_colinear = h[13];
+  std::memcpy(&errbits, h + kCtlErr, sizeof errbits);
+  const int64_t* info = h + kCtlInfo;
+  const uint64_t n_cells = static_cast<uint64_t>(info[1]), n_mapped = static_cast<uint64_t>(info[2]),
+                 n_cands = static_cast<uint64_t>(info[3]);
+  const int64_t n_minimizers = info[4], n_anchors_thread = info[5], n_minimizers_warp_l = info[6],
+                n_bases_warp_l = info[7];
+  const int64_t pool_used = info[8], n_anchors_warp = info[9], n_long_colinear = info[10];
   if (errbits & kErrChainPool) {
     // the chaining pool was too small for this batch: grow it to what the batch asked for
     // and map the batch again (outputs are rewritten in full; counters are not yet added)
@@ -961,7 +917,9 @@ int map_finish(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_s
   trace_collect(c);
 
   const int n_listed = counts[2];                                        // reads the short thread kernel listed
-  const int n_warp = thread_path ? counts[run.long_used ? 3 : 2] : static_cast<int>(n);  // warp kernels
+  int n_rest;                                                            // reads the colinear kernels listed
+  std::memcpy(&n_rest, h + kCtlClaims, sizeof n_rest);
+  const int n_warp = !thread_path ? static_cast<int>(n) : (run.direct ? n_rest : counts[run.long_used ? 3 : 2]);
   dnaln_stats& s = c->stats;
   s.reads += static_cast<uint64_t>(n);
   s.anchors += static_cast<uint64_t>(n_anchors_thread + n_anchors_warp);
@@ -976,9 +934,9 @@ int map_finish(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_s
   s.cells += n_cells;
   s.mapped += n_mapped;
   s.candidates += n_cands;
-  // k_len64, k_score_tasks, k_choose, k_cig_slots, k_records, k_cigar_gather, pass 1 / 2,
-  // plus the SW and sorting kernels the enqueue counted
-  s.launches += 7 + (thread_path ? 5 : 1) + run.launches;
+  // k_score_tasks, k_choose, k_records, k_cigar_gather, pass 1 / 2, plus what the enqueue
+  // counted
+  s.launches += 6 + (thread_path ? 2 : 1) + run.launches;
   s.ms_seed += ev_ms(c, kEvSeed0, kEvSeed1);
   s.ms_chain += ev_ms(c, kEvChain0, kEvChain1);
   s.ms_sw_score += ev_ms(c, kEvSc0, kEvSc1);
@@ -1026,17 +984,14 @@ int run_map(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_seq_
   BatchHints hint = hint0;
   hint.caller_cigar = d_cigar != nullptr;
   if ((hint.bases < 0 || hint.max_len < 0) && c->graphs && !c->trace_on) {
-    // the batch's size first (two small kernels and one read-back), so that the rest of it
+    // the batch's size first (a small kernel and one read-back), so that the rest of it
     // can run as a graph
     cudaStream_t st = c->st;
-    DBUF(len64, int64_t, "len64", n + 1);
-    DBUF(pofs, int64_t, "pofs", n + 1);
-    DBUF(info, unsigned long long, "info", 11);
-    CK(cudaMemsetAsync(info, 0, sizeof(unsigned long long), st));
-    k_len64<<<nblk(n + 1), 256, 0, st>>>(d_seq_len, n, len64, info);
-    if (int e = exclusive_scan(c, len64, pofs, n + 1)) return e;
-    CK(cudaMemcpyAsync(c->h_info, pofs + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(c->h_info + 1, info, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    int64_t* const total = c->d_ctl + kCtlOps;  // the longest read in the next word
+    CK(cudaMemsetAsync(total, 0, 2 * sizeof(int64_t), st));
+    launch_read_totals(st, d_seq_len, n, reinterpret_cast<unsigned long long*>(total + 1),
+                       reinterpret_cast<unsigned long long*>(total));
+    CK(cudaMemcpyAsync(c->h_info, total, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     hint.bases = c->h_info[0];
     hint.max_len = c->h_info[1];
@@ -1406,9 +1361,10 @@ int dnaln_gpu_ctx_create(int device, dnaln_ctx** out) {
   for (auto& x : c->out_free) bad(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
   for (auto& x : c->h2d_ev) bad(cudaEventCreate(&x));
   for (auto& x : c->d2h_ev) bad(cudaEventCreate(&x));
-  bad(cudaMalloc(&c->d_err, sizeof(uint32_t)));
-  bad(cudaMalloc(&c->d_count, 4 * sizeof(int)));
-  bad(cudaHostAlloc(&c->h_info, 16 * sizeof(int64_t), cudaHostAllocDefault));
+  bad(cudaMalloc(&c->d_ctl, kCtlWords * sizeof(int64_t)));
+  c->d_err = reinterpret_cast<uint32_t*>(c->d_ctl + kCtlErr);
+  c->d_count = reinterpret_cast<int*>(c->d_ctl + kCtlCount);
+  bad(cudaHostAlloc(&c->h_info, 24 * sizeof(int64_t), cudaHostAllocDefault));
   bad(cudaHostAlloc(&c->h_tune, sizeof(int), cudaHostAllocDefault));
   for (auto& x : c->tune_ev) bad(cudaEventCreate(&x));
   if (e != DNALN_OK) {
@@ -1448,8 +1404,7 @@ int dnaln_gpu_ctx_destroy(dnaln_ctx* c) {
     if (x) cudaEventDestroy(x);
   if (c->cp_in) cudaStreamDestroy(c->cp_in);
   if (c->cp_out) cudaStreamDestroy(c->cp_out);
-  if (c->d_err) cudaFree(c->d_err);
-  if (c->d_count) cudaFree(c->d_count);
+  if (c->d_ctl) cudaFree(c->d_ctl);
   if (c->h_info) cudaFreeHost(c->h_info);
   if (c->h_tune) cudaFreeHost(c->h_tune);
   for (auto& x : c->tune_ev)

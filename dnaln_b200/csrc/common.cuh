@@ -169,6 +169,35 @@ __device__ __forceinline__ int warp_exclusive_scan(int v, int* total) {
   return x - v;
 }
 
+__device__ __forceinline__ long long warp_exclusive_scan_ll(long long v, long long* total) {
+  const int lane = threadIdx.x & 31;
+  long long x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  *total = __shfl_sync(0xffffffffu, x, 31);
+  return x - v;
+}
+
+// Exclusive prefix sums over the block (a whole number of warps, at most 32); *total = the
+// block's sum. warp_total: 32 entries of shared memory, free again after the next barrier.
+__device__ __forceinline__ long long block_exclusive_scan_ll(long long v, long long* total, long long* warp_total) {
+  long long sum;
+  long long ex = warp_exclusive_scan_ll(v, &sum);
+  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if ((threadIdx.x & 31) == 0) warp_total[w] = sum;
+  __syncthreads();
+  long long all = 0;
+  for (int x = 0; x < nw; ++x) {
+    if (x < w) ex += warp_total[x];
+    all += warp_total[x];
+  }
+  *total = all;
+  return ex;
+}
+
 // Length order by counting: bins of 2^bin_shift lengths, bin 0 the longest.
 constexpr int kLengthBins = 1024;
 __host__ __device__ __forceinline__ int length_bin(int len, int bin_shift) {

@@ -10,6 +10,140 @@ namespace dnb {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / 32;
+
+// The block's sum of each of N values is added to ctr[k] by one atomic each; *last (may be
+// null) = the block's sum of the last value. 262,144 reads made 24,600 atomics on three words
+// warp by warp; now k_choose also sums the seeds and fills the CIGAR slots and k_records sums
+// the operations, which took nine launches more: k_choose 23 -> 21 us, and a batch of 64 reads
+// 269 -> 253 us, of 262,144 972 -> 876 us, with the other launches saved.
+template <int N>
+__device__ __forceinline__ void block_add(const unsigned long long (&v)[N], unsigned long long* const (&ctr)[N],
+                                          long long* last = nullptr) {
+  __shared__ unsigned long long part[N][kWarps];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const unsigned long long x = warp_sum(v[k]);
+    if ((threadIdx.x & 31) == 0) part[k][threadIdx.x >> 5] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < N) {
+    unsigned long long x = 0;
+    for (int w = 0; w < kWarps; ++w) x += part[threadIdx.x][w];
+    if (x) atomicAdd(ctr[threadIdx.x], x);
+    if (last && threadIdx.x == N - 1) *last = static_cast<long long>(x);
+  }
+}
+
+// First of the `want` entries this thread gets after *counter, one atomic per block.
+__device__ __forceinline__ int block_reserve(int want, int* counter) {
+  __shared__ int part[kWarps + 1];
+  int total;
+  const int ex = warp_exclusive_scan(want, &total);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = total;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int all = 0;
+    for (int w = 0; w < kWarps; ++w) {
+      const int x = part[w];
+      part[w] = all;
+      all += x;
+    }
+    part[kWarps] = all ? atomicAdd(counter, all) : 0;
+  }
+  __syncthreads();
+  return part[kWarps] + part[threadIdx.x >> 5] + ex;
+}
+
+// ---- packed offsets of the reads: exclusive sums of their lengths --------------------------
+// Blocks of per_block reads (a multiple of kLenTile): k_len_sums leaves each block's sum,
+// k_len_scan adds up those before its own and scans its reads. One block needs no sums.
+constexpr int kLenTile = 4 * kThreads;
+constexpr int64_t kLenBlocks = 2048;   // at most
+constexpr int64_t kLenSingle = 4 * kLenTile;  // reads one block takes
+
+int64_t len_per_block(int64_t n) {
+  if (n <= kLenSingle) return kLenSingle;
+  const int64_t tiles = (n + kLenTile - 1) / kLenTile;
+  return (tiles + kLenBlocks - 1) / kLenBlocks * kLenTile;
+}
+
+__global__ void __launch_bounds__(kThreads)
+    k_len_sums(const int32_t* __restrict__ len, int64_t n, int64_t per_block, long long* __restrict__ sums,
+               unsigned long long* __restrict__ max_len, unsigned long long* __restrict__ total) {
+  const int64_t lo = blockIdx.x * per_block, hi = lo + per_block < n ? lo + per_block : n;
+  unsigned long long sum = 0;
+  int most = 0;
+  for (int64_t i = lo + threadIdx.x; i < hi; i += kThreads) {
+    const int l = len[i] < 0 ? 0 : len[i];
+    sum += static_cast<unsigned>(l);
+    most = max(most, l);
+  }
+  __shared__ unsigned long long part[kWarps];
+  __shared__ int part_max[kWarps];
+  sum = warp_sum(sum);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0) {
+    part[threadIdx.x >> 5] = sum;
+    part_max[threadIdx.x >> 5] = most;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kWarps; ++w) {
+      sum += part[w];
+      most = max(most, part_max[w]);
+    }
+    if (sums) sums[blockIdx.x] = static_cast<long long>(sum);
+    if (most > 0) atomicMax(max_len, static_cast<unsigned long long>(most));
+    if (total && sum) atomicAdd(total, sum);
+  }
+}
+
+__global__ void __launch_bounds__(kThreads)
+    k_len_scan(const int32_t* __restrict__ len, int64_t n, int64_t per_block, const long long* __restrict__ sums,
+               int64_t* __restrict__ pofs, unsigned long long* __restrict__ max_len) {
+  __shared__ long long part[2][32];
+  long long base = 0;
+  if (blockIdx.x > 0) {
+    long long acc = 0;
+    for (int x = threadIdx.x; x < static_cast<int>(blockIdx.x); x += kThreads) acc += sums[x];
+    block_exclusive_scan_ll(acc, &base, part[0]);
+    __syncthreads();
+  }
+  const int64_t lo = blockIdx.x * per_block, hi = lo + per_block < n ? lo + per_block : n;
+  int most = 0, flip = 0;
+  for (int64_t t = lo; t < hi; t += kLenTile, flip ^= 1) {
+    const int64_t i = t + 4 * threadIdx.x;
+    int l[4];
+    long long sum = 0, total;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      l[k] = i + k < hi ? max(len[i + k], 0) : 0;
+      sum += l[k];
+      most = max(most, l[k]);
+    }
+    long long at = base + block_exclusive_scan_ll(sum, &total, part[flip]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i + k < hi) pofs[i + k] = at;
+      at += l[k];
+    }
+    base += total;
+  }
+  if (hi == n && threadIdx.x == 0) pofs[n] = base;
+  if (!sums) {  // the only block
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(max_len, static_cast<unsigned long long>(most));
+  }
+}
+
+// CIGAR operations before a read's: k_records leaves the sum of each block of kThreads reads
+// and of each kOpGroup blocks, k_cigar_gather adds up those before its own.
+constexpr int kOpGroup = 64;
+__host__ __device__ __forceinline__ int64_t op_blocks_for(int64_t n) { return (n + kThreads - 1) / kThreads; }
+__host__ __device__ __forceinline__ int64_t op_groups_for(int64_t n) {
+  return (op_blocks_for(n) + kOpGroup - 1) / kOpGroup;
+}
 
 // SW task of candidate c of read r: query = forward or reverse-complement codes, target
 // window = genome[wstart, wstart + len + 2bw) with N outside the candidate's contig
@@ -41,29 +175,25 @@ __global__ void k_score_tasks(int64_t n, const int64_t* __restrict__ pofs, const
   const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int nc = r < n ? cb.n_cand[r] : 0;
   const int want = nc >= 2 ? nc : 0;
-  // warp-aggregated slot reservation
-  const unsigned lane = threadIdx.x & 31;
-  int total;
-  const int ex = warp_exclusive_scan(want, &total);
-  int base = 0;
-  if (lane == 0 && total) base = atomicAdd(counter, total);
-  base = __shfl_sync(0xffffffffu, base, 0);
+  const int first = block_reserve(want, counter);
   for (int c = 0; c < want; ++c) {
     SwTask t = cand_task(r, c, pofs, seq_len, cb, ix, mc);
     t.slot = static_cast<int32_t>(r * mc.max_cand + c);
-    tasks[base + ex + c] = t;
+    tasks[first + c] = t;
   }
   // cells of the ranking pass, counted as the reference's MapStats::cells (src/mapper.cpp:139)
-  unsigned long long cells = want ? static_cast<unsigned long long>(want) * seq_len[r] * mc.W : 0ull;
-  cells = warp_sum(cells);
-  if (lane == 0 && cells) atomicAdd(ctr, cells);
+  const unsigned long long cells[1] = {want ? static_cast<unsigned long long>(want) * seq_len[r] * mc.W : 0ull};
+  unsigned long long* const to[1] = {ctr};
+  block_add(cells, to);
 }
 
 __global__ void k_choose(int64_t n, const int64_t* __restrict__ pofs, const int32_t* __restrict__ seq_len, CandBuf cb,
                          const SwResult* __restrict__ res_score, const uint32_t* __restrict__ name_hash, DevIndex ix,
                          MapConsts mc, int32_t* __restrict__ chosen, int32_t* __restrict__ s2o,
                          SwTask* __restrict__ tb_tasks, int* __restrict__ tb_counter,
-                         unsigned long long* __restrict__ ctr) {
+                         int64_t* __restrict__ cig_slot, long long* __restrict__ op_groups,
+                         const int32_t* __restrict__ n_min, const int32_t* __restrict__ n_anc,
+                         unsigned long long* __restrict__ seeds, unsigned long long* __restrict__ ctr) {
   const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   int pick_c = -1, s2 = 0, nc = 0;
   if (r < n) {
@@ -97,42 +227,34 @@ __global__ void k_choose(int64_t n, const int64_t* __restrict__ pofs, const int3
     }
     chosen[r] = pick_c;
     s2o[r] = s2;
+    cig_slot[r] = 2 * pofs[r] + r;
+    if (r < op_groups_for(n)) op_groups[r] = 0;
   }
-  const unsigned lane = threadIdx.x & 31;
-  const unsigned ball = __ballot_sync(0xffffffffu, pick_c >= 0);
-  int base = 0;
-  if (lane == 0 && ball) base = atomicAdd(tb_counter, __popc(ball));
-  base = __shfl_sync(0xffffffffu, base, 0);
+  const int at = block_reserve(pick_c >= 0 ? 1 : 0, tb_counter);
   if (pick_c >= 0) {
     SwTask t = cand_task(r, pick_c, pofs, seq_len, cb, ix, mc);
     t.slot = static_cast<int32_t>(r);
-    tb_tasks[base + __popc(ball & ((1u << lane) - 1u))] = t;
+    tb_tasks[at] = t;
   }
-  // traceback cells (src/mapper.cpp:186) and candidate count
-  unsigned long long cells = pick_c >= 0 ? static_cast<unsigned long long>(seq_len[r]) * mc.W : 0ull;
-  unsigned long long cands = static_cast<unsigned long long>(nc);
-  cells = warp_sum(cells);
-  cands = warp_sum(cands);
-  if (lane == 0) {
-    if (cells) atomicAdd(ctr, cells);
-    if (cands) atomicAdd(ctr + 2, cands);
-  }
+  // traceback cells (src/mapper.cpp:186), candidates, and the seeding's totals
+  const unsigned long long sums[4] = {
+      pick_c >= 0 ? static_cast<unsigned long long>(seq_len[r]) * mc.W : 0ull, static_cast<unsigned long long>(nc),
+      r < n ? static_cast<unsigned long long>(n_min[r]) : 0ull,
+      r < n && n_anc ? static_cast<unsigned long long>(n_anc[r]) : 0ull};
+  unsigned long long* const to[4] = {ctr, ctr + 2, seeds, seeds + 1};
+  block_add(sums, to);
 }
 
 __global__ void k_records(int64_t n, const int32_t* __restrict__ seq_len, CandBuf cb,
                           const int32_t* __restrict__ chosen, const int32_t* __restrict__ s2o,
                           const SwResult* __restrict__ res_tb, DevIndex ix, MapConsts mc,
-                          dnaln_map_record* __restrict__ out, int64_t* __restrict__ cig_count,
+                          dnaln_map_record* __restrict__ out, int32_t* __restrict__ op_count,
+                          long long* __restrict__ op_sums, long long* __restrict__ op_groups,
                           unsigned long long* __restrict__ ctr) {
   const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const unsigned ball = __ballot_sync(0xffffffffu, r < n && chosen[r < n ? r : 0] >= 0 &&
-                                                       res_tb[r < n ? r : 0].score >= mc.min_aln_score);
-  if ((threadIdx.x & 31) == 0 && ball) atomicAdd(ctr + 1, static_cast<unsigned long long>(__popc(ball)));
-  if (r > n) return;
-  if (r == n) {  // trailing element of the scan input
-    cig_count[n] = 0;
-    return;
-  }
+  int32_t ops = 0;
+  bool mapped = false;
+  if (r < n) {
   dnaln_map_record m;
   m.pos = 0;
   m.cigar_off = 0;
@@ -144,7 +266,6 @@ __global__ void k_records(int64_t n, const int32_t* __restrict__ seq_len, CandBu
   m.rev = 0;
   m.mapq = 0;
   m.pad_[0] = m.pad_[1] = 0;
-  int64_t ops = 0;
   const int c = chosen[r];
   if (c >= 0) {
     const SwResult a = res_tb[r];
@@ -167,19 +288,35 @@ __global__ void k_records(int64_t n, const int32_t* __restrict__ seq_len, CandBu
         m.mapq = static_cast<uint8_t>(static_cast<int>(q < 60.0 ? q : 60.0));
       }
       ops = (a.qb > 0 ? 1 : 0) + a.n_ops + (seq_len[r] > a.qe ? 1 : 0);
+      mapped = true;
     }
   }
   out[r] = m;
-  cig_count[r] = ops;
+  op_count[r] = ops;
+  }
+  const unsigned long long sums[2] = {mapped ? 1ull : 0ull, static_cast<unsigned long long>(ops)};
+  long long* const group = op_groups + blockIdx.x / kOpGroup;
+  unsigned long long* const to[2] = {ctr + 1, reinterpret_cast<unsigned long long*>(group)};
+  block_add(sums, to, op_sums + blockIdx.x);
 }
 
 __global__ void k_cigar_gather(int64_t n, const int64_t* __restrict__ pofs, const int32_t* __restrict__ seq_len,
                                const SwResult* __restrict__ res_tb, const uint32_t* __restrict__ cig_src,
-                               const int64_t* __restrict__ dst_off, int64_t rec_base, dnaln_map_record* __restrict__ out,
-                               uint32_t* __restrict__ dst, int64_t cap, uint32_t* __restrict__ err) {
+                               const int32_t* __restrict__ op_count, const long long* __restrict__ op_sums,
+                               const long long* __restrict__ op_groups, int64_t rec_base,
+                               dnaln_map_record* __restrict__ out, uint32_t* __restrict__ dst, int64_t cap,
+                               long long* __restrict__ total_ops, uint32_t* __restrict__ err) {
+  __shared__ long long part[2][32];
   const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int b = blockIdx.x, g = b / kOpGroup;
+  long long before = 0, base, block_ops;
+  for (int x = threadIdx.x; x < g; x += kThreads) before += op_groups[x];
+  if (static_cast<int>(threadIdx.x) < b % kOpGroup) before += op_sums[g * kOpGroup + threadIdx.x];
+  block_exclusive_scan_ll(before, &base, part[0]);
+  const int64_t cnt = r < n ? op_count[r] : 0;
+  const int64_t o = base + block_exclusive_scan_ll(cnt, &block_ops, part[1]);
+  if (threadIdx.x == 0 && blockIdx.x + 1 == gridDim.x) *total_ops = base + block_ops;
   if (r >= n) return;
-  const int64_t o = dst_off[r], cnt = dst_off[r + 1] - o;
   out[r].cigar_off = rec_base + o;
   out[r].cigar_len = static_cast<int32_t>(cnt);
   if (cnt == 0) return;
@@ -263,24 +400,47 @@ void launch_score_tasks(cudaStream_t st, int64_t n, const int64_t* pofs, const i
 
 void launch_choose(cudaStream_t st, int64_t n, const int64_t* pofs, const int32_t* seq_len, CandBuf cb,
                    const SwResult* res_score, const uint32_t* name_hash, const DevIndex& ix, const MapConsts& mc,
-                   int32_t* chosen, int32_t* s2, SwTask* tb_tasks, int* tb_counter, unsigned long long* ctr) {
+                   int32_t* chosen, int32_t* s2, SwTask* tb_tasks, int* tb_counter, int64_t* cig_slot, OpSums ops,
+                   const int32_t* n_min, const int32_t* n_anc, unsigned long long* seeds, unsigned long long* ctr) {
   if (n > 0)
     k_choose<<<blocks_for(n), kThreads, 0, st>>>(n, pofs, seq_len, cb, res_score, name_hash, ix, mc, chosen, s2,
-                                                 tb_tasks, tb_counter, ctr);
+                                                 tb_tasks, tb_counter, cig_slot, ops.groups, n_min, n_anc, seeds, ctr);
 }
 
 void launch_records(cudaStream_t st, int64_t n, const int32_t* seq_len, CandBuf cb, const int32_t* chosen,
                     const int32_t* s2, const SwResult* res_tb, const DevIndex& ix, const MapConsts& mc,
-                    dnaln_map_record* out, int64_t* cig_count, unsigned long long* ctr) {
-  k_records<<<blocks_for(n + 1), kThreads, 0, st>>>(n, seq_len, cb, chosen, s2, res_tb, ix, mc, out, cig_count, ctr);
+                    dnaln_map_record* out, OpSums ops, unsigned long long* ctr) {
+  k_records<<<blocks_for(n), kThreads, 0, st>>>(n, seq_len, cb, chosen, s2, res_tb, ix, mc, out, ops.count, ops.sums,
+                                                ops.groups, ctr);
 }
 
 void launch_cigar_gather(cudaStream_t st, int64_t n, const int64_t* pofs, const int32_t* seq_len,
-                         const SwResult* res_tb, const uint32_t* cig_src, const int64_t* dst_off, int64_t rec_base,
-                         dnaln_map_record* out, uint32_t* dst, int64_t cap, uint32_t* err) {
+                         const SwResult* res_tb, const uint32_t* cig_src, OpSums ops, int64_t rec_base,
+                         dnaln_map_record* out, uint32_t* dst, int64_t cap, long long* total_ops, uint32_t* err) {
   if (n <= 0) return;
-  k_cigar_gather<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(n, pofs, seq_len, res_tb, cig_src, dst_off,
-                                                                         rec_base, out, dst, cap, err);
+  k_cigar_gather<<<blocks_for(n), kThreads, 0, st>>>(n, pofs, seq_len, res_tb, cig_src, ops.count, ops.sums,
+                                                     ops.groups, rec_base, out, dst, cap, total_ops, err);
+}
+
+int64_t op_sum_words(int64_t n) { return op_blocks_for(n) + op_groups_for(n); }
+
+OpSums make_op_sums(int64_t n, int32_t* count, long long* words) { return {count, words, words + op_blocks_for(n)}; }
+
+int64_t len_sum_words(int64_t n) { return (n + len_per_block(n) - 1) / len_per_block(n); }
+
+int launch_read_offsets(cudaStream_t st, const int32_t* len, int64_t n, long long* sums, int64_t* pofs,
+                        unsigned long long* max_len) {
+  const int64_t per = len_per_block(n);
+  const unsigned blocks = static_cast<unsigned>((n + per - 1) / per);
+  if (blocks > 1) k_len_sums<<<blocks, kThreads, 0, st>>>(len, n, per, sums, max_len, nullptr);
+  k_len_scan<<<blocks, kThreads, 0, st>>>(len, n, per, blocks > 1 ? sums : nullptr, pofs, max_len);
+  return blocks > 1 ? 2 : 1;
+}
+
+void launch_read_totals(cudaStream_t st, const int32_t* len, int64_t n, unsigned long long* max_len,
+                        unsigned long long* total) {
+  const int64_t per = (len_per_block(n) + 3) / 4;
+  k_len_sums<<<static_cast<unsigned>((n + per - 1) / per), kThreads, 0, st>>>(len, n, per, nullptr, max_len, total);
 }
 
 void launch_align_tasks(cudaStream_t st, int64_t n, const int64_t* off, const int32_t* len, int W, SwTask* tasks,

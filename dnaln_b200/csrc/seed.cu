@@ -1021,25 +1021,32 @@ __global__ void __launch_bounds__(kChainWarps * 32, 8)
                 const int64_t* __restrict__ n_anchor, MinBuf mb, DevIndex ix, ChainParamsDev cp, CandParams cand,
                 AnchorScratch as, unsigned long long* __restrict__ pool_top, int64_t pool_cap, CandBuf cb,
                 int* __restrict__ claim, int32_t* __restrict__ big, int* __restrict__ big_n,
-                uint32_t* __restrict__ err) {
+                unsigned long long* __restrict__ info, uint32_t* __restrict__ err) {
   __shared__ ChainSmem<kSmCap> sm[kChainWarps];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t gw = static_cast<int64_t>(blockIdx.x) * kChainWarps + wib;
   const int64_t m = list ? static_cast<int64_t>(*list_n) : n;
-  if (claim) {  // work stealing: the warp takes the next read when it is done with its last
-    for (;;) {
-      int x = 0;
-      if (lane == 0) x = atomicAdd(claim, 1);
-      x = __shfl_sync(0xffffffffu, x, 0);
-      if (x >= m) break;
-      chain_read(list ? list[x] : x, pofs, seq_len, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb,
-                 big, big_n, err, sm[wib]);
+  unsigned long long mins = 0, bases = 0, anchors = 0;  // this warp's reads
+  for (int64_t x = gw;;) {
+    if (claim) {
+      int y = 0;
+      if (lane == 0) y = atomicAdd(claim, 1);
+      x = __shfl_sync(0xffffffffu, y, 0);
     }
-    return;
+    if (x >= m) break;
+    const int64_t r = list ? list[x] : x;
+    mins += static_cast<unsigned long long>(n_min[r]);
+    bases += static_cast<unsigned long long>(seq_len[r]);
+    anchors += static_cast<unsigned long long>(n_anchor[r]);
+    chain_read(r, pofs, seq_len, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, big, big_n, err,
+               sm[wib]);
+    x += static_cast<int64_t>(gridDim.x) * kChainWarps;
   }
-  for (int64_t x = gw; x < m; x += static_cast<int64_t>(gridDim.x) * kChainWarps)
-    chain_read(list ? list[x] : x, pofs, seq_len, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, big,
-               big_n, err, sm[wib]);
+  if (lane == 0 && bases) {
+    atomicAdd(info + 6, mins);
+    atomicAdd(info + 7, bases);
+    atomicAdd(info + 9, anchors);
+  }
 }
 
 // The reads k_chain_map listed for their anchor count, one warp and 25 KB of shared memory
@@ -1143,7 +1150,7 @@ void launch_chain_map(cudaStream_t st, const int64_t* pofs, const int32_t* seq_l
                       const int* list_n, const int32_t* n_min, const int64_t* n_anchor, MinBuf mb,
                       const DevIndex& ix, const ChainParamsDev& cp, const CandParams& cand, AnchorScratch as,
                       unsigned long long* pool_top, int64_t pool_cap, CandBuf cb, int* claim, int32_t* big, int* big_n,
-                      uint32_t* err) {
+                      unsigned long long* info, uint32_t* err) {
   if (n <= 0) return;
   // a count that may be known on the device only: with work stealing the resident blocks,
   // otherwise a grid-stride over a few resident waves
@@ -1163,7 +1170,7 @@ void launch_chain_map(cudaStream_t st, const int64_t* pofs, const int32_t* seq_l
   const int64_t blocks = std::min<int64_t>((n + kChainWarps - 1) / kChainWarps, cap);
   k_chain_map<<<static_cast<unsigned>(blocks), kChainWarps * 32, 0, st>>>(
       pofs, seq_len, n, list, list_n, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, claim, big, big_n,
-      err);
+      info, err);
   k_chain_big<<<static_cast<unsigned>(std::min<int64_t>(n, int64_t{8} * device_sm_count())), 32, 0, st>>>(
       pofs, seq_len, n_min, n_anchor, mb, ix, cp, cand, as, pool_top, pool_cap, cb, big, big_n, err);
 }

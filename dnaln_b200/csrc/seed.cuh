@@ -141,12 +141,12 @@ void launch_seed_list(cudaStream_t st, const char* seq, const int64_t* seq_off, 
 // warp takes its next read by an atomic add on *claim (work stealing); without, the warps
 // stride over the reads. big (n entries) and big_n (two ints zeroed by the caller: its count
 // and its claims) list reads of 257 to 1,024 anchors for a second kernel with as much shared
-// memory per warp.
+// memory per warp. info[6], [7] and [9] += the reads' minimizers, bases and anchors.
 void launch_chain_map(cudaStream_t st, const int64_t* pofs, const int32_t* seq_len, int64_t n, const int32_t* list,
                       const int* list_n, const int32_t* n_min, const int64_t* n_anchor, MinBuf mb,
                       const DevIndex& ix, const ChainParamsDev& cp, const CandParams& cand, AnchorScratch as,
                       unsigned long long* pool_top, int64_t pool_cap, CandBuf cb, int* claim, int32_t* big, int* big_n,
-                      uint32_t* err);
+                      unsigned long long* info, uint32_t* err);
 
 // Codes of both strands of reads [0, n) (seed_thread.cu): forward at codes[2*pofs[r]],
 // reverse complement right after it (src/mapper.cpp:88-99), from the ASCII reads.
@@ -192,6 +192,8 @@ void launch_read_order(cudaStream_t st, const int32_t* seq_len, const int32_t* l
 // n_anchor stay as they were). reads_per_block: 64 or
 // 128 (threads per block; same results). Returns false, launching nothing, when the
 // parameters are outside the path's range.
+// Lists of at most this many reads pass straight through the two thread kernels.
+constexpr int kSeedFewReads = 4096;
 bool seed_thread_supported(const SeedParams& sp, const ChainParamsDev& cp);
 int seed_thread_max_len();  // the longest read the short thread kernel stages
 bool launch_seed_chain_thread(cudaStream_t st, const uint8_t* codes, const int64_t* pofs,

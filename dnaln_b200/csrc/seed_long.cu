@@ -35,7 +35,7 @@ constexpr int kLMaxAnc = 256;
 constexpr int kLMaxChains = 32;
 // A list of at most this many reads goes on to the warp kernels as it is: one thread takes
 // 1.2 ms for a 1,000 bp read and its global columns, however few there are.
-constexpr int kLFew = 4096;
+constexpr int kLFew = kSeedFewReads;
 constexpr int kLMaxBand = 256;    // chaining band of the shared gap-cost table
 // column words per thread: A = anchor keys (hi, lo); B = minimizer slots (hash, pos |
 // strand << 31), later the DP words (f | maxf << 16, prev + 1) and the chain table;

@@ -76,7 +76,7 @@ struct TLayout {
 // A list of at most this many reads goes on to the next kernels as it is: one thread per read
 // takes as long for a few reads as for a wave of 56,832 (112 us at 150 bp), one warp per read
 // 30 us for 1,500 and 200 us for 20,000.
-constexpr int kTFew = 4096;
+constexpr int kTFew = kSeedFewReads;
 
 // 4-byte asynchronous copy global -> shared (both 4-byte aligned).
 __device__ __forceinline__ void cp_async4(uint32_t* dst_smem, const void* src) {
