@@ -1159,9 +1159,10 @@ struct SlotBufs {
 const char* const kSlotNames[2][6] = {{"in_seq0", "in_off0", "in_len0", "in_hash0", "out_rec0", "out_cig0"},
                                       {"in_seq1", "in_off1", "in_len1", "in_hash1", "out_rec1", "out_cig1"}};
 
-bool pop_part(dnaln_ctx* c, MapPart& pt) {
+// The next part; with own != 0 only one of that ticket.
+bool pop_part(dnaln_ctx* c, MapPart& pt, int64_t own) {
   std::lock_guard<std::mutex> g(c->qmu);
-  if (c->queue.empty()) return false;
+  if (c->queue.empty() || (own && c->queue.front().ticket != own)) return false;
   pt = c->queue.front();
   c->queue.pop_front();
   return true;
@@ -1245,17 +1246,18 @@ int compute_part(dnaln_ctx* c, int k, const MapPart& pt, const SlotBufs& sb, int
   return DNALN_OK;
 }
 
-// Drives queued parts through the two slots until the queue is empty.
-void drive_parts(dnaln_ctx* c) {
+// Drives queued parts (with own != 0, those of that ticket) through the two slots until none
+// is left.
+void drive_parts(dnaln_ctx* c, int64_t own) {
   PendingPart pend[2];
   SlotBufs sb[2];
   MapPart pt;
-  if (!pop_part(c, pt)) return;
+  if (!pop_part(c, pt, own)) return;
   int k = 0;
   int staged = stage_in(c, k, pt, sb[k]);
   for (;;) {
     MapPart nx;
-    const bool have_next = pop_part(c, nx);
+    const bool have_next = pop_part(c, nx, own);
     int next_staged = DNALN_OK;
     if (have_next) next_staged = stage_in(c, 1 - k, nx, sb[1 - k]);  // slot 1-k's inputs are free
     int64_t base = 0;
@@ -1297,6 +1299,103 @@ void drive_parts(dnaln_ctx* c) {
   finish_part(c, k, pend[k]);
 }
 
+// What the host knows of reads [a, b): their bytes' extent, bases, longest, CIGAR bound.
+// False on a negative offset or length. The sums are plain reductions the compiler can
+// vectorise; the extent is read off the ends when the reads lie one behind the other (262,144
+// reads: 320 -> 210 us).
+bool read_facts(const int64_t* off, const int32_t* len, int64_t a, int64_t b, MapPart& pt) {
+  pt.a = a;
+  pt.b = b;
+  int64_t neg = 0, gaps = 0, bases = 0;
+  int32_t most = 0;
+  for (int64_t i = a; i < b; ++i) {
+    neg |= off[i] | len[i];
+    bases += len[i];
+    most = len[i] > most ? len[i] : most;
+  }
+  if (neg < 0) return false;
+  for (int64_t i = a; i + 1 < b; ++i) gaps |= off[i + 1] - off[i] - len[i];
+  pt.lo = off[a];
+  pt.hi = off[b - 1] + len[b - 1];
+  if (gaps) {
+    for (int64_t i = a; i < b; ++i) {
+      pt.lo = std::min(pt.lo, off[i]);
+      pt.hi = std::max(pt.hi, off[i] + len[i]);
+    }
+  }
+  pt.bases = bases;
+  pt.max_len = most;
+  pt.cig_bound = 2 * bases + 3 * (b - a);  // walk ops (<= 2*len+1) + 2 clips
+  return true;
+}
+
+// A synchronous batch of at least this many bases goes in two parts, so that the second's
+// reads are copied while the first computes. Reads of 150 bp from pinned memory, one part,
+// halves, thirds: 65,536 699, 727, 921 us; 131,072 1,198, 1,110, 1,298; 262,144 2,248, 1,961,
+// 2,049; 524,288 4,155, 3,427, 3,500.
+constexpr int64_t kSplitBases = 16 << 20;
+
+// Queues a batch (see dnaln_gpu_map_submit). *alone = nothing was queued before it.
+int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_off, const int32_t* seq_len,
+                 const uint32_t* name_hash, int64_t n, const dnaln_map_params* p, dnaln_map_record* out,
+                 uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used, bool split, int64_t* ticket, bool* alone) {
+  if (!c || n < 0 || !cigar_used || !ticket || !p || (n > 0 && (!seq || !seq_off || !seq_len || !name_hash || !out)))
+    return fail(c, DNALN_ERR_INVALID_ARG, "null argument");
+  *ticket = 0;
+  *cigar_used = 0;
+  // the index-dependent checks run where the parts are driven (the index table belongs to
+  // whoever drives the device); their failures come back from dnaln_gpu_map_wait
+  if (int e = validate_map_params_basic(c, p)) return e;
+  // parts of at most sub_batch reads, with their host-side facts (lengths are known here)
+  split = split && c->sub_batch == 0 && n >= 2;
+  const int64_t S = c->sub_batch > 0 ? c->sub_batch : (split ? (n + 1) / 2 : std::max<int64_t>(n, 1));
+  std::vector<MapPart> parts;
+  for (int64_t a = 0; a < n; a += S) {
+    MapPart pt;
+    pt.index_id = id;
+    pt.seq = seq;
+    pt.seq_off = seq_off;
+    pt.seq_len = seq_len;
+    pt.name_hash = name_hash;
+    pt.p = *p;
+    pt.out = out;
+    pt.cigar = cigar;
+    pt.cigar_cap = cigar_cap;
+    pt.cigar_used = cigar_used;
+    if (!read_facts(seq_off, seq_len, a, std::min(n, a + S), pt))
+      return fail(c, DNALN_ERR_INVALID_ARG, "negative offset or length");
+    parts.push_back(pt);
+  }
+  // one part if it is small or the halves' reads are not apart in the buffer
+  if (split && (parts[0].bases + parts[1].bases < kSplitBases ||
+                std::min(parts[0].hi, parts[1].hi) > std::max(parts[0].lo, parts[1].lo))) {
+    MapPart& all = parts[0];
+    const MapPart& rest = parts[1];
+    all.b = rest.b;
+    all.lo = std::min(all.lo, rest.lo);
+    all.hi = std::max(all.hi, rest.hi);
+    all.bases += rest.bases;
+    all.max_len = std::max(all.max_len, rest.max_len);
+    all.cig_bound += rest.cig_bound;
+    parts.pop_back();
+  }
+  std::lock_guard<std::mutex> g(c->qmu);
+  const int64_t t = c->next_ticket++;
+  *ticket = t;
+  *alone = c->queue.empty();
+  if (parts.empty()) {
+    c->results[t] = DNALN_OK;
+    return DNALN_OK;
+  }
+  parts.back().last = true;
+  for (MapPart& pt : parts) {
+    pt.ticket = t;
+    c->queue.push_back(pt);
+  }
+  c->ticket_ops[t] = 0;
+  return DNALN_OK;
+}
+
 void map_worker(dnaln_ctx* c) {
   cudaSetDevice(c->device);
   std::unique_lock<std::mutex> ql(c->qmu);
@@ -1306,10 +1405,18 @@ void map_worker(dnaln_ctx* c) {
     ql.unlock();
     {
       std::lock_guard<std::mutex> g(c->mu);
-      drive_parts(c);
+      drive_parts(c, 0);
     }
     ql.lock();
   }
+}
+
+void wake_worker(dnaln_ctx* c) {
+  {
+    std::lock_guard<std::mutex> g(c->qmu);
+    if (!c->queue.empty() && !c->worker.joinable()) c->worker = std::thread(map_worker, c);
+  }
+  c->qcv.notify_all();
 }
 }  // namespace
 
@@ -2294,59 +2401,11 @@ int dnaln_gpu_map_batch_device(dnaln_ctx* c, int32_t id, const char* d_seq, cons
 int dnaln_gpu_map_submit(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_off, const int32_t* seq_len,
                          const uint32_t* name_hash, int64_t n, const dnaln_map_params* p, dnaln_map_record* out,
                          uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used, int64_t* ticket) {
-  if (!c || n < 0 || !cigar_used || !ticket || !p || (n > 0 && (!seq || !seq_off || !seq_len || !name_hash || !out)))
-    return fail(c, DNALN_ERR_INVALID_ARG, "null argument");
-  *ticket = 0;
-  *cigar_used = 0;
-  // the index-dependent checks run in the worker (the index table belongs to it while it
-  // drives the device); their failures come back from dnaln_gpu_map_wait
-  if (int e = validate_map_params_basic(c, p)) return e;
-  // parts of at most sub_batch reads, with their host-side facts (lengths are known here)
-  const int64_t S = c->sub_batch > 0 ? c->sub_batch : (n > 0 ? n : 1);
-  std::vector<MapPart> parts;
-  for (int64_t a = 0; a < n; a += S) {
-    MapPart pt;
-    pt.index_id = id;
-    pt.seq = seq;
-    pt.seq_off = seq_off;
-    pt.seq_len = seq_len;
-    pt.name_hash = name_hash;
-    pt.a = a;
-    pt.b = std::min(n, a + S);
-    pt.lo = seq_off[a];
-    pt.p = *p;
-    pt.out = out;
-    pt.cigar = cigar;
-    pt.cigar_cap = cigar_cap;
-    pt.cigar_used = cigar_used;
-    for (int64_t i = pt.a; i < pt.b; ++i) {
-      if (seq_len[i] < 0 || seq_off[i] < 0) return fail(c, DNALN_ERR_INVALID_ARG, "negative offset or length");
-      pt.lo = std::min(pt.lo, seq_off[i]);
-      pt.hi = std::max(pt.hi, seq_off[i] + seq_len[i]);
-      pt.bases += seq_len[i];
-      pt.max_len = std::max<int64_t>(pt.max_len, seq_len[i]);
-      pt.cig_bound += 2 * static_cast<int64_t>(seq_len[i]) + 3;  // walk ops (<= 2*len+1) + 2 clips
-    }
-    if (pt.hi < pt.lo) pt.hi = pt.lo;
-    parts.push_back(pt);
-  }
-  {
-    std::lock_guard<std::mutex> g(c->qmu);
-    const int64_t t = c->next_ticket++;
-    *ticket = t;
-    if (parts.empty()) {
-      c->results[t] = DNALN_OK;
-      return DNALN_OK;
-    }
-    parts.back().last = true;
-    for (MapPart& pt : parts) {
-      pt.ticket = t;
-      c->queue.push_back(pt);
-    }
-    c->ticket_ops[t] = 0;
-    if (!c->worker.joinable()) c->worker = std::thread(map_worker, c);
-  }
-  c->qcv.notify_all();
+  bool alone = false;
+  if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, false,
+                           ticket, &alone))
+    return e;
+  wake_worker(c);
   return DNALN_OK;
 }
 
@@ -2367,11 +2426,26 @@ int dnaln_gpu_map_wait(dnaln_ctx* c, int64_t ticket) {
 int dnaln_gpu_map_batch(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_off, const int32_t* seq_len,
                         const uint32_t* name_hash, int64_t n, const dnaln_map_params* p, dnaln_map_record* out,
                         uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used) {
-  int64_t ticket = 0;
-  if (int e = dnaln_gpu_map_submit(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used,
-                                   &ticket))
-    return e;
-  return dnaln_gpu_map_wait(c, ticket);
+  const auto map = [&](bool split) {
+    int64_t ticket = 0;
+    bool alone = false;
+    if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, split,
+                             &ticket, &alone))
+      return e;
+    // with nothing queued before it and the device free, the batch runs in the calling thread:
+    // a wake-up of the worker and one back cost a call of 64 reads 16 us
+    bool here = false;
+    if (alone && c->mu.try_lock()) {
+      std::lock_guard<std::mutex> g(c->mu, std::adopt_lock);
+      here = cudaSetDevice(c->device) == cudaSuccess;
+      if (here) drive_parts(c, ticket);
+    }
+    if (!here) wake_worker(c);
+    return dnaln_gpu_map_wait(c, ticket);
+  };
+  const int e = map(true);
+  // a CIGAR buffer too small for the batch is reported for the whole of it
+  return e == DNALN_ERR_CAPACITY && n > 1 && c->sub_batch == 0 ? map(false) : e;
 }
 
 }  // extern "C"

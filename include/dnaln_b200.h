@@ -126,8 +126,8 @@ typedef struct dnaln_kernel_time {
 int dnaln_gpu_set_kernel_trace(dnaln_ctx* ctx, int32_t on, const char* only);
 /* Writes min(cap, count) entries; *n_out = count of traced kernel names. */
 int dnaln_gpu_kernel_times(const dnaln_ctx* ctx, dnaln_kernel_time* out, int32_t cap, int32_t* n_out);
-/* Reads per part of a host-buffer batch (default 0: the whole batch is one part; smaller
- * parts let one synchronous call overlap its own copies, at some kernel efficiency). */
+/* Reads per part of a host-buffer batch (default 0: one part, or two for a large batch that
+ * is waited for, so that its own copies overlap; smaller parts cost kernel efficiency). */
 int dnaln_gpu_set_sub_batch(dnaln_ctx* ctx, int64_t reads);
 /* Tuning switches (none changes any result):
  *   "sub_batch"      same as dnaln_gpu_set_sub_batch;

@@ -3,10 +3,14 @@ where their blocks begin: one block of offsets and several, one group of record 
 several, blocks of more than one tile of offsets, and reads that are handed to the warp
 kernels directly and through the lists. Every copy of a read gives the record of the read
 alone, and the CIGARs lie one behind the other."""
+import ctypes as C
+import threading
+
 import numpy as np
 import pytest
 
 import dnaln_b200 as D
+from dnaln_b200._native import ptr
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +70,68 @@ def test_every_copy_of_a_read_gets_its_record(ctx, setup, n):
     if n % m == 0:
         for f in ("mapped", "candidates", "minimizers", "anchors", "cells"):
             assert st[f] == s1[f] * copies, f
+
+
+@pytest.mark.parametrize("order", ["packed", "gaps", "shuffled"])
+def test_a_large_batch_in_two_parts(ctx, setup, order):
+    """16 Mi bases and more go in two parts where the halves' reads lie apart: same results as
+    in one part, and a CIGAR buffer that is too small is refused with the same error."""
+    iid, seqs = setup
+    n = 420_000
+    batch = tiled(seqs, n)
+    if order != "packed":
+        rng = np.random.default_rng(3)
+        ln = batch.seq_len.astype(np.int64)
+        perm = rng.permutation(n) if order == "shuffled" else np.arange(n)
+        place = np.empty(n, np.int64)
+        place[perm] = np.concatenate([[0], np.cumsum(ln[perm] + 3)[:-1]])
+        seq = np.full(int((ln + 3).sum()), ord("N"), np.uint8)
+        at = np.repeat(place - batch.seq_off[:-1], ln) + np.arange(batch.seq_off[-1])
+        seq[at] = batch.seq
+        batch = (seq, place, batch.seq_len)
+    assert int(tiled(seqs, n).seq_off[-1]) >= 16 << 20
+    lib, p = ctx._lib, D.default_map_params()
+    seq, off, ln = batch if isinstance(batch, tuple) else (batch.seq, batch.seq_off[:-1].copy(), batch.seq_len)
+    seq, names = np.ascontiguousarray(seq), np.full(n, 7, np.uint32)
+
+    def run(cap):
+        rec, cig, used = np.zeros(n, D.MAP_RECORD_DTYPE), np.zeros(cap, np.uint32), C.c_int64()
+        rc = lib.dnaln_gpu_map_batch(ctx.handle, iid, ptr(seq), ptr(off), ptr(ln), ptr(names), n, C.byref(p), ptr(rec),
+                                     ptr(cig), cap, C.byref(used))
+        return rc, rec, cig[:used.value], used.value, lib.dnaln_gpu_last_error(ctx.handle)
+
+    try:
+        ctx.set_sub_batch(n)
+        want, small = run(8 * n), run(1000)
+        ctx.set_sub_batch(0)
+        got, refused = run(8 * n), run(1000)
+    finally:
+        ctx.set_sub_batch(0)
+    assert got[0] == want[0] == 0 and got[3] == want[3]
+    assert np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2])
+    assert refused[0] == small[0] != 0 and refused[3] == small[3] and refused[4] == small[4]
+
+
+def test_calls_from_threads_and_queued_batches(ctx, setup):
+    """Batches mapped in the calling thread while others are queued and mapped by other threads."""
+    iid, seqs = setup
+    batches = [tiled(seqs, n) for n in (61, 700, 5_000, 20_000)]
+    want = [ctx.map_batch(iid, b) for b in batches]
+    bad = []
+
+    def work(k):
+        for i in range(12):
+            x = (i + k) % len(batches)
+            if (i + k) % 3 == 0:
+                got = ctx.map_wait(ctx.map_submit(iid, batches[x]))
+            else:
+                got = ctx.map_batch(iid, batches[x])
+            if not (np.array_equal(got.records, want[x].records) and np.array_equal(got.cigar, want[x].cigar)):
+                bad.append((k, i))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
