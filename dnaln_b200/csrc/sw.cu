@@ -493,7 +493,7 @@ __device__ bool window_has_n(const SwTask& tk, int W, const uint8_t* __restrict_
 //    selector of two codes is two multiply-adds.
 template <int W, bool TB>
 __global__ void __launch_bounds__(kDpThreads, (TB && W <= 33) ? 12 : 1)
-    k_sw_u2(const SwTask* __restrict__ tasks, int base, int count, int n, const int* __restrict__ n_dev, int few,
+    k_sw_u2(const SwTask* __restrict__ tasks, int base, int n, const int* __restrict__ n_dev, int few,
              const uint8_t* __restrict__ qbase, const uint8_t* __restrict__ tbase, SwParams p,
              SwResult* __restrict__ res, uint32_t* __restrict__ dir, int rows_max, int* __restrict__ fb,
              int* __restrict__ claim) {
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kDpThreads, (TB && W <= 33) ? 12 : 1)
   if (threadIdx.x < 5) s_prof[threadIdx.x] = prof_biased(p, threadIdx.x);
   __syncthreads();
   if (n_dev && *n_dev <= few) return;  // a short list is the narrowest form's
-  const int nn = n_dev ? min(n, *n_dev) : n, pairs = (min(nn - base, count) + 1) / 2;
+  const int nn = n_dev ? min(n, *n_dev) : n, pairs = (nn - base + 1) / 2;
   const auto align = [&](const int lt) {  // lt: pair index within this launch
   const int ia = base + 2 * lt, ib = ia + 1;
   const bool has_b = ib < nn;
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(kDpThreads, (TB && W <= 33) ? 12 : 1)
   }
 }
 
-// Wide bands, W = CH * LANES + 1: LANES consecutive lanes of a warp share one pair of
+// W <= CH * LANES + 1: LANES consecutive lanes of a warp share one pair of
 // alignments (A and B in the 16-bit halves, as in k_sw_u2), lane c holding band cells
 // [CH c, CH c + CH) of the row in registers (the last lane also cell W - 1). Fewer cells a
 // lane: more warps and a shorter row, but its fixed work (shuffles, codes, the best row) is
@@ -658,14 +658,19 @@ __global__ void __launch_bounds__(kDpThreads, (TB && W <= 33) ? 12 : 1)
 // Resident warps per SM (sw_wide_warps), same lists: 8 cells 16 / 20 / 24 warps 185 / 176 /
 // 190 us; 32 cells 12 / 10 / 8 warps 1,333 / 1,311 / 1,200; 4 cells 20 / 24 1,262 / 1,218.
 constexpr int sw_wide_warps(int cells) { return cells == 4 ? 24 : (cells == 8 ? 20 : (cells == 16 ? 12 : 8)); }
-template <int LANES, int CH, bool TB>
+template <int W, int LANES, int CH, bool TB>
 __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
-    k_sw_wide(const SwTask* __restrict__ tasks, int base, int count, int n, const int* __restrict__ n_dev, int above, int upto,
+    k_sw_wide(const SwTask* __restrict__ tasks, int base, int n, const int* __restrict__ n_dev, int above, int upto,
               const uint8_t* __restrict__ qbase, const uint8_t* __restrict__ tbase, SwParams p,
               SwResult* __restrict__ res, uint32_t* __restrict__ dir, int rows_max, int* __restrict__ fb,
               int* __restrict__ claim) {
   static_assert(CH % 4 == 0, "a lane's cells fill whole direction words");
-  constexpr int W = CH * LANES + 1, WQ = (W + 3) / 4;
+  static_assert(W <= CH * LANES + 1, "a band's cells have lanes");
+  constexpr int WQ = (W + 3) / 4;
+  // band column W - 1: an extra cell of the last lane, or cell kLastCell of lane kLastLane, past
+  // which cells and lanes hold nothing
+  constexpr bool kExtra = W == CH * LANES + 1;
+  constexpr int kLastLane = kExtra ? LANES - 1 : (W - 1) / CH, kLastCell = kExtra ? CH : (W - 1) % CH;
   constexpr unsigned FULL = 0xffffffffu;
   if (n_dev && (*n_dev <= above || *n_dev > upto)) return;  // a list of another form's length
   __shared__ uint32_t s_prof[8];  // profile words of the five query codes
@@ -673,7 +678,7 @@ __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int c = lane % LANES;  // chunk of this lane
-  const int nn = n_dev ? min(n, *n_dev) : n, pairs = (min(nn - base, count) + 1) / 2;
+  const int nn = n_dev ? min(n, *n_dev) : n, pairs = (nn - base + 1) / 2;
   const auto align = [&](const int lt) {  // lt: pair index within this launch
   const int ia = base + 2 * lt, ib = ia + 1;
   const bool live = lt < pairs, has_b = live && ib < nn;
@@ -758,7 +763,7 @@ __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
     x_qa = qcode(qa, qla, 1 - c);
     x_qb = qcode(qb, qlb, 1 - c);
   }
-  const int end = skip ? 0 : qmax;
+  const int end = skip || c > kLastLane ? 0 : qmax;
   uint32_t* dp = TB ? DP + (d0 >> 2) * 32 - c * (WQ * 32) : nullptr;  // row i's first word of this lane
   const auto step = [&](const int t, auto steady) {
     constexpr bool kSteady = decltype(steady)::value;
@@ -804,13 +809,16 @@ __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
     }
     // local cell 0, then hand (H, E) of it to the left lane: the E input of its last cell
     uint32_t rmax = 0, dw = 0, e0;
-    const uint32_t h0 = cell2<TB>(cp, H[0], prmt(lo, hi, T[0]), H[1], E[1], hleft, f, e0, dw);
-    uint32_t hdiag = H[1];
+    const bool edge = !kExtra && c == kLastLane;
+    const bool cut0 = kLastCell == 0 && edge;
+    const uint32_t h0 = cell2<TB>(cp, H[0], prmt(lo, hi, T[0]), cut0 ? h_zero : H[1], cut0 ? kBias2 : E[1], hleft, f,
+                                  e0, dw);
+    uint32_t hdiag = H[1];  // past the band's edge a cell's diagonal is never used
     hleft = h0;
     // a lane that has not reached row 0 passes row -1's values (zero)
     uint32_t nh = __shfl_down_sync(FULL, he_ok ? h0 : h_zero, 1);
     uint32_t ne = __shfl_down_sync(FULL, he_ok ? e0 : kBias2, 1);
-    if (c == LANES - 1) {
+    if (kExtra && c == LANES - 1) {
       nh = H[CH];
       ne = E[CH];
     }
@@ -819,11 +827,16 @@ __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
       E[0] = e0;
     }
     uint32_t& top = TB ? rmax : best2;  // the row's maximum (score only: the maximum so far)
+    if (!kExtra) top = __vmaxu2(top, h0);
 #pragma unroll
-    for (int k = 1; k <= CH; ++k) {
+    for (int k = 1; k < CH + kExtra; ++k) {
       if (k == CH && c != LANES - 1) break;  // the extra cell W - 1 belongs to the last lane
-      const uint32_t hup = k == CH - 1 ? nh : (k == CH ? h_zero : H[k + 1]);
-      const uint32_t eup = k == CH - 1 ? ne : (k == CH ? kBias2 : E[k + 1]);
+      uint32_t hup = k == CH - 1 ? nh : (k == CH ? h_zero : H[k + 1]);
+      uint32_t eup = k == CH - 1 ? ne : (k == CH ? kBias2 : E[k + 1]);
+      if (k == kLastCell && edge) {
+        hup = h_zero;
+        eup = kBias2;
+      }
       uint32_t e, code = 0;
       const uint32_t h = cell2<TB>(cp, hdiag, prmt(lo, hi, T[k]), hup, eup, hleft, f, e, code);
       if (he_ok) {
@@ -832,9 +845,11 @@ __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
       }
       if constexpr (TB) {
         dw = insert_code(dw, code, k & 3);
-        if (((k & 3) == 3 || k == CH) && act) dp[(k >> 2) * 32] = dw;
+        const bool inside = (kLastLane * CH + k) / 4 < WQ || c < kLastLane;
+        if (((k & 3) == 3 || k == CH) && act && inside) dp[(k >> 2) * 32] = dw;
       }
-      if (k & 1) top = __vimax3_u16x2(top, hleft, h);
+      if (!kExtra) top = __vmaxu2(top, k > kLastCell && edge ? h_zero : h);
+      else if (k & 1) top = __vimax3_u16x2(top, hleft, h);
       else if (k == CH) top = __vmaxu2(top, h);
       hleft = h;
       hdiag = hup;
@@ -873,7 +888,7 @@ __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
   for (int t = ramp; t < steps; ++t) step(t, std::true_type{});
   // combine the lanes of the pair: larger value, then earlier row, then smaller column
   uint64_t key_a, key_b;
-  const int ncell = c == LANES - 1 ? CH + 1 : CH;
+  const int ncell = c == kLastLane ? kLastCell + 1 : CH;
   if constexpr (TB) {
     int bd_a = 0xFFF, bd_b = 0xFFF;
     const uint32_t best_a = best2 & 0xFFFFu, best_b = best2 >> 16;
@@ -889,8 +904,8 @@ __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
     key_b = static_cast<uint64_t>(best_b) << 40 | static_cast<uint64_t>(0xFFFFFu - static_cast<uint32_t>(bi_b + 1)) << 12 |
             (0xFFFu - static_cast<uint32_t>(bd_b));
   } else {
-    key_a = static_cast<uint64_t>(best2 & 0xFFFFu) << 40;
-    key_b = static_cast<uint64_t>(best2 >> 16) << 40;
+    key_a = c > kLastLane ? 0 : static_cast<uint64_t>(best2 & 0xFFFFu) << 40;
+    key_b = c > kLastLane ? 0 : static_cast<uint64_t>(best2 >> 16) << 40;
   }
 #pragma unroll
   for (int o = 1; o < LANES; o <<= 1) {
@@ -1362,6 +1377,17 @@ struct SwLaunch {
 // and 212 us; 88,000 of 50 to 1,000 rows at W = 129 1,871 and 1,307.
 constexpr int sw_narrow_cells(int W) { return W == 129 ? 16 : 8; }
 
+// Bands of registers with the forms of 32 and of fewer cells per lane.
+constexpr bool sw_has_intra(int W) { return W == 33 || W == 65 || W == 129; }
+constexpr bool sw_has_narrow(int W) { return W == 43 || sw_has_intra(W); }
+
+// Lanes per pair at `cells` a lane: a power of two, the last one with a cell more if need be.
+constexpr int sw_lanes(int W, int cells) {
+  int l = 1;
+  while (cells * l + 1 < W) l *= 2;
+  return l;
+}
+
 // Blocks of one warp for `warps` claims: all of them, up to what is resident.
 template <class Kernel>
 int dp_blocks(int64_t warps, Kernel* kernel, int smem, std::atomic<int>* resident) {
@@ -1375,20 +1401,21 @@ int dp_blocks(int64_t warps, Kernel* kernel, int smem, std::atomic<int>* residen
   return static_cast<int>(std::min<int64_t>(warps, int64_t{v > 0 ? v : 8} * device_sm_count()));
 }
 
-template <int LANES, int CH>
+template <int W, int CH>
 void run_wide(const SwLaunch& a, int count, int above, int upto) {
+  constexpr int LANES = sw_lanes(W, CH);
   const int64_t pairs = (static_cast<int64_t>(count) + 1) / 2;
   int* const claim = a.fb + (upto == INT_MAX ? 2 : 1);
   const auto run = [&](auto* kernel, int smem, std::atomic<int>* resident) {
     kernel<<<dp_blocks((pairs * LANES + 31) / 32, kernel, smem, resident), kDpThreads, smem, a.st>>>(
-        a.tasks, a.base, a.count, a.n, a.n_dev, above, upto, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb,
+        a.tasks, a.base, a.n, a.n_dev, above, upto, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb,
         claim);
   };
   constexpr int kRowBytes = 2 * (CH + 1) * kDpThreads * 4;  // the two saved best rows of each lane
   static std::atomic<int> resident[2][kMaxDevices];
   a.kt.begin(a.st, a.tb ? "k_sw_wide<tb>" : "k_sw_wide<score>");
-  if (a.tb) run(k_sw_wide<LANES, CH, true>, kRowBytes, resident[1]);
-  else run(k_sw_wide<LANES, CH, false>, 0, resident[0]);
+  if (a.tb) run(k_sw_wide<W, LANES, CH, true>, kRowBytes, resident[1]);
+  else run(k_sw_wide<W, LANES, CH, false>, 0, resident[0]);
   a.kt.end(a.st);
 }
 
@@ -1397,7 +1424,7 @@ void run_u2(const SwLaunch& a, int above) {
   const auto run = [&](auto* kernel, int smem, std::atomic<int>* resident) {
     const int64_t warps = ((static_cast<int64_t>(a.count) + 1) / 2 + 31) / 32;
     kernel<<<dp_blocks(warps, kernel, smem, resident), kDpThreads, smem, a.st>>>(
-        a.tasks, a.base, a.count, a.n, a.n_dev, above, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb, a.fb + 2);
+        a.tasks, a.base, a.n, a.n_dev, above, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb, a.fb + 2);
   };
   constexpr int kRowBytes = 2 * W * kDpThreads * 4;  // the two saved best rows of each thread
   static_assert(kRowBytes <= 48 * 1024);
@@ -1432,15 +1459,14 @@ void run_fb(const SwLaunch& a) {
 // `few`, the main form any other), the main form, the int32 kernel, the walk.
 template <int W>
 void launch_band(const SwLaunch& a, SwForm form, int few) {
-  constexpr bool kFew = W == 17 || W == 33 || W == 65 || W == 129;
   cudaMemsetAsync(a.fb, 0, kFbList * sizeof(int), a.st);
-  if constexpr (kFew) {
-    if (form == kSwIntraFew) run_wide<(W - 1) / 4, 4>(a, a.count, 0, INT_MAX);
-    else if (few > 0) run_wide<(W - 1) / 4, 4>(a, std::min(a.count, few), 0, few);
+  if (form == kSwIntraFew) run_wide<W, 4>(a, a.count, 0, INT_MAX);
+  else if (few > 0) run_wide<W, 4>(a, std::min(a.count, few), 0, few);
+  if constexpr (sw_has_intra(W)) {
+    if (form == kSwIntra) run_wide<W, 32>(a, a.count, few, INT_MAX);
   }
-  if constexpr (W == 33 || W == 65 || W == 129) {
-    if (form == kSwIntra) run_wide<(W - 1) / 32, 32>(a, a.count, few, INT_MAX);
-    if (form == kSwIntraNarrow) run_wide<(W - 1) / sw_narrow_cells(W), sw_narrow_cells(W)>(a, a.count, few, INT_MAX);
+  if constexpr (sw_has_narrow(W)) {
+    if (form == kSwIntraNarrow) run_wide<W, sw_narrow_cells(W)>(a, a.count, few, INT_MAX);
   }
   if constexpr (W != 129) {
     if (form == kSwInter) run_u2<W>(a, few);
@@ -1499,8 +1525,18 @@ size_t sw_band_bytes_per_task(int W, bool bytes_ok) {
 // best other form, us for 150-row tracebacks: W = 33 51 against 67 at 1,024 tasks, 94
 // against 91 at 16,384; W = 65 51 against 64 and, at 8,192, 97 against 85; W = 129 57
 // against 90 and, at 4,096, 117 against 95; W = 17 55 against 92 and, at 32,768, 99
-// against 97.
-int sw_few_tasks(int W) { return W == 17 ? 28672 : (W == 33 ? 14336 : (W == 65 ? 4608 : 3072)); }
+// against 97; W = 43 44 against 58 and, at 8,192, 86 against 77; W = 11 50 against 69 and, at
+// 32,768, 91 against 74.
+int sw_few_tasks(int W) {
+  switch (W) {
+    case 11: return 20480;
+    case 17: return 28672;
+    case 33: return 14336;
+    case 43: return 5120;
+    case 65: return 4608;
+    default: return 3072;  // 129
+  }
+}
 
 int sw_launches(int W, bool bytes_ok, bool tb) { return sw_uses_generic(W, bytes_ok) ? 1 : (tb ? 3 : 2); }
 
@@ -1508,17 +1544,17 @@ bool sw_has_form(int W, bool bytes_ok, SwForm form) {
   if (sw_uses_generic(W, bytes_ok)) return form == kSwInter;
   switch (form) {
     case kSwInter: return W != 129;
-    case kSwIntra: return W == 33 || W == 65 || W == 129;
-    case kSwIntraNarrow: return W == 33 || W == 65 || W == 129;
-    case kSwIntraFew: return W == 17 || W == 33 || W == 65 || W == 129;
+    case kSwIntra: return sw_has_intra(W);
+    case kSwIntraNarrow: return sw_has_narrow(W);
+    case kSwIntraFew: return true;
     default: return false;
   }
 }
 
 int sw_lanes_per_pair(int W, SwForm form) {
-  if (form == kSwIntra) return (W - 1) / 32;
-  if (form == kSwIntraNarrow) return (W - 1) / sw_narrow_cells(W);
-  if (form == kSwIntraFew) return (W - 1) / 4;
+  if (form == kSwIntra) return sw_lanes(W, 32);
+  if (form == kSwIntraNarrow) return sw_lanes(W, sw_narrow_cells(W));
+  if (form == kSwIntraFew) return sw_lanes(W, 4);
   return 1;
 }
 

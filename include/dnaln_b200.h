@@ -136,9 +136,9 @@ int dnaln_gpu_set_sub_batch(dnaln_ctx* ctx, int64_t reads);
  *   "graphs"         1 = a batch whose size the host knows (the host-buffer calls) and
  *                    whose launches repeat is captured once as a CUDA graph and replayed
  *                    (default); 0 = launched kernel by kernel;
- *   "sw_form"        banded SW kernel form where a band width has several (W = 17, 33, 65,
- *                    129): 0 = tuned per context, and the form of four cells per lane for
- *                    short task lists (default), 1 = inter-sequence, 2 = intra-sequence, 3 =
+ *   "sw_form"        banded SW kernel form where a band width has several (W = 11, 17,
+ *                    33, 43, 65, 129): 0 = tuned per context, and the form of four cells per
+ *                    lane for short task lists (default), 1 = inter-sequence, 2 = intra-sequence, 3 =
  *                    intra-sequence narrow, 4 = four cells per lane (a form the width lacks
  *                    falls back to the width's first form);
  *   "long_thread"    1 = reads the short thread kernel lists go one thread each through

@@ -57,3 +57,22 @@ def test_more_pairs_than_resident_warps(ctx, port, form, bw, n):
     finally:
         ctx.set_option("sw_form", 0)
         ctx.set_option("ungapped", 1)
+
+
+@pytest.mark.parametrize("form", [1, 3, 4])
+@pytest.mark.parametrize("scheme", [(2, 4, 4, 2, 1, 5), (2, 4, 4, 2, 1, 21), (3, 2, 0, 3, 1, 21), (2, 0, 4, 2, 0, 5)])
+def test_bands_that_end_inside_a_lane(ctx, port, form, scheme):
+    """W = 11 and 43 end in the middle of a lane's cells, with idle lanes after it."""
+    bw = scheme[5]
+    rng = np.random.default_rng(9 * form + bw)
+    qs, ts = short_tasks(rng, list(range(1, 71)) + [1, 70, 64, 2, 300, 1, 33, 500], bw)
+    ra, rb = random_tasks(rng, 150, bw)
+    try:
+        ctx.set_option("ungapped", 0)
+        ctx.set_option("sw_form", form)
+        for tb in (True, False):
+            check_same(ctx.align(qs + ra, ts + rb, tb, D.ScoreParams(*scheme)), port.align(qs + ra, ts + rb, tb, scheme),
+                       tb)
+    finally:
+        ctx.set_option("sw_form", 0)
+        ctx.set_option("ungapped", 1)
