@@ -29,6 +29,7 @@
 // one lane, and ordered by score with ties in extraction order (the reference's
 // stable_sort). Candidate loci follow src/mapper.cpp:40-62.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "seed.cuh"
@@ -258,55 +259,75 @@ struct ChainArrays {
   int32_t* prev;
   uint64_t* ord;
   uint8_t* used;
+  uint16_t* link;  // of k_chain_big's reads only
 };
 
-// The chaining DP for any lookback, in rounds of 32 predecessors (src/chain.cpp:22-45).
-// Per round one redux over score * 32 + (31 - lane): the largest score, ties to the
-// smallest lane = the nearest j; earlier (nearer) rounds win ties across rounds through
-// the strict '>' below — the reference's scan order.
-__device__ void chain_dp_rounds(const ChainArrays& a, int n, const ChainParamsDev& cp) {
+// What predecessor j adds to f[j] for anchor i: min(dq, dr, k) - cost, or kNoGain if the pair is
+// not valid. rpos < 2^31 and |qpos| < 2^30, so dr and dq fit 32 bits; their difference is
+// formed in unsigned arithmetic and used only when both passed the range tests.
+constexpr int kNoGain = INT_MIN;
+__device__ __forceinline__ int chain_gain(const ChainParamsDev& cp, uint64_t ki, uint64_t kj) {
+  const int dr = static_cast<int>(key_rpos(ki)) - static_cast<int>(key_rpos(kj)), dq = key_qpos(ki) - key_qpos(kj);
+  const int dd = static_cast<int>(dr > dq ? static_cast<uint32_t>(dr) - static_cast<uint32_t>(dq)
+                                          : static_cast<uint32_t>(dq) - static_cast<uint32_t>(dr));
+  if (key_strand(ki) != key_strand(kj) || dr > cp.max_gap || dr <= 0 || dq <= 0 || dd > cp.band) return kNoGain;
+  return min(min(dq, dr), cp.k) - cp.cost[dd];
+}
+
+// The chaining DP (src/chain.cpp:22-45), 32 anchors a tile, lane t holding row b + t. The
+// predecessors before the tile are read one after the other by all lanes, which depends on
+// nothing in the tile; then row b + s is final at step s and handed to the lanes after it. The
+// reference scans j downwards with a strict '>', so the largest score wins, ties to the
+// nearest j: here j ascends and a tie replaces. Anchors are sorted by (strand, rpos), so the
+// predecessors row b cannot reach by strand or gap no later row can.
+// The 8 reads of 600 to 770 anchors among 4,001 of 1,000 to 5,000 bases set the chaining kernels'
+// time: 472 us with a row's predecessors spread over the lanes and reduced, and the walk of more
+// than 256 anchors by one lane, 320 us with the tiles and the parallel walk; 22,000 reads of the
+// repeat genome 565 -> 471 us.
+__device__ void chain_dp_tiles(const ChainArrays& a, int n, const ChainParamsDev& cp) {
+  const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  for (int i = 0; i < n; ++i) {
-    const uint64_t ki = a.keys[i];
-    const uint32_t si = key_strand(ki);
-    const int64_t ri = key_rpos(ki), qi = key_qpos(ki);
-    int best_sc = 0, best_j = -1;
-    for (int r0 = 0; r0 < cp.lookback; r0 += 32) {
-      const int t = r0 + lane, j = i - 1 - t;
-      bool stop = true;
-      int key = INT_MIN;
-      if (t < cp.lookback && j >= 0) {
+  for (int b = 0; b < n; b += 32) {
+    const int i = b + lane;
+    const uint64_t kb = a.keys[b], ki = a.keys[min(i, n - 1)];
+    const int low = cp.lookback < b ? b - cp.lookback : 0;
+    int start = b;
+    while (start > low) {
+      const int j = start - 1 - lane;
+      bool ok = j >= low;
+      if (ok) {
         const uint64_t kj = a.keys[j];
-        const int64_t dr = ri - key_rpos(kj);
-        if (key_strand(kj) == si && dr <= cp.max_gap) {
-          stop = false;
-          const int64_t dq = qi - key_qpos(kj);
-          if (dr > 0 && dq > 0) {
-            const int64_t dd = dr > dq ? dr - dq : dq - dr;
-            if (dd <= cp.band) {
-              int64_t g = dq < dr ? dq : dr;
-              if (g > cp.k) g = cp.k;
-              const int sc = a.f[j] + static_cast<int>(g) - cp.cost[dd];
-              key = sc * 32 + (31 - lane);
-            }
-          }
-        }
+        ok = key_strand(kj) == key_strand(kb) &&
+             static_cast<int>(key_rpos(kb)) - static_cast<int>(key_rpos(kj)) <= cp.max_gap;
       }
-      const int m = __reduce_max_sync(0xffffffffu, key);
-      if (m != INT_MIN && (best_j < 0 || (m >> 5) > best_sc)) {
-        best_sc = m >> 5;
-        best_j = i - 1 - (r0 + 31 - (m & 31));
-      }
-      if (__all_sync(0xffffffffu, stop)) break;  // every later predecessor is out of range too
+      const unsigned far = ~__ballot_sync(FULL, ok);
+      const int c = far ? __ffs(far) - 1 : 32;
+      start -= c;
+      if (c < 32) break;
     }
-    if (lane == 0) {
-      if (best_j >= 0 && best_sc > cp.k) {
-        a.f[i] = best_sc;
-        a.prev[i] = best_j;
-      } else {
-        a.f[i] = cp.k;
-        a.prev[i] = -1;
+    int best = INT_MIN, bj = -1;
+#pragma unroll 4
+    for (int j = start; j < b; ++j) {
+      const int g = chain_gain(cp, ki, a.keys[j]), sc = a.f[j] + g;
+      if (g != kNoGain && sc >= best && i - j <= cp.lookback) {
+        best = sc;
+        bj = j;
       }
+    }
+    const int rows = min(32, n - b);
+    int g = chain_gain(cp, ki, kb);
+    for (int s = 0; s < rows; ++s) {
+      const int next = chain_gain(cp, ki, a.keys[min(b + s + 1, n - 1)]);
+      const int sc = __shfl_sync(FULL, max(best, cp.k), s) + g;
+      if (lane > s && g != kNoGain && sc >= best && lane - s <= cp.lookback) {
+        best = sc;
+        bj = b + s;
+      }
+      g = next;
+    }
+    if (i < n) {
+      a.f[i] = max(best, cp.k);
+      a.prev[i] = best > cp.k ? bj : -1;
     }
     __syncwarp();
   }
@@ -429,7 +450,7 @@ __device__ int extract_serial(const ChainArrays& a, int n, const ChainParamsDev&
   return m;
 }
 
-// The same chains for n <= 32 * E <= 256 anchors, found without the serial walk. Rank the
+// The same chains for n <= 32 * E <= 1024 anchors, found without the serial walk. Rank the
 // anchors by the extraction order (f descending, index ascending). The walk of end e
 // takes exactly the anchors x whose lowest-ranked descendant in the prev forest (the
 // anchors whose prev path passes through x, x included) is e: ranks of ends taken
@@ -444,8 +465,9 @@ __device__ int extract_serial(const ChainArrays& a, int n, const ChainParamsDev&
 //     are shared-memory atomics into slots at index e.
 // Chain records go to as.ch_*[c0 + e] (slot = end index) and ord[0, m) holds the final
 // order (score descending, extraction order ascending; low 32 bits = slot). The rank key
-// (desc f, index) is packed into 32 bits as (0x7FFFFF - f) << 8 | index, which needs
-// 0 <= f <= 0x7FFFFF; a read outside that (never for k <= 32) uses extract_serial.
+// (desc f, index) is packed into 32 bits as (kTopF - f) << 10 | index, which needs
+// 0 <= f <= kTopF; a read outside that (never for k <= 32) uses extract_serial.
+constexpr int kTopF = 0x3FFFFF;
 template <int E>
 __device__ int extract_par(const ChainArrays& a, int n, const ChainParamsDev& cp, const AnchorScratch& as,
                            int64_t c0) {
@@ -455,11 +477,14 @@ __device__ int extract_par(const ChainArrays& a, int n, const ChainParamsDev& cp
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int y = e * 32 + lane;
-    if (y < n) f_ok = f_ok && a.f[y] >= 0 && a.f[y] <= 0x7FFFFF;
+    if (y < n) f_ok = f_ok && a.f[y] >= 0 && a.f[y] <= kTopF;
   }
   if (!__all_sync(FULL, f_ok)) return extract_serial(a, n, cp, as, c0);
   uint64_t* claim = a.ord;  // claim keys: desc32(f) << 32 | index, min over descendants
-  uint8_t* link = a.used;   // pointer-jumping links + 1 (0 = none); every link < n <= 256
+  using Link = std::conditional_t<(E > 8), uint16_t, uint8_t>;
+  Link* link;  // pointer-jumping links + 1 (0 = none); an anchor's link is below its index
+  if constexpr (E > 8) link = a.link;
+  else link = a.used;
   int anc[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
@@ -467,7 +492,7 @@ __device__ int extract_par(const ChainArrays& a, int n, const ChainParamsDev& cp
     anc[e] = -1;
     if (y < n) {
       anc[e] = a.prev[y];
-      link[y] = static_cast<uint8_t>(anc[e] + 1);
+      link[y] = static_cast<Link>(anc[e] + 1);
       claim[y] = static_cast<uint64_t>(desc32(a.f[y])) << 32 | static_cast<uint32_t>(y);
     }
   }
@@ -489,7 +514,7 @@ __device__ int extract_par(const ChainArrays& a, int n, const ChainParamsDev& cp
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int y = e * 32 + lane;
-      if (y < n) link[y] = static_cast<uint8_t>(anc[e] + 1);
+      if (y < n) link[y] = static_cast<Link>(anc[e] + 1);
     }
     __syncwarp();
   }
@@ -504,10 +529,10 @@ __device__ int extract_par(const ChainArrays& a, int n, const ChainParamsDev& cp
     pk[e] = 0;
     sc[e] = INT_MIN;
     if (y < n) {
-      const int c = static_cast<int>(claim[y] & 0xFFu);
+      const int c = static_cast<int>(claim[y] & 0x3FFu);
       const int p = a.prev[y];
       pk[e] = c == y ? 0x80000000u | static_cast<uint32_t>(a.f[y]) : static_cast<uint32_t>(c);
-      if (p < 0 || static_cast<int>(claim[p] & 0xFFu) != c) sc[e] = a.f[c] - (p >= 0 ? a.f[p] : 0);
+      if (p < 0 || static_cast<int>(claim[p] & 0x3FFu) != c) sc[e] = a.f[c] - (p >= 0 ? a.f[p] : 0);
     }
   }
   __syncwarp();
@@ -564,99 +589,35 @@ __device__ int extract_par(const ChainArrays& a, int n, const ChainParamsDev& cp
     const unsigned b = __ballot_sync(FULL, keep[e]);
     if (keep[e]) {
       const int y = e * 32 + lane;
-      const uint32_t rank = (0x7FFFFFu - (pk[e] & 0x7FFFFFu)) << 8 | static_cast<uint32_t>(y);
+      const uint32_t rank = (kTopF - (pk[e] & kTopF)) << 10 | static_cast<uint32_t>(y);
       a.ord[m + __popc(b & ((1u << lane) - 1u))] = static_cast<uint64_t>(desc32(a.f[y])) << 32 | rank;
     }
     m += __popc(b);
   }
   __syncwarp();
   warp_sort_u64(a.ord, m);
-  for (int j = lane; j < m; j += 32) a.ord[j] = (a.ord[j] & 0xFFFFFFFF00000000ull) | (a.ord[j] & 0xFFu);
+  for (int j = lane; j < m; j += 32) a.ord[j] = (a.ord[j] & 0xFFFFFFFF00000000ull) | (a.ord[j] & 0x3FFu);
   __syncwarp();
   return m;
 }
 
 // Sorts the n anchor keys, runs the DP, extracts chains into as.ch_*[c0 + j] (j a slot
 // below n) and leaves their final order in ord[0, m) (low 32 bits = j). Returns m in
-// every lane.
+// every lane. CAP > 256: a.link holds CAP entries.
+template <int CAP>
 __device__ int chain_core(ChainArrays a, int n, const ChainParamsDev& cp, const AnchorScratch& as, int64_t c0) {
   const int lane = threadIdx.x & 31;
   warp_sort_u64(a.keys, n);
-  // DP (src/chain.cpp:22-45). For row i, lane t holds in registers the key and f of
-  // anchor i-1-t (the 32 nearest predecessors); after the row the window moves up one
-  // lane and row i enters at lane 0, so f never makes a round trip through memory on the
-  // DP's serial path. Predecessors at distance 33..lookback are read from a.keys / a.f
-  // only when the one at distance 32 has not stopped the scan: anchors are sorted by
-  // (strand, rpos), so a strand change or dr > max_gap at j holds for every farther j
-  // too (and each lane can test its own j). One redux per row takes the max of
-  // score * 64 + (63 - distance): the largest score, ties to the nearest predecessor
-  // (the reference scans j downward with a strict '>').
-  const unsigned FULL = 0xffffffffu;
-  if (cp.max_gap < (1 << 29) && chain_dp_clusters(a, n, cp)) {
-    // a lane per cluster
-  } else if (cp.lookback > 64) {
-    chain_dp_rounds(a, n, cp);
-  } else {
-  int rw = 0, qw = 0, fw = 0;
-  uint32_t sw = 0;
-  const bool two = cp.lookback > 32;
-  uint64_t ki = n > 0 ? a.keys[0] : 0;
-  for (int i = 0; i < n; ++i) {
-    const uint64_t knext = i + 1 < n ? a.keys[i + 1] : 0;
-    const uint32_t si = key_strand(ki);
-    const int ri = static_cast<int>(key_rpos(ki)), qi = key_qpos(ki);
-    // rpos < 2^31 and |qpos| < 2^30, so dr and dq fit 32 bits; dd is formed in unsigned
-    // arithmetic and used only when dr and dq passed the range tests
-    const auto score_of = [&](int rj, int qj, uint32_t sj, int fj, int t) -> int {
-      const int dr = ri - rj, dq = qi - qj;
-      const int dd = static_cast<int>(dr > dq ? static_cast<uint32_t>(dr) - static_cast<uint32_t>(dq)
-                                              : static_cast<uint32_t>(dq) - static_cast<uint32_t>(dr));
-      if (t >= cp.lookback || t >= i || sj != si || dr > cp.max_gap || dr <= 0 || dq <= 0 || dd > cp.band)
-        return INT_MIN;
-      const int g = min(min(dq, dr), cp.k);
-      return (fj + g - cp.cost[dd]) * 64 + (63 - t);
-    };
-    int c = score_of(rw, qw, sw, fw, lane);
-    if (two && i > 32) {
-      const bool live = sw == si && ri - rw <= cp.max_gap;  // lane 31: the predecessor i-32
-      if (__shfl_sync(FULL, live, 31)) {
-        __syncwarp();  // f of rows <= i-33, written by lane 0, is visible to every lane
-        const int j = i - 33 - lane;
-        if (j >= 0) {
-          const uint64_t kj = a.keys[j];
-          c = max(c, score_of(static_cast<int>(key_rpos(kj)), key_qpos(kj), key_strand(kj), a.f[j], 32 + lane));
-        }
-      }
-    }
-    const int m = __reduce_max_sync(FULL, c);
-    int fi = cp.k, pi = -1;
-    if (m != INT_MIN && (m >> 6) > cp.k) {
-      fi = m >> 6;
-      pi = i - 1 - (63 - (m & 63));
-    }
-    if (lane == 0) {
-      a.f[i] = fi;
-      a.prev[i] = pi;
-    }
-    // move the window up one lane; row i enters at lane 0
-    rw = __shfl_up_sync(FULL, rw, 1);
-    qw = __shfl_up_sync(FULL, qw, 1);
-    fw = __shfl_up_sync(FULL, fw, 1);
-    sw = __shfl_up_sync(FULL, sw, 1);
-    if (lane == 0) {
-      rw = ri;
-      qw = qi;
-      fw = fi;
-      sw = si;
-    }
-    ki = knext;
-  }
-  }
+  if (cp.max_gap >= (1 << 29) || !chain_dp_clusters(a, n, cp)) chain_dp_tiles(a, n, cp);
   __syncwarp();
   if (n <= 32) return extract_par<1>(a, n, cp, as, c0);
   if (n <= 64) return extract_par<2>(a, n, cp, as, c0);
   if (n <= 128) return extract_par<4>(a, n, cp, as, c0);
   if (n <= 256) return extract_par<8>(a, n, cp, as, c0);
+  if constexpr (CAP > 256) {
+    if (n <= 512) return extract_par<16>(a, n, cp, as, c0);
+    if (n <= 1024) return extract_par<32>(a, n, cp, as, c0);
+  }
   return extract_serial(a, n, cp, as, c0);
 }
 
@@ -793,6 +754,7 @@ struct ChainSmem {
   int32_t f[CAP];
   int32_t prev[CAP];
   uint8_t used[CAP];
+  uint16_t link[CAP > 256 ? CAP : 1];
 };
 
 // Pass 1 of read r by one warp (codes of both strands unless `encode` is false, because
@@ -904,6 +866,7 @@ __device__ void chain_read(int64_t r, const int64_t* __restrict__ pofs, const in
   a.f = small ? smw.f : as.f + a0;
   a.prev = small ? smw.prev : as.prev + a0;
   a.used = small ? smw.used : as.used + a0;
+  a.link = smw.link;
   const int64_t so = pofs[r];
   const int len = seq_len[r], nm = n_min[r], k = cp.k;
   // anchors in minimizer order x occurrence order (src/mapper.cpp:32-40)
@@ -931,7 +894,7 @@ __device__ void chain_read(int64_t r, const int64_t* __restrict__ pofs, const in
     chain_map_small(lane < na ? a.keys[lane] : ~0ULL, na, cp, cand, ix, cb, r);
     return;
   }
-  const int m = chain_core(a, na, cp, as, a0);
+  const int m = chain_core<CAP>(a, na, cp, as, a0);
   // candidate loci (src/mapper.cpp:40-62)
   const int64_t cbase = r * cand.max_cand;
   if (cand.max_cand <= 32) {
@@ -1119,7 +1082,7 @@ __global__ void __launch_bounds__(kChainWarps * 32)
     return;
   }
   ChainArrays a{as.keys + a0, as.f + a0, as.prev + a0, as.ord + a0, as.used + a0};
-  const int m = chain_core(a, static_cast<int>(na64), cp, as, a0);
+  const int m = chain_core<kSmCap>(a, static_cast<int>(na64), cp, as, a0);
   if (lane == 0) out_count[s] = m;
 }
 

@@ -47,3 +47,21 @@ def test_clusters_match_port(ctx, port, cp):
         assert np.array_equal(sr, er) and np.array_equal(sq, eq) and np.array_equal(ss, es), i
         for key in ech:
             assert np.array_equal(ch[key], ech[key]), (i, key)
+
+
+@pytest.mark.parametrize("cp", [(5000, 16, 50, 20, 2), (60, 5, 1, 0, 1), (300, 64, 80, 30, 3), (5000, 16, 0, 15, 1),
+                                (200, 16, 32, 20, 2), (200, 16, 31, 20, 2)])
+def test_long_chains_match_port(ctx, port, cp):
+    """One or two clusters of every size around the tiles of 32 rows, with ties and strays."""
+    rng = np.random.default_rng(12)
+    sets = []
+    for n in (1, 2, 31, 32, 33, 63, 64, 65, 96, 97, 255, 256, 257, 700):
+        for spread in (1, 3, 25):
+            sets.append(clustered_set(rng, [n], cp[0], spread))
+            sets.append(clustered_set(rng, [n, n // 2 + 1], cp[0], spread))
+    got = ctx.chain(sets, 15, D.ChainParams(*cp))
+    for i, ((sr, sq, ss), ch) in enumerate(got):
+        (er, eq, es), ech = port.chain(*sets[i], 15, cp)
+        assert np.array_equal(sr, er) and np.array_equal(sq, eq) and np.array_equal(ss, es), i
+        for key in ech:
+            assert np.array_equal(ch[key], ech[key]), (i, key)
