@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
   const auto step = [&](const int t, auto steady) {
     constexpr bool kSteady = decltype(steady)::value;
     const int i = t - c;
-    const bool act = static_cast<unsigned>(i) < static_cast<unsigned>(end);
+    [[maybe_unused]] const bool act = static_cast<unsigned>(i) < static_cast<unsigned>(end);
     // H, E and the target window advance once the lane has reached row 0 (rows past the
     // pair's end are N rows: they change no result and no code is stored for them); from
     // step LANES - 1 on every lane has, so the steady steps carry no per-cell guard
@@ -937,9 +937,10 @@ __global__ void __launch_bounds__(kSwThreads) k_sw_fb(const SwTask* __restrict__
                                                       const uint8_t* __restrict__ qbase,
                                                       const uint8_t* __restrict__ tbase, SwParams p,
                                                       SwResult* __restrict__ res, uint32_t* __restrict__ dir,
-                                                      int rows_max, const int* __restrict__ fb) {
+                                                      int rows_max, const int* __restrict__ fb, int above) {
   constexpr int WQ = (W + 3) / 4;
   const int nfb = fb[0];
+  if (nfb <= above) return;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nfb; j += gridDim.x * blockDim.x) {
     const int lt = fb[kFbList + j];
     const SwTask tk = tasks[base + lt];
@@ -962,13 +963,14 @@ template <int LANES, int CH, bool TB>
 __global__ void __launch_bounds__(kSwThreads)
     k_sw_fb_lanes(const SwTask* __restrict__ tasks, int base, const uint8_t* __restrict__ qbase,
                   const uint8_t* __restrict__ tbase, SwParams p, SwResult* __restrict__ res,
-                  uint32_t* __restrict__ dir, int rows_max, const int* __restrict__ fb) {
-  static_assert(CH % 4 == 0 && CH >= 8, "a lane's cells fill whole direction words");
+                  uint32_t* __restrict__ dir, int rows_max, const int* __restrict__ fb, int above, int upto) {
+  static_assert(CH % 4 == 0, "a lane's cells fill whole direction words");
   constexpr int W = CH * LANES + 1, WQ = (W + 3) / 4;
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int c = lane % LANES;
   const int nfb = fb[0];
+  if (nfb <= above || nfb > upto) return;  // a list of another form's length
   const int stride = static_cast<int>(gridDim.x * blockDim.x / LANES);
   // a warp takes 32 / LANES consecutive entries of the fallback list per round (jw, the
   // first, is warp-uniform, so every lane takes the same rounds)
@@ -1435,23 +1437,44 @@ void run_u2(const SwLaunch& a, int above) {
   a.kt.end(a.st);
 }
 
-// The int32 kernel over the listed tasks: several lanes per alignment at W = 33, 65 and 129
-// (narrow chunks: its time is one task's serial latency), else one thread, whose band fits
-// in registers. The list's length is known on the device only (usually short or empty), so
-// the kernel strides over it with a few resident waves.
+// The int32 kernel over the listed tasks. The list's length is known on the device only
+// (usually short or empty), so the kernels stride over it with a few resident waves. A short
+// list's time is one task's serial latency, so four cells a lane, whose row is the shortest; a
+// longer one's is its instructions: 8 or 16 cells, or a thread per task. Tracebacks of 150
+// rows, us, short form against the other: W = 17 56 and 102 for 500 tasks, 70 and 105 for
+// 5,000, 272 and 193 for 50,000; W = 33 53 and 77, 91 and 103, 545 and 435; W = 129 60 and
+// 105, 268 and 227, 3,262 and 1,506. (One kernel with both forms ran the longer lists 5 to 45 %
+// slower.)
 template <int W>
 void run_fb(const SwLaunch& a) {
+  constexpr bool kShort = (W - 1) % 4 == 0, kLanes = W == 33 || W == 65 || W == 129;
   constexpr int CH = W == 33 ? 8 : 16;
-  constexpr bool kLanes = W == 33 || W == 65 || W == 129;
-  constexpr int L = kLanes ? (W - 1) / CH : 1;
-  const int blocks = std::min(
-      8 * device_sm_count(), static_cast<int>((static_cast<int64_t>(a.count) * L + kSwThreads - 1) / kSwThreads));
-  const auto run = [&](auto kernel) {
-    kernel<<<blocks, kSwThreads, 0, a.st>>>(a.tasks, a.base, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb);
+  const int few = kShort ? 262144 / (W - 1) : 0;
+  const auto grid = [&](int lanes) {
+    return std::min(8 * device_sm_count(),
+                    static_cast<int>((static_cast<int64_t>(a.count) * lanes + kSwThreads - 1) / kSwThreads));
+  };
+  const auto lanes = [&](auto kernel, int l, int above, int upto) {
+    kernel<<<grid(l), kSwThreads, 0, a.st>>>(a.tasks, a.base, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max, a.fb,
+                                             above, upto);
   };
   a.kt.begin(a.st, a.tb ? "k_sw_fb<tb>" : "k_sw_fb<score>");
-  if constexpr (kLanes) a.tb ? run(k_sw_fb_lanes<L, CH, true>) : run(k_sw_fb_lanes<L, CH, false>);
-  else a.tb ? run(k_sw_fb<W, true>) : run(k_sw_fb<W, false>);
+  if constexpr (kShort) {
+    constexpr int L = (W - 1) / 4;
+    a.tb ? lanes(k_sw_fb_lanes<L, 4, true>, L, 0, few) : lanes(k_sw_fb_lanes<L, 4, false>, L, 0, few);
+  }
+  if (a.count > few) {
+    if constexpr (kLanes) {
+      constexpr int L = (W - 1) / CH;
+      a.tb ? lanes(k_sw_fb_lanes<L, CH, true>, L, few, INT_MAX) : lanes(k_sw_fb_lanes<L, CH, false>, L, few, INT_MAX);
+    } else {
+      const auto run = [&](auto kernel) {
+        kernel<<<grid(1), kSwThreads, 0, a.st>>>(a.tasks, a.base, a.qbase, a.tbase, a.p, a.res, a.dir, a.rows_max,
+                                                 a.fb, few);
+      };
+      a.tb ? run(k_sw_fb<W, true>) : run(k_sw_fb<W, false>);
+    }
+  }
   a.kt.end(a.st);
 }
 

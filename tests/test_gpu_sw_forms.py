@@ -76,3 +76,22 @@ def test_bands_that_end_inside_a_lane(ctx, port, form, scheme):
     finally:
         ctx.set_option("sw_form", 0)
         ctx.set_option("ungapped", 1)
+
+
+@pytest.mark.parametrize("bw,n", [(8, 300), (8, 17_000), (16, 300), (16, 8_192), (16, 8_200), (64, 2_000), (64, 2_100),
+                                  (21, 300)])
+def test_windows_with_n_match_port(ctx, port, bw, n):
+    """Tasks of the int32 kernel: an N in every target window, lists on both sides of the length
+    from which it takes more cells a lane."""
+    rng = np.random.default_rng(bw + n)
+    sc = (2, 4, 4, 2, 1, bw)
+    qs, ts = short_tasks(rng, rng.integers(1, 80, 300), bw)
+    for q, t in zip(qs, ts):
+        t[int(rng.integers(len(q)))] = 4
+    times = -(-n // len(qs))
+    want = (port.align(qs, ts, True, sc) * times)[:n]
+    try:
+        ctx.set_option("ungapped", 0)
+        check_same(ctx.align((qs * times)[:n], (ts * times)[:n], True, D.ScoreParams(*sc)), want, True)
+    finally:
+        ctx.set_option("ungapped", 1)
