@@ -154,7 +154,8 @@ TASK_BYTES = 48 + 32  # SW task descriptor in, result out
 def kernel_bytes(kernel: str, st: dict, mean_len: float, bw: int = 16) -> float | None:
     """Algorithmic HBM bytes of all launches of one kernel, from the batch counters in st
     (reads, minimizers, anchors, candidates, SW tasks; the warp_* counters cover the reads
-    listed for the warp-per-read kernels). None for kernels not modelled."""
+    listed for the warp-per-read kernels; sw_tasks_dp, the traceback tasks the ungapped proof
+    left to the DP kernels). None for kernels not modelled."""
     n = st["reads"]
     mins = st["minimizers"] if st.get("minimizers") else 0.18 * mean_len * n
     W = 2 * bw + 1
@@ -174,8 +175,16 @@ def kernel_bytes(kernel: str, st: dict, mean_len: float, bw: int = 16) -> float 
         # 21-B candidate out, 28 B of per-read offsets / counts
         r = st["warp_reads"]
         return st["warp_minimizers"] * 20 + st["warp_anchors"] * 4 + r * cand_per_read * 21 + r * 28
-    if kernel in ("k_sw_u2<tb>", "k_sw_wide<tb>"):  # query + window in, direction codes out, task/result
+    if kernel == "k_sketch_reads":  # codes in, 8-B minimizer out, offsets / lengths / counts
+        return n * mean_len + mins * 8 + n * 16
+    if kernel == "k_probe_reads":  # 8-B minimizer in, 16-B bucket, 4-B occurrence per anchor, 21-B candidate
+        # out, 40 B of per-read offsets / lengths / counts
+        return mins * (8 + 16) + st["anchors"] * 4 + st["candidates"] * 21 + n * 40
+    if kernel == "k_sw_ungapped<tb>":  # query + window in, task/result, the one-operation CIGAR
         t = st["sw_tasks_tb"]
+        return t * (mean_len + (mean_len + 2 * bw) + TASK_BYTES + 4)
+    if kernel in ("k_sw_u2<tb>", "k_sw_wide<tb>"):  # query + window in, direction codes out, task/result
+        t = st.get("sw_tasks_dp", st["sw_tasks_tb"])
         return t * (mean_len + (mean_len + 2 * bw) + mean_len * dir_row + TASK_BYTES)
     if kernel in ("k_sw_u2<score>", "k_sw_wide<score>"):
         t = st["sw_tasks_score"]
@@ -813,7 +822,14 @@ def run_ours(args) -> None:
     mean_len = float(np.mean(reads.seq_len))
     launches, dom_ms = ktimes[dom]
     avg_launch_ms = dom_ms / launches
-    algo = kernel_bytes(dom, dict(st, sw_tasks_tb=dom_tb_tasks), mean_len, args.bw)
+    # the share of the traceback tasks that the ungapped proof leaves to the DP kernels, from the
+    # form tuner's first batch (the counters count them all)
+    dp_share = 1.0
+    for t in ctx.sw_tuning():
+        if t["W"] == 2 * args.bw + 1 and t["traceback"] and t["tasks"] > 0:
+            dp_share = min(1.0, t["tasks"] / max(min(n_reads, BATCH), 1))
+    dom_dp_tasks = dom_tb_tasks * dp_share
+    algo = kernel_bytes(dom, dict(st, sw_tasks_tb=dom_tb_tasks, sw_tasks_dp=dom_dp_tasks), mean_len, args.bw)
     peak, peak_kind = measured_peaks()
     achieved = (algo / launches) / (avg_launch_ms / 1e3) / 1e9 if algo is not None else None
     traffic = None  # DRAM bytes per launch of this kernel from the committed ncu summary
@@ -846,7 +862,7 @@ def run_ours(args) -> None:
     roof_int = None
     if dom.startswith("k_sw_u2<tb>") or dom.startswith("k_sw_wide<tb>"):
         W = 2 * args.bw + 1
-        cells_per_launch = dom_tb_tasks * mean_len * W / launches
+        cells_per_launch = dom_dp_tasks * mean_len * W / launches
         roof_int = int_roofline(local, stream, dom, cells_per_launch, avg_launch_ms, inst_per_cell)
         one = breakdown[dom][1] / breakdown[dom][0]
         if "peak_cells_per_s" in roof_int:

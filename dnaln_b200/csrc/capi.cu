@@ -6,22 +6,23 @@
 //   k_len_scan: packed read offsets, total bases, longest read (read back first only
 //     when the caller did not give the batch's size, so the rest can run as a graph)
 //   k_encode_reads: codes of both strands of every read
-//   k_seed_chain_t: short reads one thread each (sketch, probe, anchors, chaining DP,
+//   k_sketch_reads, k_probe_reads: minimizers, and the candidate of every read whose anchors
+//     are proved to give one chain; the others are listed
+//   k_seed_chain_t: listed short reads one thread each (sketch, probe, anchors, chaining DP,
 //     chains, candidate loci); reads it cannot take are listed
 //   k_seed_chain_tl: listed long reads one thread each, longest first; what exceeds its
 //     bounds is listed again
 //   k_seed<list> + k_chain_map<list>: the reads still listed, one warp each
+//   (banded SW below: k_sw_ungapped takes the tasks proved to have no gap, the DP the rest)
 //   score-only SW over every candidate of reads with >= 2 candidates, then k_choose
 //     (best / ties / second best, fnv1a tie-break, the traceback task of each read)
 //   SW with traceback over each read's chosen candidate (chunked by scratch size), walk
-//   k_records (MAPQ, positions, soft clips), CIGAR offsets (scan), k_cigar_gather
+//   k_records (MAPQ, positions, soft clips), k_cigar_gather
 //   one read-back of the batch's totals, task counts, error flags and counters
 // Task and list counts produced on the device are consumed on the device, so the host
 // waits once per batch. The host-buffer entry points queue parts of a batch to a worker
 // thread that overlaps their copies in and out with the compute (two device slots, two
 // copy streams).
-#include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>

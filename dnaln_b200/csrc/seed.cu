@@ -21,12 +21,11 @@
 // 64-bit key (strand, rpos, qpos) so the reference's sort is a warp bitonic sort of
 // integers. The DP scans predecessors nearest-first with a `break` on strand change or
 // dr > max_gap; because anchors are sorted by (strand, rpos), the scanned predecessors
-// form one contiguous range, so the lanes test up to 32 predecessors each round
-// independently and a warp max over (score << 32 | j) picks the best with ties to the
-// nearest j, as the reference's strict '>' does. The FP64 gap cost comes from a
+// form one contiguous range. The lanes hold the rows of a tile of 32 anchors, or one cluster
+// each; ties go to the nearest j, as the reference's strict '>' does. The FP64 gap cost comes from a
 // host-computed table (exactly the reference's expression). Chains are extracted from end
-// points in (f desc, index asc) order — another bitonic sort of packed keys — walked by
-// one lane, and ordered by score with ties in extraction order (the reference's
+// points in (f desc, index asc) order (extract_par; above 1,024 anchors a sort and a walk by
+// one lane) and ordered by score with ties in extraction order (the reference's
 // stable_sort). Candidate loci follow src/mapper.cpp:40-62.
 #include <algorithm>
 #include <type_traits>

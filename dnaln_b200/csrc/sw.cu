@@ -9,23 +9,23 @@
 // with H = E = 0 for row -1 and for the fixed out-of-band cell d = W, F = H(left) = 0 at
 // each row start, and the target N-padded to qlen + W - 1.
 //
-// Kernels (inter-sequence: a thread owns whole alignments, no intra-row shuffles):
-//  * k_sw_u2<W>: two alignments per thread, one in each 16-bit half of 32-bit
+// Kernels:
+//  * k_sw_u2<W> (a thread owns whole alignments, no intra-row shuffles): two alignments per thread, one in each 16-bit half of 32-bit
 //    registers, the band row (H, E of W+1 cells, W target selectors) in registers.
 //    Values are kept biased by +16384, so every half stays positive and every add or
 //    subtract of the recurrence is one 32-bit integer add on both halves (no borrow can
 //    cross halves); E and F are DPX add-maxima (viaddmax), the other maxima unsigned 16x2
 //    max (vmaxu2 / DPX vimax3_u16x2). The substitution scores of both alignments are one
 //    prmt.b32 from an 8-byte per-row profile {s(qA, A..T) + 64, s(qB, A..T) + 64}.
-//    Direction bits come from non-negative differences (hd vs max(hd, E), ...)
-//    saturated to 0/1 with vminu2 and combined with integer multiply-adds.
+//    Direction flags are the signs of non-negative differences (cell2).
 //    With traceback it stores the direction codes and only the best cell; the walk is a
-//    separate kernel (k_sw_walk, one thread per alignment, few registers, full occupancy)
-//    so the DP kernel's register footprint does not carry the walk.
+//    separate kernel (k_sw_walk, few registers, full occupancy) so the DP kernel's
+//    register footprint does not carry the walk.
+//  * k_sw_wide<W, LANES, CH>: the same cells, several lanes per pair of alignments.
 //  * A task whose target window may contain an N (the 4-entry profile cannot score it),
 //    or whose scores or lengths do not fit the biased 16-bit range, is appended by
-//    k_sw_u2 to a device-side list; k_sw_fb runs the same cell update in int32 for the
-//    listed tasks (sw_one_reg), same outputs and codes. Genome windows that the task
+//    them to a device-side list; k_sw_fb and k_sw_fb_lanes run the same cell update in
+//    int32 for the listed tasks, same outputs and codes. Genome windows that the task
 //    builder marked N-free (kTaskNoN) skip the per-task N scan.
 //  * k_sw_any: any band width and any scores (int32, band rows in per-warp scratch).
 //
@@ -36,8 +36,7 @@
 // (kExtE), 8 + c (kNotE) and 12 + c (kExtF): the order in which cell2 gets them.
 // On every cell the walk reads, H is the positive value being traced; there it came from the
 // diagonal if h == hd (src/align.cpp:67), else from E if h == e, and otherwise from F — so
-// the walk (src/align.cpp:87-143)
-// takes the reference's steps. The best cell is the first strict maximum in row-major
+// the walk (src/align.cpp:87-143) takes the reference's steps. The best cell is the first strict maximum in row-major
 // order (per-row maximum with its first column, then strict across rows).
 #include <algorithm>
 #include <climits>
