@@ -1107,37 +1107,24 @@ __global__ void __launch_bounds__(kSwThreads)
 // Against one thread per task: 4,001 reads of 1-5 kbp 1,789 -> 236 us, 200,003 of 50-1000 bp
 // 398 -> 258, 64 of 100-300 bp 43 -> 17. Where short walks fill the SMs by themselves
 // (262,144 of 150 bp) the lanes' extra instructions cost more than the latencies they hide
-// (122 -> 181 us), so those run one thread per task.
+// (122 -> 181 us), so those run one thread per task. Short lists take a warp per task, 256 rows
+// per latency: 4,001 of 1-5 kbp 222 -> 82 us, 64 of 100-300 bp 17 -> 11; 8 lanes against 32, of
+// 150 rows 19 and 17 us at 4,096, 21 and 23 at 8,192, of 1,000 rows 62 and 53 at 8,192, 84 and 95
+// at 16,384.
 constexpr int kWalkLanes = 8;
 constexpr int kWalkMany = 98304, kWalkShort = 256;  // more tasks of at most this many rows: one thread each
-template <int W>
-__global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restrict__ tasks, int base, int count, int n,
-                                                        const int* __restrict__ n_dev,
-                                                        const uint8_t* __restrict__ qbase,
-                                                        const uint8_t* __restrict__ tbase, SwParams p,
-                                                        SwResult* __restrict__ res, const uint32_t* __restrict__ dir,
-                                                        int rows_max, uint32_t* __restrict__ cig,
-                                                        const int64_t* __restrict__ cig_off,
-                                                        uint32_t* __restrict__ err) {
+constexpr int kWalkFew = 6144;                      // up to this many tasks: a warp each
+
+// The walks of tasks [base, base + nn), G lanes each.
+template <int W, int G>
+__device__ __forceinline__ void walk_lanes(const SwTask* __restrict__ tasks, int base, int nn,
+                                           const uint8_t* __restrict__ qbase, const uint8_t* __restrict__ tbase,
+                                           const SwParams& p, SwResult* __restrict__ res,
+                                           const uint32_t* __restrict__ dir, int rows_max, uint32_t* __restrict__ cig,
+                                           const int64_t* __restrict__ cig_off, uint32_t* __restrict__ err) {
   constexpr int WQ = (W + 3) / 4;
-  constexpr int G = kWalkLanes;
-  const int nn = min(base + count, n_dev ? min(n, *n_dev) : n) - base;  // tasks of this launch
-  if (rows_max <= kWalkShort && nn > kWalkMany) {  // the launch has a thread per task then
-    const int lt = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lt >= nn) return;
-    const SwTask tk = tasks[base + lt];
-    const SwResult s = res[tk.slot];
-    SwResult r{s.score, 0, 0, 0, 0, 0, 0, 0};
-    if (s.score > 0) {
-      const PairCodes codes{pair_base(const_cast<uint32_t*>(dir), lt, rows_max, WQ), WQ, lt & 1};
-      traceback(codes, W, s.qb, s.qe, s.score, qbase + tk.q_off, tbase, tk, p, r, cig + cig_off[tk.slot],
-                2 * tk.qlen + 1, err);
-    }
-    res[tk.slot] = r;
-    return;
-  }
   const int lane = threadIdx.x & 31, gl = lane & (G - 1);
-  const unsigned gm = ((1u << G) - 1u) << (lane & ~(G - 1));
+  const unsigned gm = (G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u) << (lane & ~(G - 1));
   const int smax = max(p.match, max(-p.mismatch, -p.ambig));  // the most one step can lower v
   const int stride = static_cast<int>(gridDim.x * blockDim.x) / G;
   for (int lt = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x) / G; lt < nn; lt += stride) {
@@ -1161,7 +1148,7 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
           const int sh = code.shift(d);
           uint32_t cx = 0;  // row top - k of the block: kNotDiag in bit k, kNotE in bit 8 + k
           uint64_t qw = 0, tw = 0;  // its bases, row top - k in byte 7 - k; N past any end
-          int lost = 0;             // what the block takes from v, and 256ths of it its mismatches
+          int lost = 0;             // what the block takes from v, times 1,024, and its mismatches
           bool clean = false;
           if (top >= 0) {
             const int64_t x0 = tk.t_start + (top - (kAhead - 1)) + d;  // target of row top - 7
@@ -1175,7 +1162,7 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
               const uint64_t ok_amb = zero_bytes((qw | tw) & 0xFCFCFCFCFCFCFCFCull);
               const int n_match = __popcll(zero_bytes(qw ^ tw) & ok_amb);
               const int n_amb = kAhead - __popcll(ok_amb);
-              lost = (n_match * p.match - (kAhead - n_match - n_amb) * p.mismatch - n_amb * p.ambig) * 256 +
+              lost = (n_match * p.match - (kAhead - n_match - n_amb) * p.mismatch - n_amb * p.ambig) * 1024 +
                      (kAhead - n_match);
             } else {
 #pragma unroll
@@ -1189,20 +1176,20 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
               }
             }
           }
-          int sum = lost;  // inclusive prefix over the lanes (mismatches stay below 256)
+          int sum = lost;  // inclusive prefix over the lanes (mismatches stay below 1,024)
 #pragma unroll
           for (int o = 1; o < G; o <<= 1) {
             const int y = __shfl_up_sync(gm, sum, o, G);
             if (gl >= o) sum += y;
           }
-          const int before = (sum - lost) >> 8;  // the arithmetic shift drops the mismatches
+          const int before = (sum - lost) >> 10;  // the arithmetic shift drops the mismatches
           const bool take = clean && v - before > (kAhead - 1) * smax;
           const unsigned not_ok = (__ballot_sync(gm, !take) & gm) >> (lane & ~(G - 1));
           const int c = not_ok ? __ffs(not_ok) - 1 : G;
           if (c > 0) {
             const int t = __shfl_sync(gm, sum, c - 1, G);
-            v -= t >> 8;
-            nm += t & 255;
+            v -= t >> 10;
+            nm += t & 1023;
             run += kAhead * c;
             i -= kAhead * c;
           }
@@ -1282,6 +1269,35 @@ __global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restr
     }
     if (gl == 0) res[tk.slot] = r;
   }
+}
+
+template <int W>
+__global__ void __launch_bounds__(kSwThreads, 7) k_sw_walk(const SwTask* __restrict__ tasks, int base, int count, int n,
+                                                        const int* __restrict__ n_dev,
+                                                        const uint8_t* __restrict__ qbase,
+                                                        const uint8_t* __restrict__ tbase, SwParams p,
+                                                        SwResult* __restrict__ res, const uint32_t* __restrict__ dir,
+                                                        int rows_max, uint32_t* __restrict__ cig,
+                                                        const int64_t* __restrict__ cig_off,
+                                                        uint32_t* __restrict__ err) {
+  constexpr int WQ = (W + 3) / 4;
+  const int nn = min(base + count, n_dev ? min(n, *n_dev) : n) - base;  // tasks of this launch
+  if (rows_max <= kWalkShort && nn > kWalkMany) {  // the launch has a thread per task then
+    const int lt = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lt >= nn) return;
+    const SwTask tk = tasks[base + lt];
+    const SwResult s = res[tk.slot];
+    SwResult r{s.score, 0, 0, 0, 0, 0, 0, 0};
+    if (s.score > 0) {
+      const PairCodes codes{pair_base(const_cast<uint32_t*>(dir), lt, rows_max, WQ), WQ, lt & 1};
+      traceback(codes, W, s.qb, s.qe, s.score, qbase + tk.q_off, tbase, tk, p, r, cig + cig_off[tk.slot],
+                2 * tk.qlen + 1, err);
+    }
+    res[tk.slot] = r;
+    return;
+  }
+  if (nn <= kWalkFew) walk_lanes<W, 32>(tasks, base, nn, qbase, tbase, p, res, dir, rows_max, cig, cig_off, err);
+  else walk_lanes<W, kWalkLanes>(tasks, base, nn, qbase, tbase, p, res, dir, rows_max, cig, cig_off, err);
 }
 
 // Any band width and any scores: one alignment per thread, int32, band rows H, E in
@@ -1497,7 +1513,7 @@ void launch_band(const SwLaunch& a, SwForm form, int few) {
   if (a.tb) {
     const int lane_blocks = std::min(
         16 * device_sm_count(),
-        static_cast<int>((static_cast<int64_t>(a.count) * kWalkLanes + kSwThreads - 1) / kSwThreads));
+        static_cast<int>((static_cast<int64_t>(a.count) * 32 + kSwThreads - 1) / kSwThreads));
     const int blocks = a.rows_max <= kWalkShort && a.count > kWalkMany
                            ? std::max(lane_blocks, (a.count + kSwThreads - 1) / kSwThreads)
                            : lane_blocks;

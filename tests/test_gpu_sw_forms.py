@@ -95,3 +95,28 @@ def test_windows_with_n_match_port(ctx, port, bw, n):
         check_same(ctx.align((qs * times)[:n], (ts * times)[:n], True, D.ScoreParams(*sc)), want, True)
     finally:
         ctx.set_option("ungapped", 1)
+
+
+@pytest.mark.parametrize("times", [1, 70])
+def test_walks_over_long_runs_of_free_mismatches(ctx, port, times):
+    """Mismatches that cost nothing fill every row a walk takes at once, in lists on both sides
+    of the length up to which a task has a warp."""
+    rng = np.random.default_rng(21)
+    sc = (2, 0, 4, 2, 0, 16)
+    qs, ts = [], []
+    for i in range(90):
+        core = rng.integers(0, 4, 700 + i).astype(np.uint8)
+        q = core.copy()
+        a, m = 40 + 3 * (i % 30), 100 + 6 * i
+        q[a:a + m] = 4 if i % 2 else (q[a:a + m] + 1) % 4
+        q = q[:len(q) - 16]
+        s = int(rng.integers(0, 33))
+        qs.append(q)
+        ts.append(np.concatenate([rng.integers(0, 4, s).astype(np.uint8), core,
+                                  rng.integers(0, 4, 40).astype(np.uint8)]))
+    want = port.align(qs, ts, True, sc) * times
+    try:
+        ctx.set_option("ungapped", 0)
+        check_same(ctx.align(qs * times, ts * times, True, D.ScoreParams(*sc)), want, True)
+    finally:
+        ctx.set_option("ungapped", 1)
