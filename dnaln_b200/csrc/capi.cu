@@ -1336,10 +1336,11 @@ bool read_facts(const int64_t* off, const int32_t* len, int64_t a, int64_t b, Ma
 // 2,049; 524,288 4,155, 3,427, 3,500.
 constexpr int64_t kSplitBases = 16 << 20;
 
-// Queues a batch (see dnaln_gpu_map_submit). *alone = nothing was queued before it.
+// Queues a batch (see dnaln_gpu_map_submit). *split: may go in two parts / does. *alone =
+// nothing was queued before it.
 int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_off, const int32_t* seq_len,
                  const uint32_t* name_hash, int64_t n, const dnaln_map_params* p, dnaln_map_record* out,
-                 uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used, bool split, int64_t* ticket, bool* alone) {
+                 uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used, bool* split, int64_t* ticket, bool* alone) {
   if (!c || n < 0 || !cigar_used || !ticket || !p || (n > 0 && (!seq || !seq_off || !seq_len || !name_hash || !out)))
     return fail(c, DNALN_ERR_INVALID_ARG, "null argument");
   *ticket = 0;
@@ -1348,8 +1349,8 @@ int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_o
   // whoever drives the device); their failures come back from dnaln_gpu_map_wait
   if (int e = validate_map_params_basic(c, p)) return e;
   // parts of at most sub_batch reads, with their host-side facts (lengths are known here)
-  split = split && c->sub_batch == 0 && n >= 2;
-  const int64_t S = c->sub_batch > 0 ? c->sub_batch : (split ? (n + 1) / 2 : std::max<int64_t>(n, 1));
+  *split = *split && c->sub_batch == 0 && n >= 2;
+  const int64_t S = c->sub_batch > 0 ? c->sub_batch : (*split ? (n + 1) / 2 : std::max<int64_t>(n, 1));
   std::vector<MapPart> parts;
   for (int64_t a = 0; a < n; a += S) {
     MapPart pt;
@@ -1368,8 +1369,8 @@ int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_o
     parts.push_back(pt);
   }
   // one part if it is small or the halves' reads are not apart in the buffer
-  if (split && (parts[0].bases + parts[1].bases < kSplitBases ||
-                std::min(parts[0].hi, parts[1].hi) > std::max(parts[0].lo, parts[1].lo))) {
+  if (*split && (parts[0].bases + parts[1].bases < kSplitBases ||
+                 std::min(parts[0].hi, parts[1].hi) > std::max(parts[0].lo, parts[1].lo))) {
     MapPart& all = parts[0];
     const MapPart& rest = parts[1];
     all.b = rest.b;
@@ -1379,6 +1380,7 @@ int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_o
     all.max_len = std::max(all.max_len, rest.max_len);
     all.cig_bound += rest.cig_bound;
     parts.pop_back();
+    *split = false;
   }
   std::lock_guard<std::mutex> g(c->qmu);
   const int64_t t = c->next_ticket++;
@@ -2402,8 +2404,8 @@ int dnaln_gpu_map_batch_device(dnaln_ctx* c, int32_t id, const char* d_seq, cons
 int dnaln_gpu_map_submit(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_off, const int32_t* seq_len,
                          const uint32_t* name_hash, int64_t n, const dnaln_map_params* p, dnaln_map_record* out,
                          uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used, int64_t* ticket) {
-  bool alone = false;
-  if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, false,
+  bool alone = false, split = false;
+  if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, &split,
                            ticket, &alone))
     return e;
   wake_worker(c);
@@ -2427,10 +2429,11 @@ int dnaln_gpu_map_wait(dnaln_ctx* c, int64_t ticket) {
 int dnaln_gpu_map_batch(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_off, const int32_t* seq_len,
                         const uint32_t* name_hash, int64_t n, const dnaln_map_params* p, dnaln_map_record* out,
                         uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used) {
-  const auto map = [&](bool split) {
+  bool split = true;
+  const auto map = [&]() {
     int64_t ticket = 0;
     bool alone = false;
-    if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, split,
+    if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, &split,
                              &ticket, &alone))
       return e;
     // with nothing queued before it and the device free, the batch runs in the calling thread:
@@ -2444,9 +2447,10 @@ int dnaln_gpu_map_batch(dnaln_ctx* c, int32_t id, const char* seq, const int64_t
     if (!here) wake_worker(c);
     return dnaln_gpu_map_wait(c, ticket);
   };
-  const int e = map(true);
-  // a CIGAR buffer too small for the batch is reported for the whole of it
-  return e == DNALN_ERR_CAPACITY && n > 1 && c->sub_batch == 0 ? map(false) : e;
+  const int e = map();
+  if (e != DNALN_ERR_CAPACITY || !split) return e;
+  split = false;  // a CIGAR buffer too small for the batch is reported for the whole of it
+  return map();
 }
 
 }  // extern "C"
