@@ -1079,20 +1079,21 @@ __global__ void __launch_bounds__(kSwThreads)
       T[CH] = t_next;
     }
   }
-  // the lanes of the alignment: larger value, then earlier row, then smaller column
-  uint64_t key = static_cast<uint64_t>(best) << 40 |
-                 static_cast<uint64_t>(0xFFFFFu - static_cast<uint32_t>(bi + 1)) << 12 |
-                 (0xFFFu - static_cast<uint32_t>(bd < 0 ? 0xFFF : bd));
+  // the lanes of the alignment: larger value, then earlier row, then smaller column (rows and
+  // scores here pass 2^20 and 2^24, so a key holds 32 bits of each and the column goes beside it)
+  uint64_t key = static_cast<uint64_t>(best) << 32 | ~static_cast<uint32_t>(bi + 1);
 #pragma unroll
   for (int o = 1; o < LANES; o <<= 1) {
-    const uint64_t x = __shfl_xor_sync(FULL, key, o);
-    key = x > key ? x : key;
+    const uint64_t xk = __shfl_xor_sync(FULL, key, o);
+    const int xd = __shfl_xor_sync(FULL, bd, o);
+    if (xk > key || (xk == key && xd < bd)) {
+      key = xk;
+      bd = xd;
+    }
   }
   if (c == 0 && live) {
-    const int kb = static_cast<int>(key >> 40);
-    const int kbi = static_cast<int>(0xFFFFFu - static_cast<uint32_t>((key >> 12) & 0xFFFFFu)) - 1;
-    const int kbd = static_cast<int>(0xFFFu - static_cast<uint32_t>(key & 0xFFFu));
-    res[tk.slot] = TB ? stash(kb, kbi, kbd) : stash(kb, 0, 0);
+    const int kb = static_cast<int>(key >> 32), kbi = static_cast<int>(~static_cast<uint32_t>(key)) - 1;
+    res[tk.slot] = TB ? stash(kb, kbi, bd) : stash(kb, 0, 0);
   }
   }
 }
