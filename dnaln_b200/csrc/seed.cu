@@ -607,7 +607,9 @@ template <int CAP>
 __device__ int chain_core(ChainArrays a, int n, const ChainParamsDev& cp, const AnchorScratch& as, int64_t c0) {
   const int lane = threadIdx.x & 31;
   warp_sort_u64(a.keys, n);
-  if (cp.max_gap >= (1 << 29) || !chain_dp_clusters(a, n, cp)) chain_dp_tiles(a, n, cp);
+  // the clusters' cutoff holds while no pair gains more than k, that is while no gap cost is below
+  // zero: int(0.01 k dd + ...) is for k < 0, which the chaining entry point takes
+  if (cp.k < 0 || cp.max_gap >= (1 << 29) || !chain_dp_clusters(a, n, cp)) chain_dp_tiles(a, n, cp);
   __syncwarp();
   if (n <= 32) return extract_par<1>(a, n, cp, as, c0);
   if (n <= 64) return extract_par<2>(a, n, cp, as, c0);

@@ -1,0 +1,26 @@
+"""The chaining DP where a gap earns instead of costs: the gap cost int(0.01 k dd + 0.5 log2 dd) is
+negative for a k below zero, so a predecessor may add more than k. Many small clusters of anchors,
+against the oracle."""
+import numpy as np
+import pytest
+
+import dnaln_b200 as D
+from test_gpu_chain_clusters import clustered_set
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("k", [-30, -10, -1, 0, 1])
+def test_chaining_with_any_k_matches_port(ctx, port, k):
+    rng = np.random.default_rng(100 + k)
+    cp = (5000, 400, 50, -1000, 1)
+    sets = []
+    for clusters in (6, 8, 20):
+        sr, sq, ss = clustered_set(rng, rng.integers(3, 12, clusters), cp[0], 300)
+        sets.append((sr, (sq + rng.integers(0, 300, len(sq))).astype(np.int32), ss))
+    got = ctx.chain(sets, k, D.ChainParams(*cp))
+    for i, ((sr, sq, ss), ch) in enumerate(got):
+        (er, eq, es), ech = port.chain(*sets[i], k, cp)
+        assert np.array_equal(sr, er) and np.array_equal(sq, eq) and np.array_equal(ss, es), i
+        for key in ech:
+            assert np.array_equal(ch[key], ech[key]), (i, key)
