@@ -75,6 +75,7 @@ struct IndexRes {
   uint64_t n_keys = 0, n_pos = 0, n_buckets = 0, n_bases = 0;
   uint32_t max_count = 0;
   int32_t n_contigs = 0, k = 0, w = 0;
+  bool foreign_keys = false;  // the table (uploaded or loaded) holds keys above 2^32 that no k-mer has
   DevIndex dev{};
 };
 
@@ -669,7 +670,8 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
     const int32_t* full_list = nullptr;
     const int* full_n = nullptr;
     int32_t* rest_list = nullptr;
-    if (c->colinear && seed_colinear_supported(sp, cp, ix.dev)) {
+    // (its probe takes a key above 2^32 for an empty bucket)
+    if (c->colinear && !ix.foreign_keys && seed_colinear_supported(sp, cp, ix.dev)) {
       DBUF(rest, int32_t, "colinear_rest", n);
       DBUF(with_n, int32_t, "colinear_with_n", n);
       const int lanes = seed_colinear_lanes(n, max_len);
@@ -1126,12 +1128,13 @@ int check_contigs(dnaln_ctx* c, const uint64_t* contig_off, const uint32_t* cont
 struct TableCheck {
   uint64_t n_pos = 0, n_bases = 0, n_keys = 0;
   uint32_t max_count = 0;
-  bool ok = true;
+  bool ok = true, high_keys = false;
   void buckets(const ulonglong2* t, size_t n) {
     for (size_t i = 0; i < n; ++i) {
       if (t[i].x == kInvalidHash) continue;
       const uint64_t off = static_cast<uint32_t>(t[i].y), cnt = t[i].y >> 32;
       ok = ok && off + cnt <= n_pos;
+      high_keys = high_keys || t[i].x >> 32 != 0;
       ++n_keys;
       if (cnt > max_count) max_count = static_cast<uint32_t>(cnt);
     }
@@ -2041,6 +2044,7 @@ int dnaln_gpu_index_load(dnaln_ctx* c, const char* path, int32_t* index_id) {
   r.n_contigs = h.n_contigs;
   r.k = h.k;
   r.w = h.w;
+  r.foreign_keys = r.k <= 16 && tc.high_keys;
   register_index(c, r, h.mask, h.n_n_runs, index_id);
   return DNALN_OK;
 }
@@ -2105,6 +2109,7 @@ int dnaln_gpu_index_upload(dnaln_ctx* c, const uint8_t* genome, uint64_t n_bases
   r.n_contigs = n_contigs;
   r.k = k;
   r.w = w;
+  r.foreign_keys = k <= 16 && tc.high_keys;
   register_index(c, r, n_buckets - 1, n_runs, index_id);
   return DNALN_OK;
 }
