@@ -105,6 +105,9 @@ struct MapPart {
   uint32_t* cigar = nullptr;
   int64_t cigar_cap = 0;
   int64_t* cigar_used = nullptr;
+  // half of a batch that its caller gave whole (the ticket's other part is the other half): the
+  // results of neither are copied out before both are mapped and fit
+  bool half = false;
 };
 
 // Per-batch facts the caller may already know (host-buffer path), sparing a device read-back.
@@ -1190,17 +1193,18 @@ int stage_in(dnaln_ctx* c, int k, const MapPart& pt, SlotBufs& sb) {
   return DNALN_OK;
 }
 
-struct PendingPart {  // a part whose results are being copied out of slot k
-  bool active = false;
+struct PendingPart {  // a part whose results are in slot k: copied to the caller, or held there
+  bool active = false, copied = false;
   MapPart pt;
   int status = DNALN_OK;
+  int64_t base = 0, used = 0;  // its CIGAR operations: [base, base + used) of the batch's
 };
 
 // Records a finished part; the last part of a ticket publishes the ticket's status.
 void finish_part(dnaln_ctx* c, int k, PendingPart& pp) {
   if (!pp.active) return;
   pp.active = false;
-  if (pp.status == DNALN_OK) c->stats.ms_d2h += ev_ms(c->d2h_ev[2 * k], c->d2h_ev[2 * k + 1]);
+  if (pp.status == DNALN_OK && pp.copied) c->stats.ms_d2h += ev_ms(c->d2h_ev[2 * k], c->d2h_ev[2 * k + 1]);
   {
     std::lock_guard<std::mutex> g(c->qmu);
     const int64_t t = pp.pt.ticket;
@@ -1217,7 +1221,7 @@ void finish_part(dnaln_ctx* c, int k, PendingPart& pp) {
   if (pp.pt.last) c->qcv.notify_all();
 }
 
-// Runs part pt (inputs in slot k) and starts copying its results out. Returns the part's status.
+// Runs part pt (inputs in slot k), its results left in the slot. Returns the part's status.
 int compute_part(dnaln_ctx* c, int k, const MapPart& pt, const SlotBufs& sb, int64_t base, int64_t* used) {
   *used = 0;
   IndexRes* r = find_index(c, pt.index_id);
@@ -1238,15 +1242,25 @@ int compute_part(dnaln_ctx* c, int k, const MapPart& pt, const SlotBufs& sb, int
                       hint))
     return e;
   c->stats.ms_h2d += ev_ms(c->h2d_ev[2 * k], c->h2d_ev[2 * k + 1]);  // complete: run_map waited for it
-  if (base + *used > pt.cigar_cap || (*used > 0 && !pt.cigar))
+  if (pt.half && !pt.last) return DNALN_OK;
+  if (base + *used > pt.cigar_cap || (base + *used > 0 && !pt.cigar))
     return fail(c, DNALN_ERR_CAPACITY, "CIGAR buffer holds %lld ops, batch needs at least %lld",
                 static_cast<long long>(pt.cigar_cap), static_cast<long long>(base + *used));
+  return DNALN_OK;
+}
+
+// Starts copying the results of the part computed in slot k to its caller.
+int copy_out(dnaln_ctx* c, int k, PendingPart& pp) {
+  const MapPart& pt = pp.pt;
   CK(cudaEventRecord(c->d2h_ev[2 * k], c->cp_out));
-  CK(cudaMemcpyAsync(pt.out + pt.a, d_out, m * sizeof(dnaln_map_record), cudaMemcpyDeviceToHost, c->cp_out));
-  if (*used > 0)
-    CK(cudaMemcpyAsync(pt.cigar + base, d_cig, *used * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->cp_out));
+  CK(cudaMemcpyAsync(pt.out + pt.a, c->bufs[kSlotNames[k][4]].p, (pt.b - pt.a) * sizeof(dnaln_map_record),
+                     cudaMemcpyDeviceToHost, c->cp_out));
+  if (pp.used > 0)
+    CK(cudaMemcpyAsync(pt.cigar + pp.base, c->bufs[kSlotNames[k][5]].p, pp.used * sizeof(uint32_t),
+                       cudaMemcpyDeviceToHost, c->cp_out));
   CK(cudaEventRecord(c->d2h_ev[2 * k + 1], c->cp_out));
   CK(cudaEventRecord(c->out_free[k], c->cp_out));
+  pp.copied = true;
   return DNALN_OK;
 }
 
@@ -1278,11 +1292,19 @@ void drive_parts(dnaln_ctx* c, int64_t own) {
     // the stream is idle (run_map synchronised it after waiting for out_free[k]): the part
     // that used slot k before is fully copied out
     finish_part(c, k, pend[k]);
-    if (st == DNALN_OK) {
-      std::lock_guard<std::mutex> g(c->qmu);
-      c->ticket_ops[pt.ticket] = base + used;
-    }
+    pend[k] = PendingPart{};
     pend[k].pt = pt;
+    pend[k].base = base;
+    pend[k].used = used;
+    if (st == DNALN_OK && !(pt.half && !pt.last)) {
+      if (pt.half) st = copy_out(c, 1 - k, pend[1 - k]);  // the first half, held until now
+      if (st == DNALN_OK) st = copy_out(c, k, pend[k]);
+    }
+    {
+      std::lock_guard<std::mutex> g(c->qmu);
+      if (st == DNALN_OK) c->ticket_ops[pt.ticket] = base + used;
+      else if (pt.half) c->ticket_ops[pt.ticket] = 0;
+    }
     pend[k].status = st;
     pend[k].active = true;
     if (st != DNALN_OK) {
@@ -1339,11 +1361,11 @@ bool read_facts(const int64_t* off, const int32_t* len, int64_t a, int64_t b, Ma
 // 2,049; 524,288 4,155, 3,427, 3,500.
 constexpr int64_t kSplitBases = 16 << 20;
 
-// Queues a batch (see dnaln_gpu_map_submit). *split: may go in two parts / does. *alone =
-// nothing was queued before it.
+// Queues a batch (see dnaln_gpu_map_submit). split: it may go in two parts. *alone = nothing was
+// queued before it.
 int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_off, const int32_t* seq_len,
                  const uint32_t* name_hash, int64_t n, const dnaln_map_params* p, dnaln_map_record* out,
-                 uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used, bool* split, int64_t* ticket, bool* alone) {
+                 uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used, bool split, int64_t* ticket, bool* alone) {
   if (!c || n < 0 || !cigar_used || !ticket || !p || (n > 0 && (!seq || !seq_off || !seq_len || !name_hash || !out)))
     return fail(c, DNALN_ERR_INVALID_ARG, "null argument");
   *ticket = 0;
@@ -1352,8 +1374,8 @@ int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_o
   // whoever drives the device); their failures come back from dnaln_gpu_map_wait
   if (int e = validate_map_params_basic(c, p)) return e;
   // parts of at most sub_batch reads, with their host-side facts (lengths are known here)
-  *split = *split && c->sub_batch == 0 && n >= 2;
-  const int64_t S = c->sub_batch > 0 ? c->sub_batch : (*split ? (n + 1) / 2 : std::max<int64_t>(n, 1));
+  split = split && c->sub_batch == 0 && n >= 2;
+  const int64_t S = c->sub_batch > 0 ? c->sub_batch : (split ? (n + 1) / 2 : std::max<int64_t>(n, 1));
   std::vector<MapPart> parts;
   for (int64_t a = 0; a < n; a += S) {
     MapPart pt;
@@ -1372,8 +1394,8 @@ int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_o
     parts.push_back(pt);
   }
   // one part if it is small or the halves' reads are not apart in the buffer
-  if (*split && (parts[0].bases + parts[1].bases < kSplitBases ||
-                 std::min(parts[0].hi, parts[1].hi) > std::max(parts[0].lo, parts[1].lo))) {
+  if (split && (parts[0].bases + parts[1].bases < kSplitBases ||
+                std::min(parts[0].hi, parts[1].hi) > std::max(parts[0].lo, parts[1].lo))) {
     MapPart& all = parts[0];
     const MapPart& rest = parts[1];
     all.b = rest.b;
@@ -1383,7 +1405,8 @@ int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_o
     all.max_len = std::max(all.max_len, rest.max_len);
     all.cig_bound += rest.cig_bound;
     parts.pop_back();
-    *split = false;
+  } else if (split) {
+    for (MapPart& pt : parts) pt.half = true;
   }
   std::lock_guard<std::mutex> g(c->qmu);
   const int64_t t = c->next_ticket++;
@@ -2409,8 +2432,8 @@ int dnaln_gpu_map_batch_device(dnaln_ctx* c, int32_t id, const char* d_seq, cons
 int dnaln_gpu_map_submit(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_off, const int32_t* seq_len,
                          const uint32_t* name_hash, int64_t n, const dnaln_map_params* p, dnaln_map_record* out,
                          uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used, int64_t* ticket) {
-  bool alone = false, split = false;
-  if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, &split,
+  bool alone = false;
+  if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, false,
                            ticket, &alone))
     return e;
   wake_worker(c);
@@ -2434,28 +2457,21 @@ int dnaln_gpu_map_wait(dnaln_ctx* c, int64_t ticket) {
 int dnaln_gpu_map_batch(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_off, const int32_t* seq_len,
                         const uint32_t* name_hash, int64_t n, const dnaln_map_params* p, dnaln_map_record* out,
                         uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used) {
-  bool split = true;
-  const auto map = [&]() {
-    int64_t ticket = 0;
-    bool alone = false;
-    if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, &split,
-                             &ticket, &alone))
-      return e;
-    // with nothing queued before it and the device free, the batch runs in the calling thread:
-    // a wake-up of the worker and one back cost a call of 64 reads 16 us
-    bool here = false;
-    if (alone && c->mu.try_lock()) {
-      std::lock_guard<std::mutex> g(c->mu, std::adopt_lock);
-      here = cudaSetDevice(c->device) == cudaSuccess;
-      if (here) drive_parts(c, ticket);
-    }
-    if (!here) wake_worker(c);
-    return dnaln_gpu_map_wait(c, ticket);
-  };
-  const int e = map();
-  if (e != DNALN_ERR_CAPACITY || !split) return e;
-  split = false;  // a CIGAR buffer too small for the batch is reported for the whole of it
-  return map();
+  int64_t ticket = 0;
+  bool alone = false;
+  if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, true,
+                           &ticket, &alone))
+    return e;
+  // with nothing queued before it and the device free, the batch runs in the calling thread:
+  // a wake-up of the worker and one back cost a call of 64 reads 16 us
+  bool here = false;
+  if (alone && c->mu.try_lock()) {
+    std::lock_guard<std::mutex> g(c->mu, std::adopt_lock);
+    here = cudaSetDevice(c->device) == cudaSuccess;
+    if (here) drive_parts(c, ticket);
+  }
+  if (!here) wake_worker(c);
+  return dnaln_gpu_map_wait(c, ticket);
 }
 
 }  // extern "C"

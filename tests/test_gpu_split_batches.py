@@ -1,0 +1,67 @@
+"""Synchronous batches that go in two parts: a refusal writes nothing and is counted as in one
+part."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import dnaln_b200 as D
+from dnaln_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+N, LEN = 250_000, 150  # 37 M bases: above the size from which a batch goes in two parts
+MARK = 0x5A
+
+
+@pytest.fixture(scope="module")
+def genome():
+    return synth.make_genome(synth.GenomeSpec(n_contigs=2, contig_len=300_000, gc=0.5), 5)
+
+
+class Batch:
+    def __init__(self, genome, seed, pinned=True):
+        reads, _ = synth.make_reads(genome, synth.ReadsSpec(n_reads=N), seed)
+        assert int(reads.seq_off[-1]) == N * LEN
+        place = (lambda t: t.pin_memory()) if pinned else (lambda t: t)
+        ins = [reads.seq, reads.seq_off[:-1], reads.seq_len, reads.name_hash().view(np.int32)]
+        self.ins = [place(torch.from_numpy(np.ascontiguousarray(a))) for a in ins]
+        self.rec = place(torch.full((N, D.MAP_RECORD_DTYPE.itemsize), MARK, dtype=torch.uint8))
+        self.cig = place(torch.full((N * 16,), MARK, dtype=torch.int32))
+        self.reads = reads
+
+    def map(self, ctx, iid, cap):
+        self.rec.fill_(MARK)
+        self.cig.fill_(MARK)
+        used, p = C.c_int64(), D.default_map_params()
+        rc = ctx._lib.dnaln_gpu_map_batch(ctx.handle, iid, *(a.data_ptr() for a in self.ins), N, C.byref(p),
+                                          self.rec.data_ptr(), self.cig.data_ptr(), cap, C.byref(used))
+        return rc, used.value, ctx._lib.dnaln_gpu_last_error(ctx.handle)
+
+    def untouched(self):
+        return bool((self.rec == MARK).all()) and bool((self.cig == MARK).all())
+
+
+def test_a_refused_batch_writes_nothing(ctx, genome):
+    iid = ctx.index_build(genome)
+    b = Batch(genome, 1)
+    try:
+        ctx.set_sub_batch(N)
+        rc, used, _ = b.map(ctx, iid, N * 16)
+        assert rc == 0
+        want = b.rec.clone(), b.cig.clone()
+        whole = [b.map(ctx, iid, cap) for cap in (1000, used - 1)]
+        ctx.set_sub_batch(0)
+        assert used > N and all(r[0] != 0 for r in whole)
+        for cap, expect in zip((1000, used - 1), whole):  # short for the first part, for the second only
+            ctx.reset_stats()
+            assert b.map(ctx, iid, cap) == expect
+            assert b.untouched()
+            assert ctx.stats()["reads"] == N  # mapped once
+        for cap in (used, N * 16):
+            assert b.map(ctx, iid, cap)[:2] == (0, used)
+            assert torch.equal(b.rec, want[0]) and torch.equal(b.cig, want[1])
+    finally:
+        ctx.set_sub_batch(0)
+        ctx.index_free(iid)
