@@ -762,7 +762,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
         kt.end(st);
         warp_list = big2;
         warp_n = c->d_count + 3;
-        c->stats.launches += 1;
+        c->stats.launches += 2;
       }
     }
     if (!full_list) {

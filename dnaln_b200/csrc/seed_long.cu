@@ -46,6 +46,18 @@ constexpr int kLWordsU = kLMaxAnc / 32;
 static_assert(2 * kLMaxMin <= kLWordsB, "minimizer slots must fit region B");
 constexpr int kLWords = kLWordsA + kLWordsB + kLWordsU;
 
+// A list of at most kLFew reads, handed on. In a kernel of its own: with this loop in front,
+// k_seed_chain_tl took 3,625 us for the long ones of 60,000 reads of 50 to 1,000 bases (2 Mbp
+// repeat genome); it takes 1,579 us, at the same registers and without spills either way.
+__global__ void __launch_bounds__(256)
+    k_hand_on(const int32_t* __restrict__ list, const int* __restrict__ list_n, int32_t* __restrict__ next_list,
+              int* __restrict__ next_n) {
+  const int m = *list_n, x = blockIdx.x * 256 + threadIdx.x;
+  if (m > kLFew || x >= m) return;
+  next_list[x] = list[x];
+  if (x == 0) *next_n = m;
+}
+
 template <int W>
 __global__ void __launch_bounds__(kLT, 6)
     k_seed_chain_tl(const int32_t* __restrict__ seq_len, const int64_t* __restrict__ pofs,
@@ -74,13 +86,7 @@ __global__ void __launch_bounds__(kLT, 6)
     return reinterpret_cast<int32_t&>(B(2 * kLMaxAnc + field * kLMaxChains + c));
   };
   const int m_list = *list_n;
-  if (m_list <= kLFew) {
-    for (int64_t x = tid; x < m_list; x += stride) {
-      next_list[x] = list[x];
-      if (x == 0) *next_n = m_list;
-    }
-    return;
-  }
+  if (m_list <= kLFew) return;  // k_hand_on's
   const int k = sp.k;
   // The grid is more blocks than are resident: the first wave takes the longest reads of
   // the (longest-first) list, and the later blocks start as the first's finish. A thread
@@ -485,6 +491,7 @@ bool launch_seed_chain_long(cudaStream_t st, const int32_t* seq_len, const int64
                             int32_t* next_list, int* next_n, int min_len, bool keep_mins, uint32_t* err) {
   if (!seed_long_supported(sp, cp)) return false;
   if (threads <= 0) return true;
+  k_hand_on<<<(kLFew + 255) / 256, 256, 0, st>>>(list, list_n, next_list, next_n);
   const unsigned blocks = static_cast<unsigned>(threads / kLT);
   k_seed_chain_tl<10><<<blocks, kLT, 0, st>>>(seq_len, pofs, codes, list, list_n, ix, sp, cp, cand, cb, n_min,
                                               n_anchor, n_anc_t, scratch, next_list, next_n, min_len, keep_mins, err);

@@ -71,3 +71,12 @@ def test_listed_reads(ctx, port, lengths):
     listed = check(ctx, port, g, reads, 1, long_thread=(0,))[0]["warp_reads"] if long else None
     if long:
         assert listed > HANDED_ON and stats[0]["warp_reads"] < listed  # the thread kernel took some of the list
+
+
+@pytest.mark.parametrize("n", [1, HANDED_ON, HANDED_ON + 1])
+def test_long_lists_around_the_length_that_is_handed_on(ctx, port, n):
+    rng = np.random.default_rng(4)
+    g = genome(rng)
+    reads = many(make_reads(rng, g, 1_100, [300, 420]), 4).slice(0, n)
+    (st,) = check(ctx, port, g, reads, 0)
+    assert (st["long_reads"] > 0) == (n > HANDED_ON)
