@@ -280,6 +280,14 @@ int set_device(dnaln_ctx* c) {
   return DNALN_OK;
 }
 
+// Reads the calling thread's device without making one current or initialising it.
+bool device_is_current(const dnaln_ctx* c) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) == cudaSuccess) return dev == c->device;
+  cudaGetLastError();
+  return false;
+}
+
 int exclusive_scan(dnaln_ctx* c, const int64_t* in, int64_t* out, int64_t n);
 
 double ev_ms(cudaEvent_t a, cudaEvent_t b) {
@@ -2462,10 +2470,11 @@ int dnaln_gpu_map_batch(dnaln_ctx* c, int32_t id, const char* seq, const int64_t
   if (int e = submit_parts(c, id, seq, seq_off, seq_len, name_hash, n, p, out, cigar, cigar_cap, cigar_used, true,
                            &ticket, &alone))
     return e;
-  // with nothing queued before it and the device free, the batch runs in the calling thread:
-  // a wake-up of the worker and one back cost a call of 64 reads 16 us
+  // with nothing queued before it and the device free, the batch runs in the calling thread: a
+  // wake-up of the worker and one back cost a call of 64 reads 16 us. A thread whose current
+  // device is another one leaves it to the worker, so that its device stays current.
   bool here = false;
-  if (alone && c->mu.try_lock()) {
+  if (alone && device_is_current(c) && c->mu.try_lock()) {
     std::lock_guard<std::mutex> g(c->mu, std::adopt_lock);
     here = cudaSetDevice(c->device) == cudaSuccess;
     if (here) drive_parts(c, ticket);

@@ -65,3 +65,13 @@ def test_a_refused_batch_writes_nothing(ctx, genome):
     finally:
         ctx.set_sub_batch(0)
         ctx.index_free(iid)
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two devices to tell them apart")
+def test_the_callers_device_stays_current(genome):
+    with D.Context(1) as c:
+        iid = c.index_build(genome)
+        b = Batch(genome, 30)
+        torch.cuda.set_device(0)
+        assert b.map(c, iid, N * 16)[0] == 0
+        assert torch.cuda.current_device() == 0
