@@ -288,6 +288,14 @@ bool device_is_current(const dnaln_ctx* c) {
   return false;
 }
 
+// Whether copies from p run beside the host: page-locked memory.
+bool page_locked(const void* p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  return false;
+}
+
 int exclusive_scan(dnaln_ctx* c, const int64_t* in, int64_t* out, int64_t n);
 
 double ev_ms(cudaEvent_t a, cudaEvent_t b) {
@@ -1363,10 +1371,12 @@ bool read_facts(const int64_t* off, const int32_t* len, int64_t a, int64_t b, Ma
   return true;
 }
 
-// A synchronous batch of at least this many bases goes in two parts, so that the second's
-// reads are copied while the first computes. Reads of 150 bp from pinned memory, one part,
-// halves, thirds: 65,536 699, 727, 921 us; 131,072 1,198, 1,110, 1,298; 262,144 2,248, 1,961,
-// 2,049; 524,288 4,155, 3,427, 3,500.
+// A synchronous batch of at least this many bases in page-locked memory goes in two parts, so that
+// the second's reads are copied while the first computes. Reads of 150 bp, one part and halves, us:
+// 131,072 1,292 and 1,256; 262,144 2,319 and 2,122; 524,288 4,174 and 3,637 (thirds 921 against 727
+// for halves at 65,536, 2,049 against 1,961 at 262,144). The copies of other memory block the host,
+// so nothing overlaps and two batches of half the size remain: 131,072 2,421 and 2,736; 262,144
+// 5,355 and 5,864; 524,288 10,581 and 10,786.
 constexpr int64_t kSplitBases = 16 << 20;
 
 // Queues a batch (see dnaln_gpu_map_submit). split: it may go in two parts. *alone = nothing was
@@ -1401,9 +1411,10 @@ int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_o
       return fail(c, DNALN_ERR_INVALID_ARG, "negative offset or length");
     parts.push_back(pt);
   }
-  // one part if it is small or the halves' reads are not apart in the buffer
+  // one part if it is small, the halves' reads are not apart in the buffer or that is not page-locked
   if (split && (parts[0].bases + parts[1].bases < kSplitBases ||
-                std::min(parts[0].hi, parts[1].hi) > std::max(parts[0].lo, parts[1].lo))) {
+                std::min(parts[0].hi, parts[1].hi) > std::max(parts[0].lo, parts[1].lo) || !device_is_current(c) ||
+                !page_locked(seq))) {
     MapPart& all = parts[0];
     const MapPart& rest = parts[1];
     all.b = rest.b;

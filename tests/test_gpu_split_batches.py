@@ -67,6 +67,28 @@ def test_a_refused_batch_writes_nothing(ctx, genome):
         ctx.index_free(iid)
 
 
+@pytest.mark.parametrize("pinned", [True, False])
+def test_only_page_locked_reads_go_in_two_parts(ctx, genome, pinned):
+    iid = ctx.index_build(genome)
+    b = Batch(genome, 20, pinned)
+    try:
+        ctx.set_option("graphs", 0)
+        ctx.set_sub_batch(N)
+        assert b.map(ctx, iid, N * 16)[0] == 0
+        ctx.reset_stats()
+        assert b.map(ctx, iid, N * 16)[0] == 0
+        one = ctx.stats()["launches"]
+        ctx.set_sub_batch(0)
+        ctx.reset_stats()
+        assert b.map(ctx, iid, N * 16)[0] == 0
+        launches = ctx.stats()["launches"]
+        assert launches == one if not pinned else launches > 1.5 * one
+    finally:
+        ctx.set_sub_batch(0)
+        ctx.set_option("graphs", 1)
+        ctx.index_free(iid)
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two devices to tell them apart")
 def test_the_callers_device_stays_current(genome):
     with D.Context(1) as c:
