@@ -1372,12 +1372,17 @@ bool read_facts(const int64_t* off, const int32_t* len, int64_t a, int64_t b, Ma
 }
 
 // A synchronous batch of at least this many bases in page-locked memory goes in two parts, so that
-// the second's reads are copied while the first computes. Reads of 150 bp, one part and halves, us:
-// 131,072 1,292 and 1,256; 262,144 2,319 and 2,122; 524,288 4,174 and 3,637 (thirds 921 against 727
-// for halves at 65,536, 2,049 against 1,961 at 262,144). The copies of other memory block the host,
-// so nothing overlaps and two batches of half the size remain: 131,072 2,421 and 2,736; 262,144
-// 5,355 and 5,864; 524,288 10,581 and 10,786.
-constexpr int64_t kSplitBases = 16 << 20;
+// the second's reads are copied while the first computes, if its reads are short: the time of the
+// long reads' kernels is one read's latency, which two parts pay twice. One part and halves, us:
+//   reads of 150 bp   4.6 Mbp genome       120 Mbp repeat genome
+//   120,000           1,205 and 1,221      1,900 and 2,321
+//   180,000           1,748 and 1,690      2,599 and 2,879
+//   262,144           2,319 and 2,156      3,446 and 3,544
+//   524,288           4,255 and 3,624      6,155 and 5,835
+//   60,000 reads of 50 to 1,000 bp, 1,498 and 1,776, 7,141 and 11,828
+// The copies of memory that is not page-locked block the host, so nothing overlaps: 262,144 reads
+// 5,355 and 5,864.
+constexpr int64_t kSplitBases = 32 << 20;
 
 // Queues a batch (see dnaln_gpu_map_submit). split: it may go in two parts. *alone = nothing was
 // queued before it.
@@ -1411,8 +1416,9 @@ int submit_parts(dnaln_ctx* c, int32_t id, const char* seq, const int64_t* seq_o
       return fail(c, DNALN_ERR_INVALID_ARG, "negative offset or length");
     parts.push_back(pt);
   }
-  // one part if it is small, the halves' reads are not apart in the buffer or that is not page-locked
+  // one part unless it is large, of short reads, and its halves lie apart in page-locked memory
   if (split && (parts[0].bases + parts[1].bases < kSplitBases ||
+                std::max(parts[0].max_len, parts[1].max_len) > seed_thread_max_len() ||
                 std::min(parts[0].hi, parts[1].hi) > std::max(parts[0].lo, parts[1].lo) || !device_is_current(c) ||
                 !page_locked(seq))) {
     MapPart& all = parts[0];

@@ -21,9 +21,10 @@ def genome():
 
 
 class Batch:
-    def __init__(self, genome, seed, pinned=True):
-        reads, _ = synth.make_reads(genome, synth.ReadsSpec(n_reads=N), seed)
-        assert int(reads.seq_off[-1]) == N * LEN
+    def __init__(self, genome, seed, pinned=True, longest=LEN):
+        reads, _ = synth.make_reads(genome, synth.ReadsSpec(n_reads=N, len_min=LEN, len_max=longest,
+                                                            len_dist=2 if longest > LEN else 0), seed)
+        assert int(reads.seq_off[-1]) >= N * LEN
         place = (lambda t: t.pin_memory()) if pinned else (lambda t: t)
         ins = [reads.seq, reads.seq_off[:-1], reads.seq_len, reads.name_hash().view(np.int32)]
         self.ins = [place(torch.from_numpy(np.ascontiguousarray(a))) for a in ins]
@@ -67,10 +68,26 @@ def test_a_refused_batch_writes_nothing(ctx, genome):
         ctx.index_free(iid)
 
 
-@pytest.mark.parametrize("pinned", [True, False])
-def test_only_page_locked_reads_go_in_two_parts(ctx, genome, pinned):
+def test_halves_with_gaps_between_their_reads(ctx, genome):
     iid = ctx.index_build(genome)
-    b = Batch(genome, 20, pinned)
+    b = Batch(genome, 40)
+    try:
+        assert b.map(ctx, iid, N * 16)[0] == 0
+        want = b.rec.clone(), b.cig.clone()
+        seq = torch.full((N, LEN + 3), ord("N"), dtype=torch.uint8)
+        seq[:, :LEN] = b.ins[0][:N * LEN].view(N, LEN)
+        b.ins[0] = seq.flatten().pin_memory()
+        b.ins[1] = (torch.arange(N, dtype=torch.int64) * (LEN + 3)).pin_memory()
+        assert b.map(ctx, iid, N * 16)[0] == 0
+        assert torch.equal(b.rec, want[0]) and torch.equal(b.cig, want[1])
+    finally:
+        ctx.index_free(iid)
+
+
+@pytest.mark.parametrize("pinned,longest,parts", [(True, LEN, 2), (True, 256, 2), (True, 260, 1), (False, LEN, 1)])
+def test_only_short_page_locked_reads_go_in_two_parts(ctx, genome, pinned, longest, parts):
+    iid = ctx.index_build(genome)
+    b = Batch(genome, 20, pinned, longest)
     try:
         ctx.set_option("graphs", 0)
         ctx.set_sub_batch(N)
@@ -82,7 +99,7 @@ def test_only_page_locked_reads_go_in_two_parts(ctx, genome, pinned):
         ctx.reset_stats()
         assert b.map(ctx, iid, N * 16)[0] == 0
         launches = ctx.stats()["launches"]
-        assert launches == one if not pinned else launches > 1.5 * one
+        assert launches == one if parts == 1 else launches > 1.5 * one
     finally:
         ctx.set_sub_batch(0)
         ctx.set_option("graphs", 1)
