@@ -337,12 +337,16 @@ __device__ void chain_dp_tiles(const ChainArrays& a, int n, const ChainParamsDev
 // outside its cluster is ever a valid predecessor, so the clusters are independent, and each
 // lane runs the reference's scan with a cutoff: a predecessor j' <= j scores at most
 // max(f[0..j]) + k, so once that is <= best the strict '>' cannot hold any more. A row of
-// the warp-wide DP tests 32 predecessors of one anchor; here 32 anchors advance at once, each
-// testing the few it needs. Returns false, doing nothing, for fewer than
-// kMinClusters clusters or when one holds more than half of the anchors.
-// 262,144 reads of the 120 Mbp repeat genome, 37,000 of them chained by warps with 100
-// anchors each: k_chain_map 737 -> 646 us.
-constexpr int kMinClusters = 6;
+// the warp-wide DP advances 32 anchors of one tile step by step; here up to 32 clusters advance at
+// once, each testing the few predecessors it needs. Returns false, doing nothing, for fewer than
+// kMinClusters clusters or when one holds more than a sixth of the anchors or more than
+// kMaxCluster: its lane would run long alone, all of its lookback in every row if no two anchors
+// chain. Measured, tiles and clusters: k_chain_map of 262,144 reads of the 120 Mbp repeat genome
+// (19,970 of them, 159 anchors each) 603 and 497 us; 64 sets of 20 clusters of 45 anchors in
+// chains, the whole call, 1,542 and 1,385 us; against that 600 anchors, half of them in no chain,
+// in two clusters of 290 and four of 5, 1,306 and 2,395 us, and six clusters of 48 anchors in no
+// chain 834 and 958 us.
+constexpr int kMinClusters = 12, kMaxCluster = 48;
 __device__ bool chain_dp_clusters(const ChainArrays& a, int n, const ChainParamsDev& cp) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -365,7 +369,8 @@ __device__ bool chain_dp_clusters(const ChainArrays& a, int n, const ChainParams
   int most = 0;
   for (int c = lane; c < nc; c += 32)
     most = max(most, (c + 1 < nc ? static_cast<int>(head[c + 1]) : n) - static_cast<int>(head[c]));
-  if (2 * __reduce_max_sync(FULL, most) > n) return false;  // one lane would run most of the set
+  most = __reduce_max_sync(FULL, most);
+  if (6 * most > n || most > kMaxCluster) return false;
   int32_t* const top = reinterpret_cast<int32_t*>(head) + n;
   for (int c = lane; c < nc; c += 32) {
     const int lo = static_cast<int>(head[c]), hi = c + 1 < nc ? static_cast<int>(head[c + 1]) : n;

@@ -24,3 +24,19 @@ def test_chaining_with_any_k_matches_port(ctx, port, k):
         assert np.array_equal(sr, er) and np.array_equal(sq, eq) and np.array_equal(ss, es), i
         for key in ech:
             assert np.array_equal(ch[key], ech[key]), (i, key)
+
+
+def test_cluster_counts_and_sizes_at_the_rules_edges(ctx, port):
+    """11, 12 and 13 clusters, the largest of 47 to 49 anchors and about a sixth of all."""
+    rng = np.random.default_rng(7)
+    cp = (300, 16, 50, 20, 1)
+    sets = [clustered_set(rng, [m] * c, cp[0], 10) for c in (11, 12, 13) for m in (1, 4, 20)]
+    sets += [clustered_set(rng, [m] + [20] * 13, cp[0], 10) for m in (47, 48, 49, 50, 51, 52, 53, 54)]
+    sets += [clustered_set(rng, [m] * 14, cp[0], 10) for m in (47, 48, 49)]
+    sets += [clustered_set(rng, [10] + [1] * k, cp[0], 10) for k in (49, 50, 51)]
+    got = ctx.chain(sets, 15, D.ChainParams(*cp))
+    for i, ((sr, sq, ss), ch) in enumerate(got):
+        (er, eq, es), ech = port.chain(*sets[i], 15, cp)
+        assert np.array_equal(sr, er) and np.array_equal(sq, eq) and np.array_equal(ss, es), i
+        for key in ech:
+            assert np.array_equal(ch[key], ech[key]), (i, key)
