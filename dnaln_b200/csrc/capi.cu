@@ -621,7 +621,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   // chaining pool's fill, [10] long reads the colinear kernel finished
   unsigned long long* info = reinterpret_cast<unsigned long long*>(c->d_ctl + kCtlInfo);
   // [0] reads the colinear kernels listed, [1] work-stealing claims of the warp chaining kernel,
-  // [2] reads it listed for their anchor count, [3] claims of those, [4] reads with an N
+  // [2] reads it listed for their anchor count, [3] claims of those
   int* claims = reinterpret_cast<int*>(c->d_ctl + kCtlClaims);
   CK(cudaMemsetAsync(c->d_ctl, 0, kCtlWords * sizeof(int64_t), st));
   unsigned long long* ctr = info + 1;  // cells, mapped, candidates (map.cuh)
@@ -692,7 +692,6 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
     // (its probe takes a key above 2^32 for an empty bucket)
     if (c->colinear && !ix.foreign_keys && seed_colinear_supported(sp, cp, ix.dev)) {
       DBUF(rest, int32_t, "colinear_rest", n);
-      DBUF(with_n, int32_t, "colinear_with_n", n);
       const int lanes = seed_colinear_lanes(n, max_len);
       // in length order a warp's lanes end together; several lanes a read are taken where all
       // reads are resident at once, and the order only costs its two launches
@@ -708,11 +707,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       kt.end(st);
       kt.begin(st, "k_probe_reads");
       launch_probe_reads(st, pofs, d_seq_len, n, lanes, mb.hash, sk_counts, ix.dev, sp, cp, cand, cb, n_min, n_anchor,
-                         n_anc_t, mb, rest, claims, with_n, claims + 4, seed_thread_max_len(), info + 10, c->d_err);
-      kt.end(st);
-      kt.begin(st, "k_seed<list>");
-      launch_seed_list(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, with_n, claims + 4, codes, ix.dev, sp,
-                       mb, n_min, n_anchor, c->d_err);
+                         n_anc_t, mb, rest, claims, seed_thread_max_len(), info + 10, c->d_err);
       kt.end(st);
       c->stats.launches += 2;
       full_list = rest_list = rest;
@@ -781,12 +776,13 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
         c->stats.launches += 2;
       }
     }
-    if (!full_list) {
-      kt.begin(st, "k_seed<list>");
-      launch_seed_list(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, warp_list, warp_n, codes, ix.dev, sp,
-                       mb, n_min, n_anchor, c->d_err);
-      kt.end(st);
-    }
+    // after the colinear kernels only the reads left unsketched for an N. (Before the thread kernels,
+    // for all such reads, this sketched 95,000 reads a second time that those kernels then did a
+    // third time: 100,000 reads with 2 % N 1,606 us, so 1,325.)
+    kt.begin(st, "k_seed<list>");
+    launch_seed_list(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, warp_list, warp_n, full_list != nullptr,
+                     codes, ix.dev, sp, mb, n_min, n_anchor, c->d_err);
+    kt.end(st);
   } else {
     kt.begin(st, "k_seed");
     launch_seed(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, codes, ix.dev, sp, mb, n_min, n_anchor,

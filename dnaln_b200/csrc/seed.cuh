@@ -127,11 +127,12 @@ void launch_seed(cudaStream_t st, const char* seq, const int64_t* seq_off, int64
                  const int64_t* pofs, int64_t n, uint8_t* codes, const DevIndex& ix, const SeedParams& sp, MinBuf mb,
                  int32_t* n_min, int64_t* n_anchor, uint32_t* err);
 
-// Pass 1 for the reads list[0, *list_n) only (n_max >= *list_n), codes already written.
+// Pass 1 for the reads list[0, *list_n) only (n_max >= *list_n), codes already written; with
+// `marked`, for those of them whose n_anchor is below 0.
 void launch_seed_list(cudaStream_t st, const char* seq, const int64_t* seq_off, int64_t seq_base,
                       const int32_t* seq_len, const int64_t* pofs, int64_t n_max, const int32_t* list,
-                      const int* list_n, uint8_t* codes, const DevIndex& ix, const SeedParams& sp, MinBuf mb,
-                      int32_t* n_min, int64_t* n_anchor, uint32_t* err);
+                      const int* list_n, bool marked, uint8_t* codes, const DevIndex& ix, const SeedParams& sp,
+                      MinBuf mb, int32_t* n_min, int64_t* n_anchor, uint32_t* err);
 
 // Pass 2: anchors, chaining, candidates of the reads [0, n), or with a list of the reads
 // list[0, *list_n) (n = the list's size). n_anchor[r] = the read's anchor count (pass 1);
@@ -165,7 +166,7 @@ void launch_encode_reads_bulk(cudaStream_t st, const char* seq, const int64_t* s
 // launch_probe_reads: candidates, n_min, n_anc_t and n_anchor = 0 of the reads found to have
 // one chain; the others are appended to list (*list_n = 0 before), with their minimizers in
 // mb, n_min and n_anchor as launch_seed_list leaves them, or, where an N kept them from being
-// sketched, to n_list as well (*n_list_n = 0 before; launch_seed_list is theirs). *long_done
+// sketched, n_min = 0 and n_anchor = -1 (launch_seed_list takes them by that mark). *long_done
 // += finished reads longer than long_len.
 bool seed_colinear_supported(const SeedParams& sp, const ChainParamsDev& cp, const DevIndex& ix);
 int seed_colinear_lanes(int64_t n, int64_t max_len);
@@ -176,7 +177,7 @@ void launch_probe_reads(cudaStream_t st, const int64_t* pofs, const int32_t* seq
                         const uint64_t* mins, const int32_t* counts, const DevIndex& ix, const SeedParams& sp,
                         const ChainParamsDev& cp, const CandParams& cand, CandBuf cb, int32_t* n_min,
                         int64_t* n_anchor, int32_t* n_anc_t, MinBuf mb, int32_t* list, int* list_n,
-                        int32_t* n_list, int* n_list_n, int long_len, unsigned long long* long_done, uint32_t* err);
+                        int long_len, unsigned long long* long_done, uint32_t* err);
 // order = the reads of list[0, *list_n) (all n without a list; n at least the list's
 // length), longest first by length bin; bins: 2 * kLengthBins zeros.
 void launch_read_order(cudaStream_t st, const int32_t* seq_len, const int32_t* list, const int* list_n, int n,

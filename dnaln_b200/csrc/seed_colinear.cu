@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kCThreads)
                   const uint64_t* __restrict__ mins, const int32_t* __restrict__ counts, DevIndex ix, SeedParams sp,
                   ChainParamsDev cp, CandParams cand, CandBuf cb, int32_t* __restrict__ n_min,
                   int64_t* __restrict__ n_anchor, int32_t* __restrict__ n_anc_t, MinBuf mb, int32_t* __restrict__ list,
-                  int* __restrict__ list_n, int32_t* __restrict__ n_list, int* __restrict__ n_list_n, int long_len,
+                  int* __restrict__ list_n, int long_len,
                   unsigned long long* __restrict__ long_done, uint32_t* __restrict__ err) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int kWarps = kCThreads / 32;
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(kCThreads)
       __syncwarp();
     }
     if (bad) {
-      // its minimizers and their buckets for the warp kernels (an N read's are still to be made)
+      // its minimizers and their buckets for the warp kernels (an N read's are still to be made: -1)
       int64_t anchors = 0;
       const bool sketched = total >= 0;
       for (int j0 = 0; j0 < total && sketched; j0 += 32) {
@@ -553,9 +553,8 @@ __global__ void __launch_bounds__(kCThreads)
       }
       if (lane == 0) {
         mine[listed] = static_cast<int32_t>(r);
-        if (!sketched) n_list[atomicAdd(n_list_n, 1)] = static_cast<int32_t>(r);
         n_min[r] = sketched ? total : 0;
-        n_anchor[r] = anchors;
+        n_anchor[r] = sketched ? anchors : -1;
         n_anc_t[r] = 0;
       }
       if (++listed == 32) flush();
@@ -648,12 +647,12 @@ void launch_probe_reads(cudaStream_t st, const int64_t* pofs, const int32_t* seq
                         const uint64_t* mins, const int32_t* counts, const DevIndex& ix, const SeedParams& sp,
                         const ChainParamsDev& cp, const CandParams& cand, CandBuf cb, int32_t* n_min,
                         int64_t* n_anchor, int32_t* n_anc_t, MinBuf mb, int32_t* list, int* list_n,
-                        int32_t* n_list, int* n_list_n, int long_len, unsigned long long* long_done, uint32_t* err) {
+                        int long_len, unsigned long long* long_done, uint32_t* err) {
   const unsigned blocks = static_cast<unsigned>(
       std::min<int64_t>((n + kCThreads / 32 - 1) / (kCThreads / 32), int64_t{32} * device_sm_count()));
   const auto run = [&](auto kernel) {
     kernel<<<blocks, kCThreads, 0, st>>>(pofs, seq_len, n, mins, counts, ix, sp, cp, cand, cb, n_min, n_anchor, n_anc_t,
-                                         mb, list, list_n, n_list, n_list_n, long_len, long_done, err);
+                                         mb, list, list_n, long_len, long_done, err);
   };
   switch (lanes) {
     case 4: return run(k_probe_reads<kCW, 4>);

@@ -80,3 +80,25 @@ def test_long_lists_around_the_length_that_is_handed_on(ctx, port, n):
     reads = many(make_reads(rng, g, 1_100, [300, 420]), 4).slice(0, n)
     (st,) = check(ctx, port, g, reads, 0)
     assert (st["long_reads"] > 0) == (n > HANDED_ON)
+
+
+@pytest.mark.parametrize("times,lengths", [(1, [100, 150]), (1, [150, 300, 600]), (5, [100, 150]), (5, [150, 300, 600])])
+def test_reads_with_an_n(ctx, port, times, lengths):
+    """Every read has an N, so none is sketched for the colinear check: lists that are handed on and
+    lists the thread kernels take, with reads too rich in anchors for those."""
+    rng = np.random.default_rng(5)
+    g = genome(rng)
+    base = make_reads(rng, g, 1_000, lengths)
+    seqs = []
+    for i in range(len(base)):
+        q = bytearray(base.read(i))
+        if i % 4 == 0:  # inside the tandem repeat
+            at = 60_000 + i % 30
+            q = bytearray(b"ACGTN"[c] for c in g.codes[at:at + min(len(q), 440)])
+        q[int(rng.integers(len(q)))] = ord("N")
+        seqs.append(bytes(q))
+    reads = D.ReadBatch.from_lists(seqs * times, [b"r%d" % i for i in range(times * len(seqs))])
+    on, off = check(ctx, port, g, reads, 1)[0], check(ctx, port, g, reads, 0)[0]
+    for f in ("mapped", "candidates", "minimizers", "anchors"):
+        assert on[f] == off[f], f
+    assert 0 < on["warp_reads"] and (on["warp_reads"] == len(reads)) == (times == 1)
