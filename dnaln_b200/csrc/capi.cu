@@ -169,7 +169,7 @@ struct dnaln_ctx {
   bool stop = false;
   bool warp_seed_only = false;  // option: every read through the warp-per-read seeding kernels
   bool length_order = true;     // option: SW tasks of mixed-length batches run longest first
-  bool ungapped = true;         // option: SW tasks proved to have no gap skip the DP
+  int ungapped = 1;  // option: SW tasks proved to have no gap skip the DP (1: of long lists, 2: of any list)
   bool colinear = true;         // option: reads with one colinear chain skip the full seeding kernels
   bool long_thread = true;      // option: listed long reads one thread each before the warp kernels
   // option "work_stealing": the warp chaining kernel takes reads by atomic claims on
@@ -428,7 +428,8 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
                       const uint8_t* qbase, const uint8_t* tbase, const SwParams& sp, SwResult* res, int rows_max,
                       uint32_t* cig, const int64_t* cig_off, bool by_length) {
   if (n_max <= 0) return DNALN_OK;
-  const bool ungapped = c->ungapped && sw_ungapped_supported(sp, bytes_ok);
+  const bool ungapped = c->ungapped && sw_ungapped_supported(sp, bytes_ok) &&
+                        (c->ungapped == 2 || sw_ungapped_pays(sp.W, bytes_ok, n_max));
   // a list that fills no more than a warp per scheduler takes as long as its longest task
   // in any order
   if (sw_has_form(sp.W, bytes_ok, kSwIntraFew) && n_max <= int64_t{4} * device_sm_count() * 256 / (sp.W - 1))
@@ -1675,7 +1676,7 @@ int dnaln_gpu_set_option(dnaln_ctx* c, const char* name, int64_t value) {
     return DNALN_OK;
   }
   if (k == "ungapped") {
-    c->ungapped = value != 0;
+    c->ungapped = value == 2 ? 2 : (value != 0 ? 1 : 0);
     return DNALN_OK;
   }
   if (k == "length_order") {

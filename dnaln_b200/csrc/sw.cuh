@@ -55,6 +55,8 @@ bool launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int
 // ---- tasks without a gap, proved from bit vectors (sw_ungapped.cu) ------------------------
 // True when the scores and the band meet the proof's preconditions.
 bool sw_ungapped_supported(const SwParams& p, bool bytes_ok);
+// Whether the proof's pass is worth its time in front of the DP of up to n tasks.
+bool sw_ungapped_pays(int W, bool bytes_ok, int64_t n);
 // Writes the result (and, with tb, the one-operation CIGAR) of every task proved to align
 // by diagonal steps only, and appends the others to todo (capacity n, *todo_n = 0 before).
 // hist (may be null) counts the listed tasks per length bin.

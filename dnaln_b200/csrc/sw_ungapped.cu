@@ -306,6 +306,20 @@ bool sw_ungapped_supported(const SwParams& p, bool bytes_ok) {
          p.mismatch <= p.match + p.ge && p.match * kRun >= std::min(p.mismatch, p.oe);
 }
 
+// The DP of a short list takes one task's latency, whether a fifth or all of the list is left to it,
+// so the pass in front of it is lost time unless it proves every task, as it may of a handful.
+// Tracebacks of 150 rows, a fifth of them with a gap, us without and with the pass:
+//   W = 11   8,192 67 and 80, 20,000 96 and 86       W = 43   2,048 63 and 74, 4,096 75 and 74
+//   W = 17   8,192 80 and 92, 20,000 111 and 102     W = 65   2,048 69 and 82, 4,096 83 and 83
+//   W = 33   4,096 73 and 84, 8,192 83 and 86,       W = 129  512 71 and 86, 2,048 90 and 88
+//            20,000 176 and 111
+// and 64 tasks of 1,000 rows at W = 33 275 and 334. One task that is proved 59 and 31 (1,000 rows
+// 245 and 54), one that is not 63 and 72. The widths without a form for short lists run a thread
+// per task (k_sw_any), which any task spared is worth.
+bool sw_ungapped_pays(int W, bool bytes_ok, int64_t n) {
+  return n <= 4 || n > sw_few_tasks(W) / 2 || !sw_has_form(W, bytes_ok, kSwIntraFew);
+}
+
 void launch_sw_ungapped(cudaStream_t st, bool tb, const SwTask* tasks, int n, const int* n_dev, const uint8_t* qbase,
                         const uint8_t* tbase, const SwParams& p, SwResult* res, uint32_t* cig, const int64_t* cig_off,
                         SwTask* todo, int* todo_n, int* hist, int bin_shift) {

@@ -148,7 +148,8 @@ int dnaln_gpu_set_sub_batch(dnaln_ctx* ctx, int64_t reads);
  *   "colinear"       1 = reads whose anchors are checked, as they are found, to form one
  *                    colinear chain skip the chaining DP (default); 0 = every read runs it;
  *   "ungapped"       1 = banded SW tasks proved from bit vectors to align by diagonal steps
- *                    only skip the DP kernels (default); 0 = every task runs the DP;
+ *                    only skip the DP kernels, in lists long enough for the proof to pay
+ *                    (default); 2 = in any list; 0 = every task runs the DP;
  *   "seed_block"     reads per block of the thread-per-read seeding kernel: 0 = tuned
  *                    (default, dnaln_gpu_seed_tuning), 64 or 128;
  *   "encode_bulk"    1 = the codes of both strands are made in shared memory, tiles of
