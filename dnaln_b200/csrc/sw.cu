@@ -111,8 +111,14 @@ __device__ __forceinline__ uint32_t prof_biased(const SwParams& p, uint32_t qc) 
 
 __device__ __forceinline__ uint32_t pack2(uint32_t v) { return (v & 0xFFFFu) * 0x10001u; }
 
+// A cell's code, its flags STEP bits apart. diag: hd >= E and max(hd, E) >= F; from_e: the latter,
+// which is H = E on every cell the walk asks it for (H > 0 and not from the diagonal). Neither
+// waits for H: compared with H itself, k_sw_fb<43> spilled and took 181 us for 64 tasks of 150
+// rows, so 154.
+template <int STEP = 4>
 __device__ __forceinline__ uint32_t dir_code32(bool diag, bool from_e, bool e_not_ext, bool f_not_ext) {
-  return (diag ? 0u : kNotDiag) | (from_e ? 0u : kNotE) | (e_not_ext ? 0u : kExtE) | (f_not_ext ? 0u : kExtF);
+  return (diag ? 0u : 1u) | (e_not_ext ? 0u : 1u << STEP) | (from_e ? 0u : 1u << 2 * STEP) |
+         (f_not_ext ? 0u : 1u << 3 * STEP);
 }
 
 // Global store with an L2 evict-first policy: streaming data (the direction codes, read
@@ -200,6 +206,7 @@ struct CigarWriter {
 // Direction codes of the pair layout: word (i, g), g < WQ = ceil(W/4), holds cells 4g..4g+3
 // of both alignments of a thread (A in the low 16 bits, B in the high 16); the 32 pairs of a warp are interleaved word by word.
 struct PairCodes {
+  static constexpr uint32_t kFromNotE = kNotE, kEExt = kExtE, kFExt = kExtF, kAll = kCode;
   const uint32_t* D;  // this pair's first word
   int WQ, half;
   __device__ uint32_t word(int i, int d) const { return D[(static_cast<size_t>(i) * WQ + (d >> 2)) * 32]; }
@@ -208,13 +215,18 @@ struct PairCodes {
 };
 
 // Direction codes of the generic kernel: word (i, w), w < WW = ceil(W/8), holds cells
-// 8w..8w+7, the first four in the low half; 32 alignments of a warp interleaved word by word.
+// 8w..8w+7, the flags of cell 8w + c at bits c, 8 + c, 16 + c and 24 + c; 32 alignments of a warp
+// interleaved word by word. One shift places a cell's flags: two groups of four cells side by side
+// took 2,923 us for 64 tasks of 150 rows at W = 201, so 2,810.
 struct WordCodes {
+  static constexpr int kStep = 8;
+  static constexpr uint32_t kEExt = 1u << kStep, kFromNotE = 1u << 2 * kStep, kFExt = 1u << 3 * kStep,
+                            kAll = 1u | kEExt | kFromNotE | kFExt;
   const uint32_t* D;
   int WW;
   __device__ uint32_t word(int i, int d) const { return D[(static_cast<size_t>(i) * WW + (d >> 3)) * 32]; }
-  __device__ int shift(int d) const { return 4 * (d & 4) + (d & 3); }
-  __device__ uint32_t operator()(int i, int d) const { return (word(i, d) >> shift(d)) & kCode; }
+  __device__ int shift(int d) const { return d & 7; }
+  __device__ uint32_t operator()(int i, int d) const { return (word(i, d) >> shift(d)) & kAll; }
 };
 
 // High bit of each byte of x set where that byte is zero, every other bit clear.
@@ -294,7 +306,7 @@ __device__ void traceback(const Codes& code, int W, int bi, int bd, int best, co
         }
 #pragma unroll
         for (int k = 0; k < kAhead; ++k) {
-          cx[k] = (wk[k] >> sh) & kCode;
+          cx[k] = (wk[k] >> sh) & Codes::kAll;
           qa[k] = static_cast<int>((qw >> (8 * (kAhead - 1 - k))) & 0xFFu);
           const int t8 = static_cast<int>((tw >> (8 * (kAhead - 1 - k))) & 0xFFu);
           ta[k] = t8 > 3 ? 4 : t8;
@@ -332,13 +344,13 @@ __device__ void traceback(const Codes& code, int W, int bi, int bd, int best, co
     if (i < 0 || v <= 0) break;
     run = 0;
     bool ext;
-    if (!(x & kNotE)) {  // from E, an insertion: E(i,d) <- (i-1, d+1)
+    if (!(x & Codes::kFromNotE)) {  // from E, an insertion: E(i,d) <- (i-1, d+1)
       do {
         if (i < 0 || d >= W) {
           atomicOr(err, kErrTracebackBounds);
           goto done;
         }
-        ext = (code(i, d) & kExtE) != 0;
+        ext = (code(i, d) & Codes::kEExt) != 0;
         v += ext ? p.ge : p.oe;
         ++run;
         --i;
@@ -351,7 +363,7 @@ __device__ void traceback(const Codes& code, int W, int bi, int bd, int best, co
           atomicOr(err, kErrTracebackBounds);
           goto done;
         }
-        ext = (code(i, d) & kExtF) != 0;
+        ext = (code(i, d) & Codes::kFExt) != 0;
         v += ext ? p.ge : p.oe;
         ++run;
         --d;
@@ -439,7 +451,7 @@ __device__ SwResult sw_one_reg(const SwTask& tk, const uint8_t* __restrict__ qba
       H[d] = h;
       E[d] = e;
       if constexpr (TB) {
-        dw |= dir_code32(h == hd, h == e, eo >= ee, fo >= fe) << (d & 3);
+        dw |= dir_code32(hd >= e && m1 >= f, m1 >= f, eo >= ee, fo >= fe) << (d & 3);
         if ((d & 3) == 3 || d == W - 1) {
           reinterpret_cast<uint16_t*>(DP + (static_cast<size_t>(i) * WQ + (d >> 2)) * 32)[half] =
               static_cast<uint16_t>(dw);
@@ -1015,7 +1027,7 @@ __global__ void __launch_bounds__(kSwThreads)
       f = max(fo, fe);
       const int m1 = max(hd, e0);
       h0 = max(max(m1, f), 0);
-      if constexpr (TB) dw = dir_code32(h0 == hd, h0 == e0, eo >= ee, fo >= fe);
+      if constexpr (TB) dw = dir_code32(hd >= e0 && m1 >= f, m1 >= f, eo >= ee, fo >= fe);
       rmax = h0;
       hleft = h0;
       hdiag = hup;
@@ -1047,7 +1059,7 @@ __global__ void __launch_bounds__(kSwThreads)
         E[k] = e;
       }
       if constexpr (TB) {
-        dw |= dir_code32(h == hd, h == e, eo >= ee, fo >= fe) << (k & 3);
+        dw |= dir_code32(hd >= e && m1 >= f, m1 >= f, eo >= ee, fo >= fe) << (k & 3);
         if ((k & 3) == 3) {
           if (act) reinterpret_cast<uint16_t*>(DP + (static_cast<size_t>(i) * WQ + ((d0 + k) >> 2)) * 32)[half] =
               static_cast<uint16_t>(dw);
@@ -1344,7 +1356,7 @@ __global__ void __launch_bounds__(kSwThreads) k_sw_any(const SwTask* __restrict_
       Hs[d * 32] = h;
       Es[d * 32] = e;
       if (TB) {
-        dw |= dir_code32(h == hd, h == e, eo >= ee, fo >= fe) << (4 * (d & 4) + (d & 3));
+        dw |= dir_code32<WordCodes::kStep>(hd >= e && m1 >= f, m1 >= f, eo >= ee, fo >= fe) << (d & 7);
         if ((d & 7) == 7 || d == W - 1) {
           D[(static_cast<size_t>(i) * WW + (d >> 3)) * 32] = dw;
           dw = 0;
