@@ -1469,15 +1469,16 @@ void run_u2(const SwLaunch& a, int above) {
 // (usually short or empty), so the kernels stride over it with a few resident waves. A short
 // list's time is one task's serial latency, so four cells a lane, whose row is the shortest; a
 // longer one's is its instructions: 8 or 16 cells, or a thread per task. Tracebacks of 150
-// rows, us, short form against the other: W = 17 56 and 102 for 500 tasks, 70 and 105 for
-// 5,000, 272 and 193 for 50,000; W = 33 53 and 77, 91 and 103, 545 and 435; W = 129 60 and
-// 105, 268 and 227, 3,262 and 1,506. (One kernel with both forms ran the longer lists 5 to 45 %
-// slower.)
+// rows, us, short form against the other: W = 17 54 and 89 for 500 tasks, 91 and 93 for 12,000,
+// 111 and 95 for 16,000; W = 33 54 and 74 for 500, 89 and 103 for 6,000, 111 and 105 for 8,000;
+// W = 65 54 and 105, 91 and 107 for 3,000, 115 and 107 for 4,000; W = 129 60 and 105, 105 and 105
+// for 1,500, 132 and 107 for 2,000 (rows of 1,000 and scores alone cross at the same lengths).
+// (One kernel with both forms ran the longer lists 5 to 45 % slower.)
 template <int W>
 void run_fb(const SwLaunch& a) {
   constexpr bool kShort = (W - 1) % 4 == 0, kLanes = W == 33 || W == 65 || W == 129;
   constexpr int CH = W == 33 ? 8 : 16;
-  const int few = kShort ? 262144 / (W - 1) : 0;
+  const int few = kShort ? 196608 / (W - 1) : 0;
   const auto grid = [&](int lanes) {
     return std::min(8 * device_sm_count(),
                     static_cast<int>((static_cast<int64_t>(a.count) * lanes + kSwThreads - 1) / kSwThreads));
