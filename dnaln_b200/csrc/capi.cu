@@ -144,7 +144,8 @@ struct dnaln_ctx {
   std::map<int32_t, IndexRes> idx;
   int32_t next_id = 1;
   std::map<std::string, DevBuf> bufs;
-  int64_t* d_ctl = nullptr;    // kCtlWords counters; the next two point into it
+  int64_t* d_ctl = nullptr;    // kCtlWords counters and kCtlBase; the next two point into it
+  int64_t ctl_base = -1;       // the value at kCtlBase
   uint32_t* d_err = nullptr;   // kernel error flags
   int* d_count = nullptr;      // [0] score tasks, [1] traceback tasks, [2] reads listed for the warp path
   int64_t* h_info = nullptr;   // pinned read-back slots
@@ -408,6 +409,7 @@ constexpr int kCtlCount = 12;   // d_count: 4 ints
 constexpr int kCtlClaims = 14;  // 6 ints, see map_enqueue
 constexpr int kCtlErr = 17;     // d_err
 constexpr int kCtlWords = 18;
+constexpr int kCtlBase = 18;    // past the cleared words: what is added to every record's cigar_off
 
 inline unsigned nblk(int64_t n, int t = 256) { return static_cast<unsigned>((n + t - 1) / t); }
 
@@ -869,7 +871,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
     if (!d_cigar) return DNALN_ERR_OOM;
   }
   kt.begin(st, "k_cigar_gather");
-  launch_cigar_gather(st, n, pofs, d_seq_len, res_tb, cig_tb, ops, hint.cigar_base, d_out, d_cigar, cigar_cap,
+  launch_cigar_gather(st, n, pofs, d_seq_len, res_tb, cig_tb, ops, c->d_ctl + kCtlBase, d_out, d_cigar, cigar_cap,
                       reinterpret_cast<long long*>(c->d_ctl + kCtlOps), c->d_err);
   kt.end(st);
   CK(cudaEventRecord(c->ev[kEvPost1], st));
@@ -977,7 +979,7 @@ std::string graph_key(const dnaln_ctx* c, const IndexRes& ix, const char* d_seq,
   put(&ix.dev, sizeof ix.dev);  // every pointer and dimension of the index the kernels take
   const void* ptrs[] = {d_seq, d_seq_off, d_seq_len, d_hash, d_out, d_cigar, c->st};
   put(ptrs, sizeof ptrs);
-  const int64_t nums[] = {n, hint.seq_base, hint.bases, hint.max_len, hint.cigar_base, cigar_cap, c->pool_cap,
+  const int64_t nums[] = {n, hint.seq_base, hint.bases, hint.max_len, cigar_cap, c->pool_cap,
                           static_cast<int64_t>(c->dir_cap_bytes), c->sw_mode, c->warp_seed_only, c->long_thread,
                           c->length_order, c->ungapped, c->colinear, c->stealing, c->encode_bulk, c->seed_block,
                           c->seed_tune.tuned ? c->seed_tune.reads_per_block : 0};
@@ -1015,6 +1017,14 @@ int run_map(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_seq_
     hint.bases = c->h_info[0];
     hint.max_len = c->h_info[1];
     c->stats.launches += 1;
+  }
+  // a later part's place among the batch's CIGARs depends on the reads before it: handed over on the
+  // device, so that the part's graph serves other reads too
+  if (c->ctl_base != hint.cigar_base) {
+    c->h_info[kCtlBase] = hint.cigar_base;
+    c->ctl_base = -1;
+    CK(cudaMemcpyAsync(c->d_ctl + kCtlBase, c->h_info + kCtlBase, sizeof(int64_t), cudaMemcpyHostToDevice, c->st));
+    c->ctl_base = hint.cigar_base;
   }
   const bool graphable = c->graphs && hint.bases >= 0 && hint.max_len >= 0 && !c->trace_on && !hint.retry;
   std::string key;
@@ -1519,7 +1529,7 @@ int dnaln_gpu_ctx_create(int device, dnaln_ctx** out) {
   for (auto& x : c->out_free) bad(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
   for (auto& x : c->h2d_ev) bad(cudaEventCreate(&x));
   for (auto& x : c->d2h_ev) bad(cudaEventCreate(&x));
-  bad(cudaMalloc(&c->d_ctl, kCtlWords * sizeof(int64_t)));
+  bad(cudaMalloc(&c->d_ctl, (kCtlWords + 1) * sizeof(int64_t)));
   c->d_err = reinterpret_cast<uint32_t*>(c->d_ctl + kCtlErr);
   c->d_count = reinterpret_cast<int*>(c->d_ctl + kCtlCount);
   bad(cudaHostAlloc(&c->h_info, 24 * sizeof(int64_t), cudaHostAllocDefault));

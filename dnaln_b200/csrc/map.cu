@@ -303,7 +303,7 @@ __global__ void k_records(int64_t n, const int32_t* __restrict__ seq_len, CandBu
 __global__ void k_cigar_gather(int64_t n, const int64_t* __restrict__ pofs, const int32_t* __restrict__ seq_len,
                                const SwResult* __restrict__ res_tb, const uint32_t* __restrict__ cig_src,
                                const int32_t* __restrict__ op_count, const long long* __restrict__ op_sums,
-                               const long long* __restrict__ op_groups, int64_t rec_base,
+                               const long long* __restrict__ op_groups, const int64_t* __restrict__ rec_base,
                                dnaln_map_record* __restrict__ out, uint32_t* __restrict__ dst, int64_t cap,
                                long long* __restrict__ total_ops, uint32_t* __restrict__ err) {
   __shared__ long long part[2][32];
@@ -317,7 +317,7 @@ __global__ void k_cigar_gather(int64_t n, const int64_t* __restrict__ pofs, cons
   const int64_t o = base + block_exclusive_scan_ll(cnt, &block_ops, part[1]);
   if (threadIdx.x == 0 && blockIdx.x + 1 == gridDim.x) *total_ops = base + block_ops;
   if (r >= n) return;
-  out[r].cigar_off = rec_base + o;
+  out[r].cigar_off = *rec_base + o;
   out[r].cigar_len = static_cast<int32_t>(cnt);
   if (cnt == 0) return;
   if (o + cnt > cap) {  // the caller's buffer is too small: the call reports the size it needs
@@ -415,7 +415,7 @@ void launch_records(cudaStream_t st, int64_t n, const int32_t* seq_len, CandBuf 
 }
 
 void launch_cigar_gather(cudaStream_t st, int64_t n, const int64_t* pofs, const int32_t* seq_len,
-                         const SwResult* res_tb, const uint32_t* cig_src, OpSums ops, int64_t rec_base,
+                         const SwResult* res_tb, const uint32_t* cig_src, OpSums ops, const int64_t* rec_base,
                          dnaln_map_record* out, uint32_t* dst, int64_t cap, long long* total_ops, uint32_t* err) {
   if (n <= 0) return;
   k_cigar_gather<<<blocks_for(n), kThreads, 0, st>>>(n, pofs, seq_len, res_tb, cig_src, ops.count, ops.sums,

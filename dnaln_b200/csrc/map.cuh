@@ -52,12 +52,12 @@ void launch_records(cudaStream_t st, int64_t n, const int32_t* seq_len, CandBuf 
                     dnaln_map_record* out, OpSums ops, unsigned long long* ctr);
 
 // Writes each mapped read's CIGAR (leading S, the walk's ops reversed, trailing S) at
-// dst + the operations of the reads before it, and sets out[r].cigar_off (plus rec_base) and
+// dst + the operations of the reads before it, and sets out[r].cigar_off (plus *rec_base) and
 // cigar_len; a CIGAR that would end past cap ops is not written and sets kErrOutputCapacity.
 // *total_ops = all operations.
 // cig_src slot of read r is 2 * pofs[r] + r.
 void launch_cigar_gather(cudaStream_t st, int64_t n, const int64_t* pofs, const int32_t* seq_len,
-                         const SwResult* res_tb, const uint32_t* cig_src, OpSums ops, int64_t rec_base,
+                         const SwResult* res_tb, const uint32_t* cig_src, OpSums ops, const int64_t* rec_base,
                          dnaln_map_record* out, uint32_t* dst, int64_t cap, long long* total_ops, uint32_t* err);
 
 // GpuAligner: the tasks of n (offset, length) pairs, queries at [0, n) and targets at [n, 2n)

@@ -68,6 +68,25 @@ def test_a_refused_batch_writes_nothing(ctx, genome):
         ctx.index_free(iid)
 
 
+def test_new_reads_replay_both_parts(ctx, genome):
+    iid = ctx.index_build(genome)
+    batches = [Batch(genome, 10 + s) for s in range(4)]
+    try:
+        rose = []
+        for b in batches:
+            before = ctx.stats()["graph_launches"]
+            assert b.map(ctx, iid, N * 16)[0] == 0
+            rose.append(ctx.stats()["graph_launches"] - before)
+        assert rose[-1] == 2, rose
+        ctx.set_option("graphs", 0)
+        got = batches[-1].rec.clone(), batches[-1].cig.clone()
+        assert batches[-1].map(ctx, iid, N * 16)[0] == 0
+        assert torch.equal(batches[-1].rec, got[0]) and torch.equal(batches[-1].cig, got[1])
+    finally:
+        ctx.set_option("graphs", 1)
+        ctx.index_free(iid)
+
+
 def test_halves_with_gaps_between_their_reads(ctx, genome):
     iid = ctx.index_build(genome)
     b = Batch(genome, 40)
