@@ -144,6 +144,7 @@ struct dnaln_ctx {
   std::map<int32_t, IndexRes> idx;
   int32_t next_id = 1;
   std::map<std::string, DevBuf> bufs;
+  DevBuf index_work;  // workspace of index builds, kept up to kIndexWorkKept bytes
   int64_t* d_ctl = nullptr;    // kCtlWords counters and kCtlBase; the next two point into it
   int64_t ctl_base = -1;       // the value at kCtlBase
   uint32_t* d_err = nullptr;   // kernel error flags
@@ -238,6 +239,30 @@ int fail(dnaln_ctx* c, int code, const char* fmt, ...) {
     if (e_ != cudaSuccess) return fail(c, DNALN_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
   } while (0)
 
+// Grows b to at least `need` bytes; false (and the context error) on failure.
+bool grow(dnaln_ctx* c, DevBuf& b, const char* name, size_t need) {
+  if (b.p) cudaFree(b.p);
+  b.p = nullptr;
+  b.cap = 0;
+  if (c->fail_alloc_after >= 0 && c->fail_alloc_after-- == 0) {
+    fail(c, DNALN_ERR_OOM, "out of device memory allocating %zu bytes for %s (injected)", need, name);
+    return false;
+  }
+  size_t cap = need + need / 4;
+  if (cudaMalloc(&b.p, cap) != cudaSuccess) {
+    cudaGetLastError();
+    cap = need;
+    if (cudaMalloc(&b.p, cap) != cudaSuccess) {
+      cudaGetLastError();
+      b.p = nullptr;
+      fail(c, DNALN_ERR_OOM, "out of device memory allocating %zu bytes for %s", need, name);
+      return false;
+    }
+  }
+  b.cap = cap;
+  return true;
+}
+
 // Grow-only device buffer; returns nullptr (and sets the context error) on failure.
 template <class T>
 T* dbuf(dnaln_ctx* c, const char* name, size_t count) {
@@ -249,25 +274,7 @@ T* dbuf(dnaln_ctx* c, const char* name, size_t count) {
       return nullptr;
     }
     ++c->epoch;  // graphs captured before may reference the old buffer
-    if (b.p) cudaFree(b.p);
-    b.p = nullptr;
-    b.cap = 0;
-    if (c->fail_alloc_after >= 0 && c->fail_alloc_after-- == 0) {
-      fail(c, DNALN_ERR_OOM, "out of device memory allocating %zu bytes for %s (injected)", need, name);
-      return nullptr;
-    }
-    size_t cap = need + need / 4;
-    if (cudaMalloc(&b.p, cap) != cudaSuccess) {
-      cudaGetLastError();
-      cap = need;
-      if (cudaMalloc(&b.p, cap) != cudaSuccess) {
-        cudaGetLastError();
-        b.p = nullptr;
-        fail(c, DNALN_ERR_OOM, "out of device memory allocating %zu bytes for %s", need, name);
-        return nullptr;
-      }
-    }
-    b.cap = cap;
+    if (!grow(c, b, name, need)) return nullptr;
   }
   return static_cast<T*>(b.p);
 }
@@ -1558,6 +1565,7 @@ int dnaln_gpu_ctx_destroy(dnaln_ctx* c) {
   for (auto& kv : c->idx) free_index(kv.second);
   for (auto& kv : c->bufs)
     if (kv.second.p) cudaFree(kv.second.p);
+  if (c->index_work.p) cudaFree(c->index_work.p);
   if (c->cp_in) cudaStreamSynchronize(c->cp_in);
   if (c->cp_out) cudaStreamSynchronize(c->cp_out);
   for (auto& x : c->ev)
@@ -1790,7 +1798,9 @@ int dnaln_gpu_index_build(dnaln_ctx* c, const uint8_t* genome, uint64_t n_bases,
   e = build_index_on_device(
       c->st, static_cast<const uint8_t*>(m.genome.p), n_bases, static_cast<const uint64_t*>(m.coff.p),
       static_cast<const uint32_t*>(m.clen.p), contig_len, n_contigs, k, w,
-      [&](size_t bytes) -> void* { return dbuf<uint8_t>(c, "index_work", bytes); },
+      [&](size_t bytes) -> void* {  // apart from bufs: no graph refers to it, so its growth drops none
+        return c->index_work.cap >= bytes || grow(c, c->index_work, "index_work", bytes) ? c->index_work.p : nullptr;
+      },
       [&](size_t bytes) -> void* {
         DevBuf built;
         return dalloc(c, m, built, bytes) == DNALN_OK ? built.p : nullptr;
@@ -1800,10 +1810,10 @@ int dnaln_gpu_index_build(dnaln_ctx* c, const uint8_t* genome, uint64_t n_bases,
   m.positions = DevBuf{b.positions, b.n_pos * sizeof(uint32_t)};
   m.nruns = DevBuf{b.n_runs, static_cast<size_t>(b.n_n_runs) * sizeof(uint2)};
   // the workspace stays for the next build of a genome this size, unless it is large
-  if (c->bufs["index_work"].cap > kIndexWorkKept) {
+  if (c->index_work.cap > kIndexWorkKept) {
     cudaStreamSynchronize(c->st);
-    cudaFree(c->bufs["index_work"].p);
-    c->bufs.erase("index_work");
+    cudaFree(c->index_work.p);
+    c->index_work = DevBuf{};
   }
   if (e != DNALN_OK) {
     cudaStreamSynchronize(c->st);
