@@ -695,6 +695,35 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       launch_encode_reads(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, codes);
     kt.end(st);
     c->stats.launches += 1;
+    const auto seed_t = [&](const int32_t* list, const int* list_n, int reads_per_block) {
+      return launch_seed_chain_thread(st, codes, pofs, d_seq_len, list, list_n, n, ix.dev, sp, cp, cand, cb, n_min,
+                                      n_anchor, n_anc_t, big_list, big_n, c->d_err, reads_per_block);
+    };
+    int rpb = c->seed_block ? c->seed_block : (c->seed_tune.tuned ? c->seed_tune.reads_per_block : 0);
+    if (rpb == 0 && (n < kSeedTuneReads || c->capturing)) rpb = 128;  // too small to time, or no host waits now
+    if (rpb == 0) {
+      // the reads-per-block tuner, over all reads of the batch (of the list the colinear kernels
+      // leave, a few reads that are handed on say nothing): each block size once untimed (a kernel's
+      // first launch also loads it), then each timed. The batch's own launches follow and rewrite
+      // all outputs; the list of reads handed on is cleared before each run.
+      const int sizes[2] = {64, 128};
+      for (int x = 0; x < 4; ++x) {
+        CK(cudaMemsetAsync(big_n, 0, sizeof(int), st));
+        if (x >= 2) CK(cudaEventRecord(c->tune_ev[x - 2], st));
+        if (!seed_t(nullptr, nullptr, sizes[x & 1]))
+          return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
+        if (x >= 2) CK(cudaEventRecord(c->tune_ev[x], st));
+      }
+      CK(cudaMemsetAsync(big_n, 0, sizeof(int), st));
+      CK(cudaEventSynchronize(c->tune_ev[3]));
+      dnaln_seed_tuning& t = c->seed_tune;
+      t.ms_64 = ev_ms(c->tune_ev[0], c->tune_ev[2]);
+      t.ms_128 = ev_ms(c->tune_ev[1], c->tune_ev[3]);
+      t.reads_per_block = rpb = t.ms_64 < t.ms_128 ? 64 : 128;
+      t.reads = n;
+      t.tuned = 1;
+      c->stats.launches += 4;
+    }
     // reads whose anchors form one colinear chain; the others are listed for the full kernels
     const int32_t* full_list = nullptr;
     const int* full_n = nullptr;
@@ -729,41 +758,10 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       warp_n = claims;
       run.direct = true;
     } else {
-      const auto seed_t = [&](int rpb) {
-        return launch_seed_chain_thread(st, codes, pofs, d_seq_len, full_list, full_n, n, ix.dev, sp, cp, cand, cb,
-                                        n_min, n_anchor, n_anc_t, big_list, big_n, c->d_err, rpb);
-      };
-      int rpb = c->seed_block ? c->seed_block : (c->seed_tune.tuned ? c->seed_tune.reads_per_block : 0);
-      if (rpb == 0 && (n < kSeedTuneReads || c->capturing)) rpb = 128;  // too small to time, or no host waits now
-      if (rpb == 0) {
-        // the reads-per-block tuner: each block size once untimed (a kernel's first launch
-        // also loads it), then each timed; every run rewrites the same outputs (the list of
-        // reads handed on is cleared before each), so the last run's stand
-        const int sizes[2] = {64, 128};
-        for (int x = 0; x < 2; ++x) {
-          CK(cudaMemsetAsync(big_n, 0, sizeof(int), st));
-          if (!seed_t(sizes[x])) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
-        }
-        for (int x = 0; x < 2; ++x) {
-          CK(cudaMemsetAsync(big_n, 0, sizeof(int), st));
-          CK(cudaEventRecord(c->tune_ev[x], st));
-          if (!seed_t(sizes[x])) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
-          CK(cudaEventRecord(c->tune_ev[x + 2], st));
-        }
-        CK(cudaEventSynchronize(c->tune_ev[3]));
-        dnaln_seed_tuning& t = c->seed_tune;
-        t.ms_64 = ev_ms(c->tune_ev[0], c->tune_ev[2]);
-        t.ms_128 = ev_ms(c->tune_ev[1], c->tune_ev[3]);
-        t.reads_per_block = t.ms_64 < t.ms_128 ? 64 : 128;
-        t.reads = n;
-        t.tuned = 1;
-        c->stats.launches += 3;
-      } else {
-        kt.begin(st, "k_seed_chain_t");
-        const bool ok = seed_t(rpb);
-        kt.end(st);
-        if (!ok) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
-      }
+      kt.begin(st, "k_seed_chain_t");
+      const bool ok = seed_t(full_list, full_n, rpb);
+      kt.end(st);
+      if (!ok) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
       if (c->long_thread && seed_long_supported(sp, cp) && max_len > seed_thread_max_len()) {
         // long reads one thread each, in length order; what exceeds its bounds goes on
         const int64_t lt = seed_long_threads(n);
