@@ -35,6 +35,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <thread>
 #include <vector>
@@ -120,6 +121,13 @@ struct BatchHints {
   bool caller_cigar = false;  // the CIGARs go to the caller's buffer (not the internal one)
 };
 
+// What a list of SW tasks was launched with, for retune_sw.
+struct SwRun {
+  int key = -1;         // of its tuned form; -1: none was tuned
+  bool listed = false;  // the no-gap proof listed the tasks the DP took (else it took all)
+  int64_t chunk = 0;    // tasks of a launch, at most
+};
+
 // Host facts of an enqueued batch that its completion needs.
 struct MapRun {
   int64_t B = 0, max_len = 0, cigar_cap = 0;
@@ -127,6 +135,7 @@ struct MapRun {
   bool thread_path = false, long_used = false;
   bool direct = false;  // the reads the colinear kernels listed went straight to the warp kernels
   uint64_t launches = 0;  // kernels the enqueue issued (counted again at each graph replay)
+  SwRun sw[2];            // score only, traceback
 };
 
 struct CachedGraph {  // an instantiated batch graph and the buffer epoch it was captured at
@@ -188,6 +197,7 @@ struct dnaln_ctx {
   // tuned on the first batch that needs it, 1 = inter-sequence, 2 = intra-sequence
   int sw_mode = 0;
   std::map<int, dnaln_sw_tuning> sw_tune;
+  std::set<int> sw_retune;  // keys to be tuned again (retune_sw)
   cudaEvent_t tune_ev[kSwForms + 1] = {};
   int* h_tune = nullptr;  // pinned read-back of a device task count
   int64_t pool_cap = 0;   // entries of the warp-path chaining pool (grown from the batches' use)
@@ -432,10 +442,11 @@ int check_device_errors(dnaln_ctx* c, uint32_t bits) {
 // proved to align without a gap (option "ungapped"), then the DP kernels over the rest, in
 // length order when by_length (a thread's two alignments and a warp's 64 then have similar
 // lengths, so no lane idles through a long partner's rows), chunked so the direction-bit
-// scratch stays within dir_cap_bytes.
+// scratch stays within dir_cap_bytes. *todo_n (0 before) counts the tasks the proof leaves.
 int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks, int n_max, const int* n_dev,
                       const uint8_t* qbase, const uint8_t* tbase, const SwParams& sp, SwResult* res, int rows_max,
-                      uint32_t* cig, const int64_t* cig_off, bool by_length) {
+                      uint32_t* cig, const int64_t* cig_off, bool by_length, int* todo_n, SwRun& run_of) {
+  run_of = SwRun{};
   if (n_max <= 0) return DNALN_OK;
   const bool ungapped = c->ungapped && sw_ungapped_supported(sp, bytes_ok) &&
                         (c->ungapped == 2 || sw_ungapped_pays(sp.W, bytes_ok, n_max));
@@ -444,21 +455,21 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
   if (sw_has_form(sp.W, bytes_ok, kSwIntraFew) && n_max <= int64_t{4} * device_sm_count() * 256 / (sp.W - 1))
     by_length = false;
   if (ungapped || (by_length && n_max > 1)) {
-    // [0] listed tasks, then the length bins' counts and the places taken of each
     const KernelTrace kt = tracer(c);
-    DBUF(cnt, int, "sw_todo_n", 2 + 2 * kLengthBins);
-    CK(cudaMemsetAsync(cnt, 0, (by_length ? 2 + 2 * kLengthBins : 1) * sizeof(int), c->st));
-    int* hist = by_length ? cnt + 2 : nullptr;
+    DBUF(bins, int, "sw_bins", 2 * kLengthBins);  // the length bins' counts and the places taken of each
+    if (by_length) CK(cudaMemsetAsync(bins, 0, 2 * kLengthBins * sizeof(int), c->st));
+    int* hist = by_length ? bins : nullptr;
     const int bin_shift = length_bin_shift(rows_max);
     if (ungapped) {
       DBUF(todo, SwTask, "sw_todo", n_max);
       kt.begin(c->st, tb ? "k_sw_ungapped<tb>" : "k_sw_ungapped<score>");
-      launch_sw_ungapped(c->st, tb, tasks, n_max, n_dev, qbase, tbase, sp, res, cig, cig_off, todo, cnt, hist,
+      launch_sw_ungapped(c->st, tb, tasks, n_max, n_dev, qbase, tbase, sp, res, cig, cig_off, todo, todo_n, hist,
                          bin_shift);
       kt.end(c->st);
       c->stats.launches += 1;
       tasks = todo;
-      n_dev = cnt;
+      n_dev = todo_n;
+      run_of.listed = true;
     } else {
       kt.begin(c->st, "k_length_bins");
       launch_length_bins(c->st, tasks, n_max, n_dev, hist, bin_shift);
@@ -509,8 +520,10 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
   if (c->sw_mode != 0 && sw_has_form(sp.W, bytes_ok, static_cast<SwForm>(c->sw_mode - 1))) {
     form = static_cast<SwForm>(c->sw_mode - 1);
   } else if (forms.size() > 1) {
+    run_of.key = key;
+    run_of.chunk = chunk;
     auto it = c->sw_tune.find(key);
-    if (it != c->sw_tune.end()) form = static_cast<SwForm>(it->second.form);
+    if (it != c->sw_tune.end() && !c->sw_retune.count(key)) form = static_cast<SwForm>(it->second.form);
     else if (c->capturing) return fail(c, DNALN_ERR_CUDA, "capture stopped: a kernel form is still to be tuned");
     else tune = true;
   }
@@ -560,8 +573,8 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
           form = forms[x];
         }
       }
-      // a sample of a few tasks times launch overheads, not the forms: keep the width's
-      // first form (inter-sequence where it has one)
+      // a sample of a few tasks times launch overheads, not the forms: the width's first form
+      // (inter-sequence where it has one) until a list has enough (retune_sw)
       if (live < kSwTuneMinTasks) form = forms.front();
       t.ms_inter = sw_has_form(sp.W, bytes_ok, kSwInter) ? ms[kSwInter] : -1.0;
       t.ms_intra = sw_has_form(sp.W, bytes_ok, kSwIntra) ? ms[kSwIntra] : -1.0;
@@ -570,12 +583,23 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
       t.lanes_per_pair = sw_lanes_per_pair(sp.W, form);
       t.tasks = live;
       c->sw_tune[key] = t;
+      c->sw_retune.erase(key);
       continue;
     }
     if (!run(form)) return fail(c, DNALN_ERR_DEVICE, "SW launch without its scratch (W=%d)", sp.W);
   }
   CK(cudaGetLastError());
   return DNALN_OK;
+}
+
+// A form chosen from a sample too small to time it is chosen again by the next batch, once a list
+// had enough tasks (`tasks` went to the DP); graphs of the former choice go with it.
+void retune_sw(dnaln_ctx* c, const SwRun& r, int64_t tasks) {
+  if (r.key < 0 || std::min(tasks, r.chunk) < kSwTuneMinTasks) return;
+  const auto it = c->sw_tune.find(r.key);
+  if (it == c->sw_tune.end() || it->second.tasks >= kSwTuneMinTasks || c->sw_retune.count(r.key)) return;
+  c->sw_retune.insert(r.key);
+  ++c->epoch;
 }
 
 // ord = the reads of a list (or all n), longest first by length bin.
@@ -631,7 +655,8 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   // chaining pool's fill, [10] long reads the colinear kernel finished
   unsigned long long* info = reinterpret_cast<unsigned long long*>(c->d_ctl + kCtlInfo);
   // [0] reads the colinear kernels listed, [1] work-stealing claims of the warp chaining kernel,
-  // [2] reads it listed for their anchor count, [3] claims of those
+  // [2] reads it listed for their anchor count, [3] claims of those, [4] and [5] score and traceback
+  // tasks the no-gap proof left
   int* claims = reinterpret_cast<int*>(c->d_ctl + kCtlClaims);
   CK(cudaMemsetAsync(c->d_ctl, 0, kCtlWords * sizeof(int64_t), st));
   unsigned long long* ctr = info + 1;  // cells, mapped, candidates (map.cuh)
@@ -839,7 +864,8 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
   launch_score_tasks(st, n, pofs, d_seq_len, cb, ix.dev, mc, sc_tasks, c->d_count, ctr);
   kt.end(st);
   if (int e = launch_sw_chunked(c, false, bytes_ok, sc_tasks, static_cast<int>(n * MC), c->d_count, codes,
-                                ix.dev.genome, swp, res_sc, static_cast<int>(max_len), nullptr, nullptr, by_length))
+                                ix.dev.genome, swp, res_sc, static_cast<int>(max_len), nullptr, nullptr, by_length,
+                                claims + 4, run.sw[0]))
     return e;
   CK(cudaEventRecord(c->ev[kEvSc1], st));
 
@@ -859,7 +885,8 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
                 cig_slot, ops, n_min, thread_path ? n_anc_t : nullptr, info + 4, ctr);
   kt.end(st);
   if (int e = launch_sw_chunked(c, true, bytes_ok, tb_tasks, static_cast<int>(n), c->d_count + 1, codes,
-                                ix.dev.genome, swp, res_tb, static_cast<int>(max_len), cig_tb, cig_slot, by_length))
+                                ix.dev.genome, swp, res_tb, static_cast<int>(max_len), cig_tb, cig_slot, by_length,
+                                claims + 5, run.sw[1]))
     return e;
   CK(cudaEventRecord(c->ev[kEvTb1], st));
 
@@ -943,8 +970,10 @@ int map_finish(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_s
   trace_collect(c);
 
   const int n_listed = counts[2];                                        // reads the short thread kernel listed
-  int n_rest;                                                            // reads the colinear kernels listed
-  std::memcpy(&n_rest, h + kCtlClaims, sizeof n_rest);
+  int claims[6];                                                         // see map_enqueue
+  std::memcpy(claims, h + kCtlClaims, sizeof claims);
+  const int n_rest = claims[0];                                          // reads the colinear kernels listed
+  for (int x = 0; x < 2; ++x) retune_sw(c, run.sw[x], run.sw[x].listed ? claims[4 + x] : counts[x]);
   const int n_warp = !thread_path ? static_cast<int>(n) : (run.direct ? n_rest : counts[run.long_used ? 3 : 2]);
   dnaln_stats& s = c->stats;
   s.reads += static_cast<uint64_t>(n);
@@ -2384,7 +2413,7 @@ int dnaln_gpu_align(dnaln_ctx* c, const uint8_t* q, const int64_t* q_off, const 
   DBUF(d_tasks, SwTask, "al_tasks", n);
   DBUF(d_res, SwResult, "al_res", n);
   DBUF(d_out, dnaln_align_result, "al_out", n);
-  CK(cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), st));
+  CK(cudaMemsetAsync(c->d_ctl, 0, kCtlWords * sizeof(int64_t), st));
   CK(cudaMemcpyAsync(d_off, q_off, n * sizeof(int64_t), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_off + n, t_off, n * sizeof(int64_t), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_len, q_len, n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
@@ -2407,8 +2436,10 @@ int dnaln_gpu_align(dnaln_ctx* c, const uint8_t* q, const int64_t* q_off, const 
   if (tb)  // each task's room for 2 * qlen + 1 operations
     if (int e = exclusive_scan(c, d_cnt, d_slot, n + 1)) return e;
   CK(cudaEventRecord(c->ev[tb ? kEvTb0 : kEvSc0], st));
+  SwRun run;
+  int* const todo_n = reinterpret_cast<int*>(c->d_ctl + kCtlClaims);
   if (int e = launch_sw_chunked(c, tb, sw_bytes_ok(*sp), d_tasks, static_cast<int>(n), nullptr, d_q, d_t, swp, d_res,
-                                rows_max, d_cig, d_slot, by_length))
+                                rows_max, d_cig, d_slot, by_length, todo_n, run))
     return e;
   CK(cudaEventRecord(c->ev[tb ? kEvTb1 : kEvSc1], st));
   int64_t total = 0;
@@ -2429,12 +2460,15 @@ int dnaln_gpu_align(dnaln_ctx* c, const uint8_t* q, const int64_t* q_off, const 
       CK(cudaMemcpyAsync(cigar, d_final, total * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   }
   CK(cudaMemcpyAsync(out, d_out, n * sizeof(dnaln_align_result), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(c->h_info, c->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(c->h_info, c->d_ctl, kCtlWords * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   trace_collect(c);
   uint32_t bits;
-  std::memcpy(&bits, c->h_info, sizeof bits);
+  std::memcpy(&bits, c->h_info + kCtlErr, sizeof bits);
   if (int e = check_device_errors(c, bits)) return e;
+  int left;
+  std::memcpy(&left, c->h_info + kCtlClaims, sizeof left);
+  retune_sw(c, run, run.listed ? left : n);
   if (cigar_used) *cigar_used = total;
   c->stats.cells += static_cast<uint64_t>(bases) * W;
   if (tb) {
