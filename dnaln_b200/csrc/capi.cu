@@ -538,10 +538,11 @@ int launch_sw_chunked(dnaln_ctx* c, bool tb, bool bytes_ok, const SwTask* tasks,
   for (int64_t b = 0; b < n_max; b += chunk) {
     const int cnt = static_cast<int>(n_max - b < chunk ? n_max - b : chunk);
     const auto run = [&](SwForm f) {
-      const bool ok = launch_sw(c->st, tb, bytes_ok, tasks, static_cast<int>(b), cnt, n_max, n_dev, qbase, tbase, sp,
-                                res, dir, rows_max, cig, cig_off, band, fb, c->d_err, &kt, f, b == 0 ? few : 0);
-      c->stats.launches += static_cast<uint64_t>(sw_launches(sp.W, bytes_ok, tb)) + (b == 0 && few > 0 ? 1 : 0);
-      return ok;
+      const int launched = launch_sw(c->st, tb, bytes_ok, tasks, static_cast<int>(b), cnt, n_max, n_dev, qbase, tbase,
+                                     sp, res, dir, rows_max, cig, cig_off, band, fb, c->d_err, &kt, f,
+                                     b == 0 ? few : 0);
+      c->stats.launches += static_cast<uint64_t>(std::max(launched, 0));
+      return launched >= 0;
     };
     if (b == 0 && tune) {
       // every form once untimed first: a kernel's first launch in a process also loads it
@@ -786,6 +787,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
       kt.begin(st, "k_seed_chain_t");
       const bool ok = seed_t(full_list, full_n, rpb);
       kt.end(st);
+      c->stats.launches += 1;
       if (!ok) return fail(c, DNALN_ERR_CUDA, "thread-per-read seeding kernel could not be configured");
       if (c->long_thread && seed_long_supported(sp, cp) && max_len > seed_thread_max_len()) {
         // long reads one thread each, in length order; what exceeds its bounds goes on
@@ -816,11 +818,13 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
     launch_seed_list(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, warp_list, warp_n, full_list != nullptr,
                      codes, ix.dev, sp, mb, n_min, n_anchor, c->d_err);
     kt.end(st);
+    c->stats.launches += 1;
   } else {
     kt.begin(st, "k_seed");
     launch_seed(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, codes, ix.dev, sp, mb, n_min, n_anchor,
                 c->d_err);
     kt.end(st);
+    c->stats.launches += 1;
   }
   CK(cudaEventRecord(c->ev[kEvSeed1], st));
   CK(cudaGetLastError());
@@ -989,9 +993,9 @@ int map_finish(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_s
   s.cells += n_cells;
   s.mapped += n_mapped;
   s.candidates += n_cands;
-  // k_score_tasks, k_choose, k_records, k_cigar_gather, pass 1 / 2, plus what the enqueue
-  // counted
-  s.launches += 6 + (thread_path ? 2 : 1) + run.launches;
+  // k_chain_map, k_chain_big, k_score_tasks, k_choose, k_records, k_cigar_gather, plus what the
+  // enqueue counted
+  s.launches += 6 + run.launches;
   s.ms_seed += ev_ms(c, kEvSeed0, kEvSeed1);
   s.ms_chain += ev_ms(c, kEvChain0, kEvChain1);
   s.ms_sw_score += ev_ms(c, kEvSc0, kEvSc1);
@@ -2471,6 +2475,7 @@ int dnaln_gpu_align(dnaln_ctx* c, const uint8_t* q, const int64_t* q_off, const 
   retune_sw(c, run, run.listed ? left : n);
   if (cigar_used) *cigar_used = total;
   c->stats.cells += static_cast<uint64_t>(bases) * W;
+  c->stats.launches += tb ? 3 : 2;  // k_align_tasks; k_align_counts and k_align_gather, or k_align_scores
   if (tb) {
     c->stats.sw_tasks_tb += static_cast<uint64_t>(n);
     c->stats.ms_sw_tb += ev_ms(c, kEvTb0, kEvTb1);

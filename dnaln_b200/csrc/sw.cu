@@ -1475,7 +1475,7 @@ void run_u2(const SwLaunch& a, int above) {
 // for 1,500, 132 and 107 for 2,000 (rows of 1,000 and scores alone cross at the same lengths).
 // (One kernel with both forms ran the longer lists 5 to 45 % slower.)
 template <int W>
-void run_fb(const SwLaunch& a) {
+int run_fb(const SwLaunch& a) {  // the kernels launched
   constexpr bool kShort = (W - 1) % 4 == 0, kLanes = W == 33 || W == 65 || W == 129;
   constexpr int CH = W == 33 ? 8 : 16;
   const int few = kShort ? 196608 / (W - 1) : 0;
@@ -1505,15 +1505,22 @@ void run_fb(const SwLaunch& a) {
     }
   }
   a.kt.end(a.st);
+  return (kShort ? 1 : 0) + (a.count > few ? 1 : 0);
 }
 
 // One band width: the form for short lists (few > 0: it takes a device count of at most
-// `few`, the main form any other), the main form, the int32 kernel, the walk.
+// `few`, the main form any other), the main form, the int32 kernel, the walk. Returns the kernels
+// launched.
 template <int W>
-void launch_band(const SwLaunch& a, SwForm form, int few) {
+int launch_band(const SwLaunch& a, SwForm form, int few) {
   cudaMemsetAsync(a.fb, 0, kFbList * sizeof(int), a.st);
-  if (form == kSwIntraFew) run_wide<W, 4>(a, a.count, 0, INT_MAX);
-  else if (few > 0) run_wide<W, 4>(a, std::min(a.count, few), 0, few);
+  int launched = 1;  // the main form
+  if (form == kSwIntraFew) {
+    run_wide<W, 4>(a, a.count, 0, INT_MAX);
+  } else if (few > 0) {
+    run_wide<W, 4>(a, std::min(a.count, few), 0, few);
+    ++launched;
+  }
   if constexpr (sw_has_intra(W)) {
     if (form == kSwIntra) run_wide<W, 32>(a, a.count, few, INT_MAX);
   }
@@ -1523,7 +1530,7 @@ void launch_band(const SwLaunch& a, SwForm form, int few) {
   if constexpr (W != 129) {
     if (form == kSwInter) run_u2<W>(a, few);
   }
-  run_fb<W>(a);
+  launched += run_fb<W>(a);
   if (a.tb) {
     const int lane_blocks = std::min(
         16 * device_sm_count(),
@@ -1535,7 +1542,9 @@ void launch_band(const SwLaunch& a, SwForm form, int few) {
     k_sw_walk<W><<<blocks, kSwThreads, 0, a.st>>>(a.tasks, a.base, a.count, a.n, a.n_dev, a.qbase, a.tbase, a.p,
                                                   a.res, a.dir, a.rows_max, a.cig, a.cig_off, a.err);
     a.kt.end(a.st);
+    ++launched;
   }
+  return launched;
 }
 
 }  // namespace
@@ -1590,8 +1599,6 @@ int sw_few_tasks(int W) {
   }
 }
 
-int sw_launches(int W, bool bytes_ok, bool tb) { return sw_uses_generic(W, bytes_ok) ? 1 : (tb ? 3 : 2); }
-
 bool sw_has_form(int W, bool bytes_ok, SwForm form) {
   if (sw_uses_generic(W, bytes_ok)) return form == kSwInter;
   switch (form) {
@@ -1610,13 +1617,13 @@ int sw_lanes_per_pair(int W, SwForm form) {
   return 1;
 }
 
-bool launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int base, int count, int n,
-               const int* n_dev, const uint8_t* qbase, const uint8_t* tbase, const SwParams& p, SwResult* res,
-               uint32_t* dir, int rows_max, uint32_t* cig, const int64_t* cig_off, int* band, int* fb,
-               uint32_t* err, const KernelTrace* kt, SwForm form, int few) {
-  if (count <= 0) return true;
+int launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int base, int count, int n,
+              const int* n_dev, const uint8_t* qbase, const uint8_t* tbase, const SwParams& p, SwResult* res,
+              uint32_t* dir, int rows_max, uint32_t* cig, const int64_t* cig_off, int* band, int* fb, uint32_t* err,
+              const KernelTrace* kt, SwForm form, int few) {
+  if (count <= 0) return 0;
   const bool generic = sw_uses_generic(p.W, bytes_ok);
-  if ((tb && !dir) || (generic && !band) || (!generic && !fb) || (base % kSwTaskGroup) != 0) return false;
+  if ((tb && !dir) || (generic && !band) || (!generic && !fb) || (base % kSwTaskGroup) != 0) return -1;
   // the kernels bound their tasks by n (and the device count): a launch covers tasks
   // [base, base + count) only, so that no thread of a grid rounded up past `count` takes a
   // task of the next chunk, whose scratch this launch does not hold
@@ -1628,12 +1635,12 @@ bool launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int
     if (!sw_has_form(p.W, bytes_ok, form)) form = p.W == 129 ? kSwIntra : kSwInter;
     if (!sw_has_form(p.W, bytes_ok, kSwIntraFew)) few = 0;
     switch (p.W) {
-      case 11: launch_band<11>(a, form, few); return true;
-      case 17: launch_band<17>(a, form, few); return true;
-      case 33: launch_band<33>(a, form, few); return true;
-      case 43: launch_band<43>(a, form, few); return true;
-      case 65: launch_band<65>(a, form, few); return true;
-      case 129: launch_band<129>(a, form, few); return true;
+      case 11: return launch_band<11>(a, form, few);
+      case 17: return launch_band<17>(a, form, few);
+      case 33: return launch_band<33>(a, form, few);
+      case 43: return launch_band<43>(a, form, few);
+      case 65: return launch_band<65>(a, form, few);
+      case 129: return launch_band<129>(a, form, few);
       default: break;
     }
   }
@@ -1646,7 +1653,7 @@ bool launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int
     k_sw_any<false><<<blocks, kSwThreads, 0, st>>>(tasks, base, n, n_dev, qbase, tbase, p, res, dir, rows_max, cig,
                                                   cig_off, band, err);
   if (kt) kt->end(st);
-  return true;
+  return 1;
 }
 
 }  // namespace dnb

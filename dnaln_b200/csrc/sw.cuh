@@ -21,9 +21,6 @@ size_t sw_dir_bytes_per_task(int W, int rows_max);
 // Band-row scratch per task of the generic kernel (0 when a register kernel runs).
 size_t sw_band_bytes_per_task(int W, bool bytes_ok);
 
-// Kernels one launch_sw call issues (for launch accounting).
-int sw_launches(int W, bool bytes_ok, bool tb);
-
 // Kernel forms of the register-resident bands, all with the same results: inter-sequence
 // (k_sw_u2, a thread holds the whole band row of two alignments; W != 129) and intra-
 // sequence (k_sw_wide, the row of a pair spread over lanes in a skewed wavefront: (W - 1) /
@@ -45,12 +42,12 @@ int sw_lanes_per_pair(int W, SwForm form);
 // sw_dir_bytes_per_task(W, rows_max) and sw_band_bytes_per_task(W, bytes_ok); `fb`
 // (count + kSwFbHead ints) lists the tasks the 16-bit kernel hands to the int32 one; kt (may be
 // null) times each kernel; few > 0 (needs n_dev) lets kSwIntraFew take the whole launch when
-// *n_dev <= few. Returns false, launching nothing, when a needed scratch pointer
-// is null or base is misaligned.
-bool launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int base, int count, int n,
-               const int* n_dev, const uint8_t* qbase, const uint8_t* tbase, const SwParams& p, SwResult* res,
-               uint32_t* dir, int rows_max, uint32_t* cig, const int64_t* cig_off, int* band, int* fb,
-               uint32_t* err, const KernelTrace* kt, SwForm form = kSwInter, int few = 0);
+// *n_dev <= few. Returns the kernels launched, or -1, launching nothing, when a needed scratch
+// pointer is null or base is misaligned.
+int launch_sw(cudaStream_t st, bool tb, bool bytes_ok, const SwTask* tasks, int base, int count, int n,
+              const int* n_dev, const uint8_t* qbase, const uint8_t* tbase, const SwParams& p, SwResult* res,
+              uint32_t* dir, int rows_max, uint32_t* cig, const int64_t* cig_off, int* band, int* fb, uint32_t* err,
+              const KernelTrace* kt, SwForm form = kSwInter, int few = 0);
 
 // ---- tasks without a gap, proved from bit vectors (sw_ungapped.cu) ------------------------
 // True when the scores and the band meet the proof's preconditions.
