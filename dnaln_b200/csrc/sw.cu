@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(kDpThreads, (TB && W <= 33) ? 12 : 1)
   const uint32_t zero = kBias - static_cast<uint32_t>(p.oe);
   uint32_t best2 = h_zero, best_a = zero, best_b = zero;
   int bi_a = -1, bi_b = -1;
-  extern __shared__ uint32_t sw_rows[];
+  extern __shared__ __align__(16) uint32_t sw_rows[];  // k_sw_wide stores 16 bytes at a time
   uint32_t* const row_a = sw_rows + threadIdx.x;
   uint32_t* const row_b = sw_rows + W * kDpThreads + threadIdx.x;
   int buf_a = 0, buf_b = 1;
@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(kDpThreads, TB ? sw_wide_warps(CH) : 1)
   for (int k = 0; k <= CH; ++k) T[k] = skip ? 0u : tc2(d0 + k);  // row 0
   uint32_t best2 = h_zero;
   int bi_a = -1, bi_b = -1;
-  extern __shared__ uint32_t sw_rows[];
+  extern __shared__ __align__(16) uint32_t sw_rows[];  // k_sw_wide stores 16 bytes at a time
   uint4* const row_a = reinterpret_cast<uint4*>(sw_rows) + threadIdx.x;  // cells 4g .. 4g + 3 at [g * kDpThreads]
   uint4* const row_b = row_a + CH / 4 * kDpThreads;
   uint32_t* const last_a = sw_rows + 2 * CH * kDpThreads + threadIdx.x;  // cell CH
