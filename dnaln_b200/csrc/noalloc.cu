@@ -161,10 +161,12 @@ extern "C" int dnaln_gpu_align_noalloc(const uint8_t* d_q, const int64_t* d_q_of
   const size_t dir_t = tb ? sw_dir_bytes_per_task(p.W, rows) : 0;
   const size_t band_t = sw_band_bytes_per_task(p.W, bytes_ok);
   // scratch per group of kSwTaskGroup tasks: descriptors, CIGAR offsets, results,
-  // direction codes, band rows, int32-path task list (one more int for its count)
+  // direction codes, band rows, int32-path task list (whose head lies in the reserve)
   const int64_t G = kSwTaskGroup;
   const size_t per_group = G * (sizeof(SwTask) + sizeof(int64_t) + sizeof(SwResult) + dir_t + band_t + sizeof(int));
-  const size_t avail = kNoAllocScratchBytes - kHeader - 6 * 256;
+  constexpr size_t kReserve = 6 * 256;  // five arrays rounded up to 256 bytes, and the list's head
+  static_assert(5 * 255 + kSwFbHead * sizeof(int) <= kReserve);
+  const size_t avail = kNoAllocScratchBytes - kHeader - kReserve;
   const int64_t groups = static_cast<int64_t>(avail / per_group);
   if (groups < 1) return DNALN_ERR_INVALID_ARG;  // one group of this query length / band does not fit 64 MiB
   const int64_t chunk = std::min<int64_t>(groups * G, ((n + G - 1) / G) * G);
