@@ -621,11 +621,15 @@ bool seed_colinear_supported(const SeedParams& sp, const ChainParamsDev& cp, con
          ix.mask <= 0xFFFFFFFFull;
 }
 
+// As many lanes a read as keep all reads resident at once, each with 32 bases and more. k_sketch_reads,
+// us, with the next smaller number and with this: 20,000 reads of 150 bases (2) 20.8 and 20.7,
+// 4,557 of 100 to 300 (4) 14.5 and 13.7, 800 of 300 to 1,000 (16) 18.9 and 14.6, 4,001 of 1,000 to
+// 5,000 (16) 77.8 and 59.8.
 int seed_colinear_lanes(int64_t n, int64_t max_len) {
   const int64_t want = static_cast<int64_t>(device_sm_count()) * 6 * kCThreads;  // resident lanes
   int g = 1;
   while (g < 32 && n * g * 2 <= want && max_len / (2 * g) >= 32) g *= 2;
-  return g == 2 ? 1 : (g == 16 ? 8 : g);
+  return g;
 }
 
 void launch_sketch_reads(cudaStream_t st, const uint8_t* codes, const int64_t* pofs, const int32_t* seq_len,
@@ -636,8 +640,10 @@ void launch_sketch_reads(cudaStream_t st, const uint8_t* codes, const int64_t* p
     kernel<<<blocks, kCThreads, 0, st>>>(codes, pofs, seq_len, order, n, sp.k, mins, counts);
   };
   switch (lanes) {
+    case 2: return run(k_sketch_reads<kCW, 2>);
     case 4: return run(k_sketch_reads<kCW, 4>);
     case 8: return run(k_sketch_reads<kCW, 8>);
+    case 16: return run(k_sketch_reads<kCW, 16>);
     case 32: return run(k_sketch_reads<kCW, 32>);
     default: return run(k_sketch_reads<kCW, 1>);
   }
@@ -655,8 +661,10 @@ void launch_probe_reads(cudaStream_t st, const int64_t* pofs, const int32_t* seq
                                          mb, list, list_n, long_len, long_done, err);
   };
   switch (lanes) {
+    case 2: return run(k_probe_reads<kCW, 2>);
     case 4: return run(k_probe_reads<kCW, 4>);
     case 8: return run(k_probe_reads<kCW, 8>);
+    case 16: return run(k_probe_reads<kCW, 16>);
     case 32: return run(k_probe_reads<kCW, 32>);
     default: return run(k_probe_reads<kCW, 1>);
   }
