@@ -1,6 +1,6 @@
 // capi.cu — the C ABI (include/dnaln_b200.h): contexts, HBM-resident genome indexes, and
-// the orchestration of each batch through the kernels of seed_thread.cu, seed_long.cu,
-// seed.cu, sw.cu and map.cu.
+// the orchestration of each batch through the kernels of seed_colinear.cu, seed_thread.cu,
+// seed_long.cu, seed.cu, sw_ungapped.cu, sw.cu and map.cu.
 //
 // One batch (Mapper::map, src/mapper.cpp:75-223) is enqueued on the context's stream as:
 //   k_len_scan: packed read offsets, total bases, longest read (read back first only
@@ -12,17 +12,18 @@
 //     chains, candidate loci); reads it cannot take are listed
 //   k_seed_chain_tl: listed long reads one thread each, longest first; what exceeds its
 //     bounds is listed again
-//   k_seed<list> + k_chain_map<list>: the reads still listed, one warp each
-//   (banded SW below: k_sw_ungapped takes the tasks proved to have no gap, the DP the rest)
+//   k_seed<list>, k_chain_map<list>, k_chain_big: the reads still listed, one warp each
+//   (banded SW below: of long lists k_sw_ungapped takes the tasks proved to have no gap, the DP
+//   the rest)
 //   score-only SW over every candidate of reads with >= 2 candidates, then k_choose
 //     (best / ties / second best, fnv1a tie-break, the traceback task of each read)
 //   SW with traceback over each read's chosen candidate (chunked by scratch size), walk
 //   k_records (MAPQ, positions, soft clips), k_cigar_gather
 //   one read-back of the batch's totals, task counts, error flags and counters
 // Task and list counts produced on the device are consumed on the device, so the host
-// waits once per batch. The host-buffer entry points queue parts of a batch to a worker
-// thread that overlaps their copies in and out with the compute (two device slots, two
-// copy streams).
+// waits once per batch. The host-buffer entry points queue a batch, in parts, to be driven through
+// two device slots with two copy streams, so that the copies in and out overlap the compute: by the
+// worker thread, or by the calling thread where it waits for the batch anyway and nothing else runs.
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
@@ -194,7 +195,7 @@ struct dnaln_ctx {
   int seed_block = 0;
   dnaln_seed_tuning seed_tune{};
   // SW kernel form per (band width, traceback, read-length bucket): option "sw_form" 0 =
-  // tuned on the first batch that needs it, 1 = inter-sequence, 2 = intra-sequence
+  // tuned on the first batch that needs it, else 1 + the SwForm
   int sw_mode = 0;
   std::map<int, dnaln_sw_tuning> sw_tune;
   std::set<int> sw_retune;  // keys to be tuned again (retune_sw)
@@ -1326,7 +1327,7 @@ int copy_out(dnaln_ctx* c, int k, PendingPart& pp) {
 }
 
 // Drives queued parts (with own != 0, those of that ticket) through the two slots until none
-// is left.
+// is left: in the worker, or in a thread that waits for that ticket.
 void drive_parts(dnaln_ctx* c, int64_t own) {
   PendingPart pend[2];
   SlotBufs sb[2];

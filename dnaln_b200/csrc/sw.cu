@@ -10,8 +10,9 @@
 // each row start, and the target N-padded to qlen + W - 1.
 //
 // Kernels:
-//  * k_sw_u2<W> (a thread owns whole alignments, no intra-row shuffles): two alignments per thread, one in each 16-bit half of 32-bit
-//    registers, the band row (H, E of W+1 cells, W target selectors) in registers.
+//  * k_sw_u2<W> (a thread owns whole alignments, no intra-row shuffles): two alignments per
+//    thread, one in each 16-bit half of 32-bit registers, the band row (H, E of W+1 cells, W
+//    target selectors) in registers.
 //    Values are kept biased by +16384, so every half stays positive and every add or
 //    subtract of the recurrence is one 32-bit integer add on both halves (no borrow can
 //    cross halves); E and F are DPX add-maxima (viaddmax), the other maxima unsigned 16x2
@@ -33,11 +34,12 @@
 //   kNotDiag: H > hd                           kNotE: H > E
 //   kExtE: E extends E(i-1,d+1) (ee > eo)      kExtF: F extends F(i,d-1) (fe > fo)
 // The codes of four neighbouring cells share 16 bits, cell c's at bits c (kNotDiag), 4 + c
-// (kExtE), 8 + c (kNotE) and 12 + c (kExtF): the order in which cell2 gets them.
+// (kExtE), 8 + c (kNotE) and 12 + c (kExtF): the order in which cell2 gets them. (k_sw_any's: see
+// WordCodes.)
 // On every cell the walk reads, H is the positive value being traced; there it came from the
 // diagonal if h == hd (src/align.cpp:67), else from E if h == e, and otherwise from F — so
-// the walk (src/align.cpp:87-143) takes the reference's steps. The best cell is the first strict maximum in row-major
-// order (per-row maximum with its first column, then strict across rows).
+// the walk (src/align.cpp:87-143) takes the reference's steps. The best cell is the first strict
+// maximum in row-major order (per-row maximum with its first column, then strict across rows).
 #include <algorithm>
 #include <climits>
 #include <type_traits>
@@ -204,7 +206,8 @@ struct CigarWriter {
 };
 
 // Direction codes of the pair layout: word (i, g), g < WQ = ceil(W/4), holds cells 4g..4g+3
-// of both alignments of a thread (A in the low 16 bits, B in the high 16); the 32 pairs of a warp are interleaved word by word.
+// of both alignments of a thread (A in the low 16 bits, B in the high 16); the 32 pairs of a warp
+// are interleaved word by word.
 struct PairCodes {
   static constexpr uint32_t kFromNotE = kNotE, kEExt = kExtE, kFExt = kExtF, kAll = kCode;
   const uint32_t* D;  // this pair's first word

@@ -23,13 +23,13 @@ size_t sw_band_bytes_per_task(int W, bool bytes_ok);
 
 // Kernel forms of the register-resident bands, all with the same results: inter-sequence
 // (k_sw_u2, a thread holds the whole band row of two alignments; W != 129) and intra-
-// sequence (k_sw_wide, the row of a pair spread over lanes in a skewed wavefront: (W - 1) /
-// 32 lanes of 32 cells, or, narrow, (W - 1) / 16 lanes of 16 cells; W = 33, 65, 129). The
-// generic kernel (other widths or scores) has the inter form only.
-constexpr int kSwFbHead = 3;  // ints before the fallback list's entries
+// sequence (k_sw_wide, the row of a pair spread over lanes in a skewed wavefront): 32 cells a
+// lane (W = 33, 65, 129), narrow, 8 (W = 33, 43, 65) or 16 (W = 129), and few, 4 (every register
+// width). The generic kernel (other widths or scores) has the inter form only.
+constexpr int kSwFbHead = 3;  // ints before the fallback list's entries: its length, two claim counters
 enum SwForm : int { kSwInter = 0, kSwIntra = 1, kSwIntraNarrow = 2, kSwIntraFew = 3 };
 constexpr int kSwForms = 3;  // forms the tuner times: kSwIntraFew is chosen by the task count
-// Task count up to which kSwIntraFew ((W - 1) / 4 lanes of 4 cells) runs.
+// Task count up to which kSwIntraFew runs.
 int sw_few_tasks(int W);
 bool sw_has_form(int W, bool bytes_ok, SwForm form);
 int sw_lanes_per_pair(int W, SwForm form);

@@ -50,7 +50,11 @@ namespace dnb {
 namespace {
 
 constexpr int kThreads = 128;
-constexpr int kBlocksPerSm = 12;  // grid-stride: a few resident waves, whatever the capacity of the list
+// Grid-stride: a few resident waves, whatever the capacity of the list. At 6, 12 and 24, us: 262,144
+// tasks of 150 rows 142, 136 and 130, 100,003 of 50 to 1,000 rows at W = 129 381, 330 and 316, an
+// empty list (the scores of a batch without ties) 6.1, 7.0 and 8.1; the first batch's kernels
+// together 985, 955 and 973.
+constexpr int kBlocksPerSm = 12;
 constexpr int kRun = 14;          // longest match run test 2 allows off d0
 constexpr int kNear = 15;         // intervals of fewer rows may hold no aligned block of 8
 

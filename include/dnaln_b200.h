@@ -126,8 +126,9 @@ typedef struct dnaln_kernel_time {
 int dnaln_gpu_set_kernel_trace(dnaln_ctx* ctx, int32_t on, const char* only);
 /* Writes min(cap, count) entries; *n_out = count of traced kernel names. */
 int dnaln_gpu_kernel_times(const dnaln_ctx* ctx, dnaln_kernel_time* out, int32_t cap, int32_t* n_out);
-/* Reads per part of a host-buffer batch (default 0: one part, or two for a large batch that
- * is waited for, so that its own copies overlap; smaller parts cost kernel efficiency). */
+/* Reads per part of a host-buffer batch (default 0: one part, or two for a large batch of short
+ * reads in page-locked memory that is waited for, so that the second half's copy in overlaps;
+ * smaller parts cost kernel efficiency). */
 int dnaln_gpu_set_sub_batch(dnaln_ctx* ctx, int64_t reads);
 /* Tuning switches (none changes any result):
  *   "sub_batch"      same as dnaln_gpu_set_sub_batch;
@@ -175,12 +176,13 @@ int dnaln_gpu_set_option(dnaln_ctx* ctx, const char* name, int64_t value);
  * grouping per task group, src/align_simd.cpp:50-70): band widths with more than one
  * register-resident kernel form — inter-sequence (a thread holds the band rows of two
  * alignments; W = 33, 65 and the other register widths) and intra-sequence (a pair's row
- * spread over lanes in a skewed wavefront: (W - 1) / 32 lanes of 32 cells, or narrow,
- * (W - 1) / 16 lanes of 16 cells; W = 33, 65, 129) — have every form timed on the first
+ * spread over lanes in a skewed wavefront: 32 cells a lane, W = 33, 65, 129, or narrow, 8
+ * cells, W = 33, 43, 65, or 16, W = 129) — have every form timed on the first
  * batch of each (band width, traceback or score-only, read-length bucket <= 256 / <= 1024
  * / longer) a context maps, and the fastest runs from then on (`tasks` says how large the
- * timed sample was; a sample under 4,096 tasks keeps the width's first form, inter-sequence
- * where it has one). All forms give identical results. ms_* = -1 for a form the width
+ * timed sample was; a sample under 4,096 tasks takes the width's first form, inter-sequence
+ * where it has one, until a list has as many: the forms are then timed again). All forms
+ * give identical results. ms_* = -1 for a form the width
  * lacks. Writes min(cap, count) entries; *n_out = count. */
 typedef struct {
   int32_t W, traceback, len_bucket, form; /* form: 0 inter-sequence, 1 intra-sequence, 2 intra narrow */
@@ -193,8 +195,8 @@ typedef struct {
 int dnaln_gpu_sw_tuning(const dnaln_ctx* ctx, dnaln_sw_tuning* out, int32_t cap, int32_t* n_out);
 /* The reads-per-block tuner of the thread-per-read seeding kernel (no reference
  * counterpart): on the first batch of at least 32,768 reads a context maps (option
- * "seed_block" 0, the default), the kernel runs with 64 and with 128 reads per block, each
- * timed, and the faster size is used from then on. Both give identical results. */
+ * "seed_block" 0, the default), the kernel runs over all its reads with 64 and with 128 reads
+ * per block, each timed, and the faster size is used from then on. Both give identical results. */
 typedef struct {
   int32_t tuned;            /* 0 until a batch was timed */
   int32_t reads_per_block;  /* the size chosen */
@@ -318,8 +320,9 @@ int dnaln_gpu_int_peak(int32_t device, int32_t mode, void* stream, double* threa
  * n reads, ASCII, read r = seq[seq_off[r] .. + seq_len[r]); name_hash[r] = FNV-1a of the
  * read name (src/common.hpp:136-140, dnaln_fnv1a below), the tie-break between equal
  * best candidates. Records go to out[r]; CIGARs to `cigar` (capacity cigar_cap ops;
- * the sum over reads of 2*len+3 always suffices; DNALN_ERR_CAPACITY if it is short).
- * Page-locked buffers (dnaln_gpu_host_alloc) make the copies asynchronous. */
+ * the sum over reads of 2*len+3 always suffices; DNALN_ERR_CAPACITY if it is short, with
+ * nothing written unless sub_batch is set). Page-locked buffers (dnaln_gpu_host_alloc) make
+ * the copies asynchronous. The calling thread's current device stays as it is. */
 int dnaln_gpu_map_batch(dnaln_ctx* ctx, int32_t index_id, const char* seq, const int64_t* seq_off,
                         const int32_t* seq_len, const uint32_t* name_hash, int64_t n, const dnaln_map_params* p,
                         dnaln_map_record* out, uint32_t* cigar, int64_t cigar_cap, int64_t* cigar_used);
