@@ -807,12 +807,11 @@ __device__ void seed_read(int64_t r, bool encode, const char* __restrict__ seq, 
   }
 }
 
-// One warp per read: reads [0, n), or with a list the reads list[0, *list_n) (grid-stride), of which
-// `marked` takes those with n_anchor < 0 only.
+// One warp per read: reads [0, n), or with a list the reads list[0, *list_n) (grid-stride).
 __global__ void __launch_bounds__(kSeedWarps * 32)
     k_seed(const char* __restrict__ seq, const int64_t* __restrict__ seq_off, int64_t seq_base,
            const int32_t* __restrict__ seq_len, const int64_t* __restrict__ pofs, int64_t n,
-           const int32_t* __restrict__ list, const int* __restrict__ list_n, bool marked, uint8_t* __restrict__ codes,
+           const int32_t* __restrict__ list, const int* __restrict__ list_n, uint8_t* __restrict__ codes,
            DevIndex ix, SeedParams sp, MinBuf mb, int32_t* __restrict__ n_min, int64_t* __restrict__ n_anchor,
            uint32_t* __restrict__ err) {
   __shared__ SketchSmem sm[kSeedWarps];
@@ -824,7 +823,25 @@ __global__ void __launch_bounds__(kSeedWarps * 32)
   }
   const int m = *list_n;
   for (int64_t x = gw; x < m; x += static_cast<int64_t>(gridDim.x) * kSeedWarps)
-    if (!marked || n_anchor[list[x]] < 0) seed_read(list[x], false, seq, seq_off, seq_base, seq_len, pofs, codes, ix, sp, mb, n_min, n_anchor, err, sm[wib]);
+    seed_read(list[x], false, seq, seq_off, seq_base, seq_len, pofs, codes, ix, sp, mb, n_min, n_anchor, err, sm[wib]);
+}
+
+// The reads of a list whose n_anchor is below 0. (As a test in k_seed it cost that kernel a block
+// per SM, 64 -> 77 registers: 262,144 reads of 50 to 1,000 bases 1,983 -> 2,370 us.)
+__global__ void __launch_bounds__(kSeedWarps * 32)
+    k_seed_marked(const char* __restrict__ seq, const int64_t* __restrict__ seq_off, int64_t seq_base,
+                  const int32_t* __restrict__ seq_len, const int64_t* __restrict__ pofs,
+                  const int32_t* __restrict__ list, const int* __restrict__ list_n, uint8_t* __restrict__ codes,
+                  DevIndex ix, SeedParams sp, MinBuf mb, int32_t* __restrict__ n_min, int64_t* __restrict__ n_anchor,
+                  uint32_t* __restrict__ err) {
+  __shared__ SketchSmem sm[kSeedWarps];
+  const int wib = threadIdx.x >> 5, m = *list_n;
+  for (int64_t x = static_cast<int64_t>(blockIdx.x) * kSeedWarps + wib; x < m;
+       x += static_cast<int64_t>(gridDim.x) * kSeedWarps) {
+    const int32_t r = list[x];
+    if (n_anchor[r] < 0)
+      seed_read(r, false, seq, seq_off, seq_base, seq_len, pofs, codes, ix, sp, mb, n_min, n_anchor, err, sm[wib]);
+  }
 }
 
 // Pass 2 of read r by one warp.
@@ -1101,7 +1118,7 @@ void launch_seed(cudaStream_t st, const char* seq, const int64_t* seq_off, int64
   if (n <= 0) return;
   const int64_t blocks = (n + kSeedWarps - 1) / kSeedWarps;
   k_seed<<<static_cast<unsigned>(blocks), kSeedWarps * 32, 0, st>>>(seq, seq_off, seq_base, seq_len, pofs, n, nullptr,
-                                                                   nullptr, false, codes, ix, sp, mb, n_min, n_anchor, err);
+                                                                   nullptr, codes, ix, sp, mb, n_min, n_anchor, err);
 }
 
 void launch_seed_list(cudaStream_t st, const char* seq, const int64_t* seq_off, int64_t seq_base,
@@ -1111,8 +1128,13 @@ void launch_seed_list(cudaStream_t st, const char* seq, const int64_t* seq_off, 
   if (n_max <= 0) return;
   // grid-stride over a list whose length is only known on the device: a few resident waves
   const int64_t blocks = std::min<int64_t>((n_max + kSeedWarps - 1) / kSeedWarps, int64_t{8} * device_sm_count());
+  if (marked) {
+    k_seed_marked<<<static_cast<unsigned>(blocks), kSeedWarps * 32, 0, st>>>(
+        seq, seq_off, seq_base, seq_len, pofs, list, list_n, codes, ix, sp, mb, n_min, n_anchor, err);
+    return;
+  }
   k_seed<<<static_cast<unsigned>(blocks), kSeedWarps * 32, 0, st>>>(seq, seq_off, seq_base, seq_len, pofs, n_max,
-                                                                   list, list_n, marked, codes, ix, sp, mb, n_min, n_anchor,
+                                                                   list, list_n, codes, ix, sp, mb, n_min, n_anchor,
                                                                    err);
 }
 
