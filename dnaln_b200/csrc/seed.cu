@@ -21,9 +21,9 @@
 // 64-bit key (strand, rpos, qpos) so the reference's sort is a warp bitonic sort of
 // integers. The DP scans predecessors nearest-first with a `break` on strand change or
 // dr > max_gap; because anchors are sorted by (strand, rpos), the scanned predecessors
-// form one contiguous range. The lanes hold the rows of a tile of 32 anchors, or one cluster
-// each; ties go to the nearest j, as the reference's strict '>' does. The FP64 gap cost comes from a
-// host-computed table (exactly the reference's expression). Chains are extracted from end
+// form one contiguous range. The lanes hold one row's nearest predecessors, the rows of a tile of
+// 32 anchors, or one cluster each; ties go to the nearest j, as the reference's strict '>' does. The
+// FP64 gap cost comes from a host-computed table (exactly the reference's expression). Chains are extracted from end
 // points in (f desc, index asc) order (extract_par; above 1,024 anchors a sort and a walk by
 // one lane) and ordered by score with ties in extraction order (the reference's
 // stable_sort). Candidate loci follow src/mapper.cpp:40-62.
@@ -332,6 +332,74 @@ __device__ void chain_dp_tiles(const ChainArrays& a, int n, const ChainParamsDev
   }
 }
 
+// The chaining DP (src/chain.cpp:22-45) row by row, for lookbacks up to 64. For row i, lane t holds
+// in registers the key and f of anchor i-1-t (the 32 nearest predecessors); after the row the
+// window moves up one lane and row i enters at lane 0, so f never makes a round trip through
+// memory on the DP's serial path. Predecessors at distance 33..lookback are read from a.keys /
+// a.f only when the one at distance 32 has not stopped the scan: anchors are sorted by
+// (strand, rpos), so a strand change or dr > max_gap at j holds for every farther j too (and
+// each lane can test its own j). One redux per row takes the max of score * 64 + (63 -
+// distance): the largest score, ties to the nearest predecessor (the reference scans j
+// downward with a strict '>').
+__device__ __forceinline__ void chain_dp_rows(const ChainArrays& a, int n, const ChainParamsDev& cp) {
+  const int lane = threadIdx.x & 31;
+  const unsigned FULL = 0xffffffffu;
+  int rw = 0, qw = 0, fw = 0;
+  uint32_t sw = 0;
+  const bool two = cp.lookback > 32;
+  uint64_t ki = n > 0 ? a.keys[0] : 0;
+  for (int i = 0; i < n; ++i) {
+    const uint64_t knext = i + 1 < n ? a.keys[i + 1] : 0;
+    const uint32_t si = key_strand(ki);
+    const int ri = static_cast<int>(key_rpos(ki)), qi = key_qpos(ki);
+    // rpos < 2^31 and |qpos| < 2^30, so dr and dq fit 32 bits; dd is formed in unsigned
+    // arithmetic and used only when dr and dq passed the range tests
+    const auto score_of = [&](int rj, int qj, uint32_t sj, int fj, int t) -> int {
+      const int dr = ri - rj, dq = qi - qj;
+      const int dd = static_cast<int>(dr > dq ? static_cast<uint32_t>(dr) - static_cast<uint32_t>(dq)
+                                              : static_cast<uint32_t>(dq) - static_cast<uint32_t>(dr));
+      if (t >= cp.lookback || t >= i || sj != si || dr > cp.max_gap || dr <= 0 || dq <= 0 || dd > cp.band)
+        return INT_MIN;
+      const int g = min(min(dq, dr), cp.k);
+      return (fj + g - cp.cost[dd]) * 64 + (63 - t);
+    };
+    int c = score_of(rw, qw, sw, fw, lane);
+    if (two && i > 32) {
+      const bool live = sw == si && ri - rw <= cp.max_gap;  // lane 31: the predecessor i-32
+      if (__shfl_sync(FULL, live, 31)) {
+        __syncwarp();  // f of rows <= i-33, written by lane 0, is visible to every lane
+        const int j = i - 33 - lane;
+        if (j >= 0) {
+          const uint64_t kj = a.keys[j];
+          c = max(c, score_of(static_cast<int>(key_rpos(kj)), key_qpos(kj), key_strand(kj), a.f[j], 32 + lane));
+        }
+      }
+    }
+    const int m = __reduce_max_sync(FULL, c);
+    int fi = cp.k, pi = -1;
+    if (m != INT_MIN && (m >> 6) > cp.k) {
+      fi = m >> 6;
+      pi = i - 1 - (63 - (m & 63));
+    }
+    if (lane == 0) {
+      a.f[i] = fi;
+      a.prev[i] = pi;
+    }
+    // move the window up one lane; row i enters at lane 0
+    rw = __shfl_up_sync(FULL, rw, 1);
+    qw = __shfl_up_sync(FULL, qw, 1);
+    fw = __shfl_up_sync(FULL, fw, 1);
+    sw = __shfl_up_sync(FULL, sw, 1);
+    if (lane == 0) {
+      rw = ri;
+      qw = qi;
+      fw = fi;
+      sw = si;
+    }
+    ki = knext;
+  }
+}
+
 // The chaining DP of an anchor set that falls into many clusters (maximal runs of one strand
 // with no step over max_gap: a read's loci in a repeat), a lane per cluster. No anchor
 // outside its cluster is ever a valid predecessor, so the clusters are independent, and each
@@ -350,6 +418,11 @@ constexpr int kMinClusters = 12, kMaxCluster = 48;
 __device__ bool chain_dp_clusters(const ChainArrays& a, int n, const ChainParamsDev& cp) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
+  // one locus, as most reads: too short for so many clusters
+  if (n < kMinClusters) return false;
+  if (key_strand(a.keys[0]) == key_strand(a.keys[n - 1]) &&
+      static_cast<int64_t>(key_rpos(a.keys[n - 1])) - key_rpos(a.keys[0]) <= int64_t{kMinClusters - 1} * cp.max_gap)
+    return false;
   uint32_t* const head = reinterpret_cast<uint32_t*>(a.ord);  // cluster starts, then max(f[0..i]) at n + i
   int nc = 0;
   for (int base = 0; base < n; base += 32) {
@@ -614,7 +687,14 @@ __device__ int chain_core(ChainArrays a, int n, const ChainParamsDev& cp, const 
   warp_sort_u64(a.keys, n);
   // the clusters' cutoff holds while no pair gains more than k, that is while no gap cost is below
   // zero: int(0.01 k dd + ...) is for k < 0, which the chaining entry point takes
-  if (cp.k < 0 || cp.max_gap >= (1 << 29) || !chain_dp_clusters(a, n, cp)) chain_dp_tiles(a, n, cp);
+  if (cp.k < 0 || cp.max_gap >= (1 << 29) || !chain_dp_clusters(a, n, cp)) {
+    // Up to 256 anchors row by row (a row's packed score holds while k does not exceed 1,024): 262,144
+    // reads of 50 to 1,000 bases, all of them chained here, k_chain_map 3,104 us, in tiles 3,732.
+    // More in tiles: 4,001 reads of 1,000 to 5,000 bases, 8 of them of 600 to 770 anchors, 472 us row
+    // by row, 320 in tiles.
+    if (CAP == kSmCap && n <= kSmCap && cp.lookback <= 64 && cp.k >= 0 && cp.k <= 1024) chain_dp_rows(a, n, cp);
+    else chain_dp_tiles(a, n, cp);
+  }
   __syncwarp();
   if (n <= 32) return extract_par<1>(a, n, cp, as, c0);
   if (n <= 64) return extract_par<2>(a, n, cp, as, c0);

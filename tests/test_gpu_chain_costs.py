@@ -40,3 +40,25 @@ def test_cluster_counts_and_sizes_at_the_rules_edges(ctx, port):
         assert np.array_equal(sr, er) and np.array_equal(sq, eq) and np.array_equal(ss, es), i
         for key in ech:
             assert np.array_equal(ch[key], ech[key]), (i, key)
+
+
+@pytest.mark.parametrize("k,lookback", [(15, 50), (15, 64), (15, 65), (15, 31), (15, 0), (1024, 50), (1025, 50),
+                                        (1_000_000, 50)])
+def test_sets_around_256_anchors_match_port(ctx, port, k, lookback):
+    """Sets of 0, 1 and about 32, 64 and 256 anchors in one cluster and in some: those chained row by
+    row and those in tiles, with packed scores of every size."""
+    rng = np.random.default_rng(k + lookback)
+    cp = (5000, 16, lookback, 20, 1)
+    sets = [tuple(np.zeros(0, t) for t in (np.uint32, np.int32, np.uint32))]
+    for n in (1, 2, 11, 12, 13, 31, 32, 33, 34, 63, 64, 65, 97, 128, 255, 256, 257, 300):
+        for spread in (2, 30, 200):
+            sets.append(clustered_set(rng, [n], cp[0], spread))
+            if n > 20:
+                sets.append(clustered_set(rng, [n - 12] + [1] * 12, cp[0], spread))
+    sets.append(sets[0])
+    got = ctx.chain(sets, k, D.ChainParams(*cp))
+    for i, ((sr, sq, ss), ch) in enumerate(got):
+        (er, eq, es), ech = port.chain(*sets[i], k, cp)
+        assert np.array_equal(sr, er) and np.array_equal(sq, eq) and np.array_equal(ss, es), i
+        for key in ech:
+            assert np.array_equal(ch[key], ech[key]), (i, key)
