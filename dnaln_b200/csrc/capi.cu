@@ -814,7 +814,7 @@ int map_enqueue(dnaln_ctx* c, IndexRes& ix, const char* d_seq, const int64_t* d_
     }
     // after the colinear kernels only the reads left unsketched for an N. (Before the thread kernels,
     // for all such reads, this sketched 95,000 reads a second time that those kernels then did a
-    // third time: 100,000 reads with 2 % N 1,606 us, so 1,325.)
+    // third time: 100,000 reads with 2 % N 1,606 us, here 1,325.)
     kt.begin(st, "k_seed<list>");
     launch_seed_list(st, d_seq, d_seq_off, hint.seq_base, d_seq_len, pofs, n, warp_list, warp_n, full_list != nullptr,
                      codes, ix.dev, sp, mb, n_min, n_anchor, c->d_err);

@@ -116,7 +116,7 @@ __device__ __forceinline__ uint32_t pack2(uint32_t v) { return (v & 0xFFFFu) * 0
 // A cell's code, its flags STEP bits apart. diag: hd >= E and max(hd, E) >= F; from_e: the latter,
 // which is H = E on every cell the walk asks it for (H > 0 and not from the diagonal). Neither
 // waits for H: compared with H itself, k_sw_fb<43> spilled and took 181 us for 64 tasks of 150
-// rows, so 154.
+// rows, like this 154.
 template <int STEP = 4>
 __device__ __forceinline__ uint32_t dir_code32(bool diag, bool from_e, bool e_not_ext, bool f_not_ext) {
   return (diag ? 0u : 1u) | (e_not_ext ? 0u : 1u << STEP) | (from_e ? 0u : 1u << 2 * STEP) |
@@ -220,7 +220,7 @@ struct PairCodes {
 // Direction codes of the generic kernel: word (i, w), w < WW = ceil(W/8), holds cells
 // 8w..8w+7, the flags of cell 8w + c at bits c, 8 + c, 16 + c and 24 + c; 32 alignments of a warp
 // interleaved word by word. One shift places a cell's flags: two groups of four cells side by side
-// took 2,923 us for 64 tasks of 150 rows at W = 201, so 2,810.
+// took 2,923 us for 64 tasks of 150 rows at W = 201, this 2,810.
 struct WordCodes {
   static constexpr int kStep = 8;
   static constexpr uint32_t kEExt = 1u << kStep, kFromNotE = 1u << 2 * kStep, kFExt = 1u << 3 * kStep,

@@ -18,7 +18,10 @@ def launched(ctx, call):
     with profile(activities=[ProfilerActivity.CUDA]) as p:
         call()
         torch.cuda.synchronize()
-    return ctx.stats()["launches"], sum("dnb::" in e.name for e in p.events())
+    names = [e.name for e in p.events()]
+    if not names:
+        pytest.skip("no kernel trace here (another profiler may hold it)")
+    return ctx.stats()["launches"], sum("dnb::" in n for n in names)
 
 
 @pytest.fixture(scope="module")
